@@ -21,7 +21,7 @@
 //
 // Choices at or beyond the number of experts are identity experts: they take no row in the grouping (slot_row -1) and
 // the sum takes the token's own input for them.
-#include "common.cuh"
+#include "tc_common.cuh"
 
 #define ROUTE_WARPS 8
 // One warp's dot product of a weight row with the token's inputs (float32 in shared memory), summed over the warp.
@@ -80,93 +80,125 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_logits_kernel(float* __r
   if (lane == 0) logits[(size_t)t * (E + 1) + e] = acc;
 }
 
-// The same dot products for ROUTE_TOKENS tokens at once: a weight row is read once for all of them, and every token's sum has
-// the order route_dot gives it (a lane's elements ascending, then the warp's tree), so the logits do not depend on which kernel
-// formed them.  xs: [ROUTE_TOKENS][d] float32 in shared memory.
+// The same dot products for ROUTE_TOKENS tokens and ROUTE_ROWS rows of the router at once: a weight is converted once for all tokens, an
+// input once for all rows, and every (token, row) sum has the order route_dot gives it (a lane's elements ascending, then the warp's
+// tree), so the logits do not depend on which kernel formed them.  xs: [ROUTE_TOKENS][d] in shared memory, as stored.
 #define ROUTE_TOKENS 8
-template <typename TW>
-__device__ __forceinline__ void route_dot_tokens(const TW* __restrict__ w, const float* __restrict__ xs, int d, int lane, float (&acc)[ROUTE_TOKENS]) {
+#define ROUTE_ROWS 4
+template <typename T, int N>
+__device__ __forceinline__ void load_floats(const T* p, float (&f)[N]) {       // N elements, 16-byte pieces
+  constexpr int PER = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int i = 0; i < N / PER; ++i) {
+    const uint4 v = *(const uint4*)(p + i * PER);
+    const T* e = (const T*)&v;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) f[i * PER + k] = to_f(e[k]);
+  }
+}
+template <typename T, typename TW>
+__device__ __forceinline__ void route_dot_tile(const TW* const (&w)[ROUTE_ROWS], const T* __restrict__ xs, int d, int lane,
+                                               float (&acc)[ROUTE_ROWS][ROUTE_TOKENS]) {
   constexpr int VEC = 16 / (int)sizeof(TW);
 #pragma unroll
-  for (int t = 0; t < ROUTE_TOKENS; ++t) acc[t] = 0.f;
-  int i = 0;
-  if ((d % VEC) == 0 && (((uintptr_t)w) & 15) == 0) {
-    for (i = lane * VEC; i + 7 * 32 * VEC < d; i += 8 * 32 * VEC) {
-      uint4 wv[8];
+  for (int r = 0; r < ROUTE_ROWS; ++r)
 #pragma unroll
-      for (int u = 0; u < 8; ++u) wv[u] = *(const uint4*)(w + i + u * 32 * VEC);
+    for (int t = 0; t < ROUTE_TOKENS; ++t) acc[r][t] = 0.f;
+  bool vec = (d % VEC) == 0 && (d % (16 / (int)sizeof(T))) == 0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const TW* p = (const TW*)&wv[u];
-        float wf[VEC];
+  for (int r = 0; r < ROUTE_ROWS; ++r) vec = vec && (((uintptr_t)w[r]) & 15) == 0;
+  if (vec) {
+    // (VEC is 8 or 4 elements and a lane's pieces lie 32 * VEC apart, as in route_dot)
+#pragma unroll 2
+    for (int i = lane * VEC; i < d; i += 32 * VEC) {
+      float wf[ROUTE_ROWS][VEC];
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) wf[k] = to_f(p[k]);
+      for (int r = 0; r < ROUTE_ROWS; ++r) load_floats<TW, VEC>(w[r] + i, wf[r]);
 #pragma unroll
-        for (int t = 0; t < ROUTE_TOKENS; ++t) {
-          const float4* x4 = (const float4*)(xs + (size_t)t * d + i + u * 32 * VEC);
+      for (int t = 0; t < ROUTE_TOKENS; ++t) {
+        float xf[VEC];
+        if (VEC * sizeof(T) >= 16) load_floats<T, VEC>(xs + (size_t)t * d + i, xf);
+        else {
 #pragma unroll
-          for (int k4 = 0; k4 < VEC / 4; ++k4) {
-            const float4 xv = x4[k4];
-            acc[t] = fmaf(wf[4 * k4], xv.x, acc[t]); acc[t] = fmaf(wf[4 * k4 + 1], xv.y, acc[t]);
-            acc[t] = fmaf(wf[4 * k4 + 2], xv.z, acc[t]); acc[t] = fmaf(wf[4 * k4 + 3], xv.w, acc[t]);
-          }
+          for (int k = 0; k < VEC; ++k) xf[k] = to_f(xs[(size_t)t * d + i + k]);
         }
+#pragma unroll
+        for (int r = 0; r < ROUTE_ROWS; ++r)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) acc[r][t] = fmaf(wf[r][k], xf[k], acc[r][t]);
       }
     }
-    for (; i < d; i += 32 * VEC) {
-      const uint4 wv = *(const uint4*)(w + i);
-      const TW* p = (const TW*)&wv;
+  } else if ((d % VEC) == 0) {
+    // rows that route_dot would read in pieces but this kernel cannot: the same order, element by element
 #pragma unroll
-      for (int k = 0; k < VEC; ++k) {
-        const float wf = to_f(p[k]);
+    for (int r = 0; r < ROUTE_ROWS; ++r) {
+      const bool piece = (((uintptr_t)w[r]) & 15) == 0;
+      for (int i = piece ? lane * VEC : lane; i < d; i += piece ? 32 * VEC : 32)
+        for (int k = 0; k < (piece ? VEC : 1); ++k) {
+          const float wv = to_f(w[r][i + k]);
 #pragma unroll
-        for (int t = 0; t < ROUTE_TOKENS; ++t) acc[t] = fmaf(wf, xs[(size_t)t * d + i + k], acc[t]);
-      }
+          for (int t = 0; t < ROUTE_TOKENS; ++t) acc[r][t] = fmaf(wv, to_f(xs[(size_t)t * d + i + k]), acc[r][t]);
+        }
     }
   } else {
-    for (i = lane; i + 7 * 32 < d; i += 8 * 32) {
-      float wv[8];
+    for (int i = lane; i < d; i += 32) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) wv[u] = to_f(w[i + u * 32]);
+      for (int r = 0; r < ROUTE_ROWS; ++r) {
+        const float wv = to_f(w[r][i]);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-#pragma unroll
-        for (int t = 0; t < ROUTE_TOKENS; ++t) acc[t] = fmaf(wv[u], xs[(size_t)t * d + i + u * 32], acc[t]);
+        for (int t = 0; t < ROUTE_TOKENS; ++t) acc[r][t] = fmaf(wv, to_f(xs[(size_t)t * d + i]), acc[r][t]);
       }
-    }
-    for (; i < d; i += 32) {
-      const float wf = to_f(w[i]);
-#pragma unroll
-      for (int t = 0; t < ROUTE_TOKENS; ++t) acc[t] = fmaf(wf, xs[(size_t)t * d + i], acc[t]);
     }
   }
 #pragma unroll
-  for (int t = 0; t < ROUTE_TOKENS; ++t) acc[t] = warp_sum(acc[t]);
+  for (int r = 0; r < ROUTE_ROWS; ++r)
+#pragma unroll
+    for (int t = 0; t < ROUTE_TOKENS; ++t) acc[r][t] = warp_sum(acc[r][t]);
 }
 
-// Many tokens: a CTA takes ROUTE_TOKENS tokens and eight rows, so the router's matrix is read once per group of tokens
-// instead of once per token.  d a multiple of 4 (16-byte reads of the tokens' rows in shared memory).
+// Many tokens: a CTA takes ROUTE_TOKENS tokens and walks over all rows, four rows a warp at a time.  What bounds it is the
+// multiply-adds with the conversions around them: a row alone (eight tokens in float32 in shared memory, so 16 bytes read there for
+// four multiply-adds) took 170 us for 2,048 tokens x 65 rows x 2,048.
 template <typename T, typename TW>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_logits_tokens_kernel(float* __restrict__ logits, const T* __restrict__ h, int ld_h,
                                                                              const TW* __restrict__ wr, const TW* __restrict__ wg, int d,
                                                                              int E, int T_all) {
-  extern __shared__ __align__(16) float xs_tokens[];
+  extern __shared__ __align__(16) unsigned char xs_raw[];
+  T* xs = (T*)xs_raw;
   pdl_wait();
   pdl_launch_dependents();
   const int t0 = blockIdx.x * ROUTE_TOKENS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < ROUTE_TOKENS * d; i += blockDim.x) {
-    const int t = i / d, c = i - t * d;
-    xs_tokens[i] = t0 + t < T_all ? to_f(h[(size_t)(t0 + t) * ld_h + c]) : 0.f;
+  constexpr int PER = 16 / (int)sizeof(T);
+  if (d % PER == 0 && ld_h % PER == 0 && (((uintptr_t)h) & 15) == 0) {
+    const int pieces = d / PER;
+    for (int i = threadIdx.x; i < ROUTE_TOKENS * pieces; i += blockDim.x) {
+      const int t = i / pieces, c = (i - t * pieces) * PER;
+      *(uint4*)(xs + (size_t)t * d + c) = t0 + t < T_all ? *(const uint4*)(h + (size_t)(t0 + t) * ld_h + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  } else {
+    for (int i = threadIdx.x; i < ROUTE_TOKENS * d; i += blockDim.x) {
+      const int t = i / d, c = i - t * d;
+      xs[i] = t0 + t < T_all ? h[(size_t)(t0 + t) * ld_h + c] : from_f<T>(0.f);
+    }
   }
   __syncthreads();
-  const int e = blockIdx.y * ROUTE_WARPS + warp;
-  if (e >= E + (wg ? 1 : 0)) return;
-  float acc[ROUTE_TOKENS];
-  route_dot_tokens(e < E ? wr + (size_t)e * d : wg, xs_tokens, d, lane, acc);
-  if (lane == 0) {
+  const int rows = E + (wg ? 1 : 0);
+  for (int e0 = warp * ROUTE_ROWS; e0 < rows; e0 += ROUTE_WARPS * ROUTE_ROWS) {
+    const TW* w[ROUTE_ROWS];
 #pragma unroll
-    for (int t = 0; t < ROUTE_TOKENS; ++t)
-      if (t0 + t < T_all) logits[(size_t)(t0 + t) * (E + 1) + e] = acc[t];
+    for (int r = 0; r < ROUTE_ROWS; ++r) {
+      const int e = e0 + r < rows ? e0 + r : rows - 1;
+      w[r] = e < E ? wr + (size_t)e * d : wg;
+    }
+    float acc[ROUTE_ROWS][ROUTE_TOKENS];
+    route_dot_tile<T, TW>(w, xs, d, lane, acc);
+    if (lane == 0) {
+#pragma unroll
+      for (int r = 0; r < ROUTE_ROWS; ++r)
+#pragma unroll
+        for (int t = 0; t < ROUTE_TOKENS; ++t)
+          if (e0 + r < rows && t0 + t < T_all) logits[(size_t)(t0 + t) * (E + 1) + e0 + r] = acc[r][t];
+    }
   }
 }
 
@@ -283,7 +315,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(int* __rest
 }
 
 // logits_ws: room for T * (E + 1) floats, or null.  With it, the logits are formed in a launch of their own: for steps of up to
-// 256 tokens over (tokens x groups of eight rows) CTAs, for longer ones over (groups of eight tokens x groups of eight rows); the
+// 256 tokens over (tokens x groups of eight rows) CTAs, for longer ones a CTA per eight tokens; the
 // result is the same whichever kernel forms them (same sums, same order).
 extern "C" int qv_moe_route(int* top_idx, float* top_w, float* gate_out, const void* h, int ld_h, const void* wr, const void* wg,
                             float* logits_ws, int T, int d, int E, int top, int dt, int w_dt, const float* correction, float w_scale,
@@ -296,10 +328,10 @@ extern "C" int qv_moe_route(int* top_idx, float* top_w, float* gate_out, const v
   if (smem > 48 * 1024) return QV_ERR_TOO_LARGE;
   const bool split = logits_ws && T <= 256;
   // more tokens: the logits by groups of tokens, where the group's rows fit shared memory
-  const size_t tsmem = (size_t)ROUTE_TOKENS * d * sizeof(float);
-  const bool tokens = logits_ws && !split && d % 4 == 0 && tsmem <= 160 * 1024;
+  const size_t tsmem = (size_t)ROUTE_TOKENS * d * (dt == QV_DT_BF16 ? 2 : 4);
+  const bool tokens = logits_ws && !split && d % 4 == 0 && (size_t)ROUTE_TOKENS * d * sizeof(float) <= 160 * 1024;
   const dim3 lgrid(T, (E + (wg ? 1 : 0) + ROUTE_WARPS - 1) / ROUTE_WARPS);
-  const dim3 tgrid((T + ROUTE_TOKENS - 1) / ROUTE_TOKENS, (E + (wg ? 1 : 0) + ROUTE_WARPS - 1) / ROUTE_WARPS);
+  const dim3 tgrid((T + ROUTE_TOKENS - 1) / ROUTE_TOKENS);
 #define ROUTE(TT, TW)                                                                                                        \
   do {                                                                                                                       \
     if (split) {                                                                                                             \
@@ -350,35 +382,77 @@ extern "C" int qv_moe_route_table(int* top_idx, float* top_w, const int* table, 
   return qv_launch(moe_route_table_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, top_idx, top_w, table, ids, n, top, vocab, E);
 }
 
-// One block.  tiles: [max_tiles][3] = (expert or -1, first sorted row, rows).
+// One block.  tiles: [max_tiles][3] = (expert or -1, first sorted row, rows).  Its time is that of a few trips to memory and through
+// shared memory: the first GROUP_KEEP choices of a thread and their ranks stay in registers, experts' offsets and tiles come from a scan
+// by all threads (25 us for 12,288 choices when one thread walked over the experts and wrote the tiles).
+#define GROUP_KEEP 12
 __global__ void __launch_bounds__(1024) moe_group_kernel(int* __restrict__ row_token, int* __restrict__ slot_row, int* __restrict__ tiles,
                                                          int max_tiles, const int* __restrict__ top_idx, int* __restrict__ rank_tmp,
                                                          int R, int top, int E, int bm) {
   extern __shared__ int cnt[];               // E counts, then E offsets
+  __shared__ int part_rows[32], part_tiles[32], total_tiles;
   pdl_wait();
   pdl_launch_dependents();
   int* off = cnt + E;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < E; e += 1024) cnt[e] = 0;
   __syncthreads();
-  for (int r = threadIdx.x; r < R; r += blockDim.x)
+  int mine[GROUP_KEEP], rank[GROUP_KEEP];
+#pragma unroll
+  for (int i = 0; i < GROUP_KEEP; ++i) {
+    const int r = threadIdx.x + i * 1024;
+    mine[i] = r < R ? top_idx[r] : E;
+  }
+#pragma unroll
+  for (int i = 0; i < GROUP_KEEP; ++i) rank[i] = mine[i] < E ? atomicAdd(&cnt[mine[i]], 1) : 0;
+  for (int r = threadIdx.x + GROUP_KEEP * 1024; r < R; r += 1024)
     if (top_idx[r] < E) rank_tmp[r] = atomicAdd(&cnt[top_idx[r]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, n = 0;
-    for (int e = 0; e < E; ++e) {
-      off[e] = o;
-      for (int r0 = 0; r0 < cnt[e] && n < max_tiles; r0 += bm, ++n) {
-        tiles[3 * n] = e;
-        tiles[3 * n + 1] = o + r0;
-        tiles[3 * n + 2] = cnt[e] - r0 < bm ? cnt[e] - r0 : bm;
-      }
-      o += cnt[e];
+  int row_base = 0, tile_base = 0;           // of the experts ahead of this round of 1024
+  for (int e0 = 0; e0 < E; e0 += 1024) {
+    const int e = e0 + threadIdx.x;
+    const int n = e < E ? cnt[e] : 0, nt = (n + bm - 1) / bm;
+    int rows = n, nts = nt;                  // inclusive sums over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, rows, o), b = __shfl_up_sync(0xffffffffu, nts, o);
+      if (lane >= o) { rows += a; nts += b; }
     }
-    for (; n < max_tiles; ++n) { tiles[3 * n] = -1; tiles[3 * n + 1] = 0; tiles[3 * n + 2] = 0; }
+    if (lane == 31) { part_rows[warp] = rows; part_tiles[warp] = nts; }
+    __syncthreads();
+    int rows_before = row_base, tiles_before = tile_base, rows_all = 0, tiles_all = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) { rows_before += part_rows[w]; tiles_before += part_tiles[w]; }
+      rows_all += part_rows[w];
+      tiles_all += part_tiles[w];
+    }
+    if (e < E) {
+      const int first = rows_before + rows - n;
+      off[e] = first;
+      int at = tiles_before + nts - nt;
+      for (int r0 = 0; r0 < n && at < max_tiles; r0 += bm, ++at) {
+        tiles[3 * at] = e;
+        tiles[3 * at + 1] = first + r0;
+        tiles[3 * at + 2] = n - r0 < bm ? n - r0 : bm;
+      }
+    }
+    row_base += rows_all;
+    tile_base += tiles_all;
+    if (threadIdx.x == 0) total_tiles = tile_base;
+    __syncthreads();
   }
-  __syncthreads();
-  for (int r = threadIdx.x; r < R; r += blockDim.x) {
-    if (top_idx[r] >= E) { slot_row[r] = -1; continue; }       // an identity expert
+  for (int n = total_tiles + threadIdx.x; n < max_tiles; n += 1024) { tiles[3 * n] = -1; tiles[3 * n + 1] = 0; tiles[3 * n + 2] = 0; }
+#pragma unroll
+  for (int i = 0; i < GROUP_KEEP; ++i) {
+    const int r = threadIdx.x + i * 1024;
+    if (r >= R) break;
+    if (mine[i] >= E) { slot_row[r] = -1; continue; }          // an identity expert
+    const int pos = off[mine[i]] + rank[i];
+    slot_row[r] = pos;
+    row_token[pos] = r / top;
+  }
+  for (int r = threadIdx.x + GROUP_KEEP * 1024; r < R; r += 1024) {
+    if (top_idx[r] >= E) { slot_row[r] = -1; continue; }
     const int pos = off[top_idx[r]] + rank_tmp[r];
     slot_row[r] = pos;
     row_token[pos] = r / top;
@@ -389,9 +463,17 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(int* __restrict__ row_t
 #define MOE_BN 64
 #define MOE_BK 16
 
-#define MOE_TC_BM 64       // rows of a tile of the tensor-core kernel
-
-extern "C" int qv_moe_tile_rows(int tensor_cores) { return tensor_cores ? MOE_TC_BM : MOE_BM; }
+// Rows of a tile of grouped rows.  Tensor cores: a tile is the narrow operand of one accumulator and every tile of an expert reads the
+// expert's matrices once, so a tile should hold all rows of a usual expert; the shared memory that its room takes is taken from the
+// stages in flight.  R rows over E experts (0: not known): 32 for steps of up to 32 tokens (there the tokens themselves are the operand),
+// else the first of 64, 128, 256 that holds 4/3 of the mean (counts scatter around it).
+extern "C" int qv_moe_tile_rows(int tensor_cores, int tokens, int R, int E) {
+  if (!tensor_cores) return MOE_BM;
+  if (tokens <= 0 || E <= 0) return 64;
+  if (tokens <= 32) return 32;
+  const long long want = (4LL * R + 3LL * E - 1) / (3LL * E);
+  return want <= 64 ? 64 : want <= 128 ? 128 : 256;
+}
 
 extern "C" int qv_moe_max_tiles(int R, int E, int bm) {
   const int a = (R + bm - 1) / bm + E;
@@ -403,6 +485,7 @@ extern "C" int qv_moe_group(int* row_token, int* slot_row, int* tiles, const int
   if (T <= 0) return 0;
   if (E > 8192 || bm <= 0) return QV_ERR_UNSUPPORTED;
   const int R = T * top;
+  if (E > 4096) cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 2 * (int)sizeof(int));
   return qv_launch(moe_group_kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), (cudaStream_t)stream, row_token, slot_row, tiles,
                    qv_moe_max_tiles(R, E, bm), top_idx, rank_tmp, R, top, E, bm);
 }
@@ -516,186 +599,340 @@ extern "C" int qv_moe_experts(int up, void* out, int ld_out, const void* a, int 
 }
 
 // ---------------------------------------------------------------- the experts' products on the tensor cores (bfloat16)
-// Tile of 64 grouped rows x 64 columns, k in steps of BK through a cp.async ring of STAGES buffers; four warps, each
-// 32 x 32 as mma.sync m16n8k16 with float32 accumulators; rows of A are gathered by row_token (UP) while they
-// are copied, rows past the tile's end and k past K are zero-filled.  K must be a multiple of 8.
-#define TC_BN 64
+// Weights are the 128-row operand of tcgen05.mma, a tile's grouped rows (or, for steps of up to 32 tokens, all tokens) the narrow one,
+// so an expert's matrices are read once per tile of rows whatever the number of rows, and rows are padded to 16 only.  One CTA per SM
+// walks over (tile, block of features) items, features fastest: the CTAs at work share a tile's rows in L2 and stream different weights.
+//   warp 0      weights by contiguous bulk copies (packed tiles), rows by TMA in boxes of 32 rows x 64 k, through a ring of STAGES
+//   warp 1      tcgen05.mma, accumulators double-buffered in tensor memory
+//   warps 2..5  epilogue of the item before: activation, stores (a thread holds a feature, columns are rows)
+// Gated up product: the 128 rows are 16 gate rows and the 16 up rows of the same features in turn, so a warp holds both halves.
+// What bounds it: the matrices' bytes (few rows an expert) or what an SM takes in from L2 (16 KB of weights and the rows' tile a k
+// block).
+struct ExpertsArgs {
+  void* out;
+  const uint8_t* w1;
+  const uint8_t* w2;
+  const int* row_token;
+  const int* tiles;
+  int* err;
+  int max_tiles, N, K, ld_out;
+  int tokens;                                // > 0: the rows of the narrow operand are the tokens, and row_token says which a row is
+  GluAct glu;
+};
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void ldsm4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(s));
-}
-__device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+  return r;
 }
 
-template <int MODE, int BK, int STAGES>
-__global__ void __launch_bounds__(128) moe_experts_tc_kernel(void* __restrict__ out_, int ld_out, const bf16* __restrict__ a, int ld_a,
-                                                             const bf16* __restrict__ w1, const bf16* __restrict__ w2,
-                                                             const int* __restrict__ row_token, const int* __restrict__ tiles, int N, int K,
-                                                             GluAct glu) {
-  constexpr bool GATHER = MODE != 0;         // modes as in moe_experts_kernel
-  constexpr bool UP = MODE == 1;
-  constexpr int LD = BK + 8;                 // padded row of a staged tile: ldmatrix without bank conflicts
-  constexpr int PIECES = BK / 8;             // 16-byte pieces of a row
-  constexpr int TILE = 64 * LD;              // elements of one staged 64-row tile
-  extern __shared__ __align__(16) unsigned char moe_smem[];
-  bf16* As = (bf16*)moe_smem;                // [STAGES][64][LD]
-  bf16* B1 = As + STAGES * TILE;             // [STAGES][64][LD]
-  bf16* B2 = B1 + STAGES * TILE;             // [STAGES][64][LD] (UP)
-  pdl_wait();
+template <int MODE, int RT, int STAGES>
+__global__ void __launch_bounds__(192) moe_experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const ExpertsArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  constexpr int W_BYTES = BM * BK * 2;               // 128 weight rows x 64 k
+  constexpr int STAGE_BYTES = W_BYTES + RT * BK * 2;
+  constexpr int TMEM_COLS = 2 * RT;
+  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(ring + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;               // [2]
+  uint64_t* acc_empty = acc_full + 2;                // [2]
+  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
-  const int e = tiles[3 * blockIdx.y];
-  if (e < 0) return;
-  const int row0 = tiles[3 * blockIdx.y + 1], rows = tiles[3 * blockIdx.y + 2];
-  const int n0 = blockIdx.x * TC_BN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  // weights are packed: [expert][N/64][K/64] tiles of 64 rows x 64 k, each 8 KB contiguous (zero-padded at the edges)
-  static_assert(BK == 64, "a stage is one packed tile");
-  const int NT = (N + 63) / 64, KT = (K + 63) / 64;
-  const bf16* W1 = w1 + ((size_t)e * NT + blockIdx.x) * KT * 4096;
-  const bf16* W2 = UP ? w2 + ((size_t)e * NT + blockIdx.x) * KT * 4096 : nullptr;
-  auto stage = [&](int buf, int k0) {
-    if (k0 < K) {
-      const size_t tile_off = (size_t)(k0 / 64) * 4096;
-      for (int c = tid; c < 64 * PIECES; c += 128) {
-        const int r = c / PIECES, pc = c - r * PIECES, k = k0 + pc * 8;
-        const bool kin = k < K, aok = r < rows && kin;
-        const size_t src_row = aok ? (GATHER ? (size_t)row_token[row0 + r] : (size_t)(row0 + r)) : 0;
-        cp_async16(As + buf * TILE + r * LD + pc * 8, a + src_row * ld_a + (kin ? k : 0), aok ? 16 : 0);
-        cp_async16(B1 + buf * TILE + r * LD + pc * 8, W1 + tile_off + c * 8, 16);
-        if (UP) cp_async16(B2 + buf * TILE + r * LD + pc * 8, W2 + tile_off + c * 8, 16);
+  pdl_wait();                                        // the tile table, the rows and the output belong to the kernels ahead until here
+  const int NT = (p.N + 63) / 64, KT = (p.K + BK - 1) / BK;
+  const int blocks = MODE == 1 ? NT : (NT + 1) / 2;  // items of a tile: 64 features of two matrices, or 128 of one
+  const int items = p.max_tiles * blocks;
+
+  if (warp == 0) {
+    const bool leader = elect_one();
+    int it = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+      const int t = item / blocks, fb = item - t * blocks;
+      const int e = p.tiles[3 * t];
+      if (e < 0) break;
+      const int row0 = p.tokens ? 0 : p.tiles[3 * t + 1], rows = p.tokens ? p.tokens : p.tiles[3 * t + 2];
+      const int boxes = (rows + 31) / 32;
+      const int halves = MODE == 1 ? 2 : (2 * fb + 1 < NT ? 2 : 1);        // 8 KB weight tiles a stage
+      const uint8_t* w1 = p.w1 + ((size_t)e * NT + (MODE == 1 ? fb : 2 * fb)) * KT * 8192;
+      const uint8_t* w2 = MODE == 1 ? p.w2 + ((size_t)e * NT + fb) * KT * 8192 : w1 + (size_t)KT * 8192;
+      for (int kb = 0; kb < KT; ++kb, ++it) {
+        const int s = it % STAGES;
+        if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.err, 31)) { ok = false; break; }
+        if (leader) {
+          uint8_t* dst = ring + s * STAGE_BYTES;
+          mbar_expect_tx(&full[s], halves * 8192 + boxes * 4096);
+          const uint8_t* s1 = w1 + (size_t)kb * 8192;
+          const uint8_t* s2 = w2 + (size_t)kb * 8192;
+          if (MODE == 1) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {            // 16 gate rows, then the 16 up rows of the same features
+              bulk_load_1d(dst + q * 4096, s1 + q * 2048, &full[s], 2048);
+              bulk_load_1d(dst + q * 4096 + 2048, s2 + q * 2048, &full[s], 2048);
+            }
+          } else {
+            bulk_load_1d(dst, s1, &full[s], 8192);
+            if (halves == 2) bulk_load_1d(dst + 8192, s2, &full[s], 8192);
+          }
+          for (int x = 0; x < boxes; ++x) tma_load_2d(dst + W_BYTES + x * 4096, &map_a, &full[s], kb * BK, row0 + 32 * x);
+        }
+        __syncwarp();
       }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");      // one group a stage, empty past the end, so the counts below hold
-  };
-  float acc1[2][4][4] = {}, acc2[UP ? 2 : 1][4][4] = {};
-  const int nk = (K + BK - 1) / BK;
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    int it = 0, local = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; ok && item < items; item += gridDim.x, ++local) {
+      const int t = item / blocks;
+      if (p.tiles[3 * t] < 0) break;
+      const int rows = p.tokens ? p.tokens : p.tiles[3 * t + 2];
+      const uint32_t idesc = umma_idesc(BM, (rows + 15) & ~15);
+      const int b = local & 1;
+      ok = mbar_wait(&acc_empty[b], ((local >> 1) & 1) ^ 1, p.err, 34);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + (uint32_t)(b * RT);
+      for (int kb = 0; kb < KT; ++kb, ++it) {
+        const int s = it % STAGES;
+        ok = mbar_wait(&full[s], (it / STAGES) & 1, p.err, 32);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(ring + s * STAGE_BYTES);
+        const uint64_t da = umma_desc(a_addr), db = umma_desc(a_addr + W_BYTES);
+        if (leader) {
 #pragma unroll
-  for (int st = 0; st < STAGES - 1; ++st) stage(st, st * BK);
-  for (int kt = 0; kt < nk; ++kt) {
-    const int buf = kt % STAGES;
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();                         // stage kt has landed for everyone; the buffer refilled next was read a round ago
-    stage((kt + STAGES - 1) % STAGES, (kt + STAGES - 1) * BK);
-    const bf16* Ab = As + buf * TILE;
-    const bf16* B1b = B1 + buf * TILE;
-    const bf16* B2b = B2 + buf * TILE;
-#pragma unroll
-    for (int ks = 0; ks < BK / 16; ++ks) {
-      uint32_t af[2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-        ldsm4(af[mt][0], af[mt][1], af[mt][2], af[mt][3], Ab + (wm * 32 + mt * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
-#pragma unroll
-      for (int pr = 0; pr < 2; ++pr) {
-        const int n = wn * 32 + pr * 16 + (lane >> 4) * 8 + (lane & 7), k = ks * 16 + ((lane >> 3) & 1) * 8;
-        uint32_t b[4];
-        ldsm4(b[0], b[1], b[2], b[3], B1b + n * LD + k);
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          mma16816(acc1[mt][pr * 2], af[mt], b[0], b[1]);
-          mma16816(acc1[mt][pr * 2 + 1], af[mt], b[2], b[3]);
+          for (int kk = 0; kk < BK / 16; ++kk) umma_f16(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(&empty[s]);
         }
-        if (UP) {
-          ldsm4(b[0], b[1], b[2], b[3], B2b + n * LD + k);
+        __syncwarp();
+      }
+      if (leader) umma_commit(&acc_full[b]);
+      __syncwarp();
+    }
+  } else {
+    const int q = warp & 3;
+    int local = 0;
+    for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
+      const int t = item / blocks, fb = item - t * blocks;
+      if (p.tiles[3 * t] < 0) break;
+      const int row0 = p.tiles[3 * t + 1], rows = p.tiles[3 * t + 2];
+      const int b = local & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (local >> 1) & 1, p.err, 33))) break;     // (the MMA warp then gives up too)
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * RT);
+      const int feat = MODE == 1 ? fb * 64 + q * 16 + (lane & 15) : fb * 128 + q * 32 + lane;
+#pragma unroll 1
+      for (int c0 = 0; c0 < rows; c0 += 16) {
+        uint32_t r[16];
+        if (p.tokens) {
 #pragma unroll
-          for (int mt = 0; mt < 2; ++mt) {
-            mma16816(acc2[mt][pr * 2], af[mt], b[0], b[1]);
-            mma16816(acc2[mt][pr * 2 + 1], af[mt], b[2], b[3]);
+          for (int j = 0; j < 16; ++j) {
+            int col = p.row_token[row0 + (c0 + j < rows ? c0 + j : 0)];
+            if ((unsigned)col >= (unsigned)p.tokens) col = 0;
+            r[j] = tmem_ld1(taddr + col);
+          }
+          tmem_wait_ld();
+        } else {
+          tmem_ld16(taddr + c0, r);
+          tmem_wait_ld();
+        }
+        if (MODE == 1) {
+          // a lane of the lower half gives its gate value of the odd row for the up value of the even row
+          const int up = lane >> 4;
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const float give = __uint_as_float(up ? r[j] : r[j + 1]);
+            const float got = __shfl_xor_sync(0xffffffffu, give, 16);
+            const float g = up ? got : __uint_as_float(r[j]), u = up ? __uint_as_float(r[j + 1]) : got;
+            const int row = c0 + j + up;
+            if (row < rows && feat < p.N)
+              ((bf16*)p.out)[(size_t)(row0 + row) * p.ld_out + feat] = __float2bfloat16_rn(glu_apply(g, u, p.glu));
+          }
+        } else if (feat < p.N) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (c0 + j >= rows) break;
+            const float v = __uint_as_float(r[j]);
+            const size_t at = (size_t)(row0 + c0 + j) * p.ld_out + feat;
+            if (MODE == 2) ((bf16*)p.out)[at] = __float2bfloat16_rn(fmaxf(v, 0.f) * fmaxf(v, 0.f));
+            else ((float*)p.out)[at] = v;
           }
         }
+        __syncwarp();
       }
+      tc_fence_before();
+      mbar_arrive(&acc_empty[b]);
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  // accumulator (mt, nt): rows wm*32 + mt*16 + lane/4 (+8), columns wn*32 + nt*8 + 2*(lane%4) (+1)
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int r = wm * 32 + mt * 16 + (lane >> 2) + half * 8;
-      if (r >= rows) continue;
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int n = n0 + wn * 32 + nt * 8 + 2 * (lane & 3) + j;
-          if (n >= N) continue;
-          const float v = acc1[mt][nt][half * 2 + j];
-          if (UP) ((bf16*)out_)[(size_t)(row0 + r) * ld_out + n] = __float2bfloat16_rn(glu_apply(v, acc2[mt][nt][half * 2 + j], glu));
-          else if (MODE == 2) ((bf16*)out_)[(size_t)(row0 + r) * ld_out + n] = __float2bfloat16_rn(fmaxf(v, 0.f) * fmaxf(v, 0.f));
-          else ((float*)out_)[(size_t)(row0 + r) * ld_out + n] = v;
-        }
-      }
-    }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
+}
+
+// out[r] = a[row_token[r]]: the rows in grouped order, for the boxes above (16-byte pieces; rows beyond the last choice copy any row).
+__global__ void __launch_bounds__(256) moe_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ a, int ld16, int pieces,
+                                                         const int* __restrict__ row_token, int R, int T) {
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int r = blockIdx.x; r < R; r += gridDim.x) {
+    int t = row_token[r];
+    if ((unsigned)t >= (unsigned)T) t = 0;
+    for (int i = threadIdx.x; i < pieces; i += blockDim.x) out[(size_t)r * pieces + i] = a[(size_t)t * ld16 + i];
+  }
+}
+
+static int moe_sms() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0, v = 0;
+    n = (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) ? v : 148;
+  }
+  return n;
+}
+
+template <int MODE, int RT, int STAGES>
+static int moe_experts_launch(const CUtensorMap& map, const ExpertsArgs& p, cudaStream_t st) {
+  constexpr int smem = STAGES * (BM * BK * 2 + RT * BK * 2) + 1024 + 256;
+  auto kernel = moe_experts_tc_kernel<MODE, RT, STAGES>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int NT = (p.N + 63) / 64;
+  const long long items = (long long)p.max_tiles * (MODE == 1 ? NT : (NT + 1) / 2);
+  if (items > 0x40000000LL) return QV_ERR_TOO_LARGE;
+  return qv_launch(kernel, dim3((unsigned)(items < moe_sms() ? items : moe_sms())), dim3(192), (size_t)smem, st, map, p);
+}
+
+// w [E][N][K] -> the packed tiles (see qv_moe_experts_tc), zero where a matrix ends.  K a multiple of 8, w on 16 bytes.
+__global__ void __launch_bounds__(256) moe_pack_kernel(uint4* __restrict__ out, const bf16* __restrict__ w, int N, int K, int NT, int KT) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const size_t tile = ((size_t)blockIdx.z * NT + blockIdx.y) * KT + blockIdx.x;
+  const bf16* src = w + (size_t)blockIdx.z * N * K;
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    const int r = i >> 3, c = i & 7, n = blockIdx.y * 64 + r, k = blockIdx.x * 64 + c * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (n < N && k < K) v = *(const uint4*)(src + (size_t)n * K + k);
+    out[tile * 512 + r * 8 + (c ^ (r & 7))] = v;
+  }
+}
+
+extern "C" int qv_moe_pack_experts(void* out, const void* w, int E, int N, int K, void* stream) {
+  if (E <= 0 || N <= 0 || K < 8 || (K & 7) || (((uintptr_t)out | (uintptr_t)w) & 15)) return QV_ERR_UNSUPPORTED;
+  const int NT = (N + 63) / 64, KT = (K + 63) / 64;
+  if (E > 65535 || NT > 65535) return QV_ERR_TOO_LARGE;
+  return qv_launch(moe_pack_kernel, dim3(KT, NT, E), dim3(256), 0, (cudaStream_t)stream, (uint4*)out, (const bf16*)w, N, K, NT, KT);
 }
 
 // As qv_moe_experts for bfloat16 operands, on the tensor cores, with the experts' matrices packed in tiles of 64 x 64
-// ([E][ceil(N/64)][ceil(K/64)][64][64], zero-padded: what a stage copies is 8 KB in one piece, which memory delivers
-// several times faster than 64 rows that lie a whole matrix row apart).  The tile table must have been made for tiles
-// of qv_moe_tile_rows(1) rows.  Refuses rows of `a` that do not start on 16 bytes.
-extern "C" int qv_moe_experts_tc(int up, void* out, int ld_out, const void* a, int ld_a, const void* w1, const void* w2,
+// ([E][ceil(N/64)][ceil(K/64)][64][64], zero-padded, the eight 16-byte chunks of row r at chunk ^ (r % 8): the image the product
+// reads from shared memory).  tile_rows: what the tile table was made for (32, 64, 128 or 256).  a_rows: the rows of `a`.
+// gathered: room for R rows of K elements, for up products of more than 32 tokens.  Refuses rows of `a` that do not start on 16 bytes.
+extern "C" int qv_moe_experts_tc(int up, void* out, int ld_out, const void* a, int ld_a, int a_rows, const void* w1, const void* w2,
                                  const int* row_token, const int* tiles, int R, int E, int N, int K, int act, float limit, float slope,
-                                 void* stream) {
+                                 int tile_rows, void* gathered, int* err, void* stream) {
   if (R <= 0) return 0;
-  if (act < 0 || act > 2) return QV_ERR_UNSUPPORTED;
-  const GluAct glu = {act, limit, slope};
+  if (act < 0 || act > 2 || up < 0 || up > 2 || N <= 0 || K < 8 || (K & 7)) return QV_ERR_UNSUPPORTED;
   if ((ld_a & 7) || (((uintptr_t)a | (uintptr_t)w1 | (uintptr_t)w2) & 15)) return QV_ERR_UNSUPPORTED;
-  const int max_tiles = qv_moe_max_tiles(R, E, MOE_TC_BM);
-  if (max_tiles > 65535) return QV_ERR_TOO_LARGE;
-  dim3 grid((N + TC_BN - 1) / TC_BN, max_tiles);
+  const bool direct = up && a_rows <= 32;
   cudaStream_t st = (cudaStream_t)stream;
-  // k in steps of 64 through three stages: a row of a weight tile is then a whole 128-byte line and two stages of
-  // copies are in flight while one is multiplied
-  constexpr int BK = 64, STAGES = 3;
-  const size_t smem = (size_t)STAGES * 64 * (BK + 8) * 2 * (up == 1 ? 3 : 2);
-  if (up == 1) {
-    cudaFuncSetAttribute(moe_experts_tc_kernel<1, BK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return qv_launch(moe_experts_tc_kernel<1, BK, STAGES>, grid, dim3(128), smem, st, out, ld_out, (const bf16*)a, ld_a, (const bf16*)w1,
-                     (const bf16*)w2, row_token, tiles, N, K, glu);
+  ExpertsArgs p;
+  p.out = out; p.w1 = (const uint8_t*)w1; p.w2 = (const uint8_t*)w2; p.row_token = row_token; p.tiles = tiles; p.err = err;
+  p.max_tiles = qv_moe_max_tiles(R, E, tile_rows); p.N = N; p.K = K; p.ld_out = ld_out; p.tokens = direct ? a_rows : 0;
+  p.glu = {act, limit, slope};
+  CUtensorMap map;
+  if (up && !direct) {
+    if (!gathered || ((uintptr_t)gathered & 15)) return QV_ERR_UNSUPPORTED;
+    const int pieces = K / 8;
+    const int rc = qv_launch(moe_gather_kernel, dim3(R < 148 * 16 ? R : 148 * 16), dim3(pieces >= 256 ? 256 : pieces >= 128 ? 128 : 64), 0, st,
+                             (uint4*)gathered, (const uint4*)a, ld_a / 8, pieces, row_token, R, a_rows);
+    if (rc) return rc;
+    if (!make_map(&map, gathered, R, K, K, 32)) return QV_ERR_UNSUPPORTED;
+  } else if (!make_map(&map, a, direct ? a_rows : R, K, ld_a, 32)) {
+    return QV_ERR_UNSUPPORTED;
   }
-  if (up == 2) {
-    cudaFuncSetAttribute(moe_experts_tc_kernel<2, BK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return qv_launch(moe_experts_tc_kernel<2, BK, STAGES>, grid, dim3(128), smem, st, out, ld_out, (const bf16*)a, ld_a, (const bf16*)w1,
-                     (const bf16*)w2, row_token, tiles, N, K, glu);
-  }
-  cudaFuncSetAttribute(moe_experts_tc_kernel<0, BK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return qv_launch(moe_experts_tc_kernel<0, BK, STAGES>, grid, dim3(128), smem, st, out, ld_out, (const bf16*)a, ld_a, (const bf16*)w1,
-                   (const bf16*)w2, row_token, tiles, N, K, glu);
+#define EXPERTS_TC(RT, ST)                                                                    \
+  do {                                                                                        \
+    if (up == 1) return moe_experts_launch<1, RT, ST>(map, p, st);                            \
+    if (up == 2) return moe_experts_launch<2, RT, ST>(map, p, st);                            \
+    return moe_experts_launch<0, RT, ST>(map, p, st);                                         \
+  } while (0)
+  if (tile_rows == 32) EXPERTS_TC(32, 10);
+  if (tile_rows == 64) EXPERTS_TC(64, 8);
+  if (tile_rows == 128) EXPERTS_TC(128, 6);
+  if (tile_rows == 256) EXPERTS_TC(256, 4);
+#undef EXPERTS_TC
+  return QV_ERR_UNSUPPORTED;
 }
 
 // delta [T, d] float32.  mix, shared, h (the tokens' inputs, read for identity experts): [T, d] in the compute type or null; gate
-// [T] float32 or null.
-template <typename T>
+// [T] float32 or null.  VEC elements a thread: 4 where all rows allow 16-byte (8-byte) accesses.  It moves the choices' float32 rows
+// once; one element a thread kept too few bytes in flight (2,048 tokens x 6 choices x 2,048: 44 us).
+template <typename T, int VEC>
 __global__ void __launch_bounds__(256) moe_combine_kernel(float* __restrict__ delta, const T* __restrict__ mix, const float* __restrict__ y,
                                                           const int* __restrict__ slot_row, const float* __restrict__ top_w,
                                                           const T* __restrict__ shared, const float* __restrict__ gate, int d, int top,
                                                           const float* __restrict__ s_mix, const float* __restrict__ s_ff,
                                                           const T* __restrict__ h, int ld_h) {
+  struct alignas(sizeof(T) * VEC) PackT { T v[VEC]; };
+  struct alignas(4 * VEC) PackF { float v[VEC]; };
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
   const float g = gate ? gate[t] : 1.f;
-  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < d; i += gridDim.y * blockDim.x) {
-    float routed = 0.f;
+  for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; i < d; i += gridDim.y * blockDim.x * VEC) {
+    float routed[VEC] = {};
+#pragma unroll 4
     for (int j = 0; j < top; ++j) {
       const int r = slot_row[(size_t)t * top + j];
-      const float yv = r >= 0 ? y[(size_t)r * d + i] : (h ? to_f(h[(size_t)t * ld_h + i]) : 0.f);
-      routed = fmaf(top_w[(size_t)t * top + j], yv, routed);
+      const float w = top_w[(size_t)t * top + j];
+      PackF yv = {};
+      if (r >= 0) {
+        yv = *(const PackF*)(y + (size_t)r * d + i);
+      } else if (h) {
+        const PackT hv = *(const PackT*)(h + (size_t)t * ld_h + i);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) yv.v[k] = to_f(hv.v[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) routed[k] = fmaf(w, yv.v[k], routed[k]);
     }
-    float v = routed;
-    if (shared) v = fmaf(g, to_f(shared[(size_t)t * d + i]), v);
-    if (s_ff) v *= s_ff[i];
-    if (mix) v = fmaf(to_f(mix[(size_t)t * d + i]), s_mix ? s_mix[i] : 1.f, v);
-    delta[(size_t)t * d + i] = v;
+    PackT sv = {}, mv = {};
+    if (shared) sv = *(const PackT*)(shared + (size_t)t * d + i);
+    if (mix) mv = *(const PackT*)(mix + (size_t)t * d + i);
+    PackF o;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+      float v = routed[k];
+      if (shared) v = fmaf(g, to_f(sv.v[k]), v);
+      if (s_ff) v *= s_ff[i + k];
+      if (mix) v = fmaf(to_f(mv.v[k]), s_mix ? s_mix[i + k] : 1.f, v);
+      o.v[k] = v;
+    }
+    *(PackF*)(delta + (size_t)t * d + i) = o;
   }
 }
 
@@ -703,8 +940,13 @@ extern "C" int qv_moe_combine(float* delta, const void* mix, const float* y, con
                               const void* shared, const float* gate, int T, int d, int top, int dt, const float* s_mix,
                               const float* s_ff, const void* h, int ld_h, void* stream) {
   if (T <= 0) return 0;
-  QV_DISPATCH_DT(dt, TT,
-                 return qv_launch(moe_combine_kernel<TT>, dim3(T, T < 256 ? (d + 255) / 256 : 1), dim3(256), 0, (cudaStream_t)stream, delta, (const TT*)mix, y, slot_row,
-                                  top_w, (const TT*)shared, gate, d, top, s_mix, s_ff, (const TT*)h, ld_h));
+  const bool vec = d % 4 == 0 && ld_h % 4 == 0 && ((((uintptr_t)delta | (uintptr_t)y | (uintptr_t)mix | (uintptr_t)shared | (uintptr_t)h) & 15) == 0);
+  const int per = vec ? 1024 : 256;
+  const dim3 grid(T, T < 256 ? (d + per - 1) / per : 1);
+#define COMBINE(TT, V)                                                                                                                \
+  return qv_launch(moe_combine_kernel<TT, V>, grid, dim3(256), 0, (cudaStream_t)stream, delta, (const TT*)mix, y, slot_row, top_w,    \
+                   (const TT*)shared, gate, d, top, s_mix, s_ff, (const TT*)h, ld_h)
+  QV_DISPATCH_DT(dt, TT, if (vec) COMBINE(TT, 4); COMBINE(TT, 1));
+#undef COMBINE
   return QV_ERR_UNSUPPORTED;
 }

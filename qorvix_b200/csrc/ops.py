@@ -69,9 +69,10 @@ _ARGTYPES = {
     "qv_gated_group_norm": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _I, _V],
     "qv_moe_route": [_V, _V, _V, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _F, _I, _I, _I, _V],
     "qv_moe_max_tiles": [_I, _I, _I],
-    "qv_moe_tile_rows": [_I],
+    "qv_moe_tile_rows": [_I, _I, _I, _I],
     "qv_moe_group": [_V, _V, _V, _V, _V, _I, _I, _I, _I, _V],
-    "qv_moe_experts_tc": [_I, _V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _F, _F, _V],
+    "qv_moe_experts_tc": [_I, _V, _I, _V, _I, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _F, _F, _I, _V, _V, _V],
+    "qv_moe_pack_experts": [_V, _V, _I, _I, _I, _V],
     "qv_moe_experts": [_I, _V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _F, _V],
     "qv_moe_combine": [_V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _V, _V, _V, _I, _V],
     "qv_moe_route_table": [_V, _V, _V, _V, _I, _I, _I, _I, _V],
@@ -1133,9 +1134,10 @@ def moe_route(top_idx, top_w, gate_out, h, w_router, w_gate, correction=None, w_
         add_launches(1)
 
 
-def moe_tile_rows(tensor_cores: bool) -> int:
-    """Rows of a tile of grouped rows: what the tile table is made for (the two experts' kernels differ)."""
-    return int(_lib("moe").qv_moe_tile_rows(1 if tensor_cores else 0))
+def moe_tile_rows(tensor_cores: bool, tokens: int = 0, rows: int = 0, experts: int = 0) -> int:
+    """Rows of a tile of grouped rows: what the tile table is made for (the two experts' kernels differ, and the tensor-core kernel
+    takes the tiles that suit a step of `tokens` tokens with `rows` choices over `experts` experts, where these are given)."""
+    return int(_lib("moe").qv_moe_tile_rows(1 if tensor_cores else 0, tokens, rows, experts))
 
 
 def moe_max_tiles(rows: int, experts: int, tile_rows: int) -> int:
@@ -1153,28 +1155,38 @@ def moe_group(row_token, slot_row, tiles, top_idx, scratch, experts: int, tile_r
 
 
 def moe_pack_experts(w: torch.Tensor) -> torch.Tensor:
-    """Experts' matrices [E, N, K] (bfloat16) as tiles of 64 rows x 64 k, [E, ceil(N/64), ceil(K/64), 64, 64],
-    zero-padded at the edges: the layout the tensor-core kernel copies a stage from in one piece."""
+    """Experts' matrices [E, N, K] (bfloat16) as tiles of 64 rows x 64 k, [E, ceil(N/64), ceil(K/64), 64, 64], zero-padded at the
+    edges, the eight 16-byte chunks of a tile's row r in the order chunk ^ (r % 8): the layout the tensor-core kernel's products read
+    from shared memory, copied there in contiguous pieces."""
+    _need_cuda(w)
+    assert w.dtype == torch.bfloat16
     E, N, K = w.shape
-    Np, Kp = -(-N // 64) * 64, -(-K // 64) * 64
-    if (Np, Kp) != (N, K):
-        w = torch.nn.functional.pad(w, (0, Kp - K, 0, Np - N))
-    return w.view(E, Np // 64, 64, Kp // 64, 64).permute(0, 1, 3, 2, 4).contiguous()
+    out = torch.empty((E, -(-N // 64), -(-K // 64), 64, 64), device=w.device, dtype=w.dtype)
+    w = w.contiguous()
+    _check(_lib("moe").qv_moe_pack_experts(_ptr(out), _ptr(w), E, N, K, _stream()), "moe_pack_experts")
+    return out
 
 
-def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0) -> None:
+def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0, tile_rows: int = 0) -> None:
     """The experts' products on the tensor cores (bfloat16); up as for moe_experts.  p1, p2: matrices packed by moe_pack_experts; the sizes
-    follow from out [R, N] and a [., K]; the tile table was made for tiles of moe_tile_rows(True) rows."""
+    follow from out [R, N] and a [., K]; the tile table was made for tiles of `tile_rows` rows (0: moe_tile_rows(True))."""
     _need_cuda(out, a, p1, p2, row_token, tiles)
     R, N = out.shape
     K = a.shape[1]
     E = p1.shape[0]
     assert a.dtype == p1.dtype == torch.bfloat16 and a.stride(1) == 1 and out.stride(1) == 1 and a.stride(0) % 8 == 0
     assert p1.is_contiguous() and tuple(p1.shape[1:]) == (-(-N // 64), -(-K // 64), 64, 64) and R == row_token.numel()
-    assert out.dtype == (torch.bfloat16 if up else torch.float32)
-    rc = _lib("moe").qv_moe_experts_tc(int(up), _ptr(out), out.stride(0), _ptr(a), a.stride(0), _ptr(p1), _ptr(p2),
-                                       _ptr(row_token), _ptr(tiles), R, E, N, K, act, float(limit), float(slope), _stream())
+    assert p2 is None or (p2.is_contiguous() and p2.shape == p1.shape and p2.dtype == p1.dtype)
+    assert out.dtype == (torch.bfloat16 if up else torch.float32) and (up or a.shape[0] == R)
+    tile_rows = tile_rows or moe_tile_rows(True)
+    gathers = bool(up) and a.shape[0] > 32                     # the rows in grouped order, for the up products of longer steps
+    gathered = torch.empty((R, K), device=a.device, dtype=a.dtype) if gathers else None
+    rc = _lib("moe").qv_moe_experts_tc(int(up), _ptr(out), out.stride(0), _ptr(a), a.stride(0), a.shape[0], _ptr(p1), _ptr(p2),
+                                       _ptr(row_token), _ptr(tiles), R, E, N, K, act, float(limit), float(slope), tile_rows,
+                                       _ptr(gathered), _ptr(_tc_buffers(a.device)["err"]), _stream())
     _check(rc, "moe_experts_tc")
+    if gathers:
+        add_launches(1)
 
 
 def moe_experts(up, out, a, w1, w2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0) -> None:
