@@ -142,6 +142,7 @@ struct ScanArgs {
   float* state; long long slot_stride;    // per slot: [H][tiles][dk * 32 (+ dk + 1 for GATED_MAX)]
   const int* seg_q_start; const int* seg_slot;
   int H, dk, dv;
+  int chunk_from;                         // segments of at least this many tokens are linear_scan_chunk_kernel's (INT_MAX: none)
 };
 
 __host__ __device__ inline int scan_tile_floats(int kind, int dk, int vt = SCAN_VT) { return dk * vt + (kind == SCAN_GATED_MAX ? dk + 1 : 0); }
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(SCAN_VT * SCAN_WARPS) linear_scan_kernel(ScanA
   float* red = ns + dk;                    // [SCAN_WARPS][32]
   float* sc = red + SCAN_WARPS * SCAN_VT;  // [2]: n . q, spare
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len >= a.chunk_from) return;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk);
   for (int i = threadIdx.x; i < dk * SCAN_VT; i += blockDim.x) S[i] = st[i];
   float m = 0.f;
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(SCAN_VT * SCAN_WARPS) linear_scan_reg_kernel(S
   float* ge = gt + SCAN_CH;                        // [SCAN_CH] exp(-m) (GATED_MAX)
   float* gm = ge + SCAN_CH;                        // [SCAN_CH] scratch of the running maximum
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len >= a.chunk_from) return;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk, VT);
   float S[RPT];
 #pragma unroll
@@ -427,15 +430,489 @@ __global__ void __launch_bounds__(SCAN_VT * SCAN_WARPS) linear_scan_reg_kernel(S
   }
 }
 
+// ---------------------------------------------------------------- portions: tokens in chunks, on the tensor cores (bfloat16 q, k, v)
+// Within a chunk of 64 tokens, with the decays' running logarithm F_t (from the chunk's start), the running maximum m_t and S_0 the state
+// ahead of the chunk:
+//   y_t   = A_t S_0^T q_t + sum_{j <= t} W_tj v_j        W_tj = exp(G_t + H_j) b_j (q_t . k_j),  A_t = exp(G_t + m_0)
+//   S_end = A_63 S_0 + sum_j (c_j v_j) k_j^T             c_j  = exp(G_63 + H_j) b_j
+// GATED_MAX: G_t = F_t - m_t, H_j = log i_j - F_j, b_j = 1, m_t = F_t + max(m_0, max_{j <= t} H_j), and n . q is n_0's share plus the rows'
+// sums of W.  DECAY: G_t = F_t, H_j = -F_j, b_j = dt_j, m_0 = 0.  Every exponent is <= 0; F, m, G and H are kept in float64, so that the
+// difference of two long sums is as good as a short one; for W, G and H are kept as pairs of float32.
+// All four products are mma.sync with float32 sums whose one operand holds bfloat16 values as they are stored (q, k, v) and whose other
+// is a float32 quantity (state, W, c v) in three bfloat16 terms that hold its 24 bits: what was float32 in the token-by-token kernel is
+// as exact here.
+// A CTA owns a (segment, head, tile of VT value columns) and keeps its state in registers as S^T: a warp has 16 columns and a slice of
+// 16 NK key rows, laid out so that the accumulators of the update are, term by term, the second operand of S^T q without any exchange.
+// Products with S_0 are split over the key slices, so the slices' sums meet in shared memory.  Eight warps hold the state (first S^T q,
+// then the update), eight form W and W v (then the sums and the output); one of these, whose part of W is empty, works out the next chunk's
+// gates; the next chunk's
+// q, k, v arrive by cp.async (a bulk copy a row takes its issuing warp 50 clocks, three times what the chunk may take): a chunk is two stretches between CTA barriers.  n is kept like a value column of ones.
+// The tensor cores cut the sums' low bits off as they add; so long sums are taken in short runs that are added in float32, a term's small
+// parts apart from its large one, and the update apart from the state.
+// What bounds it: a chunk's chain of products and the two barriers (a prompt has only heads x tiles CTAs); mma.sync issues a product in
+// some 8 clocks a scheduler.  2,048 tokens of 4 heads of 256 x 512: 2,573 us token by token, 180 in chunks; portions of 777, 583 and
+// 583 tokens of 64 heads of 128 x 64: 897 and 130 us.
+#define LC_C 64
+__device__ __forceinline__ void lc_ldsm4(uint32_t* r, const void* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void lc_ldsm4t(uint32_t* r, const void* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void lc_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// x and y as three bfloat16 terms each (x in the lower half of a word)
+__device__ __forceinline__ void lc_split3(float x, float y, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    t[i] = *(const uint32_t*)&h;
+    x -= __low2float(h);
+    y -= __high2float(h);
+  }
+}
+
+__device__ __forceinline__ void lc_cp16(void* dst, const void* src, bool live) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ float2 lc_pair(double x) {
+  const float hi = (float)x;
+  return make_float2(hi, (float)(x - (double)hi));
+}
+// exp(x + y) of two such numbers whose sum is small beside them (Knuth's two-sum: what the first sum's rounding dropped)
+__device__ __forceinline__ float lc_exp_sum(float2 x, float2 y) {
+  const float s = x.x + y.x, b = s - x.x;
+  const float e = (x.x - (s - b)) + (y.x - b);
+  return expf(s + (e + (x.y + y.y)));
+}
+
+struct LcGates {                           // what a chunk's gates amount to
+  float2 G[LC_C], H[LC_C];                           // a number and what rounding it to float32 left over
+  float b[LC_C], A[LC_C], c[LC_C], em[LC_C];         // em: exp(-m_t)
+  bf16 ct[3][LC_C];                                  // c in three terms
+  float A_end, m_end, pad[2];
+};
+#define LC_GATE_WARP 9                     // of the eight that form W: its 16 x 32 tokens lie above the diagonal
+#define LC_BATCH 512                       // tokens whose gates' logarithms are worked out together, by all threads
+
+template <int VT, int NK> struct LcShape {
+  static constexpr int SLICES = VT == 16 ? 8 : 4;    // key slices; warps = slices x (VT / 16)
+  static constexpr int DKP = SLICES * 16 * NK;
+  static constexpr int LDQ = DKP + 8, LDV = VT + 8, LDR = VT + 8;
+  static constexpr int STAGE = 2 * LC_C * LDQ * 2;                                     // bytes: q and k of a chunk
+  static constexpr int RED = (SLICES + 2) * LC_C * LDR * 4;                            // the slices' sums, and W v's two
+  static constexpr int V = LC_C * LDV * 2;
+  static constexpr int BYTES = 2 * STAGE + RED + 5 * V + 2 * (int)sizeof(LcGates) + LC_C * 2 * 4 + SLICES * LC_C * 4 + 2 * LC_BATCH * 4;
+};
+
+#define LC_THREADS 512
+template <int KIND, int VT, int NK>
+__global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanArgs a) {
+  typedef LcShape<VT, NK> Sh;
+  constexpr int SLICES = Sh::SLICES, DKP = Sh::DKP, LDQ = Sh::LDQ, LDV = Sh::LDV, LDR = Sh::LDR;
+  extern __shared__ __align__(16) unsigned char lc_smem[];
+  unsigned char* stages = lc_smem;                                   // [2][q | k]
+  float* red = (float*)(lc_smem + 2 * Sh::STAGE);                    // [SLICES + 2][64][LDR]
+  bf16* vbuf = (bf16*)(lc_smem + 2 * Sh::STAGE + Sh::RED);           // [2][64][LDV]
+  bf16* vs = vbuf + 2 * LC_C * LDV;                                  // [3][64][LDV] terms of c_j v_j
+  LcGates* gates = (LcGates*)(vs + 3 * LC_C * LDV);                  // [2]
+  float* rowsum = (float*)(gates + 2);                               // [64][2]
+  float* nq = rowsum + LC_C * 2;                                     // [SLICES][64] the slices' shares of A_t n_0 . q_t
+  float* lfb = nq + SLICES * LC_C;                                   // [LC_BATCH] log of the decay
+  float* lib = lfb + LC_BATCH;                                       // [LC_BATCH] log of the input gate | step size
+  pdl_wait();
+  pdl_launch_dependents();
+  const int s = blockIdx.x, h = blockIdx.y, tile = blockIdx.z;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len < a.chunk_from) return;
+  const int dk = a.dk, dv = a.dv;
+  const int tiles = (dv + VT - 1) / VT;
+  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk, VT);
+  const bf16* qb = (const bf16*)a.q + (size_t)(h / a.q_group) * dk;
+  const bf16* kb = (const bf16*)a.k + (size_t)(h / a.q_group) * dk;
+  const bf16* vb = (const bf16*)a.v + (size_t)h * dv + tile * VT;
+  const int nchunks = (len + LC_C - 1) / LC_C;
+  const int slice = warp % SLICES, half = (warp / SLICES) * 16;      // of the state's warps: key rows, value columns
+  const int k0 = slice * 16 * NK;
+  const int g8 = lane >> 2, t4 = lane & 3, mi = lane >> 3, r8 = lane & 7;
+
+  // chunk c's q, k, v (zeros beyond the segment and beyond dk): a thread copies the same 16 bytes of every few rows
+  constexpr int PQ = DKP / 8, PV = VT / 8, RSTEP = LC_THREADS / PQ;
+  const int qrow = tid / PQ, qpc = tid % PQ, vrow = tid / PV, vpc = tid % PV;
+  const bf16* qp = qb + (size_t)(q0 + qrow) * a.ld_q + qpc * 8;
+  const bf16* kp = kb + (size_t)(q0 + qrow) * a.ld_k + qpc * 8;
+  const bf16* vp = vb + (size_t)(q0 + vrow) * a.ld_v + vpc * 8;
+  const bool q_in = qpc * 8 < dk, v_in = vrow < LC_C && tile * VT + vpc * 8 < dv;
+  auto issue = [&](int c) {
+    bf16* qs = (bf16*)(stages + (c & 1) * Sh::STAGE) + qrow * LDQ + qpc * 8;
+    const int left = len - c * LC_C;
+#pragma unroll
+    for (int i = 0; i < LC_C / RSTEP; ++i) {
+      const bool live = q_in && qrow + i * RSTEP < left;
+      lc_cp16(qs + i * RSTEP * LDQ, live ? qp + (size_t)(i * RSTEP) * a.ld_q : (const bf16*)a.q, live);
+      lc_cp16(qs + (LC_C + i * RSTEP) * LDQ, live ? kp + (size_t)(i * RSTEP) * a.ld_k : (const bf16*)a.k, live);
+    }
+    if (vrow < LC_C) {
+      const bool live = v_in && vrow < left;
+      lc_cp16(vbuf + ((c & 1) * LC_C + vrow) * LDV + vpc * 8, live ? vp : (const bf16*)a.v, live);
+    }
+    qp += (size_t)LC_C * a.ld_q;
+    kp += (size_t)LC_C * a.ld_k;
+    vp += (size_t)LC_C * a.ld_v;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the gates of chunk c, by one warp: two neighbouring tokens a lane, sums and maxima by scans over the warp
+  const float b1 = a.p1 ? a.p1[h] : 0.f, b2 = a.p2 ? a.p2[h] : 0.f, b3 = a.p3 ? a.p3[h] : 0.f;
+  const float rate = KIND == SCAN_DECAY ? expf(b2) : 0.f;
+  double m_run = 0.0;
+  if (KIND == SCAN_GATED_MAX) m_run = (double)st[dk * VT + dk];
+  // the logarithms of a batch of tokens' gates, a token a thread
+  auto work_logs = [&](int first) {
+    for (int i = tid; i < LC_BATCH && first + i < len; i += LC_THREADS) {
+      const size_t row = (size_t)(q0 + first + i);
+      if (KIND == SCAN_GATED_MAX) {
+        const float zf = a.cap * tanhf((a.g2[row * a.ld_g2 + h] + b2) / a.cap);
+        lfb[i] = fminf(zf, 0.f) - log1pf(expf(-fabsf(zf)));
+        lib[i] = a.cap * tanhf((a.g1[row * a.ld_g1 + h] + b1) / a.cap);
+      } else {
+        const float z = a.g1[row * a.ld_g1 + h] + b1;
+        lib[i] = z > 20.f ? z : log1pf(expf(z));
+      }
+    }
+  };
+  auto work_gates = [&](int c) {
+    LcGates& gt = gates[c & 1];
+    double lf[2], li[2];
+    float bb[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = c * LC_C + 2 * lane + i, tb = t % LC_BATCH;
+      lf[i] = 0.0; li[i] = -1e30; bb[i] = KIND == SCAN_DECAY ? 0.f : 1.f;      // a token beyond the segment: keeps all, adds nothing
+      if (t < len) {
+        if (KIND == SCAN_GATED_MAX) {
+          lf[i] = (double)lfb[tb];
+          li[i] = (double)lib[tb];
+        } else {
+          bb[i] = lib[tb];
+          lf[i] = -(double)rate * (double)bb[i];
+        }
+      }
+    }
+    double sum = lf[0] + lf[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+    }
+    double F[2], Hh[2], G[2], m[2] = {0.0, 0.0};
+    F[1] = sum;
+    F[0] = sum - lf[1];
+    if (KIND == SCAN_GATED_MAX) {
+      Hh[0] = li[0] - F[0]; Hh[1] = li[1] - F[1];
+      double mx = fmax(Hh[0], Hh[1]);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, mx, o);
+        if (lane >= o) mx = fmax(mx, up);
+      }
+      const double ahead = __shfl_up_sync(0xffffffffu, mx, 1);
+      const double before = lane ? fmax(m_run, ahead) : m_run;
+      m[0] = F[0] + fmax(before, Hh[0]);
+      m[1] = F[1] + fmax(m_run, mx);
+      G[0] = F[0] - m[0]; G[1] = F[1] - m[1];
+    } else {
+      Hh[0] = -F[0]; Hh[1] = -F[1];
+      G[0] = F[0]; G[1] = F[1];
+    }
+    const double G_end = __shfl_sync(0xffffffffu, G[1], 31), m_end = __shfl_sync(0xffffffffu, m[1], 31);
+    const float c0 = expf((float)(G_end + Hh[0])) * bb[0], c1 = expf((float)(G_end + Hh[1])) * bb[1];
+    uint32_t terms[3];
+    lc_split3(c0, c1, terms);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) *(uint32_t*)(gt.ct[x] + 2 * lane) = terms[x];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = 2 * lane + i;
+      gt.G[t] = lc_pair(G[i]);
+      gt.H[t] = lc_pair(Hh[i]);
+      gt.b[t] = bb[i];
+      gt.A[t] = expf((float)(G[i] + m_run));
+      gt.c[t] = i ? c1 : c0;
+      gt.em[t] = KIND == SCAN_GATED_MAX ? expf((float)-m[i]) : 1.f;
+    }
+    if (lane == 0) { gt.A_end = expf((float)(G_end + m_run)); gt.m_end = (float)m_end; }
+    m_run = m_end;
+  };
+
+  issue(0);
+  work_logs(0);
+  __syncthreads();
+  if (warp == LC_GATE_WARP) work_gates(0);
+  const bool has_n = KIND == SCAN_GATED_MAX && half == 0;            // n is kept like one more value column, all ones
+  float nT[2 * NK][4] = {};
+  float sT[2 * NK][4];                               // S^T: value columns half + g8 (+ 8), key rows k0 + 8 nt + 2 t4 (+ 1)
+  if (warp < 8) {
+#pragma unroll
+    for (int nt = 0; nt < 2 * NK; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = half + g8 + (i >> 1) * 8;
+        sT[nt][i] = k < dk ? st[k * VT + col] : 0.f;
+        if (has_n && g8 == 0 && i < 2 && k < dk) nT[nt][i] = st[dk * VT + k];
+      }
+  }
+
+  for (int c = 0; c < nchunks; ++c) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // chunk c and its gates are in place; everyone is done with chunk c - 1
+    if (c + 1 < nchunks) issue(c + 1);
+    const bf16* qs = (const bf16*)(stages + (c & 1) * Sh::STAGE);
+    const bf16* ks = qs + LC_C * LDQ;
+    const bf16* vc = vbuf + (c & 1) * LC_C * LDV;
+    const LcGates& gt = gates[c & 1];
+    if (warp < 8) {
+      // c_j v_j in three terms, for the update
+      for (int i = tid; i < LC_C * VT / 2; i += 256) {
+        const int t = i / (VT / 2), cc = (i - t * (VT / 2)) * 2;
+        const float cj = gt.c[t];
+        uint32_t w[3];
+        lc_split3(cj * to_f(vc[t * LDV + cc]), cj * to_f(vc[t * LDV + cc + 1]), w);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) *(uint32_t*)(vs + (x * LC_C + t) * LDV + cc) = w[x];
+      }
+      // this slice's share of A_t q_t S_0
+      uint32_t b0[NK][2][3], b1t[NK][2][3];          // [key step][column tile][term]
+#pragma unroll
+      for (int kk = 0; kk < NK; ++kk)
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          lc_split3(sT[2 * kk][2 * nb], sT[2 * kk][2 * nb + 1], b0[kk][nb]);
+          lc_split3(sT[2 * kk + 1][2 * nb], sT[2 * kk + 1][2 * nb + 1], b1t[kk][nb]);
+        }
+      uint32_t n0[NK][3], n1[NK][3];                 // n's: column 0 of a tile of eight
+      if (has_n) {
+#pragma unroll
+        for (int kk = 0; kk < NK; ++kk) {
+          lc_split3(nT[2 * kk][0], nT[2 * kk][1], n0[kk]);
+          lc_split3(nT[2 * kk + 1][0], nT[2 * kk + 1][1], n1[kk]);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float hi[2][4] = {}, lo[2][4] = {}, nh[4] = {}, nl[4] = {};
+#pragma unroll
+        for (int kk = 0; kk < NK; ++kk) {
+          uint32_t af[4];
+          lc_ldsm4(af, qs + (m * 16 + (mi & 1) * 8 + r8) * LDQ + k0 + kk * 16 + (mi >> 1) * 8);
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) {
+            lc_mma(lo[nb], af, b0[kk][nb][2], b1t[kk][nb][2]);
+            lc_mma(hi[nb], af, b0[kk][nb][0], b1t[kk][nb][0]);
+            lc_mma(lo[nb], af, b0[kk][nb][1], b1t[kk][nb][1]);
+          }
+          if (has_n) {
+            lc_mma(nl, af, n0[kk][2], n1[kk][2]);
+            lc_mma(nh, af, n0[kk][0], n1[kk][0]);
+            lc_mma(nl, af, n0[kk][1], n1[kk][1]);
+          }
+        }
+        const float a_lo = gt.A[m * 16 + g8], a_hi = gt.A[m * 16 + g8 + 8];
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          float* d = red + ((size_t)slice * LC_C + m * 16 + g8) * LDR + half + nb * 8 + 2 * t4;
+          *(float2*)d = make_float2(a_lo * (hi[nb][0] + lo[nb][0]), a_lo * (hi[nb][1] + lo[nb][1]));
+          *(float2*)(d + 8 * LDR) = make_float2(a_hi * (hi[nb][2] + lo[nb][2]), a_hi * (hi[nb][3] + lo[nb][3]));
+        }
+        if (has_n && t4 == 0) {
+          nq[slice * LC_C + m * 16 + g8] = a_lo * (nh[0] + nl[0]);
+          nq[slice * LC_C + m * 16 + g8 + 8] = a_hi * (nh[2] + nl[2]);
+        }
+      }
+    } else {
+      if (warp == LC_GATE_WARP && c + 1 < nchunks) work_gates(c + 1);
+      // W = q k^T of 16 tokens x 32 tokens, decayed, and its product with v
+      const int mt = (warp - 8) >> 1, j0 = (warp & 1) * 32;
+      float hi[VT / 8][4] = {}, lo[VT / 8][4] = {};
+      float rs[2] = {0.f, 0.f};
+      if (j0 <= mt * 16 + 15) {
+        float w[4][4] = {};
+#pragma unroll
+        for (int k4 = 0; k4 < DKP; k4 += 64) {       // runs of four products, added up in float32
+          float part[4][4] = {};
+#pragma unroll
+          for (int kk = k4; kk < k4 + 64; kk += 16) {
+            uint32_t af[4], bq[4];
+            lc_ldsm4(af, qs + (mt * 16 + (mi & 1) * 8 + r8) * LDQ + kk + (mi >> 1) * 8);
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+              lc_ldsm4(bq, ks + (j0 + pr * 16 + (mi >> 1) * 8 + r8) * LDQ + kk + (mi & 1) * 8);
+              lc_mma(part[2 * pr], af, bq[0], bq[1]);
+              lc_mma(part[2 * pr + 1], af, bq[2], bq[3]);
+            }
+          }
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) w[nt][x] += part[nt][x];
+        }
+        const float2 Gt[2] = {gt.G[mt * 16 + g8], gt.G[mt * 16 + g8 + 8]};
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj) {
+            const int j = j0 + nt * 8 + 2 * t4 + jj;
+            const float2 Hj = gt.H[j];
+            const float bj = KIND == SCAN_DECAY ? gt.b[j] : 1.f;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const float f = j <= mt * 16 + g8 + r * 8 ? w[nt][2 * r + jj] * (lc_exp_sum(Gt[r], Hj) * bj) : 0.f;
+              w[nt][2 * r + jj] = f;
+              rs[r] += f;
+            }
+          }
+        }
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          uint32_t t0[3], t1[3], t2[3], t3[3];
+          lc_split3(w[2 * kk][0], w[2 * kk][1], t0);
+          lc_split3(w[2 * kk][2], w[2 * kk][3], t1);
+          lc_split3(w[2 * kk + 1][0], w[2 * kk + 1][1], t2);
+          lc_split3(w[2 * kk + 1][2], w[2 * kk + 1][3], t3);
+#pragma unroll
+          for (int nb = 0; nb < VT / 16; ++nb) {
+            uint32_t bv[4];
+            lc_ldsm4t(bv, vc + (j0 + kk * 16 + (mi & 1) * 8 + r8) * LDV + nb * 16 + (mi >> 1) * 8);
+#pragma unroll
+            for (int x = 2; x >= 0; --x) {
+              const uint32_t af[4] = {t0[x], t1[x], t2[x], t3[x]};
+              lc_mma(x ? lo[2 * nb] : hi[2 * nb], af, bv[0], bv[1]);
+              lc_mma(x ? lo[2 * nb + 1] : hi[2 * nb + 1], af, bv[2], bv[3]);
+            }
+          }
+        }
+      }
+      if (KIND == SCAN_GATED_MAX) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 1);
+          rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 2);
+          if (t4 == 0) rowsum[(mt * 16 + g8 + x * 8) * 2 + (warp & 1)] = rs[x];
+        }
+      }
+#pragma unroll
+      for (int nb = 0; nb < VT / 8; ++nb) {
+        float* d = red + ((size_t)(SLICES + (warp & 1)) * LC_C + mt * 16 + g8) * LDR + nb * 8 + 2 * t4;
+        *(float2*)d = make_float2(hi[nb][0] + lo[nb][0], hi[nb][1] + lo[nb][1]);
+        *(float2*)(d + 8 * LDR) = make_float2(hi[nb][2] + lo[nb][2], hi[nb][3] + lo[nb][3]);
+      }
+    }
+    __syncthreads();                                 // the terms of c v and all sums are in place
+    if (warp < 8) {
+      float up[2 * NK][4] = {}, lo[2 * NK][4] = {}, nu[2 * NK][4] = {};
+#pragma unroll
+      for (int kk = 0; kk < LC_C; kk += 16) {
+        uint32_t af[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) lc_ldsm4t(af[x], vs + (x * LC_C + kk + (mi >> 1) * 8 + r8) * LDV + half + (mi & 1) * 8);
+#pragma unroll
+        for (int nb = 0; nb < NK; ++nb) {
+          uint32_t bk[4];
+          lc_ldsm4t(bk, ks + (kk + (mi & 1) * 8 + r8) * LDQ + k0 + nb * 16 + (mi >> 1) * 8);
+#pragma unroll
+          for (int x = 2; x >= 0; --x) {
+            lc_mma(x ? lo[2 * nb] : up[2 * nb], af[x], bk[0], bk[1]);
+            lc_mma(x ? lo[2 * nb + 1] : up[2 * nb + 1], af[x], bk[2], bk[3]);
+          }
+          if (has_n) {
+#pragma unroll
+            for (int x = 2; x >= 0; --x) {           // row 0: c
+              const uint32_t ca[4] = {g8 == 0 ? *(const uint32_t*)(gt.ct[x] + kk + 2 * t4) : 0u, 0u,
+                                      g8 == 0 ? *(const uint32_t*)(gt.ct[x] + kk + 8 + 2 * t4) : 0u, 0u};
+              lc_mma(nu[2 * nb], ca, bk[0], bk[1]);
+              lc_mma(nu[2 * nb + 1], ca, bk[2], bk[3]);
+            }
+          }
+        }
+      }
+      const float ae = gt.A_end;
+#pragma unroll
+      for (int nt = 0; nt < 2 * NK; ++nt)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          sT[nt][x] = fmaf(ae, sT[nt][x], up[nt][x] + lo[nt][x]);
+          if (has_n) nT[nt][x] = fmaf(ae, nT[nt][x], nu[nt][x]);
+        }
+    } else {
+      for (int i = tid - 256; i < LC_C * VT / 4; i += 256) {
+        const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
+        if (c * LC_C + t >= len || tile * VT + cc >= dv) continue;
+        float4 y = *(const float4*)(red + (size_t)t * LDR + cc);
+#pragma unroll
+        for (int sl = 1; sl < SLICES + 2; ++sl) {
+          const float4 z = *(const float4*)(red + ((size_t)sl * LC_C + t) * LDR + cc);
+          y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
+        }
+        y.x *= a.q_scale; y.y *= a.q_scale; y.z *= a.q_scale; y.w *= a.q_scale;
+        if (KIND == SCAN_GATED_MAX) {
+          float dot = rowsum[2 * t] + rowsum[2 * t + 1];
+#pragma unroll
+          for (int sl = 0; sl < SLICES; ++sl) dot += nq[sl * LC_C + t];
+          dot *= a.q_scale;
+          const float den = fmaxf(fabsf(dot), gt.em[t]) + 1e-6f;
+          y.x /= den; y.y /= den; y.z /= den; y.w /= den;
+        } else {
+          const bf16* vr = vc + t * LDV + cc;
+          y.x = fmaf(b3, to_f(vr[0]), y.x); y.y = fmaf(b3, to_f(vr[1]), y.y); y.z = fmaf(b3, to_f(vr[2]), y.z); y.w = fmaf(b3, to_f(vr[3]), y.w);
+        }
+        *(float4*)(a.out + (size_t)(q0 + c * LC_C + t) * a.ld_out + (size_t)h * dv + tile * VT + cc) = y;
+      }
+    }
+    // the logarithms of the batch that begins with chunk c + 2 (the present one's last gates were worked out ahead of the barrier)
+    if ((c + 2) % (LC_BATCH / LC_C) == 0) work_logs((c + 2) * LC_C);
+  }
+  if (warp < 8) {
+#pragma unroll
+    for (int nt = 0; nt < 2 * NK; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = half + g8 + (i >> 1) * 8;
+        if (k < dk) st[k * VT + col] = sT[nt][i];
+        if (has_n && g8 == 0 && i < 2 && k < dk) st[dk * VT + k] = nT[nt][i];
+      }
+  }
+  if (KIND == SCAN_GATED_MAX && tid == 0) st[dk * VT + dk] = gates[(nchunks - 1) & 1].m_end;
+}
+
+template <int KIND, int VT, int NK>
+static int launch_scan_chunk(const ScanArgs& a, dim3 grid, cudaStream_t st) {
+  auto kernel = linear_scan_chunk_kernel<KIND, VT, NK>;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LcShape<VT, NK>::BYTES);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return qv_launch(kernel, grid, dim3(LC_THREADS), (size_t)LcShape<VT, NK>::BYTES, st, a);
+}
+
 extern "C" long long qv_linear_scan_state_floats(int kind, int H, int dk, int dv) {
   const int vt = scan_vt(dk);
   return (long long)H * ((dv + vt - 1) / vt) * scan_tile_floats(kind, dk, vt);
 }
 
+// max_q_len, min_q_len: the longest and the shortest segment (0: not known; a shortest segment that is not known costs a launch).
+#define SCAN_CHUNK_FROM 16
 extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, int ld_q, int q_group, const void* k, int ld_k,
                               const void* v, int ld_v, const float* g1, int ld_g1, const float* g2, int ld_g2, const float* p1,
                               const float* p2, const float* p3, float cap, float q_scale, float* state, long long slot_stride,
-                              const int* seg_q_start, const int* seg_slot, int S, int H, int dk, int dv, int dt, void* stream) {
+                              const int* seg_q_start, const int* seg_slot, int S, int max_q_len, int min_q_len, int H, int dk, int dv, int dt,
+                              void* stream) {
   if (S <= 0) return 0;
   if (kind != SCAN_GATED_MAX && kind != SCAN_DECAY) return QV_ERR_UNSUPPORTED;
   if (H <= 0 || dk <= 0 || dv <= 0 || q_group <= 0 || H > 65535) return QV_ERR_UNSUPPORTED;
@@ -447,8 +924,23 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
   a.out = out; a.ld_out = ld_out; a.q = q; a.ld_q = ld_q; a.q_group = q_group; a.k = k; a.ld_k = ld_k; a.v = v; a.ld_v = ld_v;
   a.g1 = g1; a.ld_g1 = ld_g1; a.g2 = g2; a.ld_g2 = ld_g2; a.p1 = p1; a.p2 = p2; a.p3 = p3; a.cap = cap; a.q_scale = q_scale;
   a.state = state; a.slot_stride = slot_stride; a.seg_q_start = seg_q_start; a.seg_slot = seg_slot; a.H = H; a.dk = dk; a.dv = dv;
+  a.chunk_from = 0x7fffffff;
   dim3 grid(S, H, tiles);
   cudaStream_t st = (cudaStream_t)stream;
+  // Portions of SCAN_CHUNK_FROM tokens and more take the tensor cores, the step's other segments the token-by-token kernel: which kernel a
+  // segment runs through depends on its own length alone.  bfloat16 only (the 32-bit path keeps one order of sums for every cut).
+  if (dt == QV_DT_BF16 && max_q_len >= SCAN_CHUNK_FROM && dk <= 256 && dk % 8 == 0 && dv % 8 == 0 && ld_q % 8 == 0 && ld_k % 8 == 0 &&
+      ld_v % 8 == 0 && ld_out % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0) {
+    a.chunk_from = SCAN_CHUNK_FROM;
+    int rc;
+    if (kind == SCAN_GATED_MAX)
+      rc = vt == 16 ? launch_scan_chunk<SCAN_GATED_MAX, 16, 2>(a, grid, st)
+                    : dk <= 64 ? launch_scan_chunk<SCAN_GATED_MAX, 32, 1>(a, grid, st) : launch_scan_chunk<SCAN_GATED_MAX, 32, 2>(a, grid, st);
+    else
+      rc = vt == 16 ? launch_scan_chunk<SCAN_DECAY, 16, 2>(a, grid, st)
+                    : dk <= 64 ? launch_scan_chunk<SCAN_DECAY, 32, 1>(a, grid, st) : launch_scan_chunk<SCAN_DECAY, 32, 2>(a, grid, st);
+    if (rc || min_q_len >= SCAN_CHUNK_FROM) return rc;
+  }
   if (dk <= 8 * 32) {                      // the state fits the registers
     const size_t esz = dt == QV_DT_F32 ? 4 : 2;
     const size_t rowpad = (size_t)((dk + 7) & ~7);

@@ -1,0 +1,92 @@
+"""The recurrences over portions (chunks of 64 tokens on the tensor cores) against float64 token by token, at the edges of chunks and of the
+kernel's sizes, beside short segments that the token-by-token kernel takes; and no further off than that kernel is."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from qorvix_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+def context(lens, chunked=True):
+    S = len(lens)
+    qs = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+    return SimpleNamespace(num_segments=S, num_tokens=sum(lens), max_q_len=max(lens) if chunked else 1, seg_len=list(lens), seg_q_start=qs,
+                           seg_slot=torch.arange(S, dtype=torch.int32, device="cuda").flip(0).contiguous())
+
+
+def plain(kind, q, k, v, g1, g2, p1, p2, p3, cap, scale, S, n, m):
+    """One head in float64: q, k [T, dk], v [T, dv], state S [dk, dv], n [dk], m."""
+    ys = []
+    for t in range(q.shape[0]):
+        if kind == ops.SCAN_GATED_MAX:
+            li = cap * torch.tanh((g1[t] + p1) / cap)
+            lf = torch.nn.functional.logsigmoid(cap * torch.tanh((g2[t] + p2) / cap))
+            new = torch.maximum(lf + m, li)
+            a, b, m = torch.exp(lf + m - new), torch.exp(li - new), new
+        else:
+            dt = torch.nn.functional.softplus(g1[t] + p1)
+            a, b = torch.exp(-torch.exp(p2) * dt), dt
+        S = a * S + b * torch.outer(k[t], v[t])
+        n = a * n + b * k[t]
+        y = scale * (q[t] @ S)
+        if kind == ops.SCAN_GATED_MAX:
+            y = y / (torch.maximum((scale * (n @ q[t])).abs(), torch.exp(-m)) + 1e-6)
+        else:
+            y = y + p3 * v[t]
+        ys.append(y)
+    return torch.stack(ys), S, n, m
+
+
+@pytest.mark.parametrize("kind", [ops.SCAN_GATED_MAX, ops.SCAN_DECAY])
+@pytest.mark.parametrize("dk,dv,H,qg,lens,shift", [(8, 8, 2, 1, [16, 1, 65], 0.0), (64, 40, 3, 1, [63, 15, 64], 2.0), (72, 24, 2, 2, [130, 2, 17], -3.0),
+                                                   (128, 64, 2, 1, [200, 128], 4.0), (136, 48, 1, 1, [127, 16], 0.0), (256, 16, 2, 1, [129, 1, 33], 3.0)])
+def test_chunks_against_float64(kind, dk, dv, H, qg, lens, shift):
+    g = torch.Generator(device="cuda").manual_seed(dk + dv)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, cap, scale = sum(lens), 6.0, dk ** -0.5
+    width = (H // qg) * dk
+    both = rnd(T, 2 * width).to(torch.bfloat16)                # q and k as columns of one product
+    q, k, v = both[:, :width], both[:, width:], rnd(T, H * dv).to(torch.bfloat16)
+    g1, g2 = rnd(T, H) * 2 - (2.0 if kind == ops.SCAN_DECAY else 0.0), rnd(T, H) * 2 + shift
+    p1, p2, p3 = rnd(H), rnd(H), rnd(H)
+    floats = ops.linear_scan_state_floats(kind, H, dk, dv)
+    start = torch.zeros(len(lens), floats, device="cuda")
+    gated = kind == ops.SCAN_GATED_MAX
+    args = lambda out, state, ctx: ops.linear_scan(kind, out, q, k, v, g1, g2 if gated else None, p1, p2 if True else None, None if gated else p3, cap,
+                                                   scale, state, ctx, H, dk, dv, q_group=qg)
+    # a state that earlier tokens left: the same tokens once, token by token
+    args(torch.empty(T, H * dv, device="cuda"), start, context(lens, chunked=False))
+    outs, states = [], []
+    for chunked in (True, False):
+        state, out = start.clone(), torch.full((T, H * dv), float("nan"), device="cuda")
+        args(out, state, context(lens, chunked))
+        outs.append(out.double())
+        states.append(state)
+    vt = 16 if 128 < dk <= 256 else 32
+    tiles = -(-dv // vt)
+    def state_of(state, s, h):
+        per = dk * vt + (dk + 1 if gated else 0)
+        block = state[s].view(H, tiles, per)[h].double()
+        S = block[:, : dk * vt].reshape(tiles, dk, vt).permute(1, 0, 2).reshape(dk, tiles * vt)[:, :dv]
+        return S, block[0, dk * vt: dk * vt + dk] if gated else torch.zeros(dk, dtype=F64, device="cuda"), block[0, -1] if gated else None
+    errors = torch.zeros(2, 2, dtype=F64)
+    norms = torch.zeros(2, dtype=F64)
+    at = 0
+    for s, n_tok in enumerate(lens):
+        slot = len(lens) - 1 - s
+        for h in range(H):
+            rows, kh = slice(at, at + n_tok), slice((h // qg) * dk, (h // qg) * dk + dk)
+            S0, n0, m0 = state_of(start, slot, h)
+            y, S1, _, _ = plain(kind, q[rows, kh].double(), k[rows, kh].double(), v[rows, h * dv:(h + 1) * dv].double(), g1[rows, h].double(),
+                                g2[rows, h].double(), p1[h].double(), p2[h].double(), p3[h].double(), cap, scale, S0, n0, m0)
+            norms += torch.stack([(y ** 2).sum(), (S1 ** 2).sum()]).cpu()
+            for i in range(2):
+                errors[i] += torch.stack([((outs[i][rows, h * dv:(h + 1) * dv] - y) ** 2).sum(), ((state_of(states[i], slot, h)[0] - S1) ** 2).sum()]).cpu()
+        at += n_tok
+    rel = (errors / norms).sqrt()
+    # a float32 sum of some 64 to 256 products that cancel: a few 1e-7; the chunks may not be further off than token by token
+    assert bool((rel[0] <= torch.maximum(1.2 * rel[1], torch.full((2,), 3e-7, dtype=F64))).all()), rel.tolist()
