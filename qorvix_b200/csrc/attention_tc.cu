@@ -64,6 +64,12 @@ struct AttnArgs {
   int segments, q_pairs, items;                      // items = H x segments x q_pairs (some of them empty)
   int paired;                                        // 1: an item is two query tiles; 0: one (q_pairs then counts tiles)
   float scale_log2;
+  // keys and values as rows of one matrix instead of pages (ROPE > 0): a segment's first row there, the key it is (a multiple of
+  // KT), the first column of the values, and a gate whose sigmoid multiplies the output (or null)
+  const int* row_off = nullptr;
+  const int* row_key = nullptr;
+  const bf16* gate = nullptr;
+  int ld_gate = 0, v_col = 0, min_len = 0;           // segments of fewer than min_len tokens are left out
 };
 
 // bar.sync over the `count` threads that name barrier `id`
@@ -75,6 +81,7 @@ struct Item {
   const int* bt;                                     // the segment's row of the block table
   int h, kvh, q0, qlen, tile0, pos0;                 // tile0: first row of tile A in its segment (B: tile0 + 128)
   int k_last, tile_begin;                            // the last key any row of the item sees; its first key tile
+  int row0;                                          // (ROPE > 0) the row of key 0
   int n_a, n_b;                                      // key tiles of A and of B (0: no B; else n_a or n_a + 1)
 };
 
@@ -89,10 +96,11 @@ __device__ __forceinline__ bool item_at(const AttnArgs& a, int idx, Item& t) {
   t.q0 = a.seg_q_start[seg];
   t.qlen = a.seg_q_start[seg + 1] - t.q0;
   t.tile0 = (a.q_pairs - 1 - y) * (PAIRED ? 2 * QT : QT);
-  if (t.tile0 >= t.qlen) return false;
+  if (t.tile0 >= t.qlen || t.qlen < a.min_len) return false;
   t.pos0 = a.seg_pos0[seg];
   t.kvh = t.h / (a.H / a.Hkv);
   t.bt = a.block_table + (size_t)seg * a.max_blocks;
+  t.row0 = a.row_off ? a.row_off[seg] - a.row_key[seg] : 0;
   const int rows = t.qlen - t.tile0;                 // of both tiles
   const int last_a = t.pos0 + t.tile0 + (rows < QT ? rows : QT) - 1;
   int k_first = 0;
@@ -126,21 +134,26 @@ struct Walk {
   }
 };
 
-template <int HD, bool PAIRED>
+// ROPE > 0: queries and keys have ROPE further entries (the queries' behind each head's, the keys' one row for all heads, map_kr);
+// keys and values are rows of a matrix (map_kv, boxes of KT rows), each segment's padded with rows of zeros to whole tiles.
+template <int HD, bool PAIRED, int ROPE>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                                       const __grid_constant__ CUtensorMap map_kv, const AttnArgs a) {
+                                                                       const __grid_constant__ CUtensorMap map_kv,
+                                                                       const __grid_constant__ CUtensorMap map_kr, const AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int NH = HD / 64;                        // 64-element halves of the head
-  constexpr int Q_BYTES = QT * HD * 2;               // [NH][128 rows][64]
-  constexpr int K_BYTES = KT * HD * 2;               // [NH][128 keys][64]
+  constexpr int NHK = (HD + ROPE) / 64;              // and of a query or key
+  constexpr int Q_BYTES = QT * (HD + ROPE) * 2;      // [NHK][128 rows][64]
+  constexpr int K_BYTES = KT * (HD + ROPE) * 2;      // [NHK][128 keys][64]
+  constexpr int V_BYTES = KT * HD * 2;               // [NH][128 keys][64]
   constexpr int HALF_BYTES = 128 * 128;              // one [128][64] bf16 tile
   static_assert(2 * KT + 2 * HD <= 512, "S and O of both query tiles must fit tensor memory");
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = base;                                // tiles A and B
-  constexpr int K_ST = PAIRED ? K_ST_PAIRS : K_ST_SINGLE;
+  constexpr int K_ST = PAIRED || ROPE ? K_ST_PAIRS : K_ST_SINGLE;
   uint8_t* sK = sQ + (PAIRED ? 2 : 1) * Q_BYTES;     // K_ST stages
   uint8_t* sV = sK + K_ST * K_BYTES;                 // V_ST stages
-  uint64_t* bars = (uint64_t*)(sV + V_ST * K_BYTES);
+  uint64_t* bars = (uint64_t*)(sV + V_ST * V_BYTES);
   uint64_t* q_full = bars;                           // [2]: one per query tile, like the next four
   uint64_t* q_empty = bars + 2;
   uint64_t* s_full = bars + 4;
@@ -202,7 +215,28 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
     int s = 0;                                       // the ring's stage, and how often it has been round
     uint32_t lap = 0;
     bool alive = true;
-    while (alive && walk.next(a, t)) {
+    constexpr int ROWS_BYTES[2] = {K_BYTES, V_BYTES};
+    while (ROPE > 0 && alive && walk.next(a, t)) {
+      for (int j = 0; j < t.n_a; ++j) {
+        alive = mbar_wait(&empty[s], (lap & 1) ^ 1, a.err, 11);
+        if (!alive) break;
+        const int row = t.row0 + (t.tile_begin + j) * KT;
+        if (leader) {
+          mbar_expect_tx(&full[s], ROWS_BYTES[which]);
+          uint8_t* dst = ring + s * ROWS_BYTES[which];
+          const int col = (which ? a.v_col : 0) + t.h * HD;
+#pragma unroll
+          for (int hf = 0; hf < NH; ++hf) tma_load_2d(dst + hf * HALF_BYTES, &map_kv, &full[s], col + hf * 64, row);
+          if (which == 0) {
+#pragma unroll
+            for (int hf = NH; hf < NHK; ++hf) tma_load_2d(dst + hf * HALF_BYTES, &map_kr, &full[s], (hf - NH) * 64, row);
+          }
+        }
+        __syncwarp();
+        if (++s == stages) { s = 0; ++lap; }
+      }
+    }
+    while (ROPE == 0 && alive && walk.next(a, t)) {
       const int last_block = t.k_last & ~15;
       const int n = t.n_b > t.n_a ? t.n_b : t.n_a;
       for (int j = 0; j < n; ++j) {
@@ -239,8 +273,8 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           if (!alive) break;
           if (leader) {
             mbar_expect_tx(&q_full[x], Q_BYTES);
-            for (int f = 0; f < NH; ++f)
-              tma_load_2d(sQ + x * Q_BYTES + f * HALF_BYTES, &map_q, &q_full[x], t.h * HD + f * 64, t.q0 + t.tile0 + x * QT);
+            for (int f = 0; f < NHK; ++f)
+              tma_load_2d(sQ + x * Q_BYTES + f * HALF_BYTES, &map_q, &q_full[x], t.h * (HD + ROPE) + f * 64, t.q0 + t.tile0 + x * QT);
           }
           __syncwarp();
           ++loads[x];
@@ -268,7 +302,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         const uint32_t d = tmem + (uint32_t)(x * KT);
         if (leader) {
 #pragma unroll
-        for (int hf = 0; hf < NH; ++hf) {
+        for (int hf = 0; hf < NHK; ++hf) {
           const uint64_t dq = umma_desc(smem_u32(sQ + qx * Q_BYTES + hf * HALF_BYTES));
           const uint64_t dk = umma_desc(smem_u32(sK + ks * K_BYTES + hf * HALF_BYTES));
 #pragma unroll
@@ -293,7 +327,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         if (leader) {
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk) {
-          const uint32_t v_addr = smem_u32(sV + vs * K_BYTES + (kk * 16) * 128);
+          const uint32_t v_addr = smem_u32(sV + vs * V_BYTES + (kk * 16) * 128);
           const uint32_t p_col = (uint32_t)(((kk * 16) / 64) * 64 + ((kk * 16) % 64) / 2);
           umma_f16_ts(o, p + p_col, umma_desc_mn(v_addr, HALF_BYTES), idesc_pv, (kk > 0 || j > 0) ? 1u : 0u);
         }
@@ -492,11 +526,22 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         const bool store = ok && row_in_seg < t.qlen;
         const float inv = store ? 1.f / l : 0.f;
         bf16* orow = a.out + (size_t)(t.q0 + (store ? row_in_seg : 0)) * a.ld_out + (size_t)t.h * HD + wg * OPT;
+        const bf16* grow = ROPE > 0 && a.gate ? a.gate + (size_t)(t.q0 + (store ? row_in_seg : 0)) * a.ld_gate + (size_t)t.h * HD + wg * OPT : nullptr;
 #pragma unroll 1
         for (int c = 0; c < OPT; c += 32) {
           uint32_t v[32];
           tmem_ld32(o_addr + c, v);
           tmem_wait_ld();
+          if (ROPE > 0 && grow && store) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              const uint4 gv = *(const uint4*)(grow + c + i);
+              const bf16* ge = (const bf16*)&gv;
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                v[i + u] = __float_as_uint(__uint_as_float(v[i + u]) * (1.0f / (1.0f + expf(-to_f(ge[u])))));
+            }
+          }
           if (store) {
 #pragma unroll
             for (int i = 0; i < 32; i += 8)
@@ -527,14 +572,16 @@ int device_sms() {
   return sms;
 }
 
-template <int HD, bool PAIRED>
-int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const AttnArgs& args, cudaStream_t st) {
+template <int HD, bool PAIRED, int ROPE = 0>
+int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mkr, const AttnArgs& args, cudaStream_t st) {
   // two Q tiles, the rings of keys and values, 256 bytes of barriers, 2 KB for what a row's threads exchange, 1 KB to align
-  constexpr int smem = 2 * QT * HD * 2 + (K_ST_PAIRS + V_ST) * KT * HD * 2 + 256 + 2048 + 1024;
+  constexpr int smem = ROPE ? (QT + K_ST_PAIRS * KT) * (HD + ROPE) * 2 + V_ST * KT * HD * 2 + 256 + 2048 + 1024
+                            : 2 * QT * HD * 2 + (K_ST_PAIRS + V_ST) * KT * HD * 2 + 256 + 2048 + 1024;
   static_assert(QT * HD * 2 + (K_ST_SINGLE + V_ST) * KT * HD * 2 <= 2 * QT * HD * 2 + (K_ST_PAIRS + V_ST) * KT * HD * 2, "one layout's room serves both");
   static_assert(smem <= 227 * 1024, "more shared memory than a CTA can have");
   static bool configured = false;
-  auto kernel = attn_prefill_tc_kernel<HD, PAIRED>;
+  static_assert(!ROPE || !PAIRED, "two query tiles with their further entries do not fit");
+  auto kernel = attn_prefill_tc_kernel<HD, PAIRED, ROPE>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
@@ -542,7 +589,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const AttnArgs& args, 
   }
   // one CTA per SM, or one per item when there are fewer
   const int ctas = args.items < device_sms() ? args.items : device_sms();
-  return qv_launch(kernel, dim3(ctas), dim3(ATTN_THREADS), (size_t)smem, st, mq, mkv, args);
+  return qv_launch(kernel, dim3(ctas), dim3(ATTN_THREADS), (size_t)smem, st, mq, mkv, mkr, args);
 }
 
 }  // namespace
@@ -583,6 +630,34 @@ extern "C" int qv_attn_prefill_tc(void* out, int ld_out, const void* q, int ld_q
   a.ld_out = ld_out; a.max_blocks = max_blocks; a.H = H; a.Hkv = Hkv; a.page = page; a.window = window;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.segments = S; a.q_pairs = (int)q_pairs; a.items = (int)(H * S * q_pairs); a.paired = paired;
-  if (hd == 128) return paired ? launch<128, true>(mq, mkv, a, (cudaStream_t)stream) : launch<128, false>(mq, mkv, a, (cudaStream_t)stream);
-  return paired ? launch<64, true>(mq, mkv, a, (cudaStream_t)stream) : launch<64, false>(mq, mkv, a, (cudaStream_t)stream);
+  if (hd == 128) return paired ? launch<128, true>(mq, mkv, mkv, a, (cudaStream_t)stream) : launch<128, false>(mq, mkv, mkv, a, (cudaStream_t)stream);
+  return paired ? launch<64, true>(mq, mkv, mkv, a, (cudaStream_t)stream) : launch<64, false>(mq, mkv, mkv, a, (cudaStream_t)stream);
+}
+
+// Prompt portions whose keys and values lie as rows of one matrix `kv` [rows][ld_kv]: the H heads' keys of 128 entries from column 0,
+// their values of 128 from column v_col, and a rotated key part of 64 that all heads share in `kr` [rows][64]; queries of 192 a head (the
+// rotated part behind).  Segment s has keys row_key[s] .. in rows row_off[s] .., padded with zeros to a multiple of 128 rows (row_key a
+// multiple of 128 too).  Segments of fewer than min_len tokens are left out.  gate [T][ld_gate]: its sigmoid multiplies the output.
+// One query tile an item (two with their rotated parts do not fit shared memory).  Bounded like the paged kernel, by a tile's chain of
+// softmax and products.
+extern "C" int qv_attn_rows_tc(void* out, int ld_out, const void* q, int ld_q, int T, const void* kv, long long ld_kv, int v_col, const void* kr,
+                               long long rows, const int* row_off, const int* row_key, const void* gate, int ld_gate,
+                               const int* seg_q_start, const int* seg_pos0, int S, int max_q_len, int min_len, int H, int window, float scale,
+                               int* err, void* stream) {
+  if (S <= 0 || max_q_len <= 0 || rows <= 0) return 0;
+  if (H <= 0 || (ld_q & 7) || (ld_out & 7) || (ld_kv & 7) || (v_col & 7) || (gate && ((ld_gate & 7) || ((uintptr_t)gate & 15))) ||
+      (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)kr) & 15) || rows > 0x7fffffffLL || v_col + H * 128 > ld_kv)
+    return QV_ERR_UNSUPPORTED;
+  const long long q_tiles = (max_q_len + QT - 1) / QT;
+  if ((long long)H * S * q_tiles > (1LL << 30)) return QV_ERR_TOO_LARGE;
+  CUtensorMap mq, mkv, mkr;
+  if (!make_map(&mq, q, T, H * 192, ld_q, QT) || !make_map(&mkv, kv, rows, v_col + H * 128, ld_kv, KT) || !make_map(&mkr, kr, rows, 64, 64, KT))
+    return QV_ERR_UNSUPPORTED;
+  AttnArgs a;
+  a.out = (bf16*)out; a.seg_q_start = seg_q_start; a.seg_pos0 = seg_pos0; a.block_table = nullptr; a.err = err;
+  a.ld_out = ld_out; a.max_blocks = 0; a.H = H; a.Hkv = H; a.page = KT; a.window = window;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.segments = S; a.q_pairs = (int)q_tiles; a.items = (int)(H * S * q_tiles); a.paired = 0;
+  a.row_off = row_off; a.row_key = row_key; a.gate = (const bf16*)gate; a.ld_gate = ld_gate; a.v_col = v_col; a.min_len = min_len;
+  return launch<128, false, 64>(mq, mkv, mkr, a, (cudaStream_t)stream);
 }

@@ -712,3 +712,44 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
   return qv_launch(heads_gemm_kernel<false>, dim3((dv + 63) / 64, (T + 63) / 64, H), dim3(128), 0, st, (bf16*)out, ld_out, dv,
                    (const bf16*)lat, H * rank, rank, (const bf16*)wuv, (const bf16*)nullptr, 0, 0, T, dv, rank, 0);
 }
+
+// ---------------------------------------------------------------- portions: the latents as rows, for keys and values formed per head
+// Copies the cached rows that the segments of at least min_len tokens see into c [rows][rank] and kr [rows][dr], a warp a row: segment s
+// from key row_key[s] (the window's first key, rounded down to a multiple of 128; 0 without a window) in rows row_off[s] .., padded with
+// rows of zeros to a multiple of 128.  The first block also writes row_off and row_key [S].
+__device__ __forceinline__ int lt_first_key(int pos0, int window) { return window > 0 && pos0 + 1 > window ? (pos0 + 1 - window) & ~127 : 0; }
+__global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict__ c, uint4* __restrict__ kr, int* __restrict__ row_off,
+                                                              int* __restrict__ row_key, const uint4* __restrict__ cache, int rank16, int dr16,
+                                                              const int* __restrict__ seg_q_start, const int* __restrict__ seg_pos0,
+                                                              const int* __restrict__ block_table, int max_blocks, int S, int min_len, int page,
+                                                              int window, int rows) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
+    int off = 0, key = -1, seg = 0;                 // key -1: a row of zeros
+    for (int s = 0; s < S; ++s) {
+      const int len = seg_q_start[s + 1] - seg_q_start[s], pos0 = seg_pos0[s], first = lt_first_key(pos0, window);
+      const int n = len >= min_len ? pos0 + len - first : 0, padded = (n + 127) & ~127;
+      if (r >= off && r < off + padded) { seg = s; key = r - off < n ? first + r - off : -1; }
+      if (r == 0 && lane == 0) { row_off[s] = off; row_key[s] = first; }
+      off += padded;
+    }
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const uint4* src = nullptr;
+    if (key >= 0) src = cache + ((size_t)block_table[(size_t)seg * max_blocks + key / page] * page + key % page) * (rank16 + dr16);
+    for (int i = lane; i < rank16; i += 32) c[(size_t)r * rank16 + i] = src ? src[i] : zero;
+    for (int i = lane; i < dr16; i += 32) kr[(size_t)r * dr16 + i] = src ? src[rank16 + i] : zero;
+  }
+}
+
+extern "C" int qv_latent_rows_out(void* c, void* kr, int* row_off, int* row_key, const void* cache, int rank, int dr, const int* seg_q_start,
+                                  const int* seg_pos0, const int* block_table, int max_blocks, int S, int min_len, int page, int window, int rows,
+                                  void* stream) {
+  if (S <= 0 || rows <= 0) return 0;
+  if (rank % 8 || dr % 8 || (((uintptr_t)c | (uintptr_t)kr | (uintptr_t)cache) & 15)) return QV_ERR_UNSUPPORTED;
+  const int blocks = (rows + 7) / 8;
+  return qv_launch(latent_rows_out_kernel, dim3(blocks < 148 * 8 ? blocks : 148 * 8), dim3(256), 0, (cudaStream_t)stream, (uint4*)c, (uint4*)kr,
+                   row_off, row_key, (const uint4*)cache, rank / 8, dr / 8, seg_q_start, seg_pos0, block_table, max_blocks, S, min_len, page, window,
+                   rows);
+}

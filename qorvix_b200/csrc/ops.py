@@ -63,6 +63,8 @@ _ARGTYPES = {
     "qv_latent_attention_generic": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V, _V],
     "qv_latent_tc_workspace_bytes": [_I, _I, _I, _I, _I],
     "qv_latent_attention_tc": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _V, _V, _I, _V],
+    "qv_latent_rows_out": [_V, _V, _V, _V, _V, _I, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V],
+    "qv_attn_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _I, _V, _L, _V, _V, _V, _I, _V, _V, _I, _I, _I, _I, _I, _F, _V, _V],
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
     "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V],
@@ -685,14 +687,81 @@ def latent_attention_tc(out, q, gate, cache_layer, wuk_t, wuv, ctx, block_table,
     return True
 
 
+LATENT_EXPAND_FROM = 32                    # segments of at least this many tokens form keys and values per head
+LATENT_EXPAND_BYTES = 1 << 30              # the most that their rows may take
+
+
+def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale) -> int:
+    """Latent attention of the step's portions with every head's keys and values formed once (kv_up: packed tiles and number of rows of
+    [all heads' key matrices; all heads' value matrices], applied to the rows that the portions see) and flash attention on the tensor
+    cores over them.  A query then multiplies dn + dr + dv entries a key instead of 2 rank + dr; it pays for portions of
+    LATENT_EXPAND_FROM tokens and more.  Takes the segments from the first such one on; returns how many leading segments it left out (all
+    of them: nothing was done, where a size, a type or the room for the rows does not allow it)."""
+    S = ctx.num_segments
+    lens, pos0 = getattr(ctx, "seg_len", None), getattr(ctx, "seg_start_pos", None)
+    if (kv_up is None or q.dtype != torch.bfloat16 or not lens or not pos0 or getattr(ctx, "captured", False) or dn != 128 or dv != 128 or dr != 64
+            or rank % 8 or q.stride(0) % 8 or out.stride(0) % 8 or cache_layer.dtype != torch.bfloat16
+            or (gate is not None and (gate.dtype != torch.bfloat16 or gate.stride(0) % 8 or gate.data_ptr() % 16))
+            or q.data_ptr() % 16 or out.data_ptr() % 16):
+        return S
+    first = next((i for i, n in enumerate(lens) if n >= LATENT_EXPAND_FROM), S)
+    if first == S:
+        return S
+    rows = 0
+    for n, p in zip(lens[first:], pos0[first:]):
+        lo = (p + 1 - window) & ~127 if window > 0 and p + 1 > window else 0
+        rows += (p + n - lo + 127) & ~127
+    packed, features = kv_up
+    if rows * (rank + dr + features) * 2 > LATENT_EXPAND_BYTES:
+        return S
+    _need_cuda(out, q, gate, cache_layer, block_table)
+    _i32(block_table, "block_table")
+    dev = q.device
+    c = torch.empty((rows, rank), device=dev, dtype=torch.bfloat16)
+    kr = torch.empty((rows, dr), device=dev, dtype=torch.bfloat16)
+    kv = torch.empty((rows, features), device=dev, dtype=torch.bfloat16)
+    where = torch.empty((2, S - first), device=dev, dtype=torch.int32)
+    starts, firsts, tables = ctx.seg_q_start[first:], ctx.seg_pos0[first:], block_table[first:]
+    _check(_lib("latent_attention").qv_latent_rows_out(
+        _ptr(c), _ptr(kr), _ptr(where[0]), _ptr(where[1]), _ptr(cache_layer), rank, dr, _ptr(starts), _ptr(firsts), _ptr(tables),
+        block_table.shape[-1], S - first, 1, page, window, rows, _stream()), "latent_rows_out")
+    gemm(kv, c, None, packed, features)
+    _check(_lib("attention_tc").qv_attn_rows_tc(
+        _ptr(out), out.stride(0), _ptr(q), q.stride(0), q.shape[0], _ptr(kv), kv.stride(0), H * dn, _ptr(kr), rows, _ptr(where[0]), _ptr(where[1]),
+        _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(starts), _ptr(firsts), S - first, max(lens[first:]), 1, H, window, scale,
+        _ptr(_tc_buffers(dev)["err"]), _stream()), "attn_rows_tc")
+    return first
+
+
 def latent_attention(out, q, gate, cache_layer, wuk, wuv, ctx, block_table, H, dn, dr, dv, rank, page, window, scale, wuk_t=None, sink=None,
-                     weight_terms: int = 1) -> None:
-    """Latent attention of every token of the step: the tensor-core kernels for bfloat16 where they take the sizes (and
-    the transposed key matrices wuk_t [H, rank, dn] are given), else (and for float32) the CUDA-core kernel."""
+                     weight_terms: int = 1, kv_up=None) -> None:
+    """Latent attention of every token of the step.  bfloat16: portions form keys and values per head where the sizes allow it and kv_up is
+    given (see latent_attention_expanded; softmax weights of one term, no sinks), other segments take the tensor-core kernels over the
+    latents themselves (with the transposed key matrices wuk_t [H, rank, dn]), else (and for float32) the CUDA-core kernel."""
+    if kv_up is not None and sink is None and weight_terms == 1:
+        left = latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale)
+        if left == 0:
+            return
+        if left < ctx.num_segments:                # the segments ahead of the first portion
+            tokens = sum(ctx.seg_len[:left])
+            ctx = _LeadingSegments(ctx, left, tokens)
+            out, q, gate, block_table = out[:tokens], q[:tokens], gate[:tokens] if gate is not None else None, block_table[:left]
     if q.dtype == torch.bfloat16 and latent_attention_tc(out, q, gate, cache_layer, wuk_t, wuv, ctx, block_table, H, dn, dr, dv, rank,
                                                          page, window, scale, sink=sink, weight_terms=weight_terms):
         return
     latent_attention_generic(out, q, gate, cache_layer, wuk, wuv, ctx, block_table, H, dn, dr, dv, rank, page, window, scale, sink=sink)
+
+
+class _LeadingSegments:
+    """What the latent kernels read of a step's context, for its first `n` segments."""
+
+    def __init__(self, ctx, n: int, tokens: int):
+        self.num_segments, self.num_tokens = n, tokens
+        self.seg_len, self.seg_start_pos = list(ctx.seg_len[:n]), list(ctx.seg_start_pos[:n])
+        self.max_q_len = max(self.seg_len)
+        self.max_ctx_len = max(a + b for a, b in zip(self.seg_len, self.seg_start_pos))
+        self.seg_q_start, self.seg_pos0 = ctx.seg_q_start[: n + 1], ctx.seg_pos0[:n]
+        self.tok_pos, self.tok_seg = ctx.tok_pos[:tokens], ctx.tok_seg[:tokens]
 
 
 # ------------------------------------------------------------------ recurrent mixers

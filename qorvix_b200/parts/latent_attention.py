@@ -45,6 +45,11 @@ class LatentAttention(Mixer):
         # the tensor-core kernels read each head's key matrix with the latent index outermost
         self.k_up_t = (self.k_up.view(self.H, self.dn, self.rank).transpose(1, 2).contiguous()
                        if self.k_up.dtype == torch.bfloat16 else None)
+        # portions form every head's keys and values once: one product of the latents with both matrices
+        self.kv_up = None
+        if rt.dtype == torch.bfloat16 and self.k_up.dtype == torch.bfloat16 and (self.dn, self.dr, self.dv) == (128, 64, 128):
+            up = Linear(torch.cat([self.k_up, self.v_up], dim=0))
+            self.kv_up = (up.packed, up.out_features) if up.packed is not None else None
         self.o_proj = Linear(source.get(spec.o_proj))
         self.position = build_part("position", spec.position, source, rt)
         self.sink = source.get(spec.sink, dtype=torch.float32) if getattr(spec, "sink", None) is not None else None
@@ -77,7 +82,7 @@ class LatentAttention(Mixer):
         gate = proj[:, self.gate_off: self.gate_off + H * dv] if self.gate_off is not None else None
         out = torch.empty((proj.shape[0], H * dv), device=proj.device, dtype=self.rt.dtype)
         ops.latent_attention(out, q, gate, cache.tensor, self.k_up, self.v_up, ctx, bt,
-                             H, dn, dr, dv, rank, cache.page_size, self.window, self.scale, wuk_t=self.k_up_t, sink=self.sink, weight_terms=self.weight_terms)
+                             H, dn, dr, dv, rank, cache.page_size, self.window, self.scale, wuk_t=self.k_up_t, sink=self.sink, weight_terms=self.weight_terms, kv_up=self.kv_up)
         return self.o_proj(out, out_dtype=self.rt.dtype)
 
 

@@ -1,0 +1,75 @@
+"""Latent attention of portions whose keys and values are formed per head, against float64 over the same cache rows: portions that end
+inside, at and behind a tile of 128 queries or keys, far into their requests, behind single tokens and before them, with and without
+window and gate, pages out of order; and which segments take that path."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from qorvix_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+H, DN, DR, DV = 3, 128, 64, 128
+
+
+def context(lens, past):
+    i32 = dict(dtype=torch.int32, device="cuda")
+    return SimpleNamespace(num_segments=len(lens), num_tokens=sum(lens), max_q_len=max(lens), max_ctx_len=max(a + b for a, b in zip(lens, past)),
+                           seg_len=list(lens), seg_start_pos=list(past), captured=False,
+                           seg_q_start=torch.tensor([0] + lens, **i32).cumsum(0).to(torch.int32), seg_pos0=torch.tensor(past, **i32),
+                           tok_pos=torch.cat([torch.arange(p, p + n, **i32) for n, p in zip(lens, past)]),
+                           tok_seg=torch.repeat_interleave(torch.arange(len(lens), **i32), torch.tensor(lens, device="cuda")).to(torch.int32))
+
+
+@pytest.mark.parametrize("lens,past,window,gated,rank", [
+    ([32], [0], 0, True, 64), ([127, 128, 129], [0, 1, 300], 0, False, 128), ([1, 1, 200], [40, 700, 60], 0, True, 64),
+    ([260, 1, 33], [128, 90, 511], 0, True, 64), ([140, 64], [500, 130], 100, False, 64), ([300], [255], 128, True, 512), ([40, 31], [3, 9], 1, True, 64)])
+def test_portions_against_float64(lens, past, window, gated, rank):
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    T, page, S = sum(lens), 16, len(lens)
+    ctx = context(lens, past)
+    blocks = -(-ctx.max_ctx_len // page)
+    table = torch.randperm(S * blocks, generator=g, device="cuda").to(torch.int32).view(S, blocks)
+    cache = rnd(S * blocks + 1, page, rank + DR)
+    proj = rnd(T, H * (DN + DR) + 8)
+    q = proj[:, : H * (DN + DR)]
+    gate = rnd(T, H * DV) if gated else None
+    wuk, wuv = rnd(H * DN, rank).mul_(rank ** -0.5), rnd(H * DV, rank).mul_(rank ** -0.5)
+    up = torch.cat([wuk, wuv])
+    out = torch.full((T, H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
+    scale = (DN + DR) ** -0.5
+    left = ops.latent_attention_expanded(out, q, gate, cache, (ops.pack_weight(up), up.shape[0]), ctx, table, H, DN, DR, DV, rank, page, window, scale)
+    ops.check_kernel_errors()
+    assert left == next(i for i, n in enumerate(lens) if n >= ops.LATENT_EXPAND_FROM)
+    ops.latent_attention(out, q, gate, cache, wuk, wuv, ctx, table, H, DN, DR, DV, rank, page, window, scale,
+                         wuk_t=wuk.view(H, DN, rank).transpose(1, 2).contiguous(), kv_up=(ops.pack_weight(up), up.shape[0]))
+    ops.check_kernel_errors()
+    at = 0
+    for s, (n, p) in enumerate(zip(lens, past)):
+        rows = cache[table[s].long()].reshape(-1, rank + DR)[: p + n].double()
+        c, kr = rows[:, :rank], rows[:, rank:]
+        qs = q[at: at + n].double().view(n, H, DN + DR)
+        i, j = torch.arange(p, p + n, device="cuda")[:, None], torch.arange(p + n, device="cuda")[None, :]
+        hidden = (j > i) | ((i - j >= window) if window else False)
+        for h in range(H):
+            k, v = c @ wuk[h * DN:(h + 1) * DN].double().T, c @ wuv[h * DV:(h + 1) * DV].double().T
+            sc = (qs[:, h, :DN] @ k.T + qs[:, h, DN:] @ kr.T) * scale
+            want = torch.softmax(sc.masked_fill(hidden, float("-inf")), dim=1) @ v
+            if gated:
+                want = want * torch.sigmoid(gate[at: at + n, h * DV:(h + 1) * DV].double())
+            got = out[at: at + n, h * DV:(h + 1) * DV].double()
+            # keys and values rounded to bfloat16 (2^-9 of each: scores of order one move by some 2^-9, weights with them), weights and
+            # output rounded once more
+            assert float((got - want).norm() / want.norm()) < 8e-3, (s, h)
+        at += n
+
+
+def test_what_stays_with_the_latents():
+    ctx = context([1, 5, 31], [9, 0, 4])
+    args = (torch.empty(37, H * DV, device="cuda", dtype=torch.bfloat16), torch.empty(37, H * (DN + DR), device="cuda", dtype=torch.bfloat16), None,
+            torch.empty(9, 16, 64 + DR, device="cuda", dtype=torch.bfloat16), (None, H * (DN + DV)))
+    table = torch.zeros(3, 3, device="cuda", dtype=torch.int32)
+    assert ops.latent_attention_expanded(*args, ctx, table, H, DN, DR, DV, 64, 16, 0, 1.0) == 3           # short segments
+    ctx.seg_len = [1, 5, 1 << 21]
+    assert ops.latent_attention_expanded(*args, ctx, table, H, DN, DR, DV, 64, 16, 0, 1.0) == 3           # rows beyond the room for them
