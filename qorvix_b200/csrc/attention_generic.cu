@@ -15,7 +15,10 @@
 
 #define MAX_HD 512
 
-template <typename T>
+// NREG: output entries a lane holds (head sizes up to 32 NREG).  VEC: the heads' rows start on 16 bytes and are whole 16-byte pieces.
+// A warp's time is that of its loads, so those of a key's row go out 64 entries at a time and the values of several keys
+// together; what is added in which order does not change by it.
+template <typename T, int NREG, bool VEC>
 __global__ void __launch_bounds__(128) attention_generic_kernel(
     T* __restrict__ out, int ld_out, const T* __restrict__ q, int ld_q, const T* __restrict__ cache,
     const int* __restrict__ tok_pos, const int* __restrict__ tok_seg,
@@ -25,6 +28,8 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x * 4 + warp;
   const int t = blockIdx.y;
+  pdl_wait();
+  pdl_launch_dependents();
   if (h >= H) return;                            // whole warp leaves together
   float* qs = qs_all + (size_t)warp * hd;
   const T* qrow = q + (size_t)t * ld_q + (size_t)h * hd;
@@ -39,7 +44,7 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
   const size_t v_off = (size_t)Hkv * page * hd;
   const size_t head_off = (size_t)kvh * page * hd;
 
-  constexpr int NREG = MAX_HD / 32;
+  constexpr int KEYS = NREG <= 4 ? 8 : 2;        // keys whose values are fetched together
   float o[NREG];
 #pragma unroll
   for (int j = 0; j < NREG; ++j) o[j] = 0.f;
@@ -54,7 +59,24 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
       base = (size_t)bt[tk / page] * page_elems + head_off + (size_t)(tk % page) * hd;
       const T* kp = cache + base;
       float dot = 0.f;
-      for (int i = 0; i < hd; ++i) dot = fmaf(qs[i], to_f(kp[i]), dot);
+      if (VEC) {
+        constexpr int PER = 16 / (int)sizeof(T), GO = 64 / PER;     // pieces of 16 bytes
+        for (int i0 = 0; i0 < hd; i0 += 64) {
+          uint4 kv[GO];
+#pragma unroll
+          for (int u = 0; u < GO; ++u)
+            if (i0 + u * PER < hd) kv[u] = *(const uint4*)(kp + i0 + u * PER);
+#pragma unroll
+          for (int u = 0; u < GO; ++u) {
+            if (i0 + u * PER >= hd) break;
+            const T* e = (const T*)&kv[u];
+#pragma unroll
+            for (int x = 0; x < PER; ++x) dot = fmaf(qs[i0 + u * PER + x], to_f(e[x]), dot);
+          }
+        }
+      } else {
+        for (int i = 0; i < hd; ++i) dot = fmaf(qs[i], to_f(kp[i]), dot);
+      }
       s = dot * scale;
     }
     const float m_new = fmaxf(m, warp_max(s));   // finite: the block holds at least one valid key
@@ -64,15 +86,25 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
 #pragma unroll
     for (int j = 0; j < NREG; ++j) o[j] *= corr;
     const int nk = pos - kb + 1 < 32 ? pos - kb + 1 : 32;
-    for (int j = 0; j < nk; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      const size_t bj = __shfl_sync(0xffffffffu, (unsigned long long)base, j);
-      if (pj == 0.f) continue;                   // masked (before the window) or underflowed: adds nothing
-      const T* vp = cache + bj + v_off;
+    for (int j0 = 0; j0 < nk; j0 += KEYS) {
+      float pj[KEYS], v[KEYS][NREG];
 #pragma unroll
-      for (int r = 0; r < NREG; ++r) {
-        const int i = lane + 32 * r;
-        if (i < hd) o[r] = fmaf(pj, to_f(vp[i]), o[r]);
+      for (int j = 0; j < KEYS; ++j) {
+        pj[j] = __shfl_sync(0xffffffffu, p, (j0 + j) & 31);
+        const size_t bj = __shfl_sync(0xffffffffu, (unsigned long long)base, (j0 + j) & 31);
+        if (j0 + j >= nk) pj[j] = 0.f;
+        const T* vp = cache + bj + v_off;
+#pragma unroll
+        for (int r = 0; r < NREG; ++r) {
+          const int i = lane + 32 * r;
+          v[j][r] = pj[j] != 0.f && i < hd ? to_f(vp[i]) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < KEYS; ++j) {
+        if (pj[j] == 0.f) continue;              // masked (before the window) or underflowed: adds nothing
+#pragma unroll
+        for (int r = 0; r < NREG; ++r) o[r] = fmaf(pj[j], v[j][r], o[r]);
       }
     }
     m = m_new;
@@ -110,9 +142,17 @@ extern "C" int qv_attention_generic(void* out, int ld_out, const void* q, int ld
     return 0;
   }
   const size_t smem = (size_t)4 * hd * sizeof(float);
-  QV_DISPATCH_DT(dt, TT,
-                 attention_generic_kernel<TT><<<grid, 128, smem, (cudaStream_t)stream>>>(
-                     (TT*)out, ld_out, (const TT*)q, ld_q, (const TT*)cache, tok_pos, tok_seg,
-                     block_table, max_blocks, H, Hkv, hd, page, window, scale));
-  return qv_launch_status();
+  const bool vec = hd % (dt == QV_DT_F32 ? 4 : 8) == 0 && ((uintptr_t)cache & 15) == 0;
+#define AG_LAUNCH(TT, NR, V)                                                                                                     \
+  return qv_launch(attention_generic_kernel<TT, NR, V>, grid, dim3(128), smem, (cudaStream_t)stream, (TT*)out, ld_out, (const TT*)q, ld_q, \
+                   (const TT*)cache, tok_pos, tok_seg, block_table, max_blocks, H, Hkv, hd, page, window, scale)
+  QV_DISPATCH_DT(dt, TT, {
+    if (!vec) AG_LAUNCH(TT, MAX_HD / 32, false);
+    if (hd <= 32) AG_LAUNCH(TT, 1, true);
+    if (hd <= 64) AG_LAUNCH(TT, 2, true);
+    if (hd <= 128) AG_LAUNCH(TT, 4, true);
+    AG_LAUNCH(TT, MAX_HD / 32, true);
+  });
+#undef AG_LAUNCH
+  return QV_ERR_UNSUPPORTED;
 }
