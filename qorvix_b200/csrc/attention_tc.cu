@@ -136,18 +136,26 @@ struct Walk {
 
 // ROPE > 0: queries and keys have ROPE further entries (the queries' behind each head's, the keys' one row for all heads, map_kr);
 // keys and values are rows of a matrix (map_kv, boxes of KT rows), each segment's padded with rows of zeros to whole tiles.
-template <int HD, bool PAIRED, int ROPE>
+//
+// DIFF: one softmax map a "head" (a.H counts both maps of every head), queries and keys of 64 entries, values of HD that two maps share,
+// all three as columns of the cache's rows (map_kv: [rows of all pages][G (2 x 64 + HD)], boxes of 16 rows).  Weights enter P.V as three
+// bfloat16 terms that hold their 24 bits: the large one and the middle one over the thread's share of S, the small one in the room that
+// a second query tile's output would take.  All sixteen softmax warps work on the one tile, four threads a row (1,500 tokens behind 500, 16 heads, window 1,024: 106 us; with two
+// threads a row 160, the mma.sync kernel 184).  The normalised rows leave in float32, [tokens][a.H][HD], for diff_rows_kernel.
+template <int HD, bool PAIRED, int ROPE, bool DIFF>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                        const __grid_constant__ CUtensorMap map_kv,
                                                                        const __grid_constant__ CUtensorMap map_kr, const AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int NH = HD / 64;                        // 64-element halves of the head
-  constexpr int NHK = (HD + ROPE) / 64;              // and of a query or key
-  constexpr int Q_BYTES = QT * (HD + ROPE) * 2;      // [NHK][128 rows][64]
-  constexpr int K_BYTES = KT * (HD + ROPE) * 2;      // [NHK][128 keys][64]
+  constexpr int HDK = DIFF ? 64 : HD + ROPE;         // entries of a query or key
+  constexpr int NHK = HDK / 64;
+  constexpr int Q_BYTES = QT * HDK * 2;              // [NHK][128 rows][64]
+  constexpr int K_BYTES = KT * HDK * 2;              // [NHK][128 keys][64]
   constexpr int V_BYTES = KT * HD * 2;               // [NH][128 keys][64]
   constexpr int HALF_BYTES = 128 * 128;              // one [128][64] bf16 tile
   static_assert(2 * KT + 2 * HD <= 512, "S and O of both query tiles must fit tensor memory");
+  constexpr int WGS = DIFF ? 4 : 2;                  // softmax warpgroups that share a query tile's rows (keys KT / WGS each)
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = base;                                // tiles A and B
   constexpr int K_ST = PAIRED || ROPE ? K_ST_PAIRS : K_ST_SINGLE;
@@ -179,7 +187,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
   if (threadIdx.x == 0) {
     for (int x = 0; x < 2; ++x) {
       mbar_init(&q_full[x], 1); mbar_init(&q_empty[x], 1);
-      mbar_init(&s_full[x], 1); mbar_init(&p_full[x], 256); mbar_init(&pv_done[x], 1);
+      mbar_init(&s_full[x], 1); mbar_init(&p_full[x], WGS * 128); mbar_init(&pv_done[x], 1);
     }
     for (int i = 0; i < K_ST; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < V_ST; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
@@ -195,6 +203,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;                  // columns 0..255: S of A and of B (P over the first half of each)
   const uint32_t tmem_o = tmem + 2 * KT;             // 2 x HD columns: the output rows of A and of B
+  const uint32_t tmem_lo = tmem_o + HD;              // DIFF: the weights' small terms, 64 columns per S buffer
 
   Walk<PAIRED> walk{0, (int)blockIdx.x, (int)gridDim.x};
   Item t;
@@ -243,17 +252,20 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         int key0 = (t.tile_begin + j) * KT + (lane & 7) * 16;
         if (key0 > last_block) key0 = last_block;              // keys nobody sees: any valid page will do
         const int pg = t.bt[key0 / a.page];                    // fetched before the wait: its latency is the wait's
-        const int my_row = ((pg * 2 + which) * a.Hkv + t.kvh) * a.page + (key0 % a.page);
+        const int my_row = DIFF ? pg * a.page + key0 % a.page : ((pg * 2 + which) * a.Hkv + t.kvh) * a.page + (key0 % a.page);
+        const int col0 = !DIFF ? 0 : which ? a.Hkv * 128 + t.kvh * HD : t.kvh * 128 + (t.h & 1) * 64;
+        const int halves = DIFF && which == 0 ? 1 : NH;
+        const int bytes = which ? V_BYTES : K_BYTES;
         alive = mbar_wait(&empty[s], (lap & 1) ^ 1, a.err, 11);
         if (!alive) break;
-        if (leader) mbar_expect_tx(&full[s], K_BYTES);
+        if (leader) mbar_expect_tx(&full[s], bytes);
 #pragma unroll
         for (int blk = 0; blk < KT / 16; ++blk) {
           const int row = __shfl_sync(0xffffffffu, my_row, blk);
           if (leader) {
 #pragma unroll
             for (int hf = 0; hf < NH; ++hf)
-              tma_load_2d(ring + s * K_BYTES + hf * HALF_BYTES + blk * 16 * 128, &map_kv, &full[s], hf * 64, row);
+              if (hf < halves) tma_load_2d(ring + s * bytes + hf * HALF_BYTES + blk * 16 * 128, &map_kv, &full[s], col0 + hf * 64, row);
           }
         }
         __syncwarp();
@@ -274,7 +286,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           if (leader) {
             mbar_expect_tx(&q_full[x], Q_BYTES);
             for (int f = 0; f < NHK; ++f)
-              tma_load_2d(sQ + x * Q_BYTES + f * HALF_BYTES, &map_q, &q_full[x], t.h * (HD + ROPE) + f * 64, t.q0 + t.tile0 + x * QT);
+              tma_load_2d(sQ + x * Q_BYTES + f * HALF_BYTES, &map_q, &q_full[x], t.h * HDK + f * 64, t.q0 + t.tile0 + x * QT);
           }
           __syncwarp();
           ++loads[x];
@@ -324,7 +336,21 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         // P [128 rows][128 keys] in tensor memory, two keys per column, each softmax warpgroup's 64 keys at the
         // start of its share of S; V [128 keys][HD] MN-major
         const uint32_t o = tmem_o + (uint32_t)(qx * HD), p = tmem + (uint32_t)(x * KT);
-        if (leader) {
+        if (DIFF && leader) {
+          // the small terms first, so that they are added up before the large ones join them
+#pragma unroll
+          for (int term = 2; term >= 0; --term) {
+#pragma unroll
+            for (int kk = 0; kk < KT / 16; ++kk) {
+              const uint32_t v_addr = smem_u32(sV + vs * V_BYTES + (kk * 16) * 128);
+              const int wgk = (kk * 16) / 32, within = ((kk * 16) % 32) / 2;
+              const uint32_t pt = term == 2 ? tmem_lo + (uint32_t)(x * 64 + wgk * 16 + within) : p + (uint32_t)(wgk * 32 + term * 16 + within);
+              umma_f16_ts(o, pt, umma_desc_mn(v_addr, HALF_BYTES), idesc_pv, (term < 2 || kk > 0 || j > 0) ? 1u : 0u);
+            }
+          }
+          umma_commit(&pv_done[x]);
+          umma_commit(&v_empty[vs]);
+        } else if (leader) {
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk) {
           const uint32_t v_addr = smem_u32(sV + vs * V_BYTES + (kk * 16) * 128);
@@ -375,16 +401,16 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
     }
   } else if (warp >= 4) {
     // softmax: thread = (query row of tile x, half of the tile's keys)
-    constexpr int KPT = KT / 2;                        // keys of a tile per thread
-    constexpr int OPT = HD / 2;                        // output columns per thread
-    const int x = (warp - 4) >> 3;
-    const int wg = ((warp - 4) >> 2) & 1;              // which half of the keys and of the output columns
+    constexpr int KPT = KT / WGS;                      // keys of a tile per thread
+    constexpr int OPT = HD / WGS;                      // output columns per thread
+    const int x = DIFF ? 0 : (warp - 4) >> 3;
+    const int wg = ((warp - 4) >> 2) & (WGS - 1);      // which share of the keys and of the output columns
     const int qd = warp & 3;                           // the quarter of tensor memory's lanes this warp may touch
     const int r = qd * 32 + lane;
     const uint32_t lane_base = (uint32_t)(qd * 32) << 16;
     const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(x * HD + wg * OPT);
-    bf16* mx_x = (bf16*)(xchg + (x * 4 + qd) * 256);
-    float* l_x = (float*)(xchg + (x * 4 + qd) * 256);
+    bf16* mx_x = (bf16*)(xchg + (x * 4 + qd) * (128 * WGS));
+    float* l_x = (float*)(xchg + (x * 4 + qd) * (128 * WGS));
     const int bar_id = 1 + x * 4 + qd;
     int n_t = 0;                                       // this tile's key tiles so far: its barriers' phases
     bool ok = true;
@@ -411,7 +437,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           tc_fence_after();
           uint32_t sv[KPT];
           tmem_ld32(s_addr, sv);
-          tmem_ld32(s_addr + 32, sv + 32);
+          if (KPT > 32) tmem_ld32(s_addr + 32, sv + KPT - 32);
           tmem_wait_ld();
           if (all_visible) {
             // four independent chains: one chain of dependent maxima would cost more than the loads did
@@ -436,10 +462,12 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           // it for the other and takes the larger.  (The reference maximum need not be the exact one:
           // any common value at or above the true maximum less 2^RESCALE_STEP serves.)
           const bf16 mine = __float2bfloat16_ru(mx);
-          bf16* slot = mx_x + (n_t & 1) * 64;
+          bf16* slot = mx_x + (n_t & 1) * (32 * WGS);
           slot[wg * 32 + lane] = mine;
-          named_barrier(bar_id, 64);
-          mx = fmaxf(__bfloat162float(mine), __bfloat162float(slot[(wg ^ 1) * 32 + lane]));
+          named_barrier(bar_id, 32 * WGS);
+          mx = __bfloat162float(mine);
+#pragma unroll
+          for (int o = 1; o < WGS; ++o) mx = fmaxf(mx, __bfloat162float(slot[(wg ^ o) * 32 + lane]));
         }
         if (!ok) continue;
         float corr = 1.f;
@@ -473,6 +501,38 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         // only columns that have been read), and their sum
         const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
         float sum = 0.f;
+        if (DIFF) {
+          // the whole share is read before the first term goes over it; 16 scores at a time become 3 x 8 words
+          uint32_t sv[KPT];
+          tmem_ld32(s_addr, sv);
+          tmem_wait_ld();
+          const uint32_t lo_addr = tmem_lo + lane_base + (uint32_t)(buf * 64 + wg * (KPT / 2));
+#pragma unroll
+          for (int c = 0; c < KPT; c += 16) {
+            uint32_t w0[8], w1[8], w2[8];
+            float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float e[2];
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const int key = key_base + c + i + u;
+                e[u] = all_visible || (key >= lo && key <= hi) ? fast_exp2(fmaf(__uint_as_float(sv[c + i + u]), a.scale_log2, neg_m)) : 0.f;
+              }
+              s4[(i >> 1) & 3] += e[0] + e[1];
+              const __nv_bfloat162 h = __floats2bfloat162_rn(e[0], e[1]);
+              const float r0 = e[0] - __low2float(h), r1 = e[1] - __high2float(h);
+              const __nv_bfloat162 m2 = __floats2bfloat162_rn(r0, r1);
+              w0[i >> 1] = *(const uint32_t*)&h;
+              w1[i >> 1] = *(const uint32_t*)&m2;
+              w2[i >> 1] = pack2_bf16(r0 - __low2float(m2), r1 - __high2float(m2));
+            }
+            sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            tmem_st8(s_addr + (uint32_t)(c >> 1), w0);
+            tmem_st8(s_addr + KPT / 2 + (uint32_t)(c >> 1), w1);
+            tmem_st8(lo_addr + (uint32_t)(c >> 1), w2);
+          }
+        } else
 #pragma unroll
         for (int c = 0; c < KPT; c += 32) {
           uint32_t sv[32], w[16];
@@ -512,11 +572,13 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         // the row's sum: both threads' parts, added in the same order by both.  A barrier first (the
         // maxima of the last two tiles lie in the bytes the sums go to) and one after (the next
         // item's maxima go to the same bytes).
-        named_barrier(bar_id, 64);
+        named_barrier(bar_id, 32 * WGS);
         l_x[wg * 32 + lane] = l;
-        named_barrier(bar_id, 64);
+        named_barrier(bar_id, 32 * WGS);
         l = l_x[lane] + l_x[32 + lane];
-        named_barrier(bar_id, 64);
+#pragma unroll
+        for (int o = 2; o < WGS; ++o) l += l_x[o * 32 + lane];
+        named_barrier(bar_id, 32 * WGS);
       }
       if (ok) {
         ok = PAIRED ? __all_sync(0xffffffffu, mbar_wait(&pv_done[x], (uint32_t)((n_t - 1) & 1), a.err, 20))
@@ -532,6 +594,16 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           uint32_t v[32];
           tmem_ld32(o_addr + c, v);
           tmem_wait_ld();
+          if (DIFF) {
+            if (store) {
+              float* frow = (float*)a.out + ((size_t)(t.q0 + row_in_seg) * a.H + t.h) * HD + wg * OPT;
+#pragma unroll
+              for (int i = 0; i < 32; i += 4)
+                *(float4*)(frow + c + i) = make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv, __uint_as_float(v[i + 2]) * inv,
+                                                       __uint_as_float(v[i + 3]) * inv);
+            }
+            continue;
+          }
           if (ROPE > 0 && grow && store) {
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
@@ -572,16 +644,18 @@ int device_sms() {
   return sms;
 }
 
-template <int HD, bool PAIRED, int ROPE = 0>
+template <int HD, bool PAIRED, int ROPE = 0, bool DIFF = false>
 int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mkr, const AttnArgs& args, cudaStream_t st) {
   // two Q tiles, the rings of keys and values, 256 bytes of barriers, 2 KB for what a row's threads exchange, 1 KB to align
-  constexpr int smem = ROPE ? (QT + K_ST_PAIRS * KT) * (HD + ROPE) * 2 + V_ST * KT * HD * 2 + 256 + 2048 + 1024
+  constexpr int smem = DIFF ? (QT + K_ST_SINGLE * KT) * 64 * 2 + V_ST * KT * HD * 2 + 256 + 2048 + 1024
+                       : ROPE ? (QT + K_ST_PAIRS * KT) * (HD + ROPE) * 2 + V_ST * KT * HD * 2 + 256 + 2048 + 1024
                             : 2 * QT * HD * 2 + (K_ST_PAIRS + V_ST) * KT * HD * 2 + 256 + 2048 + 1024;
   static_assert(QT * HD * 2 + (K_ST_SINGLE + V_ST) * KT * HD * 2 <= 2 * QT * HD * 2 + (K_ST_PAIRS + V_ST) * KT * HD * 2, "one layout's room serves both");
   static_assert(smem <= 227 * 1024, "more shared memory than a CTA can have");
   static bool configured = false;
   static_assert(!ROPE || !PAIRED, "two query tiles with their further entries do not fit");
-  auto kernel = attn_prefill_tc_kernel<HD, PAIRED, ROPE>;
+  static_assert(!DIFF || (!PAIRED && !ROPE && HD == 128), "one tile of one map an item");
+  auto kernel = attn_prefill_tc_kernel<HD, PAIRED, ROPE, DIFF>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
@@ -660,4 +734,47 @@ extern "C" int qv_attn_rows_tc(void* out, int ld_out, const void* q, int ld_q, i
   a.segments = S; a.q_pairs = (int)q_tiles; a.items = (int)(H * S * q_tiles); a.paired = 0;
   a.row_off = row_off; a.row_key = row_key; a.gate = (const bf16*)gate; a.ld_gate = ld_gate; a.v_col = v_col; a.min_len = min_len;
   return launch<128, false, 64>(mq, mkv, mkr, a, (cudaStream_t)stream);
+}
+
+// Both maps of a head joined: rows [T][2 H][128] float32 (map 1, map 2 of head 0, ...) -> out[t, h] = d / sqrt(mean(d^2) + eps) * post,
+// d = map 1 - lam * map 2.  A warp a (token, head).
+__global__ void __launch_bounds__(256) diff_rows_kernel(bf16* __restrict__ out, int ld_out, const float4* __restrict__ rows, int n, int H, float lam,
+                                                        float eps, float post, const int* __restrict__ seg_q_start) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (unit >= n * H) return;
+  const int t = seg_q_start[0] + unit / H, h = unit % H;
+  const float4 a = rows[((size_t)t * 2 * H + 2 * h) * 32 + lane], b = rows[((size_t)t * 2 * H + 2 * h + 1) * 32 + lane];
+  const float d0 = a.x - lam * b.x, d1 = a.y - lam * b.y, d2 = a.z - lam * b.z, d3 = a.w - lam * b.w;
+  const float ss = warp_sum((d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3));
+  const float f = 1.0f / sqrtf(ss / 128.0f + eps) * post;
+  *(uint2*)(out + (size_t)t * ld_out + h * 128 + lane * 4) = make_uint2(pack2_bf16(d0 * f, d1 * f), pack2_bf16(d2 * f, d3 * f));
+}
+
+// Differential attention of prompt portions with maps of 64 and values of 128: cache rows [pages * page][G (2 x 64 + 128)], queries
+// [T][ld_q] (two maps of 64 a head), `tokens` rows from seg_q_start[0] on, workspace rows [T][2 H][128] float32.  Other sizes, pages that
+// are no multiple of 16 and unaligned operands are refused.
+extern "C" int qv_diff_attention_rows_tc(void* out, int ld_out, const void* q, int ld_q, int T, const void* cache, long long cache_rows,
+                                         const int* seg_q_start, const int* seg_pos0, const int* block_table, int max_blocks, int S, int tokens,
+                                         int max_q_len, int H, int G, int page, int window, float scale, float lam, float eps, float post,
+                                         float* rows, int* err, void* stream) {
+  if (S <= 0 || max_q_len <= 0 || tokens <= 0) return 0;
+  if (H <= 0 || G <= 0 || H % G || page % 16 || (ld_q & 7) || (ld_out & 3) ||
+      (((uintptr_t)q | (uintptr_t)cache | (uintptr_t)rows) & 15) || ((uintptr_t)out & 7) || cache_rows > 0x7fffffffLL)
+    return QV_ERR_UNSUPPORTED;
+  const long long q_tiles = (max_q_len + QT - 1) / QT;
+  if (2LL * H * S * q_tiles > (1LL << 30) || (long long)tokens * H > (1LL << 30)) return QV_ERR_TOO_LARGE;
+  const int width = G * 256;
+  CUtensorMap mq, mkv;
+  if (!make_map(&mq, q, T, H * 128, ld_q, QT) || !make_map(&mkv, cache, cache_rows, width, width, 16)) return QV_ERR_UNSUPPORTED;
+  AttnArgs a;
+  a.out = (bf16*)rows; a.seg_q_start = seg_q_start; a.seg_pos0 = seg_pos0; a.block_table = block_table; a.err = err;
+  a.ld_out = 0; a.max_blocks = max_blocks; a.H = 2 * H; a.Hkv = G; a.page = page; a.window = window;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.segments = S; a.q_pairs = (int)q_tiles; a.items = (int)(2LL * H * S * q_tiles); a.paired = 0;
+  const int rc = launch<128, false, 0, true>(mq, mkv, mkv, a, (cudaStream_t)stream);
+  if (rc) return rc;
+  return qv_launch(diff_rows_kernel, dim3((unsigned)(((long long)tokens * H + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, (bf16*)out, ld_out,
+                   (const float4*)rows, tokens, H, lam, eps, post, seg_q_start);
 }

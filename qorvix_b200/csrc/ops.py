@@ -65,6 +65,7 @@ _ARGTYPES = {
     "qv_latent_attention_tc": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _V, _V, _I, _V],
     "qv_latent_rows_out": [_V, _V, _V, _V, _V, _I, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V],
     "qv_attn_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _I, _V, _L, _V, _V, _V, _I, _V, _V, _I, _I, _I, _I, _I, _F, _V, _V],
+    "qv_diff_attention_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _V, _V, _V],
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
     "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V],
@@ -582,6 +583,34 @@ def diff_attention_splits(tokens: int, H: int, G: int, window: int, max_ctx: int
     return max(1, min(sm_count() // max(tokens * G, 1), blocks // 2, 12))
 
 
+DIFF_ROWS_FROM = 64                        # portions of at least this many tokens take the tcgen05 kernel
+DIFF_ROWS_BYTES = 1 << 30                  # the most that both maps' float32 rows may take
+
+
+def diff_attention_rows(out, q, cache_layer, ctx, block_table, first: int, H, G, n, dv, page, window, scale, lam, eps, post) -> bool:
+    """Differential attention of the step's segments from `first` on with every map as an attention of its own on the tcgen05 tensor cores
+    (weights in three bfloat16 terms, rows left in float32) and a pass that joins the maps.  For portions of DIFF_ROWS_FROM tokens and
+    more, maps of 64 and values of 128; False, nothing written, otherwise."""
+    lens = ctx.seg_len[first:]
+    T = q.shape[0]
+    if (n != 64 or dv != 128 or page % 16 or max(lens) < DIFF_ROWS_FROM or q.stride(0) % 8 or out.stride(0) % 4 or q.data_ptr() % 16
+            or out.data_ptr() % 8 or T * H * 2 * dv * 4 > DIFF_ROWS_BYTES or os.environ.get("QORVIX_DIFF_WEIGHT_TERMS") == "1"):
+        return False
+    _need_cuda(out, q, cache_layer, block_table)
+    assert q.stride(1) == 1 and out.stride(1) == 1 and out.dtype == cache_layer.dtype == torch.bfloat16
+    assert cache_layer.is_contiguous() and tuple(cache_layer.shape[1:]) == (page, G * (2 * n + dv))
+    rows = torch.empty((T, 2 * H, dv), device=q.device, dtype=torch.float32)
+    rc = _lib("attention_tc").qv_diff_attention_rows_tc(
+        _ptr(out), out.stride(0), _ptr(q), q.stride(0), T, _ptr(cache_layer), cache_layer.shape[0] * page, _ptr(ctx.seg_q_start[first:]),
+        _ptr(ctx.seg_pos0[first:]), _ptr(block_table[first:]), block_table.shape[-1], len(lens), sum(lens), max(lens), H, G, page, int(window),
+        float(scale), float(lam), float(eps), float(post), _ptr(rows), _ptr(_tc_buffers(q.device)["err"]), _stream())
+    if rc == -2:
+        return False
+    _check(rc, "diff_attention_rows")
+    add_launches(1)                                  # the pass that joins the maps
+    return True
+
+
 def diff_attention(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, window, scale, lam, eps, post) -> None:
     """Differential attention of every token of the step over its request's cache rows.  bfloat16: the tensor-core
     kernel where it takes the sizes (single tokens, which come first in a step, with tiles of 16 rows and their keys in
@@ -596,7 +625,7 @@ def diff_attention(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, win
         if n1:
             splits = diff_attention_splits(n1, H, G, window, ctx.max_ctx_len)
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start, ctx.seg_pos0, block_table, n1, 1, *args, splits=splits)
-        if ok and n1 < S:
+        if ok and n1 < S and not diff_attention_rows(out, q, cache_layer, ctx, block_table, n1, *args):
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start[n1:], ctx.seg_pos0[n1:], block_table[n1:], S - n1,
                                    max(ctx.seg_len[n1:]), *args)
         if ok:
