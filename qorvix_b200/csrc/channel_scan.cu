@@ -435,6 +435,312 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 #undef CS_LAUNCH
 }
 
+// ---------------------------------------------------------------- delta rule on the decayed state: four tokens at a time
+// With S_0 the state ahead of a block of up to four tokens, P_t the product of the decays of the block's tokens up to t (per channel) and
+// kb = beta k, the recurrence S_t = diag(g_t) S_(t-1) + kb_t e_t^T, e_t = v_t - S_(t-1)^T (g_t k_t), y_t = S_t^T q_t unrolls to
+//   e_t   = v_t - S_0^T (P_t k_t) - sum_(l < t) A_tl e_l        A_tl = sum_c k_t (g_(l+1) .. g_t) kb_l
+//   y_t   = S_0^T (P_t q_t) + sum_(l <= t) B_tl e_l             B_tl = sum_c q_t (g_(l+1) .. g_t) kb_l
+//   S_end = diag(P_end) S_0 + sum_l (g_(l+1) .. g_end kb_l) e_l^T
+// that is, the eight products with S_0 do not wait for one another, and a block costs one chain of sums and shuffles instead of four.
+// Only products of decays (each at most one) occur, no quotients; everything is float32.
+//   channel_delta_operands   x [T][H][3][n] = P_t k_t, P_t q_t, (g_(t+1) .. g_end) kb_t;  pall [T][H][n] = P_end, at a block's first token;
+//                            coef [T][H][8] = A_t0 A_t1 A_t2 -, B_t0 .. B_t3.  A warp per (token, head).
+//   channel_delta_blocks     the recurrence; a lane holds 16 rows of two columns, two warps a CTA work and two fetch (one column a lane and
+//                            four working warps: 496 us where this takes 426).
+// 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 426 in blocks, the operands 14 and 34.  Bound by a block's chain (dots,
+// shuffles, the triangular sums, the update) in one warp a scheduler.
+// Blocks are counted from the start of a request's portion, so cuts agree to rounding (the 32-bit path takes channel_scan_kernel).
+#define CD_BLOCK 4
+// A warp takes a block and a head (the warp of the block's first token; the others have nothing to do): a row of q, k and g is then read
+// once for all of the block's products.
+__global__ void __launch_bounds__(128) channel_delta_operands_kernel(float* __restrict__ x, float* __restrict__ pall, float* __restrict__ coef,
+                                                                    const float* __restrict__ q, int ld_q, const float* __restrict__ k, int ld_k,
+                                                                    const float* __restrict__ b, int ld_b, const float* __restrict__ g, int ld_g,
+                                                                    const int* __restrict__ tok_seg, const int* __restrict__ seg_q_start, int H,
+                                                                    int G, int n, float eps, float q_scale, int t_first) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = t_first + blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int seg = tok_seg[t], q0 = seg_q_start[seg], j = t - q0, left = seg_q_start[seg + 1] - q0 - j;
+  if (h >= H || j % CD_BLOCK) return;
+  const int nb = left < CD_BLOCK ? left : CD_BLOCK;
+  const int grp = h / (H / G);
+  const float* qr = q + (size_t)t * ld_q + (size_t)grp * n;
+  const float* kr = k + (size_t)t * ld_k + (size_t)grp * n;
+  const float* gr = g + (size_t)t * ld_g + (size_t)h * n;
+  float beta[CD_BLOCK];
+#pragma unroll
+  for (int u = 0; u < CD_BLOCK; ++u) beta[u] = u < nb ? 1.0f / (1.0f + expf(-b[(size_t)(t + u) * ld_b + h])) : 0.f;
+  float qq[CD_BLOCK] = {}, k2[CD_BLOCK] = {}, kk[6] = {}, qk[10] = {};      // pairs (u, l): kk at u (u - 1) / 2 + l, qk at u (u + 1) / 2 + l
+#pragma unroll 2
+  for (int i = lane; i < n; i += 32) {
+    float qv[CD_BLOCK], kv[CD_BLOCK], gv[CD_BLOCK];
+#pragma unroll
+    for (int u = 0; u < CD_BLOCK; ++u) {
+      const bool in = u < nb;
+      qv[u] = in ? qr[i + (size_t)u * ld_q] : 0.f;
+      kv[u] = in ? kr[i + (size_t)u * ld_k] : 0.f;
+      gv[u] = in ? gr[i + (size_t)u * ld_g] : 1.f;
+    }
+#pragma unroll
+    for (int u = 0; u < CD_BLOCK; ++u) {
+      qq[u] = fmaf(qv[u], qv[u], qq[u]);
+      k2[u] = fmaf(kv[u], kv[u], k2[u]);
+      float D = 1.f;                                                 // g_(l+1) .. g_u
+#pragma unroll
+      for (int l = u; l >= 0; --l) {
+        const float kd = kv[l] * D;
+        qk[u * (u + 1) / 2 + l] = fmaf(qv[u], kd, qk[u * (u + 1) / 2 + l]);
+        if (l < u) kk[u * (u - 1) / 2 + l] = fmaf(kv[u], kd, kk[u * (u - 1) / 2 + l]);
+        D *= gv[l];
+      }
+    }
+  }
+  float iq[CD_BLOCK], ik[CD_BLOCK];
+#pragma unroll
+  for (int u = 0; u < CD_BLOCK; ++u) {
+    iq[u] = q_scale / sqrtf(warp_sum(qq[u]) + eps);
+    ik[u] = 1.0f / sqrtf(warp_sum(k2[u]) + eps);
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) kk[i] = warp_sum(kk[i]);
+#pragma unroll
+  for (int i = 0; i < 10; ++i) qk[i] = warp_sum(qk[i]);
+  const size_t o = (size_t)t * H + h;
+  for (int i = lane; i < n; i += 32) {
+    float gv[CD_BLOCK], P[CD_BLOCK], suffix[CD_BLOCK];
+#pragma unroll
+    for (int u = 0; u < CD_BLOCK; ++u) gv[u] = u < nb ? gr[i + (size_t)u * ld_g] : 1.f;
+    P[0] = gv[0];
+#pragma unroll
+    for (int u = 1; u < CD_BLOCK; ++u) P[u] = P[u - 1] * gv[u];
+    suffix[CD_BLOCK - 1] = 1.f;
+#pragma unroll
+    for (int u = CD_BLOCK - 2; u >= 0; --u) suffix[u] = suffix[u + 1] * gv[u + 1];
+    pall[o * n + i] = P[CD_BLOCK - 1];
+#pragma unroll
+    for (int u = 0; u < CD_BLOCK; ++u) {
+      if (u >= nb) break;
+      const float ku = kr[i + (size_t)u * ld_k] * ik[u];
+      float* xr = x + (o + (size_t)u * H) * 3 * n + i;
+      xr[0] = P[u] * ku;
+      xr[n] = P[u] * (qr[i + (size_t)u * ld_q] * iq[u]);
+      xr[2 * n] = suffix[u] * (beta[u] * ku);
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int u = 0; u < CD_BLOCK; ++u) {
+      if (u >= nb) break;
+      float c[8] = {};
+#pragma unroll
+      for (int l = 0; l <= u; ++l) {
+        const float f = ik[l] * beta[l];
+        if (l < u) c[l] = kk[u * (u - 1) / 2 + l] * ik[u] * f;
+        c[4 + l] = qk[u * (u + 1) / 2 + l] * iq[u] * f;
+      }
+      float4* dst = (float4*)(coef + (o + (size_t)u * H) * 8);
+      dst[0] = make_float4(c[0], c[1], c[2], c[3]);
+      dst[1] = make_float4(c[4], c[5], c[6], c[7]);
+    }
+  }
+}
+
+struct ChannelDeltaArgs {
+  float* out; int ld_out;                 // [T, H * dv]
+  const float* x; const float* pall; const float* coef;
+  const float* v; int ld_v;
+  float* state; long long slot_stride;    // as ChannelScanArgs
+  const int* seg_q_start; const int* seg_slot;
+  int H, dk, dv;
+};
+
+// NB: blocks a stage, two stages.  C: columns a lane, so 4 / C warps work; two more fetch.
+template <int LPC, int NB, int C = 2>
+__global__ void __launch_bounds__(32 * (4 / C + 2)) channel_delta_blocks_kernel(ChannelDeltaArgs a) {
+  extern __shared__ __align__(16) float cd_ring[];
+  constexpr int CPT = 32 / LPC, CTA_COLS = 4 * CPT, VEC = CS_PAD * LPC, W = 4 / C;
+  constexpr int ROW = 3 * VEC + 8 + CTA_COLS;                        // floats a token takes: three vectors, factors, values
+  constexpr int BLK = CD_BLOCK * ROW + VEC;                          // a block: its tokens, then P_end
+  pdl_wait();
+  const int s = blockIdx.x, h = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lic = lane % LPC, cw = lane / LPC;
+  const int dk = a.dk, dv = a.dv, H = a.H;
+  const int tiles = (dv + CPT - 1) / CPT;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  const bool works = warp < W;
+  const int tile0 = blockIdx.z * 4 + (works ? warp * C : 0);         // of the working warps: C tiles of CPT columns
+  const int cta_col0 = blockIdx.z * CTA_COLS;
+  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile0) * (CS_ROWS * 32) + lane;
+  float S[C][CS_ROWS];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < CS_ROWS; ++i) S[c][i] = works && tile0 + c < tiles ? st[c * CS_ROWS * 32 + i * 32] : 0.f;
+  auto issue = [&](int ch) {                                         // by the last two warps, a token a warp; zeros beyond the segment
+    float* base = cd_ring + (ch & 1) * NB * BLK;
+#pragma unroll 2
+    for (int tk = warp - W; tk < NB * CD_BLOCK; tk += 2) {
+      const int j = ch * NB * CD_BLOCK + tk;
+      const bool in = j < len;
+      const size_t row = (size_t)(q0 + (in ? j : 0)) * H + h;
+      const float* src = a.x + row * 3 * dk;
+      float* blk = base + (tk / CD_BLOCK) * BLK;
+      float* dst = blk + (tk % CD_BLOCK) * ROW;
+#pragma unroll
+      for (int r = lane * 4; r < CS_ROWS * LPC; r += 128) {
+        const bool ok = in && r < dk;
+        const int off = r + (r / CS_ROWS) * (CS_PAD - CS_ROWS);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) cs_cp16(dst + v * VEC + off, ok ? src + v * dk + r : a.x, ok);
+        if (tk % CD_BLOCK == 0) cs_cp16(blk + CD_BLOCK * ROW + off, ok ? a.pall + row * dk + r : a.x, ok);
+      }
+      if (lane < 2) cs_cp16(dst + 3 * VEC + lane * 4, a.coef + row * 8 + lane * 4, in);
+      for (int cc = lane; cc < CTA_COLS; cc += 32) {
+        const bool ok = in && cta_col0 + cc < dv;
+        cs_cp4(dst + 3 * VEC + 8 + cc, ok ? a.v + (size_t)(q0 + j) * a.ld_v + (size_t)h * dv + cta_col0 + cc : a.v, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int nstages = (len + NB * CD_BLOCK - 1) / (NB * CD_BLOCK);
+  if (!works && nstages > 0) issue(0);
+  for (int ch = 0; ch < nstages; ++ch) {
+    if (!works) {
+      if (ch + 1 < nstages) {
+        issue(ch + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+    }
+    __syncthreads();
+    if (works) {
+#pragma unroll 1
+      for (int blk = 0; blk < NB; ++blk) {
+        const int j0 = (ch * NB + blk) * CD_BLOCK;
+        if (j0 >= len) break;
+        const float* d = cd_ring + (ch & 1) * NB * BLK + blk * BLK;
+        float p[CD_BLOCK][C], r[CD_BLOCK][C];
+#pragma unroll
+        for (int t = 0; t < CD_BLOCK; ++t) {
+          const float4* pk = (const float4*)(d + t * ROW + lic * CS_PAD);
+          const float4* pq = (const float4*)(d + t * ROW + VEC + lic * CS_PAD);
+          float ps[C][2] = {}, rs[C][2] = {};                        // two partial sums each
+#pragma unroll
+          for (int i = 0; i < CS_ROWS / 4; ++i) {
+            const float4 k4 = pk[i], q4 = pq[i];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              ps[c][0] = fmaf(k4.x, S[c][4 * i], ps[c][0]); ps[c][1] = fmaf(k4.y, S[c][4 * i + 1], ps[c][1]);
+              ps[c][0] = fmaf(k4.z, S[c][4 * i + 2], ps[c][0]); ps[c][1] = fmaf(k4.w, S[c][4 * i + 3], ps[c][1]);
+              rs[c][0] = fmaf(q4.x, S[c][4 * i], rs[c][0]); rs[c][1] = fmaf(q4.y, S[c][4 * i + 1], rs[c][1]);
+              rs[c][0] = fmaf(q4.z, S[c][4 * i + 2], rs[c][0]); rs[c][1] = fmaf(q4.w, S[c][4 * i + 3], rs[c][1]);
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < C; ++c) { p[t][c] = ps[c][0] + ps[c][1]; r[t][c] = rs[c][0] + rs[c][1]; }
+        }
+#pragma unroll
+        for (int o = LPC / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int t = 0; t < CD_BLOCK; ++t)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              p[t][c] += __shfl_xor_sync(0xffffffffu, p[t][c], o);
+              r[t][c] += __shfl_xor_sync(0xffffffffu, r[t][c], o);
+            }
+        float e[CD_BLOCK][C];
+#pragma unroll
+        for (int t = 0; t < CD_BLOCK; ++t) {
+          const float4 A4 = *(const float4*)(d + t * ROW + 3 * VEC), B4 = *(const float4*)(d + t * ROW + 3 * VEC + 4);
+          const float A[4] = {A4.x, A4.y, A4.z, A4.w}, B[4] = {B4.x, B4.y, B4.z, B4.w};
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const int cc = (warp * C + c) * CPT + cw;
+            float ev = d[t * ROW + 3 * VEC + 8 + cc] - p[t][c];
+#pragma unroll
+            for (int l = 0; l < t; ++l) ev = fmaf(-A[l], e[l][c], ev);
+            e[t][c] = ev;
+            float y = r[t][c];
+#pragma unroll
+            for (int l = 0; l <= t; ++l) y = fmaf(B[l], e[l][c], y);
+            if (lic == 0 && cta_col0 + cc < dv && j0 + t < len) a.out[(size_t)(q0 + j0 + t) * a.ld_out + (size_t)h * dv + cta_col0 + cc] = y;
+          }
+        }
+        const float4* pp = (const float4*)(d + CD_BLOCK * ROW + lic * CS_PAD);
+#pragma unroll
+        for (int i = 0; i < CS_ROWS / 4; ++i) {
+          const float4 g4 = pp[i];
+#pragma unroll
+          for (int c = 0; c < C; ++c) { S[c][4 * i] *= g4.x; S[c][4 * i + 1] *= g4.y; S[c][4 * i + 2] *= g4.z; S[c][4 * i + 3] *= g4.w; }
+#pragma unroll
+          for (int t = 0; t < CD_BLOCK; ++t) {
+            const float4 w4 = *(const float4*)(d + t * ROW + 2 * VEC + lic * CS_PAD + 4 * i);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              S[c][4 * i] = fmaf(w4.x, e[t][c], S[c][4 * i]); S[c][4 * i + 1] = fmaf(w4.y, e[t][c], S[c][4 * i + 1]);
+              S[c][4 * i + 2] = fmaf(w4.z, e[t][c], S[c][4 * i + 2]); S[c][4 * i + 3] = fmaf(w4.w, e[t][c], S[c][4 * i + 3]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  pdl_launch_dependents();
+  if (!works) return;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (tile0 + c < tiles)
+#pragma unroll
+      for (int i = 0; i < CS_ROWS; ++i) st[c * CS_ROWS * 32 + i * 32] = S[c][i];
+}
+
+// Floats of workspace for T tokens: x, pall and coef in this order.
+extern "C" long long qv_channel_delta_workspace_floats(int T, int H, int dk) { return (long long)T * H * (4 * (long long)dk + 8); }
+
+// The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
+// beta, g [T, H * dk] the decays, v [T, H * dv].  dk a multiple of 4, at most 256.
+extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
+                                const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
+                                long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int H, int G,
+                                int dk, int dv, float* workspace, void* stream) {
+  if (S <= 0 || T <= 0) return 0;
+  if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || dk % 4 || ((uintptr_t)workspace & 15)) return QV_ERR_UNSUPPORTED;
+  if (dk > 256) return QV_ERR_TOO_LARGE;
+  cudaStream_t st = (cudaStream_t)stream;
+  ChannelDeltaArgs a;
+  float* x = workspace;
+  float* pall = x + (size_t)T * H * 3 * dk;
+  float* coef = pall + (size_t)T * H * dk;
+  for (int done = 0; done < T; done += 65535) {
+    const int rows = T - done < 65535 ? T - done : 65535;
+    const int rc = qv_launch(channel_delta_operands_kernel, dim3(rows, (H + 3) / 4), dim3(128), 0, st, x, pall, coef, q, ld_q, k, ld_k, b, ld_b, g,
+                             ld_g, tok_seg, seg_q_start, H, G, dk, eps, q_scale, done);
+    if (rc) return rc;
+  }
+  a.out = out; a.ld_out = ld_out; a.x = x; a.pall = pall; a.coef = coef; a.v = v; a.ld_v = ld_v; a.state = state; a.slot_stride = slot_stride;
+  a.seg_q_start = seg_q_start; a.seg_slot = seg_slot; a.H = H; a.dk = dk; a.dv = dv;
+  const int lpc = cs_lanes_per_column(dk);
+  const int cta_cols = 4 * 32 / lpc;
+  const int ctas = (dv + cta_cols - 1) / cta_cols;
+  if (ctas > 65535) return QV_ERR_TOO_LARGE;
+#define CD_LAUNCH(LPC, NB)                                                                                                       \
+  do {                                                                                                                           \
+    constexpr int smem = 2 * NB * (CD_BLOCK * (3 * CS_PAD * LPC + 8 + 4 * 32 / LPC) + CS_PAD * LPC) * 4;                         \
+    cudaFuncSetAttribute(channel_delta_blocks_kernel<LPC, NB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
+    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB, 2>, dim3(S, H, ctas), dim3(128), (size_t)smem, st, a);           \
+  } while (0)
+  if (lpc == 1) CD_LAUNCH(1, 4);
+  if (lpc == 2) CD_LAUNCH(2, 4);
+  if (lpc == 4) CD_LAUNCH(4, 4);
+  if (lpc == 8) CD_LAUNCH(8, 4);
+  CD_LAUNCH(16, 2);
+#undef CD_LAUNCH
+}
+
 // ---------------------------------------------------------------- unit norm per head, weight, gate, factor
 // y [T, H * dv] float32 -> out[t, h, i] = y / sqrt(mean_i(y^2) + eps) * w[h * dv + i] * gate(g[t, h * dv + i]) * factor,
 // gate 0: sigmoid, 1: SiLU; g float32 (row stride ld_g).  One warp per (token, head); the sum's order follows dv alone.

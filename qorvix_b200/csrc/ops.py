@@ -105,6 +105,8 @@ _ARGTYPES = {
     "qv_unit_keys": [_V, _V, _V, _I, _V, _I, _V, _I, _I, _I, _F, _V],
     "qv_channel_scan_state_floats": [_I, _I, _I],
     "qv_channel_scan": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _V],
+    "qv_channel_delta_workspace_floats": [_I, _I, _I],
+    "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _V],
     "qv_head_norm_gate": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _F, _I, _V],
     "qv_bias_attn_prepare": [_V, _I, _V, _I, _I, _I, _I, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V],
     "qv_bias_attention_generic": [_V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _V, _I, _V, _V, _I, _F, _I, _V],
@@ -121,7 +123,7 @@ _ARGTYPES = {
 }
 _RESTYPES = {"qv_error_string": ctypes.c_char_p, "qv_packed_weight_bytes": c_longlong, "qv_gemm_bf16_split_slot_bytes": c_longlong,
              "qv_linear_scan_state_floats": c_longlong, "qv_latent_tc_workspace_bytes": c_longlong, "qv_diff_partial_floats": c_longlong,
-             "qv_channel_scan_state_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
+             "qv_channel_scan_state_floats": c_longlong, "qv_channel_delta_workspace_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
 _typed_libs = {}
 
 
@@ -919,6 +921,26 @@ def channel_scan(out, q, k, v, w, au, u, q_scale: float, state, ctx, H: int, dk:
         au.stride(0) if au is not None else 0, _ptr(u), u.stride(0) if u is not None else 0, float(q_scale), _ptr(state),
         state.stride(0), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, int(ctx.max_q_len), H, dk, dv, _stream())
     _check(rc, "channel_scan")
+
+
+def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: int, eps: float, q_scale: float) -> bool:
+    """The delta rule that reads the decayed state, four tokens at a time: unit vectors of q and k (q times q_scale), beta = sigmoid(b), decays
+    g, per request and head; state as channel_scan's.  False, nothing done, for key sizes the kernel does not take (multiples of 4 up to 256)."""
+    if dk % 4 or dk > 256:
+        return False
+    _need_cuda(out, q, k, v, b, g, state)
+    for t in (out, q, k, v, b, g):
+        assert t.dtype == torch.float32 and t.stride(1) == 1
+    assert state.dtype == torch.float32 and state.stride(-1) == 1
+    T = q.shape[0]
+    lib = _lib("channel_scan")
+    ws = torch.empty(int(lib.qv_channel_delta_workspace_floats(T, H, dk)), device=q.device, dtype=torch.float32)
+    rc = lib.qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
+                              _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0), _ptr(ctx.tok_seg),
+                              _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, T, H, G, dk, dv, _ptr(ws), _stream())
+    _check(rc, "channel_delta")
+    add_launches(1)
+    return True
 
 
 def head_norm_gate(out, y, gate, w, H: int, eps: float, gate_kind: int, factor: float = 1.0) -> None:

@@ -165,12 +165,15 @@ class ChannelDelta(SharedIOMixer):
         ops.channel_gates(decay, proj[:, a0:g0], self.a_up, self.dt_bias, False, ops.GATE_EXP_NEG_SOFTPLUS, 0.0, rate=self.rate)
         gate = torch.empty((T, H * dv), device=dev, dtype=torch.float32)
         ops.channel_gates(gate, proj[:, g0: g0 + self.spec.gate_rank], self.g_up, None, False, ops.GATE_LINEAR, 0.0)
-        qh = torch.empty((T, H * dk), device=dev, dtype=torch.float32)
-        kb, ug = torch.empty_like(qh), torch.empty_like(qh)
-        ops.delta_operands(qh, kb, ug, conv[:, : G * dk], conv[:, G * dk: 2 * G * dk], proj[:, b0:a0], decay, H, G, dk, self.spec.key_eps,
-                           dk ** -0.5)
         y = torch.empty((T, H * dv), device=dev, dtype=torch.float32)
-        ops.channel_scan(y, qh, kb, conv[:, 2 * G * dk:], decay, kb, ug, 1.0, scan_state, ctx, H, dk, dv)
+        q, k, v = conv[:, : G * dk], conv[:, G * dk: 2 * G * dk], conv[:, 2 * G * dk:]
+        # portions: four tokens at a time (the 32-bit path keeps one order of sums for every cut)
+        if not (self.rt.dtype == torch.bfloat16 and ctx.max_q_len >= 4
+                and ops.channel_delta(y, q, k, v, proj[:, b0:a0], decay, scan_state, ctx, H, G, dk, dv, self.spec.key_eps, dk ** -0.5)):
+            qh = torch.empty((T, H * dk), device=dev, dtype=torch.float32)
+            kb, ug = torch.empty_like(qh), torch.empty_like(qh)
+            ops.delta_operands(qh, kb, ug, q, k, proj[:, b0:a0], decay, H, G, dk, self.spec.key_eps, dk ** -0.5)
+            ops.channel_scan(y, qh, kb, v, decay, kb, ug, 1.0, scan_state, ctx, H, dk, dv)
         ops.head_norm_gate(out, y, gate, self.norm, H, self.spec.eps, ops.HEAD_GATE_SIGMOID, factor)
 
 
