@@ -138,8 +138,10 @@ def latent_attention_case(seg_lens, ctx_len, peaks, page=16, window=0, gated=Tru
     wuv = torch.randn(H * dv, rank, device="cuda", dtype=torch.bfloat16) * 0.05
     wuk_t = wuk.view(H, dn, rank).transpose(1, 2).contiguous()
     out = torch.empty(T, H * dv, device="cuda", dtype=torch.bfloat16)
+    up = torch.cat([wuk, wuv])
+    kv_up = None if sinks else (ops.pack_weight(up), up.shape[0])
     us = kb.timed_chain(lambda i: ops.latent_attention(out, q, gate, caches[i % copies], wuk, wuv, ctx, table, H, dn, dr, dv, rank, page, window,
-                                                       ATTN["scale"], wuk_t=wuk_t, **more), launches=8)
+                                                       ATTN["scale"], wuk_t=wuk_t, kv_up=kv_up, **more), launches=8)
     seen = lambda pos: min(pos + 1, window) if window else pos + 1                      # keys a query at `pos` sees
     pairs = sum(seen(ctx_len - n + i) for n in seg_lens for i in range(n))              # (query, key) pairs per head
     flops = H * pairs * (2.0 * (rank + dr) + 2.0 * rank) + T * H * 2.0 * rank * (dn + dv)
@@ -186,7 +188,7 @@ def experts_case(T, peaks, identity=0, groups=None) -> dict:
     R = T * top
     top_idx = torch.empty(T, top, device="cuda", dtype=torch.int32)
     top_w = torch.empty(T, top, device="cuda", dtype=torch.float32)
-    tile_rows = ops.moe_tile_rows(True)
+    tile_rows = ops.moe_tile_rows(True, T, R, E)
     ints = torch.empty(3 * R + 3 * ops.moe_max_tiles(R, E, tile_rows), device="cuda", dtype=torch.int32)
     row_token, slot_row, scratch, tiles = ints[:R], ints[R:2 * R], ints[2 * R:3 * R], ints[3 * R:]
     act = torch.empty(R, ff, device="cuda", dtype=torch.bfloat16)
@@ -202,8 +204,8 @@ def experts_case(T, peaks, identity=0, groups=None) -> dict:
     def run(i):
         ops.moe_route(top_idx, top_w, None, x, router, None, correction=corr, w_scale=2.5, **route)
         ops.moe_group(row_token, slot_row, tiles, top_idx, scratch, E, tile_rows)
-        ops.moe_experts_tc(True, act, x, wg[i % copies], wu[i % copies], row_token, tiles, **glu)
-        ops.moe_experts_tc(False, y, act, wd[i % copies], None, row_token, tiles)
+        ops.moe_experts_tc(True, act, x, wg[i % copies], wu[i % copies], row_token, tiles, tile_rows=tile_rows, **glu)
+        ops.moe_experts_tc(False, y, act, wd[i % copies], None, row_token, tiles, tile_rows=tile_rows)
         ops.moe_combine(delta, None, y, slot_row, top_w, None, None, identity_in=x if identity else None)
 
     us = kb.timed_chain(run, launches=6)
@@ -294,7 +296,7 @@ def table_experts_case(T, peaks) -> dict:
     R = T * top
     top_idx = torch.empty(T, top, device="cuda", dtype=torch.int32)
     top_w = torch.empty(T, top, device="cuda", dtype=torch.float32)
-    tile_rows = ops.moe_tile_rows(True)
+    tile_rows = ops.moe_tile_rows(True, T, R, E)
     ints = torch.empty(3 * R + 3 * ops.moe_max_tiles(R, E, tile_rows), device="cuda", dtype=torch.int32)
     row_token, slot_row, scratch, tiles = ints[:R], ints[R:2 * R], ints[2 * R:3 * R], ints[3 * R:]
     act = torch.empty(R, ff, device="cuda", dtype=torch.bfloat16)
@@ -305,8 +307,8 @@ def table_experts_case(T, peaks) -> dict:
     def run(i):
         ops.moe_route_table(top_idx, top_w, table, ids, E)
         ops.moe_group(row_token, slot_row, tiles, top_idx, scratch, E, tile_rows)
-        ops.moe_experts_tc(2, act, x, wu[i % copies], None, row_token, tiles)
-        ops.moe_experts_tc(0, y, act, wd[i % copies], None, row_token, tiles)
+        ops.moe_experts_tc(2, act, x, wu[i % copies], None, row_token, tiles, tile_rows=tile_rows)
+        ops.moe_experts_tc(0, y, act, wd[i % copies], None, row_token, tiles, tile_rows=tile_rows)
         ops.moe_combine(delta, None, y, slot_row, top_w, None, None, ff_scale=scale)
 
     us = kb.timed_chain(run, launches=6)
