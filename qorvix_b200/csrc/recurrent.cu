@@ -446,11 +446,11 @@ __global__ void __launch_bounds__(SCAN_VT * SCAN_WARPS) linear_scan_reg_kernel(S
 // Products with S_0 are split over the key slices, so the slices' sums meet in shared memory.  Eight warps hold the state (first S^T q,
 // then the update), eight form W and W v (then the sums and the output); one of these, whose part of W is empty, works out the next chunk's
 // gates; the next chunk's
-// q, k, v arrive by cp.async (a bulk copy a row takes its issuing warp 50 clocks, three times what the chunk may take): a chunk is two stretches between CTA barriers.  n is kept like a value column of ones.
+// q, k, v arrive by cp.async (a bulk copy a row takes its issuing warp 50 clocks, three times what the chunk may take): a chunk is two stretches between CTA barriers.  n . q is formed like a value column's.
 // The tensor cores cut the sums' low bits off as they add; so long sums are taken in short runs that are added in float32, a term's small
 // parts apart from its large one, and the update apart from the state.
 // What bounds it: a chunk's chain of products and the two barriers (a prompt has only heads x tiles CTAs); mma.sync issues a product in
-// some 8 clocks a scheduler.  2,048 tokens of 4 heads of 256 x 512: 2,573 us token by token, 180 in chunks; portions of 777, 583 and
+// some 8 clocks a scheduler.  2,048 tokens of 4 heads of 256 x 512: 2,573 us token by token, 175 in chunks; portions of 777, 583 and
 // 583 tokens of 64 heads of 128 x 64: 897 and 130 us.
 #define LC_C 64
 __device__ __forceinline__ void lc_ldsm4(uint32_t* r, const void* p) {
@@ -494,7 +494,6 @@ __device__ __forceinline__ float lc_exp_sum(float2 x, float2 y) {
 struct LcGates {                           // what a chunk's gates amount to
   float2 G[LC_C], H[LC_C];                           // a number and what rounding it to float32 left over
   float b[LC_C], A[LC_C], c[LC_C], em[LC_C];         // em: exp(-m_t)
-  bf16 ct[3][LC_C];                                  // c in three terms
   float A_end, m_end, pad[2];
 };
 #define LC_GATE_WARP 9                     // of the eight that form W: its 16 x 32 tokens lie above the diagonal
@@ -507,7 +506,7 @@ template <int VT, int NK> struct LcShape {
   static constexpr int STAGE = 2 * LC_C * LDQ * 2;                                     // bytes: q and k of a chunk
   static constexpr int RED = (SLICES + 2) * LC_C * LDR * 4;                            // the slices' sums, and W v's two
   static constexpr int V = LC_C * LDV * 2;
-  static constexpr int BYTES = 2 * STAGE + RED + 5 * V + 2 * (int)sizeof(LcGates) + LC_C * 2 * 4 + SLICES * LC_C * 4 + 2 * LC_BATCH * 4;
+  static constexpr int BYTES = 2 * STAGE + RED + 5 * V + 2 * (int)sizeof(LcGates) + LC_C * 2 * 4 + SLICES * LC_C * 4 + 2 * LC_BATCH * 4 + 2 * DKP * 4;
 };
 
 #define LC_THREADS 512
@@ -525,6 +524,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
   float* nq = rowsum + LC_C * 2;                                     // [SLICES][64] the slices' shares of A_t n_0 . q_t
   float* lfb = nq + SLICES * LC_C;                                   // [LC_BATCH] log of the decay
   float* lib = lfb + LC_BATCH;                                       // [LC_BATCH] log of the input gate | step size
+  float* ns = lib + LC_BATCH;                                        // [2][DKP] n as two sums (GATED_MAX)
   pdl_wait();
   pdl_launch_dependents();
   const int s = blockIdx.x, h = blockIdx.y, tile = blockIdx.z;
@@ -632,10 +632,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
     }
     const double G_end = __shfl_sync(0xffffffffu, G[1], 31), m_end = __shfl_sync(0xffffffffu, m[1], 31);
     const float c0 = expf((float)(G_end + Hh[0])) * bb[0], c1 = expf((float)(G_end + Hh[1])) * bb[1];
-    uint32_t terms[3];
-    lc_split3(c0, c1, terms);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) *(uint32_t*)(gt.ct[x] + 2 * lane) = terms[x];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int t = 2 * lane + i;
@@ -654,8 +650,11 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
   work_logs(0);
   __syncthreads();
   if (warp == LC_GATE_WARP) work_gates(0);
-  const bool has_n = KIND == SCAN_GATED_MAX && half == 0;            // n is kept like one more value column, all ones
-  float nT[2 * NK][4] = {};
+  // n . q is formed like one more value column's; n itself is summed by the warps of W, which have time for it (as a product of 16 rows of
+  // which one counts it was half as many again as the state's own in half of these warps: 195 us where this takes 175)
+  const bool has_n = KIND == SCAN_GATED_MAX && half == 0;
+  if (KIND == SCAN_GATED_MAX)
+    for (int i = tid; i < 2 * DKP; i += LC_THREADS) ns[i] = i < dk ? st[dk * VT + i] : 0.f;
   float sT[2 * NK][4];                               // S^T: value columns half + g8 (+ 8), key rows k0 + 8 nt + 2 t4 (+ 1)
   if (warp < 8) {
 #pragma unroll
@@ -664,7 +663,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
       for (int i = 0; i < 4; ++i) {
         const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = half + g8 + (i >> 1) * 8;
         sT[nt][i] = k < dk ? st[k * VT + col] : 0.f;
-        if (has_n && g8 == 0 && i < 2 && k < dk) nT[nt][i] = st[dk * VT + k];
       }
   }
 
@@ -699,8 +697,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
       if (has_n) {
 #pragma unroll
         for (int kk = 0; kk < NK; ++kk) {
-          lc_split3(nT[2 * kk][0], nT[2 * kk][1], n0[kk]);
-          lc_split3(nT[2 * kk + 1][0], nT[2 * kk + 1][1], n1[kk]);
+          const float* np = ns + k0 + kk * 16 + 2 * t4;
+          lc_split3(g8 ? 0.f : np[0] + np[DKP], g8 ? 0.f : np[1] + np[DKP + 1], n0[kk]);
+          lc_split3(g8 ? 0.f : np[8] + np[DKP + 8], g8 ? 0.f : np[9] + np[DKP + 9], n1[kk]);
         }
       }
 #pragma unroll
@@ -814,7 +813,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
     }
     __syncthreads();                                 // the terms of c v and all sums are in place
     if (warp < 8) {
-      float up[2 * NK][4] = {}, lo[2 * NK][4] = {}, nu[2 * NK][4] = {};
+      float up[2 * NK][4] = {}, lo[2 * NK][4] = {};
 #pragma unroll
       for (int kk = 0; kk < LC_C; kk += 16) {
         uint32_t af[3][4];
@@ -829,15 +828,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
             lc_mma(x ? lo[2 * nb] : up[2 * nb], af[x], bk[0], bk[1]);
             lc_mma(x ? lo[2 * nb + 1] : up[2 * nb + 1], af[x], bk[2], bk[3]);
           }
-          if (has_n) {
-#pragma unroll
-            for (int x = 2; x >= 0; --x) {           // row 0: c
-              const uint32_t ca[4] = {g8 == 0 ? *(const uint32_t*)(gt.ct[x] + kk + 2 * t4) : 0u, 0u,
-                                      g8 == 0 ? *(const uint32_t*)(gt.ct[x] + kk + 8 + 2 * t4) : 0u, 0u};
-              lc_mma(nu[2 * nb], ca, bk[0], bk[1]);
-              lc_mma(nu[2 * nb + 1], ca, bk[2], bk[3]);
-            }
-          }
         }
       }
       const float ae = gt.A_end;
@@ -846,9 +836,26 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           sT[nt][x] = fmaf(ae, sT[nt][x], up[nt][x] + lo[nt][x]);
-          if (has_n) nT[nt][x] = fmaf(ae, nT[nt][x], nu[nt][x]);
         }
     } else {
+      if (KIND == SCAN_GATED_MAX && ((tid - 256) & 127) * 2 < DKP) {         // n: two key rows and half the tokens a thread
+        const int kr = ((tid - 256) & 127) * 2, jb = (tid - 256) >> 7 ? 32 : 0;
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 c4 = *(const float4*)(gt.c + jb + j);
+          const float cc[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const __nv_bfloat162 kv = *(const __nv_bfloat162*)(ks + (jb + j + u) * LDQ + kr);
+            a0 = fmaf(cc[u], __low2float(kv), a0);
+            a1 = fmaf(cc[u], __high2float(kv), a1);
+          }
+        }
+        float* np = ns + (jb ? DKP : 0) + kr;
+        np[0] = fmaf(gt.A_end, np[0], a0);
+        np[1] = fmaf(gt.A_end, np[1], a1);
+      }
       for (int i = tid - 256; i < LC_C * VT / 4; i += 256) {
         const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
         if (c * LC_C + t >= len || tile * VT + cc >= dv) continue;
@@ -883,10 +890,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
       for (int i = 0; i < 4; ++i) {
         const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = half + g8 + (i >> 1) * 8;
         if (k < dk) st[k * VT + col] = sT[nt][i];
-        if (has_n && g8 == 0 && i < 2 && k < dk) st[dk * VT + k] = nT[nt][i];
       }
   }
-  if (KIND == SCAN_GATED_MAX && tid == 0) st[dk * VT + dk] = gates[(nchunks - 1) & 1].m_end;
+  if (KIND == SCAN_GATED_MAX) {
+    __syncthreads();                                 // n is whole
+    for (int i = tid; i < dk; i += LC_THREADS) st[dk * VT + i] = ns[i] + ns[DKP + i];
+    if (tid == 0) st[dk * VT + dk] = gates[(nchunks - 1) & 1].m_end;
+  }
 }
 
 template <int KIND, int VT, int NK>
