@@ -5,6 +5,7 @@ library kernel; a missing or unbuildable library raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -585,13 +586,22 @@ def diff_attention_splits(tokens: int, H: int, G: int, window: int, max_ctx: int
     return max(1, min(sm_count() // max(tokens * G, 1), blocks // 2, 12))
 
 
-DIFF_ROWS_FROM = 64                        # portions of at least this many tokens take the tcgen05 kernel
+DIFF_ROWS_FROM = 64                        # steps with a portion of at least this many tokens may take the tcgen05 kernel
+# and do from this much work on, (query, key) pairs x heads.  Below, either kernel ends before the host has launched the layer (58 us), and
+# two launches cost more of it than one (63).  16 heads over 400 tokens (1.3 M): 76 us a layer and 62; 8 heads over 200 tokens behind 800
+# in a window of 512 (0.8 M): 64 and 62; 8 heads over 400 tokens (0.6 M): 60 and 63.
+DIFF_ROWS_WORK = 3 << 18
 DIFF_ROWS_BYTES = 1 << 30                  # the most that both maps' float32 rows may take
+
+
+def _pairs(ctx, from_tokens: int, window: int) -> int:
+    """(query, key) pairs of the step's segments of at least `from_tokens` tokens (the keys of a segment's middle token for all of them)."""
+    return sum(n * min(p + n // 2 + 1, window or p + n) for n, p in zip(ctx.seg_len, ctx.seg_start_pos) if n >= from_tokens)
 
 
 def diff_attention_rows(out, q, cache_layer, ctx, block_table, first: int, H, G, n, dv, page, window, scale, lam, eps, post) -> bool:
     """Differential attention of the step's segments from `first` on with every map as an attention of its own on the tcgen05 tensor cores
-    (weights in three bfloat16 terms, rows left in float32) and a pass that joins the maps.  For portions of DIFF_ROWS_FROM tokens and
+    (weights in three bfloat16 terms, rows left in float32) and a pass that joins the maps.  For a portion of DIFF_ROWS_FROM tokens or
     more, maps of 64 and values of 128; False, nothing written, otherwise."""
     lens = ctx.seg_len[first:]
     T = q.shape[0]
@@ -603,9 +613,10 @@ def diff_attention_rows(out, q, cache_layer, ctx, block_table, first: int, H, G,
     assert cache_layer.is_contiguous() and tuple(cache_layer.shape[1:]) == (page, G * (2 * n + dv))
     rows = torch.empty((T, 2 * H, dv), device=q.device, dtype=torch.float32)
     rc = _lib("attention_tc").qv_diff_attention_rows_tc(
-        _ptr(out), out.stride(0), _ptr(q), q.stride(0), T, _ptr(cache_layer), cache_layer.shape[0] * page, _ptr(ctx.seg_q_start[first:]),
-        _ptr(ctx.seg_pos0[first:]), _ptr(block_table[first:]), block_table.shape[-1], len(lens), sum(lens), max(lens), H, G, page, int(window),
-        float(scale), float(lam), float(eps), float(post), _ptr(rows), _ptr(_tc_buffers(q.device)["err"]), _stream())
+        _ptr(out), out.stride(0), _ptr(q), q.stride(0), T, _ptr(cache_layer), cache_layer.shape[0] * page, _ptr(ctx.seg_q_start) + first * 4,
+        _ptr(ctx.seg_pos0) + first * 4, _ptr(block_table) + first * 4 * block_table.shape[-1], block_table.shape[-1], len(lens), sum(lens),
+        max(lens), H, G, page, int(window), float(scale), float(lam), float(eps), float(post), _ptr(rows),
+        _ptr(_tc_buffers(q.device)["err"]), _stream())
     if rc == -2:
         return False
     _check(rc, "diff_attention_rows")
@@ -627,7 +638,8 @@ def diff_attention(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, win
         if n1:
             splits = diff_attention_splits(n1, H, G, window, ctx.max_ctx_len)
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start, ctx.seg_pos0, block_table, n1, 1, *args, splits=splits)
-        if ok and n1 < S and not diff_attention_rows(out, q, cache_layer, ctx, block_table, n1, *args):
+        rows = ctx.max_q_len >= DIFF_ROWS_FROM and _pairs(ctx, DIFF_ROWS_FROM, window) * H >= DIFF_ROWS_WORK
+        if ok and n1 < S and not (rows and diff_attention_rows(out, q, cache_layer, ctx, block_table, n1, *args)):
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start[n1:], ctx.seg_pos0[n1:], block_table[n1:], S - n1,
                                    max(ctx.seg_len[n1:]), *args)
         if ok:
@@ -720,14 +732,19 @@ def latent_attention_tc(out, q, gate, cache_layer, wuk_t, wuv, ctx, block_table,
 
 LATENT_EXPAND_FROM = 32                    # segments of at least this many tokens form keys and values per head
 LATENT_EXPAND_BYTES = 1 << 30              # the most that their rows may take
+# and the least work that it is done for: (query, key) pairs x heads x entries they would multiply over the latents.  Below, the kernels over
+# the latents end before the host has launched the layer (69 us) and the three launches of this path take more of it (82): 16 heads of rank
+# 512, 128 tokens behind 300 (0.6 G): 98 us a layer and 83; 256 tokens (0.6 G): 101 and 81; 64 tokens behind 800 (0.9 G): 89 and 85; 8
+# heads of rank 256, 128 tokens behind 800 (0.5 G): 74 and 82, 512 tokens (0.6 G): 104 and 81.
+LATENT_EXPAND_WORK = 1 << 29
 
 
 def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale) -> int:
     """Latent attention of the step's portions with every head's keys and values formed once (kv_up: packed tiles and number of rows of
     [all heads' key matrices; all heads' value matrices], applied to the rows that the portions see) and flash attention on the tensor
-    cores over them.  A query then multiplies dn + dr + dv entries a key instead of 2 rank + dr; it pays for portions of
-    LATENT_EXPAND_FROM tokens and more.  Takes the segments from the first such one on; returns how many leading segments it left out (all
-    of them: nothing was done, where a size, a type or the room for the rows does not allow it)."""
+    cores over them.  A query then multiplies dn + dr + dv entries a key instead of 2 rank + dr.  Takes the segments from the first of
+    LATENT_EXPAND_FROM tokens on; returns how many leading segments it left out (all of them: nothing was done, where a size, a type or
+    the room for the rows does not allow it)."""
     S = ctx.num_segments
     lens, pos0 = getattr(ctx, "seg_len", None), getattr(ctx, "seg_start_pos", None)
     if (kv_up is None or q.dtype != torch.bfloat16 or not lens or not pos0 or getattr(ctx, "captured", False) or dn != 128 or dv != 128 or dr != 64
@@ -749,27 +766,32 @@ def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table
     _i32(block_table, "block_table")
     dev = q.device
     c = torch.empty((rows, rank), device=dev, dtype=torch.bfloat16)
-    kr = torch.empty((rows, dr), device=dev, dtype=torch.bfloat16)
     kv = torch.empty((rows, features), device=dev, dtype=torch.bfloat16)
-    where = torch.empty((2, S - first), device=dev, dtype=torch.int32)
-    starts, firsts, tables = ctx.seg_q_start[first:], ctx.seg_pos0[first:], block_table[first:]
+    room = torch.empty(rows * dr * 2 + (S - first) * 8, device=dev, dtype=torch.uint8)   # the rotated parts, then two lists of row numbers
+    kr = _ptr(room)
+    starts_row, firsts_row = kr + rows * dr * 2, kr + rows * dr * 2 + (S - first) * 4
+    skip = first * 4                                                                     # bytes of the left-out segments' entries (int32)
+    starts, firsts, tables = _ptr(ctx.seg_q_start) + skip, _ptr(ctx.seg_pos0) + skip, _ptr(block_table) + skip * block_table.shape[-1]
     _check(_lib("latent_attention").qv_latent_rows_out(
-        _ptr(c), _ptr(kr), _ptr(where[0]), _ptr(where[1]), _ptr(cache_layer), rank, dr, _ptr(starts), _ptr(firsts), _ptr(tables),
-        block_table.shape[-1], S - first, 1, page, window, rows, _stream()), "latent_rows_out")
+        _ptr(c), kr, starts_row, firsts_row, _ptr(cache_layer), rank, dr, starts, firsts, tables, block_table.shape[-1], S - first, 1, page,
+        window, rows, _stream()), "latent_rows_out")
     gemm(kv, c, None, packed, features)
     _check(_lib("attention_tc").qv_attn_rows_tc(
-        _ptr(out), out.stride(0), _ptr(q), q.stride(0), q.shape[0], _ptr(kv), kv.stride(0), H * dn, _ptr(kr), rows, _ptr(where[0]), _ptr(where[1]),
-        _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(starts), _ptr(firsts), S - first, max(lens[first:]), 1, H, window, scale,
+        _ptr(out), out.stride(0), _ptr(q), q.stride(0), q.shape[0], _ptr(kv), kv.stride(0), H * dn, kr, rows, starts_row, firsts_row,
+        _ptr(gate), gate.stride(0) if gate is not None else 0, starts, firsts, S - first, max(lens[first:]), 1, H, window, scale,
         _ptr(_tc_buffers(dev)["err"]), _stream()), "attn_rows_tc")
     return first
 
 
 def latent_attention(out, q, gate, cache_layer, wuk, wuv, ctx, block_table, H, dn, dr, dv, rank, page, window, scale, wuk_t=None, sink=None,
                      weight_terms: int = 1, kv_up=None) -> None:
-    """Latent attention of every token of the step.  bfloat16: portions form keys and values per head where the sizes allow it and kv_up is
-    given (see latent_attention_expanded; softmax weights of one term, no sinks), other segments take the tensor-core kernels over the
+    """Latent attention of every token of the step.  bfloat16: portions form keys and values per head where the sizes allow it, kv_up is
+    given and the work is worth it (see latent_attention_expanded; softmax weights of one term, no sinks), other segments take the tensor-core kernels over the
     latents themselves (with the transposed key matrices wuk_t [H, rank, dn]), else (and for float32) the CUDA-core kernel."""
-    if kv_up is not None and sink is None and weight_terms == 1:
+    entries = H * (2 * rank + dr)
+    if (kv_up is not None and sink is None and weight_terms == 1 and ctx.max_q_len >= LATENT_EXPAND_FROM and not ctx.captured
+            and ctx.num_tokens * ctx.max_ctx_len * entries >= LATENT_EXPAND_WORK
+            and _pairs(ctx, LATENT_EXPAND_FROM, window) * entries >= LATENT_EXPAND_WORK):
         left = latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale)
         if left == 0:
             return
@@ -1254,12 +1276,14 @@ def moe_route(top_idx, top_w, gate_out, h, w_router, w_gate, correction=None, w_
         add_launches(1)
 
 
+@functools.lru_cache(maxsize=256)           # of the sizes alone; a step asks for each of its layers
 def moe_tile_rows(tensor_cores: bool, tokens: int = 0, rows: int = 0, experts: int = 0) -> int:
     """Rows of a tile of grouped rows: what the tile table is made for (the two experts' kernels differ, and the tensor-core kernel
     takes the tiles that suit a step of `tokens` tokens with `rows` choices over `experts` experts, where these are given)."""
     return int(_lib("moe").qv_moe_tile_rows(1 if tensor_cores else 0, tokens, rows, experts))
 
 
+@functools.lru_cache(maxsize=256)
 def moe_max_tiles(rows: int, experts: int, tile_rows: int) -> int:
     return int(_lib("moe").qv_moe_max_tiles(rows, experts, tile_rows))
 
@@ -1287,10 +1311,12 @@ def moe_pack_experts(w: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0, tile_rows: int = 0) -> None:
+def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0, tile_rows: int = 0, room=None) -> None:
     """The experts' products on the tensor cores (bfloat16); up as for moe_experts.  p1, p2: matrices packed by moe_pack_experts; the sizes
-    follow from out [R, N] and a [., K]; the tile table was made for tiles of `tile_rows` rows (0: moe_tile_rows(True))."""
-    _need_cuda(out, a, p1, p2, row_token, tiles)
+    follow from out [R, N] and a [., K]; the tile table was made for tiles of `tile_rows` rows (0: moe_tile_rows(True)).  room: a tensor
+    of at least R * K * 2 bytes that up products of more than 32 tokens may write their rows in grouped order to (the down product's
+    output will do: it is written when they are done with)."""
+    _need_cuda(out, a, p1, p2, row_token, tiles, room)
     R, N = out.shape
     K = a.shape[1]
     E = p1.shape[0]
@@ -1300,10 +1326,11 @@ def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, li
     assert out.dtype == (torch.bfloat16 if up else torch.float32) and (up or a.shape[0] == R)
     tile_rows = tile_rows or moe_tile_rows(True)
     gathers = bool(up) and a.shape[0] > 32                     # the rows in grouped order, for the up products of longer steps
-    gathered = torch.empty((R, K), device=a.device, dtype=a.dtype) if gathers else None
+    if gathers and (room is None or not room.is_contiguous() or room.nbytes < R * K * 2):
+        room = torch.empty((R, K), device=a.device, dtype=a.dtype)
     rc = _lib("moe").qv_moe_experts_tc(int(up), _ptr(out), out.stride(0), _ptr(a), a.stride(0), a.shape[0], _ptr(p1), _ptr(p2),
                                        _ptr(row_token), _ptr(tiles), R, E, N, K, act, float(limit), float(slope), tile_rows,
-                                       _ptr(gathered), _ptr(_tc_buffers(a.device)["err"]), _stream())
+                                       _ptr(room) if gathers else None, _ptr(_tc_buffers(a.device)["err"]), _stream())
     _check(rc, "moe_experts_tc")
     if gathers:
         add_launches(1)

@@ -51,13 +51,14 @@ class RoutedFeedForward(FeedForward):
         ops.moe_route(top_idx, top_w, gate, x, self.router, self.shared_gate, **self.routing)
         tc = self.tensor_cores
         tile_rows = ops.moe_tile_rows(tc, T, R, s.experts)
-        ints = torch.empty(3 * R + 3 * ops.moe_max_tiles(R, s.experts, tile_rows), device=dev, dtype=torch.int32)
-        row_token, slot_row, scratch, tiles = ints[:R], ints[R: 2 * R], ints[2 * R: 3 * R], ints[3 * R:]
+        n_tiles = 3 * ops.moe_max_tiles(R, s.experts, tile_rows)
+        ints = torch.empty(3 * R + n_tiles, device=dev, dtype=torch.int32)
+        row_token, slot_row, scratch, tiles = ints.split_with_sizes((R, R, R, n_tiles))
         ops.moe_group(row_token, slot_row, tiles, top_idx, scratch, s.experts, tile_rows)
         act = torch.empty((R, s.expert_ff), device=dev, dtype=x.dtype)
         y = torch.empty((R, d), device=dev, dtype=torch.float32)
         if tc:
-            ops.moe_experts_tc(True, act, x, self.w_gate, self.w_up, row_token, tiles, tile_rows=tile_rows, **self.glu)
+            ops.moe_experts_tc(True, act, x, self.w_gate, self.w_up, row_token, tiles, tile_rows=tile_rows, room=y, **self.glu)
             ops.moe_experts_tc(False, y, act, self.w_down, None, row_token, tiles, tile_rows=tile_rows)
         else:
             ops.moe_experts(True, act, x, self.w_gate, self.w_up, row_token, tiles, **self.glu)
@@ -98,13 +99,14 @@ class TableRoutedFeedForward(FeedForward):
         ops.moe_route_table(top_idx, top_w, self.table, ctx.token_ids, s.experts)
         tc = self.tensor_cores
         tile_rows = ops.moe_tile_rows(tc, T, R, s.experts)
-        ints = torch.empty(3 * R + 3 * ops.moe_max_tiles(R, s.experts, tile_rows), device=dev, dtype=torch.int32)
-        row_token, slot_row, scratch, tiles = ints[:R], ints[R: 2 * R], ints[2 * R: 3 * R], ints[3 * R:]
+        n_tiles = 3 * ops.moe_max_tiles(R, s.experts, tile_rows)
+        ints = torch.empty(3 * R + n_tiles, device=dev, dtype=torch.int32)
+        row_token, slot_row, scratch, tiles = ints.split_with_sizes((R, R, R, n_tiles))
         ops.moe_group(row_token, slot_row, tiles, top_idx, scratch, s.experts, tile_rows)
         act = torch.empty((R, s.expert_ff), device=dev, dtype=x.dtype)
         y = torch.empty((R, d), device=dev, dtype=torch.float32)
         if tc:
-            ops.moe_experts_tc(2, act, x, self.w_up, None, row_token, tiles, tile_rows=tile_rows)
+            ops.moe_experts_tc(2, act, x, self.w_up, None, row_token, tiles, tile_rows=tile_rows, room=y)
             ops.moe_experts_tc(0, y, act, self.w_down, None, row_token, tiles, tile_rows=tile_rows)
         else:
             ops.moe_experts(2, act, x, self.w_up, None, row_token, tiles)

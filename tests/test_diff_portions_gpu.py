@@ -23,8 +23,8 @@ def run(lens, past, window, H, G, cache, table, q, lam, page=16):
     ctx = context(lens, past)
     out = torch.full((sum(lens), H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
     first = next(i for i, n in enumerate(lens) if n > 1)
-    assert ops.diff_attention_rows(out, q, cache, ctx, table, first, H, G, N, DV, page, window, 0.125, lam, 1e-5, 0.8)
     ops.diff_attention(out, q, cache, ctx, table, H, G, N, DV, page, window, 0.125, lam, 1e-5, 0.8)
+    assert ops.diff_attention_rows(out, q, cache, ctx, table, first, H, G, N, DV, page, window, 0.125, lam, 1e-5, 0.8)
     ops.check_kernel_errors()
     return out
 

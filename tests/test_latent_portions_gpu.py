@@ -39,12 +39,12 @@ def test_portions_against_float64(lens, past, window, gated, rank):
     up = torch.cat([wuk, wuv])
     out = torch.full((T, H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
     scale = (DN + DR) ** -0.5
-    left = ops.latent_attention_expanded(out, q, gate, cache, (ops.pack_weight(up), up.shape[0]), ctx, table, H, DN, DR, DV, rank, page, window, scale)
+    packed = (ops.pack_weight(up), up.shape[0])
+    ops.latent_attention(out, q, gate, cache, wuk, wuv, ctx, table, H, DN, DR, DV, rank, page, window, scale,
+                         wuk_t=wuk.view(H, DN, rank).transpose(1, 2).contiguous(), kv_up=packed)
+    left = ops.latent_attention_expanded(out, q, gate, cache, packed, ctx, table, H, DN, DR, DV, rank, page, window, scale)
     ops.check_kernel_errors()
     assert left == next(i for i, n in enumerate(lens) if n >= ops.LATENT_EXPAND_FROM)
-    ops.latent_attention(out, q, gate, cache, wuk, wuv, ctx, table, H, DN, DR, DV, rank, page, window, scale,
-                         wuk_t=wuk.view(H, DN, rank).transpose(1, 2).contiguous(), kv_up=(ops.pack_weight(up), up.shape[0]))
-    ops.check_kernel_errors()
     at = 0
     for s, (n, p) in enumerate(zip(lens, past)):
         rows = cache[table[s].long()].reshape(-1, rank + DR)[: p + n].double()
