@@ -70,6 +70,8 @@ struct AttnArgs {
   const int* row_key = nullptr;
   const bf16* gate = nullptr;
   int ld_gate = 0, v_col = 0, min_len = 0;           // segments of fewer than min_len tokens are left out
+  const bf16* cache = nullptr;                       // DIFF: the cache's rows, and how many there are
+  int cache_rows = 0;
 };
 
 // bar.sync over the `count` threads that name barrier `id`
@@ -80,7 +82,7 @@ __device__ __forceinline__ void named_barrier(int id, int count) {
 struct Item {
   const int* bt;                                     // the segment's row of the block table
   int h, kvh, q0, qlen, tile0, pos0;                 // tile0: first row of tile A in its segment (B: tile0 + 128)
-  int k_last, tile_begin;                            // the last key any row of the item sees; its first key tile
+  int k_first, k_last, tile_begin;                   // the first and the last key any row of the item sees; its first key tile
   int row0;                                          // (ROPE > 0) the row of key 0
   int n_a, n_b;                                      // key tiles of A and of B (0: no B; else n_a or n_a + 1)
 };
@@ -105,6 +107,7 @@ __device__ __forceinline__ bool item_at(const AttnArgs& a, int idx, Item& t) {
   const int last_a = t.pos0 + t.tile0 + (rows < QT ? rows : QT) - 1;
   int k_first = 0;
   if (a.window > 0) { const int f = t.pos0 + t.tile0 - a.window + 1; k_first = f > 0 ? f : 0; }
+  t.k_first = k_first;
   t.tile_begin = k_first / KT;
   t.n_a = last_a / KT - t.tile_begin + 1;
   t.n_b = 0;
@@ -140,7 +143,8 @@ struct Walk {
 // DIFF: one softmax map a "head" (a.H counts both maps of every head), queries and keys of 64 entries, values of HD that two maps share,
 // all three as columns of the cache's rows (map_kv: [rows of all pages][G (2 x 64 + HD)], boxes of 16 rows).  Weights enter P.V as three
 // bfloat16 terms that hold their 24 bits: the large one and the middle one over the thread's share of S, the small one in the room that
-// a second query tile's output would take.  All sixteen softmax warps work on the one tile, four threads a row (1,500 tokens behind 500, 16 heads, window 1,024: 106 us; with two
+// a second query tile's output would take.  Values of keys that nobody in the item sees enter as zeros: their rows may hold anything (what
+// an earlier owner of the page left behind), and a weight of zero would not keep an infinity or a NaN out of the sums.  All sixteen softmax warps work on the one tile, four threads a row (1,500 tokens behind 500, 16 heads, window 1,024: 106 us; with two
 // threads a row 160, the mma.sync kernel 184).  The normalised rows leave in float32, [tokens][a.H][HD], for diff_rows_kernel.
 template <int HD, bool PAIRED, int ROPE, bool DIFF>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -250,23 +254,53 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
       const int n = t.n_b > t.n_a ? t.n_b : t.n_a;
       for (int j = 0; j < n; ++j) {
         int key0 = (t.tile_begin + j) * KT + (lane & 7) * 16;
+        // DIFF, values: a block nobody sees is copied from behind the cache's last row (zeros); one that is seen in part is stored by
+        // the warp itself, zeros in place of the rows nobody sees
+        const bool zeros = DIFF && which && (key0 > t.k_last || key0 + 15 < t.k_first);
+        const uint32_t part = DIFF ? __ballot_sync(0xffffffffu, which && lane < 8 && !zeros && (key0 < t.k_first || key0 + 15 > t.k_last)) : 0u;
         if (key0 > last_block) key0 = last_block;              // keys nobody sees: any valid page will do
         const int pg = t.bt[key0 / a.page];                    // fetched before the wait: its latency is the wait's
-        const int my_row = DIFF ? pg * a.page + key0 % a.page : ((pg * 2 + which) * a.Hkv + t.kvh) * a.page + (key0 % a.page);
+        const int my_row = zeros ? a.cache_rows : DIFF ? pg * a.page + key0 % a.page : ((pg * 2 + which) * a.Hkv + t.kvh) * a.page + (key0 % a.page);
         const int col0 = !DIFF ? 0 : which ? a.Hkv * 128 + t.kvh * HD : t.kvh * 128 + (t.h & 1) * 64;
         const int halves = DIFF && which == 0 ? 1 : NH;
         const int bytes = which ? V_BYTES : K_BYTES;
         alive = mbar_wait(&empty[s], (lap & 1) ^ 1, a.err, 11);
         if (!alive) break;
-        if (leader) mbar_expect_tx(&full[s], bytes);
+        if (leader) {
+          if (DIFF && part) mbar_expect_more(&full[s], bytes - __popc(part) * 16 * HD * 2);
+          else mbar_expect_tx(&full[s], bytes);
+        }
 #pragma unroll
         for (int blk = 0; blk < KT / 16; ++blk) {
           const int row = __shfl_sync(0xffffffffu, my_row, blk);
-          if (leader) {
+          if (leader && !(DIFF && (part >> blk & 1))) {
 #pragma unroll
             for (int hf = 0; hf < NH; ++hf)
               if (hf < halves) tma_load_2d(ring + s * bytes + hf * HALF_BYTES + blk * 16 * 128, &map_kv, &full[s], col0 + hf * 64, row);
           }
+        }
+        if (DIFF && part) {
+          for (uint32_t left = part; left; left &= left - 1) {
+            const int blk = __ffs(left) - 1;
+            const int row = __shfl_sync(0xffffffffu, my_row, blk), first = (t.tile_begin + j) * KT + blk * 16;
+            constexpr int PIECES = HD / 8;                     // of 16 bytes a row, in the places where the copies' swizzle puts them
+            uint4 v[PIECES / 2];
+#pragma unroll
+            for (int i = 0; i < PIECES / 2; ++i) {
+              const int r = (lane + 32 * i) / PIECES, c = (lane + 32 * i) % PIECES;
+              v[i] = make_uint4(0u, 0u, 0u, 0u);
+              if (first + r >= t.k_first && first + r <= t.k_last)
+                v[i] = *(const uint4*)(a.cache + (size_t)(row + r) * (a.Hkv * (128 + HD)) + col0 + c * 8);
+            }
+#pragma unroll
+            for (int i = 0; i < PIECES / 2; ++i) {
+              const int r = (lane + 32 * i) / PIECES, c = (lane + 32 * i) % PIECES;
+              *(uint4*)(ring + s * bytes + (c >> 3) * HALF_BYTES + (blk * 16 + r) * 128 + (((c & 7) ^ (r & 7)) << 4)) = v[i];
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (leader) mbar_arrive(&full[s]);
         }
         __syncwarp();
         if (++s == stages) { s = 0; ++lap; }
@@ -773,6 +807,7 @@ extern "C" int qv_diff_attention_rows_tc(void* out, int ld_out, const void* q, i
   a.ld_out = 0; a.max_blocks = max_blocks; a.H = 2 * H; a.Hkv = G; a.page = page; a.window = window;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.segments = S; a.q_pairs = (int)q_tiles; a.items = (int)(2LL * H * S * q_tiles); a.paired = 0;
+  a.cache = (const bf16*)cache; a.cache_rows = (int)cache_rows;
   const int rc = launch<128, false, 0, true>(mq, mkv, mkv, a, (cudaStream_t)stream);
   if (rc) return rc;
   return qv_launch(diff_rows_kernel, dim3((unsigned)(((long long)tokens * H + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, (bf16*)out, ld_out,

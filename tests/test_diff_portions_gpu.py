@@ -76,3 +76,25 @@ def test_all_bits_of_the_weights_enter():
     q = (torch.randn((192, H * 2 * N), generator=g, device="cuda") * 0.05).to(torch.bfloat16)
     got, ref = run(lens, past, 0, H, G, cache, table, q, 0.7).double(), want(lens, past, 0, H, G, cache, table, q, 0.7)
     assert float((got - ref).norm() / ref.norm()) < 6e-3
+
+
+@pytest.mark.parametrize("lens,past,window", [([100], [37], 0), ([128], [0], 0), ([1, 200, 90], [20, 130, 900], 100), ([300], [1000], 64), ([70, 65], [3, 15], 1)])
+def test_rows_that_nobody_sees_may_hold_anything(lens, past, window):
+    """Rows behind a request's last token, and ahead of its first token's window, belong to whoever had the page before: infinities and NaN
+    there leave every output as it is."""
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    H, G = 4, 2
+    blocks = -(-max(a + b for a, b in zip(lens, past)) // 16) + 1
+    table = torch.randperm(len(lens) * blocks, generator=g, device="cuda").to(torch.int32).view(len(lens), blocks)
+    cache = torch.randn((len(lens) * blocks, 16, G * (2 * N + DV)), generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn((sum(lens), H * 2 * N), generator=g, device="cuda").to(torch.bfloat16)
+    clean = run(lens, past, window, H, G, cache, table, q, 0.3)
+    for s, (n, p) in enumerate(zip(lens, past)):
+        rows = cache[table[s].long()].reshape(blocks * 16, -1)
+        first = max(0, p + 1 - window) if window else 0
+        for part in (rows[p + n:], rows[:first]):
+            part[0::2] = float("inf")
+            part[1::2] = float("nan")
+        cache[table[s].long()] = rows.view(blocks, 16, -1)
+    assert bool(torch.isfinite(clean).all())
+    assert torch.equal(run(lens, past, window, H, G, cache, table, q, 0.3), clean)
