@@ -716,7 +716,8 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
 // ---------------------------------------------------------------- portions: the latents as rows, for keys and values formed per head
 // Copies the cached rows that the segments of at least min_len tokens see into c [rows][rank] and kr [rows][dr], a warp a row: segment s
 // from key row_key[s] (the window's first key, rounded down to a multiple of 128; 0 without a window) in rows row_off[s] .., padded with
-// rows of zeros to a multiple of 128.  The first block also writes row_off and row_key [S].
+// rows of zeros to a multiple of 128 (and ahead of the window: those pages may have another owner by now, and a weight of zero does not keep
+// an infinity out of a sum).  The first block also writes row_off and row_key [S].
 __device__ __forceinline__ int lt_first_key(int pos0, int window) { return window > 0 && pos0 + 1 > window ? (pos0 + 1 - window) & ~127 : 0; }
 __global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict__ c, uint4* __restrict__ kr, int* __restrict__ row_off,
                                                               int* __restrict__ row_key, const uint4* __restrict__ cache, int rank16, int dr16,
@@ -731,7 +732,7 @@ __global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict_
     for (int s = 0; s < S; ++s) {
       const int len = seg_q_start[s + 1] - seg_q_start[s], pos0 = seg_pos0[s], first = lt_first_key(pos0, window);
       const int n = len >= min_len ? pos0 + len - first : 0, padded = (n + 127) & ~127;
-      if (r >= off && r < off + padded) { seg = s; key = r - off < n ? first + r - off : -1; }
+      if (r >= off && r < off + padded) { seg = s; key = r - off < n && (window <= 0 || first + r - off > pos0 - window) ? first + r - off : -1; }
       if (r == 0 && lane == 0) { row_off[s] = off; row_key[s] = first; }
       off += padded;
     }

@@ -73,3 +73,30 @@ def test_what_stays_with_the_latents():
     assert ops.latent_attention_expanded(*args, ctx, table, H, DN, DR, DV, 64, 16, 0, 1.0) == 3           # short segments
     ctx.seg_len = [1, 5, 1 << 21]
     assert ops.latent_attention_expanded(*args, ctx, table, H, DN, DR, DV, 64, 16, 0, 1.0) == 3           # rows beyond the room for them
+
+
+@pytest.mark.parametrize("lens,past,window", [([40], [200], 0), ([140], [500], 100), ([64, 33], [130, 1000], 50), ([40], [300], 1)])
+def test_rows_that_nobody_sees_may_hold_anything(lens, past, window):
+    """Rows behind a request's last token, and ahead of its first token's window, belong to whoever had the page before."""
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    T, rank, ctx = sum(lens), 64, context(lens, past)
+    blocks = -(-ctx.max_ctx_len // 16) + 1
+    table = torch.randperm(len(lens) * blocks, generator=g, device="cuda").to(torch.int32).view(len(lens), blocks)
+    cache, q, up = rnd(len(lens) * blocks, 16, rank + DR), rnd(T, H * (DN + DR)), rnd(H * (DN + DV), rank).mul_(rank ** -0.5)
+    packed = (ops.pack_weight(up), up.shape[0])
+
+    def run():
+        out = torch.full((T, H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
+        assert ops.latent_attention_expanded(out, q, None, cache, packed, ctx, table, H, DN, DR, DV, rank, 16, window, (DN + DR) ** -0.5) == 0
+        ops.check_kernel_errors()
+        return out
+
+    clean = run()
+    for s, (n, p) in enumerate(zip(lens, past)):
+        rows = cache[table[s].long()].reshape(blocks * 16, -1)
+        for part in (rows[p + n:], rows[: max(0, p + 1 - window) if window else 0]):
+            part[0::2], part[1::2] = float("inf"), float("nan")
+        cache[table[s].long()] = rows.view(blocks, 16, -1)
+    assert bool(torch.isfinite(clean).all())
+    assert torch.equal(run(), clean)
