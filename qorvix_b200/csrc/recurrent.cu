@@ -509,6 +509,65 @@ template <int VT, int NK> struct LcShape {
   static constexpr int BYTES = 2 * STAGE + RED + 5 * V + 2 * (int)sizeof(LcGates) + LC_C * 2 * 4 + SLICES * LC_C * 4 + 2 * LC_BATCH * 4 + 2 * DKP * 4;
 };
 
+__device__ __forceinline__ bool lc_finite(float4 v) { return (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w)) <= 3.4028234e38f; }
+// The share of W v in token t's output at columns cc .. cc + 3, tokens behind t left out instead of weighted by zero: for chunks with an
+// infinite or NaN value, which may reach its own token's output and later ones but no earlier one (a weight of zero does not keep it out).
+template <int KIND, int DKP, int LDQ, int LDV>
+__device__ float4 lc_values_up_to(const bf16* qs, const bf16* vc, const LcGates& gt, int t, int cc) {
+  const bf16* ks = qs + LC_C * LDQ;
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = 0; j <= t; ++j) {
+    float dot = 0.f;
+    for (int i = 0; i < DKP; ++i) dot = fmaf(to_f(qs[t * LDQ + i]), to_f(ks[j * LDQ + i]), dot);
+    const float w = dot * (lc_exp_sum(gt.G[t], gt.H[j]) * (KIND == SCAN_DECAY ? gt.b[j] : 1.f));
+    const bf16* v = vc + j * LDV + cc;
+    y.x = fmaf(w, to_f(v[0]), y.x); y.y = fmaf(w, to_f(v[1]), y.y); y.z = fmaf(w, to_f(v[2]), y.z); y.w = fmaf(w, to_f(v[3]), y.w);
+  }
+  return y;
+}
+
+template <int LDR>
+__device__ __forceinline__ float4 lc_sums(float4 y, const float* red, int from, int to, int t, int cc) {
+#pragma unroll
+  for (int sl = from; sl < to; ++sl) {
+    const float4 z = *(const float4*)(red + ((size_t)sl * LC_C + t) * LDR + cc);
+    y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
+  }
+  return y;
+}
+// Four output columns of token t from their sums; v: the token's values there.
+template <int KIND, int VT, int SLICES>
+__device__ __forceinline__ float4 lc_output(float4 y, const float* rowsum, const float* nq, const bf16* v, const LcGates& gt, int t, float q_scale,
+                                            float b3) {
+  y.x *= q_scale; y.y *= q_scale; y.z *= q_scale; y.w *= q_scale;
+  if (KIND == SCAN_GATED_MAX) {
+    float dot = rowsum[2 * t] + rowsum[2 * t + 1];
+#pragma unroll
+    for (int sl = 0; sl < SLICES; ++sl) dot += nq[sl * LC_C + t];
+    dot *= q_scale;
+    const float den = fmaxf(fabsf(dot), gt.em[t]) + 1e-6f;
+    y.x /= den; y.y /= den; y.z /= den; y.w /= den;
+  } else {
+    y.x = fmaf(b3, to_f(v[0]), y.x); y.y = fmaf(b3, to_f(v[1]), y.y); y.z = fmaf(b3, to_f(v[2]), y.z); y.w = fmaf(b3, to_f(v[3]), y.w);
+  }
+  return y;
+}
+// A chunk's outputs where only the chunk's own values made them infinite or NaN, once more: tokens behind each left out.
+template <int KIND, int VT, int NK>
+__device__ __noinline__ void lc_write_again(float* out, int ld_out, int tokens, int cols, const float* red, const bf16* qs, const bf16* vc,
+                                            const LcGates& gt, const float* rowsum, const float* nq, float q_scale, float b3) {
+  typedef LcShape<VT, NK> Sh;
+  for (int i = threadIdx.x - 256; i < LC_C * VT / 4; i += 256) {
+    const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
+    if (t >= tokens || cc >= cols) continue;
+    const float4 past = lc_sums<Sh::LDR>(*(const float4*)(red + (size_t)t * Sh::LDR + cc), red, 1, Sh::SLICES, t, cc);
+    if (!lc_finite(past) || lc_finite(lc_sums<Sh::LDR>(past, red, Sh::SLICES, Sh::SLICES + 2, t, cc))) continue;
+    const float4 z = lc_values_up_to<KIND, Sh::DKP, Sh::LDQ, Sh::LDV>(qs, vc, gt, t, cc);
+    *(float4*)(out + (size_t)t * ld_out + cc) = lc_output<KIND, VT, Sh::SLICES>(
+        make_float4(past.x + z.x, past.y + z.y, past.z + z.z, past.w + z.w), rowsum, nq, vc + t * Sh::LDV + cc, gt, t, q_scale, b3);
+  }
+}
+
 #define LC_THREADS 512
 template <int KIND, int VT, int NK>
 __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanArgs a) {
@@ -610,9 +669,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
       const double up = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += up;
     }
+    const double sum_ahead = __shfl_up_sync(0xffffffffu, sum, 1);
     double F[2], Hh[2], G[2], m[2] = {0.0, 0.0};
     F[1] = sum;
-    F[0] = sum - lf[1];
+    F[0] = (lane ? sum_ahead : 0.0) + lf[0];         // (not sum - lf[1]: a token's gates say nothing about the token ahead of it)
     if (KIND == SCAN_GATED_MAX) {
       Hh[0] = li[0] - F[0]; Hh[1] = li[1] - F[1];
       double mx = fmax(Hh[0], Hh[1]);
@@ -856,29 +916,18 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
         np[0] = fmaf(gt.A_end, np[0], a0);
         np[1] = fmaf(gt.A_end, np[1], a1);
       }
+      bool finite = true;
       for (int i = tid - 256; i < LC_C * VT / 4; i += 256) {
         const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
         if (c * LC_C + t >= len || tile * VT + cc >= dv) continue;
-        float4 y = *(const float4*)(red + (size_t)t * LDR + cc);
-#pragma unroll
-        for (int sl = 1; sl < SLICES + 2; ++sl) {
-          const float4 z = *(const float4*)(red + ((size_t)sl * LC_C + t) * LDR + cc);
-          y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
-        }
-        y.x *= a.q_scale; y.y *= a.q_scale; y.z *= a.q_scale; y.w *= a.q_scale;
-        if (KIND == SCAN_GATED_MAX) {
-          float dot = rowsum[2 * t] + rowsum[2 * t + 1];
-#pragma unroll
-          for (int sl = 0; sl < SLICES; ++sl) dot += nq[sl * LC_C + t];
-          dot *= a.q_scale;
-          const float den = fmaxf(fabsf(dot), gt.em[t]) + 1e-6f;
-          y.x /= den; y.y /= den; y.z /= den; y.w /= den;
-        } else {
-          const bf16* vr = vc + t * LDV + cc;
-          y.x = fmaf(b3, to_f(vr[0]), y.x); y.y = fmaf(b3, to_f(vr[1]), y.y); y.z = fmaf(b3, to_f(vr[2]), y.z); y.w = fmaf(b3, to_f(vr[3]), y.w);
-        }
+        const float4 y = lc_output<KIND, VT, SLICES>(lc_sums<LDR>(*(const float4*)(red + (size_t)t * LDR + cc), red, 1, SLICES + 2, t, cc),
+                                                     rowsum, nq, vc + t * LDV + cc, gt, t, a.q_scale, b3);
         *(float4*)(a.out + (size_t)(q0 + c * LC_C + t) * a.ld_out + (size_t)h * dv + tile * VT + cc) = y;
+        finite = finite && lc_finite(y);
       }
+      if (!finite)                                   // (apart, and in a function, so that the loop above is free of it)
+        lc_write_again<KIND, VT, NK>(a.out + (size_t)(q0 + c * LC_C) * a.ld_out + (size_t)h * dv + tile * VT, a.ld_out, len - c * LC_C, dv - tile * VT, red,
+                                     qs, vc, gt, rowsum, nq, a.q_scale, b3);
     }
     // the logarithms of the batch that begins with chunk c + 2 (the present one's last gates were worked out ahead of the barrier)
     if ((c + 2) % (LC_BATCH / LC_C) == 0) work_logs((c + 2) * LC_C);

@@ -90,3 +90,43 @@ def test_chunks_against_float64(kind, dk, dv, H, qg, lens, shift):
     rel = (errors / norms).sqrt()
     # a float32 sum of some 64 to 256 products that cancel: a few 1e-7; the chunks may not be further off than token by token
     assert bool((rel[0] <= torch.maximum(1.2 * rel[1], torch.full((2,), 3e-7, dtype=F64))).all()), rel.tolist()
+
+
+@pytest.mark.parametrize("kind", [ops.SCAN_GATED_MAX, ops.SCAN_DECAY])
+@pytest.mark.parametrize("dk,dv,lens", [(64, 40, [63, 140]), (128, 64, [200]), (256, 16, [16, 129])])
+@pytest.mark.parametrize("what", ["value", "gate"])
+def test_what_is_not_finite_reaches_no_earlier_token(kind, dk, dv, lens, what):
+    """An infinite value (in one column), or a gate that is NaN, at one token a segment: the tokens ahead of it keep their outputs, and an
+    infinite value leaves the other columns of later tokens finite."""
+    g = torch.Generator(device="cuda").manual_seed(dk + dv)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, H = sum(lens), 2
+    q, k, v = (rnd(T, H * n).to(torch.bfloat16) for n in (dk, dk, dv))
+    g1, g2, p1, p2, p3 = rnd(T, H), rnd(T, H) + 2, rnd(H), rnd(H), rnd(H)
+    gated = kind == ops.SCAN_GATED_MAX
+
+    def run():
+        state = torch.zeros(len(lens), ops.linear_scan_state_floats(kind, H, dk, dv), device="cuda")
+        out = torch.full((T, H * dv), float("nan"), device="cuda")
+        ops.linear_scan(kind, out, q, k, v, g1, g2 if gated else None, p1, p2, None if gated else p3, 6.0, dk ** -0.5, state, context(lens), H, dk, dv)
+        return out
+
+    clean, at, spots = run(), 0, []
+    assert bool(torch.isfinite(clean).all())
+    for n in lens:
+        spots.append((at, at + 2 * (n // 4) + 1, at + n))      # an odd token inside a chunk
+        at += n
+    for _, t, _ in spots:
+        if what == "value":
+            v[t, 3] = float("inf")
+        else:
+            g1[t] = float("nan")
+    got = run()
+    for first, t, end in spots:
+        scale = clean[first:end].abs().max()
+        # chunks with such a value sum W v in another order: float32 sums of up to 64 products
+        assert bool(((got[first:t] - clean[first:t]).abs() <= 2e-5 * scale).all())
+        assert not bool(torch.isfinite(got[t, 3]))
+        if what == "value":
+            others = torch.arange(H * dv, device="cuda") != 3
+            assert bool(((got[first:end] - clean[first:end])[:, others].abs() <= 2e-5 * scale).all())
