@@ -734,9 +734,47 @@ LATENT_EXPAND_FROM = 32                    # segments of at least this many toke
 LATENT_EXPAND_BYTES = 1 << 30              # the most that their rows may take
 # and the least work that it is done for: (query, key) pairs x heads x entries they would multiply over the latents.  Below, the kernels over
 # the latents end before the host has launched the layer (69 us) and the three launches of this path take more of it (82): 16 heads of rank
-# 512, 128 tokens behind 300 (0.6 G): 98 us a layer and 83; 256 tokens (0.6 G): 101 and 81; 64 tokens behind 800 (0.9 G): 89 and 85; 8
+# 512, 128 tokens behind 300 (0.8 G): 98 us a layer and 83; 256 tokens (0.6 G): 101 and 81; 64 tokens behind 800 (0.9 G): 89 and 85; 8
 # heads of rank 256, 128 tokens behind 800 (0.5 G): 74 and 82, 512 tokens (0.6 G): 104 and 81.
 LATENT_EXPAND_WORK = 1 << 29
+
+
+def _latent_carried_us(lens, pos0, H: int, window: int, sms: int) -> float:
+    """About what the kernels over the latents take beside the layer's other work: tiles of 32 (token, head) rows walk over blocks of 64
+    keys, 6.6 us a block, cut into slices of keys where the tiles leave SMs idle; 19 us of merge and value matrices."""
+    if not lens:
+        return 0.0
+    tiles = sum(-(-n * H // 32) for n in lens)
+    seen = [min(p + n, window + n) if window > 0 else p + n for n, p in zip(lens, pos0)]
+    splits = max(1, min(sms // max(tiles, 1), -(-max(p + n for n, p in zip(lens, pos0)) // 64)))
+    total = sum(-(-n * H // 32) * min(p + n / 2, window or p + n) / 64 for n, p in zip(lens, pos0))
+    return 19.0 + 6.6 * max(-(-max(seen) // 64 // splits), total / sms)
+
+
+def _latent_expanded_us(lens, pos0, H: int, rank: int, features: int, window: int, sms: int) -> float:
+    """About what forming every head's keys and values takes (the product, and its rows on their way to memory) and the attention over
+    them: tiles of 128 queries walk over tiles of 128 keys, 2.1 us a tile, no slices of keys."""
+    rows, longest, total = 0, 0, 0.0
+    for n, p in zip(lens, pos0):
+        lo = (p + 1 - window) & ~127 if window > 0 and p + 1 > window else 0
+        rows += (p + n - lo + 127) & ~127
+        longest = max(longest, -(-min(p + n, window + 128 if window > 0 else p + n) // 128))
+        total += -(-n // 128) * H * (min(p + n / 2, window or p + n) / 128 + 0.5)
+    return 2.1 * max(longest, total / sms) + rows * features * (rank / 0.6e9 + 1 / 2.5e6)
+
+
+def latent_expand_pays(lens, pos0, H: int, rank: int, features: int, window: int, sms: int) -> bool:
+    """Whether the segments from the first of LATENT_EXPAND_FROM tokens on are faster with keys and values formed per head.  A few tokens
+    far into a request are not: the rows to form and the walk over them grow with the cached tokens, however few the new ones are, while the
+    kernels over the latents cut the keys over the SMs.  us a layer on the device over the latents and with keys and values formed,
+    16 heads of rank 512: 32 tokens behind 2,000 78 and 85, behind 8,000 140 and 216; 64 behind 2,000 115 and 90, behind 8,000 258 and
+    218; 128 behind 8,000 469 and 190.  8 heads of rank 256: 32 behind 8,000 88 and 175, 64 141 and 179, 128 256 and 142.  64 heads of
+    rank 512: 32 behind 2,000 176 and 151, behind 8,000 465 and 391."""
+    first = next((i for i, n in enumerate(lens) if n >= LATENT_EXPAND_FROM), len(lens))
+    if first == len(lens):
+        return False
+    apart = _latent_expanded_us(lens[first:], pos0[first:], H, rank, features, window, sms) + _latent_carried_us(lens[:first], pos0[:first], H, window, sms)
+    return apart < 0.9 * _latent_carried_us(lens, pos0, H, window, sms)
 
 
 def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale) -> int:
@@ -791,7 +829,8 @@ def latent_attention(out, q, gate, cache_layer, wuk, wuv, ctx, block_table, H, d
     entries = H * (2 * rank + dr)
     if (kv_up is not None and sink is None and weight_terms == 1 and ctx.max_q_len >= LATENT_EXPAND_FROM and not ctx.captured
             and ctx.num_tokens * ctx.max_ctx_len * entries >= LATENT_EXPAND_WORK
-            and _pairs(ctx, LATENT_EXPAND_FROM, window) * entries >= LATENT_EXPAND_WORK):
+            and _pairs(ctx, LATENT_EXPAND_FROM, window) * entries >= LATENT_EXPAND_WORK
+            and latent_expand_pays(ctx.seg_len, ctx.seg_start_pos, H, rank, H * (dn + dv), window, sm_count())):
         left = latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale)
         if left == 0:
             return

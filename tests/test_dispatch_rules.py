@@ -147,3 +147,18 @@ def test_pre_norm_block_hands_a_prepared_norm_input_only_to_parts_that_take_it(m
     ctx.next_norm = ForeignNorm()
     block(FoldingMixer(), FoldingFfn()).forward(residual, None, ctx, None)
     assert calls[-1] == ("ffn", "PreNormed", ctx.next_norm)
+
+
+def test_latent_portions_choose_by_what_either_path_costs():
+    """The faster path as measured (us a layer over the latents, with keys and values formed per head), 148 SMs."""
+    pays = lambda lens, pos0, H, rank: ops.latent_expand_pays(lens, pos0, H, rank, H * 256, 0, 148)
+    for H, rank, new, cached, carried, expanded in (
+            (16, 512, 32, 2000, 78, 85), (16, 512, 64, 2000, 115, 90), (16, 512, 128, 2000, 176, 85), (16, 512, 32, 8000, 140, 216),
+            (16, 512, 64, 8000, 258, 218), (16, 512, 128, 8000, 469, 190), (16, 512, 2048, 0, 1024, 147), (8, 256, 32, 8000, 88, 175),
+            (8, 256, 64, 8000, 141, 179), (8, 256, 128, 8000, 256, 142), (8, 256, 128, 2000, 112, 66), (64, 512, 32, 2000, 176, 151),
+            (64, 512, 32, 8000, 465, 391)):
+        assert pays([new], [cached], H, rank) == (expanded < carried), (H, rank, new, cached)
+    assert not pays([1, 31], [9, 9000], 16, 512)                                # no portion
+    assert not pays([1, 1, 32], [700, 900, 8000], 16, 512)                      # behind single tokens
+    assert pays([512, 8], [0, 8000], 16, 512)                                   # one CTA a tile over the latents: 900 us and 278
+    assert ops.latent_expand_pays([64], [8000], 8, 256, 2048, 500, 148)         # a window leaves few rows to form
