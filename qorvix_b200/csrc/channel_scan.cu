@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(128) channel_delta_operands_kernel(float* __re
                                                                     const float* __restrict__ q, int ld_q, const float* __restrict__ k, int ld_k,
                                                                     const float* __restrict__ b, int ld_b, const float* __restrict__ g, int ld_g,
                                                                     const int* __restrict__ tok_seg, const int* __restrict__ seg_q_start, int H,
-                                                                    int G, int n, float eps, float q_scale, int t_first) {
+                                                                    int G, int n, float eps, float q_scale, int t_base, int t_first) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = t_first + blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(128) channel_delta_operands_kernel(float* __re
   for (int i = 0; i < 6; ++i) kk[i] = warp_sum(kk[i]);
 #pragma unroll
   for (int i = 0; i < 10; ++i) qk[i] = warp_sum(qk[i]);
-  const size_t o = (size_t)t * H + h;
+  const size_t o = (size_t)(t - t_base) * H + h;
   for (int i = lane; i < n; i += 32) {
     float gv[CD_BLOCK], P[CD_BLOCK], suffix[CD_BLOCK];
 #pragma unroll
@@ -548,7 +548,8 @@ __global__ void __launch_bounds__(128) channel_delta_operands_kernel(float* __re
 
 struct ChannelDeltaArgs {
   float* out; int ld_out;                 // [T, H * dv]
-  const float* x; const float* pall; const float* coef;
+  const float* x; const float* pall; const float* coef;       // from token t_base on
+  int t_base;
   const float* v; int ld_v;
   float* state; long long slot_stride;    // as ChannelScanArgs
   const int* seg_q_start; const int* seg_slot;
@@ -584,7 +585,7 @@ __global__ void __launch_bounds__(32 * (4 / C + 2)) channel_delta_blocks_kernel(
     for (int tk = warp - W; tk < NB * CD_BLOCK; tk += 2) {
       const int j = ch * NB * CD_BLOCK + tk;
       const bool in = j < len;
-      const size_t row = (size_t)(q0 + (in ? j : 0)) * H + h;
+      const size_t row = (size_t)(q0 - a.t_base + (in ? j : 0)) * H + h;
       const float* src = a.x + row * 3 * dk;
       float* blk = base + (tk / CD_BLOCK) * BLK;
       float* dst = blk + (tk % CD_BLOCK) * ROW;
@@ -698,31 +699,47 @@ __global__ void __launch_bounds__(32 * (4 / C + 2)) channel_delta_blocks_kernel(
       for (int i = 0; i < CS_ROWS; ++i) st[c * CS_ROWS * 32 + i * 32] = S[c][i];
 }
 
-// Floats of workspace for T tokens: x, pall and coef in this order.
-extern "C" long long qv_channel_delta_workspace_floats(int T, int H, int dk) { return (long long)T * H * (4 * (long long)dk + 8); }
+// Floats of workspace: `lead` tokens token by token (operands of qv_channel_scan), `rest` tokens in blocks (x, pall and coef in this order).
+extern "C" long long qv_channel_delta_workspace_floats(int lead, int rest, int H, int dk) {
+  return ((long long)lead * 3 * dk + (long long)rest * (4 * (long long)dk + 8)) * H;
+}
 
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
-// beta, g [T, H * dk] the decays, v [T, H * dv].  dk a multiple of 4, at most 256.
+// beta, g [T, H * dk] the decays, v [T, H * dv].  The first S_lead segments (T_lead tokens, the longest of them max_lead) go token by token, the
+// others in blocks, for which dk is a multiple of 4, at most 256.
 extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                                 const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
-                                long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int H, int G,
-                                int dk, int dv, float* workspace, void* stream) {
+                                long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,
+                                int T_lead, int max_lead, int H, int G, int dk, int dv, float* workspace, void* stream) {
   if (S <= 0 || T <= 0) return 0;
-  if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || dk % 4 || ((uintptr_t)workspace & 15)) return QV_ERR_UNSUPPORTED;
+  if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || S_lead < 0 || S_lead > S || T_lead < 0 || T_lead > T) return QV_ERR_UNSUPPORTED;
+  if (S_lead < S && (dk % 4 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
   if (dk > 256) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
+  if (S_lead > 0) {
+    const size_t n = (size_t)T_lead * H * dk;
+    float *qh = workspace, *kb = qh + n, *ug = kb + n;
+    int rc = qv_delta_operands(qh, kb, ug, q, ld_q, k, ld_k, b, ld_b, g, ld_g, T_lead, H, G, dk, eps, q_scale, stream);
+    if (rc) return rc;
+    rc = qv_channel_scan(out, ld_out, qh, H * dk, kb, H * dk, v, ld_v, g, ld_g, kb, H * dk, ug, H * dk, 1.0f, state, slot_stride, seg_q_start,
+                         seg_slot, S_lead, max_lead, H, dk, dv, stream);
+    if (rc || S_lead == S) return rc;
+    workspace += 3 * n;
+  }
+  const size_t rest = (size_t)(T - T_lead) * H;
   ChannelDeltaArgs a;
   float* x = workspace;
-  float* pall = x + (size_t)T * H * 3 * dk;
-  float* coef = pall + (size_t)T * H * dk;
-  for (int done = 0; done < T; done += 65535) {
+  float* pall = x + rest * 3 * dk;
+  float* coef = pall + rest * dk;
+  for (int done = T_lead; done < T; done += 65535) {
     const int rows = T - done < 65535 ? T - done : 65535;
     const int rc = qv_launch(channel_delta_operands_kernel, dim3(rows, (H + 3) / 4), dim3(128), 0, st, x, pall, coef, q, ld_q, k, ld_k, b, ld_b, g,
-                             ld_g, tok_seg, seg_q_start, H, G, dk, eps, q_scale, done);
+                             ld_g, tok_seg, seg_q_start, H, G, dk, eps, q_scale, T_lead, done);
     if (rc) return rc;
   }
   a.out = out; a.ld_out = ld_out; a.x = x; a.pall = pall; a.coef = coef; a.v = v; a.ld_v = ld_v; a.state = state; a.slot_stride = slot_stride;
-  a.seg_q_start = seg_q_start; a.seg_slot = seg_slot; a.H = H; a.dk = dk; a.dv = dv;
+  a.seg_q_start = seg_q_start + S_lead; a.seg_slot = seg_slot + S_lead; a.H = H; a.dk = dk; a.dv = dv;
+  a.t_base = T_lead;
   const int lpc = cs_lanes_per_column(dk);
   const int cta_cols = 4 * 32 / lpc;
   const int ctas = (dv + cta_cols - 1) / cta_cols;
@@ -731,7 +748,7 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
   do {                                                                                                                           \
     constexpr int smem = 2 * NB * (CD_BLOCK * (3 * CS_PAD * LPC + 8 + 4 * 32 / LPC) + CS_PAD * LPC) * 4;                         \
     cudaFuncSetAttribute(channel_delta_blocks_kernel<LPC, NB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB, 2>, dim3(S, H, ctas), dim3(128), (size_t)smem, st, a);           \
+    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB, 2>, dim3(S - S_lead, H, ctas), dim3(128), (size_t)smem, st, a);           \
   } while (0)
   if (lpc == 1) CD_LAUNCH(1, 4);
   if (lpc == 2) CD_LAUNCH(2, 4);

@@ -167,16 +167,9 @@ class ChannelDelta(SharedIOMixer):
         ops.channel_gates(gate, proj[:, g0: g0 + self.spec.gate_rank], self.g_up, None, False, ops.GATE_LINEAR, 0.0)
         y = torch.empty((T, H * dv), device=dev, dtype=torch.float32)
         q, k, v = conv[:, : G * dk], conv[:, G * dk: 2 * G * dk], conv[:, 2 * G * dk:]
-        # portions: four tokens at a time (the 32-bit path keeps one order of sums for every cut).  Keys of up to 64 entries have half the
-        # work a token and the same chain a block: token by token is the faster scan there (8 heads, two portions of 345 and fewer tokens:
-        # 167 us a layer and 177), and only short portions, which end before the host has launched the layer, gain by the launch
-        # less (200 tokens: 161 and 147)
-        if not (self.rt.dtype == torch.bfloat16 and ctx.max_q_len >= 4 and (dk > 64 or ctx.max_q_len <= 256)
-                and ops.channel_delta(y, q, k, v, proj[:, b0:a0], decay, scan_state, ctx, H, G, dk, dv, self.spec.key_eps, dk ** -0.5)):
-            qh = torch.empty((T, H * dk), device=dev, dtype=torch.float32)
-            kb, ug = torch.empty_like(qh), torch.empty_like(qh)
-            ops.delta_operands(qh, kb, ug, q, k, proj[:, b0:a0], decay, H, G, dk, self.spec.key_eps, dk ** -0.5)
-            ops.channel_scan(y, qh, kb, v, decay, kb, ug, 1.0, scan_state, ctx, H, dk, dv)
+        # (the 32-bit path keeps one order of sums for every cut: token by token)
+        ops.channel_delta(y, q, k, v, proj[:, b0:a0], decay, scan_state, ctx, H, G, dk, dv, self.spec.key_eps, dk ** -0.5,
+                          blocks=self.rt.dtype == torch.bfloat16)
         ops.head_norm_gate(out, y, gate, self.norm, H, self.spec.eps, ops.HEAD_GATE_SIGMOID, factor)
 
 

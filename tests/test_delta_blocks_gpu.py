@@ -75,3 +75,32 @@ def test_blocks_against_float64(dk, dv, H, G, lens, rate):
     rel = (err / norm).sqrt()
     # sums of up to 256 float32 products: some 1e-7; four tokens at a time may not be further off than one at a time
     assert bool((rel[0] <= torch.maximum(1.2 * rel[1], torch.full((2,), 2.5e-7, dtype=torch.float64))).all()), rel.tolist()
+
+
+@pytest.mark.parametrize("dk,dv,lens", [(128, 40, [1, 1, 3, 40, 2]), (68, 24, [15, 16]), (256, 24, [1, 70]), (64, 24, [1, 40]), (128, 128, [1, 15, 2])])
+def test_short_segments_ahead_keep_their_kernel(dk, dv, lens):
+    """Segments ahead of the first portion are the token-by-token kernel's, bit for bit; the portions behind them agree to rounding."""
+    g = torch.Generator(device="cuda").manual_seed(dk + dv)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    H, G, T, ctx = 2, 1, sum(lens), context(lens)
+    q, k, v, b = rnd(T, G * dk), rnd(T, G * dk), rnd(T, H * dv), rnd(T, H)
+    decay = torch.exp(-torch.rand((T, H * dk), generator=g, device="cuda"))
+    start = rnd(len(lens), ops.channel_scan_state_floats(H, dk, dv)) * 0.1
+    results = []
+    for blocks in (True, False):
+        state, out = start.clone(), torch.full((T, H * dv), float("nan"), device="cuda")
+        assert ops.channel_delta(out, q, k, v, b, decay, state, ctx, H, G, dk, dv, 1e-6, dk ** -0.5, blocks=blocks)
+        results.append((out, state))
+    (out, state), (ref, ref_state) = results
+    lead = ops.delta_lead(lens, dk)
+    n = sum(lens[:lead])
+    slots = ctx.seg_slot.long()
+    assert torch.equal(out[:n], ref[:n]) and torch.equal(state[slots[:lead]], ref_state[slots[:lead]])
+    # float32 sums of up to 256 products in two orders, some 1e-7 each
+    assert float((out - ref).norm() / ref.norm()) < 2e-6 and float((state - ref_state).norm() / ref_state.norm()) < 2e-6
+    qh = torch.empty((T, H * dk), device="cuda")
+    kb, ug = torch.empty_like(qh), torch.empty_like(qh)
+    ops.delta_operands(qh, kb, ug, q, k, b, decay, H, G, dk, 1e-6, dk ** -0.5)
+    state, alone = start.clone(), torch.empty_like(ref)
+    ops.channel_scan(alone, qh, kb, v, decay, kb, ug, 1.0, state, ctx, H, dk, dv)
+    assert torch.equal(alone, ref) and torch.equal(state, ref_state)

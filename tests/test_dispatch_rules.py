@@ -162,3 +162,11 @@ def test_latent_portions_choose_by_what_either_path_costs():
     assert not pays([1, 1, 32], [700, 900, 8000], 16, 512)                      # behind single tokens
     assert pays([512, 8], [0, 8000], 16, 512)                                   # one CTA a tile over the latents: 900 us and 278
     assert ops.latent_expand_pays([64], [8000], 8, 256, 2048, 500, 148)         # a window leaves few rows to form
+
+
+def test_delta_rule_segments_that_go_token_by_token():
+    assert ops.delta_lead([1, 1, 1], 128) == 3 and ops.delta_lead([15], 128) == 1
+    assert ops.delta_lead([1, 1, 3, 16], 128) == 3                              # a portion does not take the single tokens with it
+    assert ops.delta_lead([300, 2], 128) == 0 and ops.delta_lead([1, 300, 2], 256) == 1
+    assert ops.delta_lead([1, 200], 64) == 2 and ops.delta_lead([200], 130) == 1  # short keys, keys that are no multiple of four
+    assert ops.delta_lead([200], 128, blocks=False) == 1 and ops.delta_lead([200], 260) == 1
