@@ -69,7 +69,8 @@ _ARGTYPES = {
     "qv_diff_attention_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _V, _V, _V],
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
-    "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V],
+    "qv_linear_scan_chunk_from": [],
+    "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_gated_group_norm": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _I, _V],
     "qv_moe_route": [_V, _V, _V, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _F, _I, _I, _I, _V],
     "qv_moe_max_tiles": [_I, _I, _I],
@@ -859,6 +860,19 @@ class _LeadingSegments:
 # ------------------------------------------------------------------ recurrent mixers
 
 SCAN_GATED_MAX, SCAN_DECAY = 0, 1
+SCAN_CHUNK_FROM = 16                       # segments of at least this many tokens go in chunks (bfloat16; qv_linear_scan_chunk_from)
+
+
+def _scan_rest(ctx):
+    """The step's leading segments of fewer than SCAN_CHUNK_FROM tokens; the longest and the shortest of the others."""
+    lens = getattr(ctx, "seg_len", None)
+    if ctx.max_q_len < SCAN_CHUNK_FROM or not lens:
+        return 0, ctx.max_q_len, 0
+    lead = 0
+    while lead < len(lens) and lens[lead] < SCAN_CHUNK_FROM:
+        lead += 1
+    rest = lens[lead:]
+    return lead, max(rest, default=0), min(rest, default=0)
 
 
 def conv_state(out, x, w, bias, tail, ctx, act: bool = True, add_input: bool = False) -> None:
@@ -897,8 +911,8 @@ def linear_scan(kind, out, q, k, v, g1, g2, p1, p2, p3, cap, q_scale, state, ctx
     rc = _lib("recurrent").qv_linear_scan(
         kind, _ptr(out), out.stride(0), _ptr(q), q.stride(0), q_group, _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(g1),
         g1.stride(0), _ptr(g2), g2.stride(0) if g2 is not None else 0, _ptr(p1), _ptr(p2), _ptr(p3), float(cap), float(q_scale),
-        _ptr(state), state.stride(0), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
-        min(getattr(ctx, "seg_len", None) or [0]), H, dk, dv, dt_code(q.dtype), _stream())
+        _ptr(state), state.stride(0), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, *_scan_rest(ctx),
+        H, dk, dv, dt_code(q.dtype), _stream())
     _check(rc, "linear_scan")
 
 

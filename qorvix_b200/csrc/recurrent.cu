@@ -965,12 +965,15 @@ extern "C" long long qv_linear_scan_state_floats(int kind, int H, int dk, int dv
   return (long long)H * ((dv + vt - 1) / vt) * scan_tile_floats(kind, dk, vt);
 }
 
-// max_q_len, min_q_len: the longest and the shortest segment (0: not known; a shortest segment that is not known costs a launch).
+// Segments from the first of SCAN_CHUNK_FROM tokens on take the chunks' kernel (those among them that are shorter leave it at once), so
+// that single tokens, which come first in a step, add no CTAs to it: lead, the segments ahead of it; rest_max, rest_min, the longest and the
+// shortest of the others (rest_min 0: not known; that costs a launch).
 #define SCAN_CHUNK_FROM 16
+extern "C" int qv_linear_scan_chunk_from(void) { return SCAN_CHUNK_FROM; }
 extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, int ld_q, int q_group, const void* k, int ld_k,
                               const void* v, int ld_v, const float* g1, int ld_g1, const float* g2, int ld_g2, const float* p1,
                               const float* p2, const float* p3, float cap, float q_scale, float* state, long long slot_stride,
-                              const int* seg_q_start, const int* seg_slot, int S, int max_q_len, int min_q_len, int H, int dk, int dv, int dt,
+                              const int* seg_q_start, const int* seg_slot, int S, int lead, int rest_max, int rest_min, int H, int dk, int dv, int dt,
                               void* stream) {
   if (S <= 0) return 0;
   if (kind != SCAN_GATED_MAX && kind != SCAN_DECAY) return QV_ERR_UNSUPPORTED;
@@ -988,17 +991,22 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
   cudaStream_t st = (cudaStream_t)stream;
   // Portions of SCAN_CHUNK_FROM tokens and more take the tensor cores, the step's other segments the token-by-token kernel: which kernel a
   // segment runs through depends on its own length alone.  bfloat16 only (the 32-bit path keeps one order of sums for every cut).
-  if (dt == QV_DT_BF16 && max_q_len >= SCAN_CHUNK_FROM && dk <= 256 && dk % 8 == 0 && dv % 8 == 0 && ld_q % 8 == 0 && ld_k % 8 == 0 &&
+  if (dt == QV_DT_BF16 && lead >= 0 && lead < S && rest_max >= SCAN_CHUNK_FROM && dk <= 256 && dk % 8 == 0 && dv % 8 == 0 && ld_q % 8 == 0 && ld_k % 8 == 0 &&
       ld_v % 8 == 0 && ld_out % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0) {
     a.chunk_from = SCAN_CHUNK_FROM;
+    ScanArgs rest = a;
+    rest.seg_q_start += lead;
+    rest.seg_slot += lead;
+    const dim3 rest_grid(S - lead, H, tiles);
     int rc;
     if (kind == SCAN_GATED_MAX)
-      rc = vt == 16 ? launch_scan_chunk<SCAN_GATED_MAX, 16, 2>(a, grid, st)
-                    : dk <= 64 ? launch_scan_chunk<SCAN_GATED_MAX, 32, 1>(a, grid, st) : launch_scan_chunk<SCAN_GATED_MAX, 32, 2>(a, grid, st);
+      rc = vt == 16 ? launch_scan_chunk<SCAN_GATED_MAX, 16, 2>(rest, rest_grid, st)
+                    : dk <= 64 ? launch_scan_chunk<SCAN_GATED_MAX, 32, 1>(rest, rest_grid, st) : launch_scan_chunk<SCAN_GATED_MAX, 32, 2>(rest, rest_grid, st);
     else
-      rc = vt == 16 ? launch_scan_chunk<SCAN_DECAY, 16, 2>(a, grid, st)
-                    : dk <= 64 ? launch_scan_chunk<SCAN_DECAY, 32, 1>(a, grid, st) : launch_scan_chunk<SCAN_DECAY, 32, 2>(a, grid, st);
-    if (rc || min_q_len >= SCAN_CHUNK_FROM) return rc;
+      rc = vt == 16 ? launch_scan_chunk<SCAN_DECAY, 16, 2>(rest, rest_grid, st)
+                    : dk <= 64 ? launch_scan_chunk<SCAN_DECAY, 32, 1>(rest, rest_grid, st) : launch_scan_chunk<SCAN_DECAY, 32, 2>(rest, rest_grid, st);
+    if (rest_min >= SCAN_CHUNK_FROM) grid.x = lead;          // none of them is left for the kernel below
+    if (rc || grid.x == 0) return rc;
   }
   if (dk <= 8 * 32) {                      // the state fits the registers
     const size_t esz = dt == QV_DT_F32 ? 4 : 2;

@@ -130,3 +130,38 @@ def test_what_is_not_finite_reaches_no_earlier_token(kind, dk, dv, lens, what):
         if what == "value":
             others = torch.arange(H * dv, device="cuda") != 3
             assert bool(((got[first:end] - clean[first:end])[:, others].abs() <= 2e-5 * scale).all())
+
+
+def test_the_length_from_which_segments_go_in_chunks():
+    assert ops._lib("recurrent").qv_linear_scan_chunk_from() == ops.SCAN_CHUNK_FROM
+    rest = lambda lens: ops._scan_rest(SimpleNamespace(seg_len=lens, max_q_len=max(lens)))
+    assert rest([1, 1, 15]) == (0, 15, 0) and rest([1, 1, 16]) == (2, 16, 16) and rest([1, 40, 3, 16]) == (1, 40, 3) and rest([16]) == (0, 16, 16)
+
+
+@pytest.mark.parametrize("kind", [ops.SCAN_GATED_MAX, ops.SCAN_DECAY])
+@pytest.mark.parametrize("lens", [[1, 1, 1, 40], [3, 15, 16], [1, 70, 2, 33], [64, 1]])
+def test_a_segment_does_not_depend_on_its_neighbours(kind, lens):
+    """Single tokens ahead of portions, short segments between and behind them: every segment's outputs and state are, bit for bit, those
+    of a step that holds it alone."""
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, H, dk, dv, S = sum(lens), 2, 64, 40, len(lens)
+    q, k, v = (rnd(T, H * n).to(torch.bfloat16) for n in (dk, dk, dv))
+    g1, g2, p1, p2, p3 = rnd(T, H), rnd(T, H) + 2, rnd(H), rnd(H), rnd(H)
+    gated = kind == ops.SCAN_GATED_MAX
+    start = rnd(S, ops.linear_scan_state_floats(kind, H, dk, dv)) * 0.1
+
+    def run(rows, state, ctx):
+        out = torch.full((rows.stop - rows.start, H * dv), float("nan"), device="cuda")
+        ops.linear_scan(kind, out, q[rows], k[rows], v[rows], g1[rows], g2[rows] if gated else None, p1, p2, None if gated else p3, 6.0, dk ** -0.5,
+                        state, ctx, H, dk, dv)
+        return out
+
+    state = start.clone()
+    whole, at = run(slice(0, T), state, context(lens)), 0
+    for s, n in enumerate(lens):
+        slot = S - 1 - s
+        one = start[slot: slot + 1].clone()
+        assert torch.equal(run(slice(at, at + n), one, context([n])), whole[at: at + n]), s
+        assert torch.equal(one[0], state[slot]), s
+        at += n
