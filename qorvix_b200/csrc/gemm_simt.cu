@@ -8,7 +8,8 @@
 // so a value does not depend on M, on the tile it falls in, or on anything else in the batch.
 //
 // Rows of both operands are staged as they lie (k contiguous, a row padded by 16 bytes so that 16-byte reads of
-// neighbouring rows miss one another's banks), STAGES - 1 tiles ahead by cp.async where the operands are float32 on 16 bytes, and
+// neighbouring rows miss one another's banks), STAGES - 1 tiles ahead by cp.async where the operands are float32 on 16 bytes, else (other
+// types, odd strides) through registers, all of a thread's elements of the next tile in flight under the present one's multiply-adds; and
 // a thread reads four k of a row at a time.  Two tile shapes: 16 x 32 (64 k, 2 x 2 outputs a thread) where 64 x 64 tiles would be few
 // or mostly padding, else 64 x 64 (32 k, 4 x 4 a thread).  Few CTAs are bound by the chain of K dependent multiply-adds and the
 // staging around it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (now 5 / 9 us, 3 rows x 192).
@@ -51,27 +52,49 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
         gs_cp16(dst + r * LD + (e % PIECES) * 4, live ? src : (const float*)W, live);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
-    } else {
-      for (int e = tid; e < ROWS * BK; e += THREADS) {
-        const int r = e / BK, k = k0 + e % BK;
-        float v = 0.f;
-        if (k < K) {
-          if (r < BM) { if (m0 + r < M) v = to_f(A[(size_t)(m0 + r) * lda + k]); }
-          else if (n0 + r - BM < N) v = to_f(W[(size_t)(n0 + r - BM) * ldw + k]);
-        }
-        dst[r * LD + e % BK] = v;
-      }
     }
   };
-  for (int t = 0; t < STAGES - 1; ++t) {
-    if (t < tiles) stage(t);
-    else if (ASYNC) asm volatile("cp.async.commit_group;" ::: "memory");
+  constexpr int PER_A = BM * BK / THREADS, PER_W = BN * BK / THREADS;
+  static_assert(BM * BK % THREADS == 0 && BN * BK % THREADS == 0, "every thread stages as many elements");
+  TA va[PER_A];
+  TW vw[PER_W];
+  auto fetch = [&](int t) {                        // tile t's elements, zeros beyond the matrices ...
+#pragma unroll
+    for (int i = 0; i < PER_A; ++i) {
+      const int e = tid + i * THREADS, r = m0 + e / BK, k = t * BK + e % BK;
+      va[i] = r < M && k < K ? A[(size_t)r * lda + k] : from_f<TA>(0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < PER_W; ++i) {
+      const int e = tid + i * THREADS, r = n0 + e / BK, k = t * BK + e % BK;
+      vw[i] = r < N && k < K ? W[(size_t)r * ldw + k] : from_f<TW>(0.f);
+    }
+  };
+  auto put = [&](int t) {                          // ... into its buffer
+    float* dst = ring[t % STAGES];
+#pragma unroll
+    for (int i = 0; i < PER_A; ++i) { const int e = tid + i * THREADS; dst[(e / BK) * LD + e % BK] = to_f(va[i]); }
+#pragma unroll
+    for (int i = 0; i < PER_W; ++i) { const int e = tid + i * THREADS; dst[(BM + e / BK) * LD + e % BK] = to_f(vw[i]); }
+  };
+  if (ASYNC) {
+    for (int t = 0; t < STAGES - 1; ++t) {
+      if (t < tiles) stage(t);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  } else if (tiles > 0) {
+    fetch(0);
+    put(0);
   }
   for (int t = 0; t < tiles; ++t) {
     if (ASYNC) asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();                               // tile t has landed; the buffer filled next was read a tile ago
-    if (t + STAGES - 1 < tiles) stage(t + STAGES - 1);
-    else if (ASYNC) asm volatile("cp.async.commit_group;" ::: "memory");
+    if (ASYNC) {
+      if (t + STAGES - 1 < tiles) stage(t + STAGES - 1);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    } else if (t + 1 < tiles) {
+      fetch(t + 1);
+    }
     const float* as = ring[t % STAGES] + ty * LD;
     const float* ws = ring[t % STAGES] + (BM + tx) * LD;
 #pragma unroll
@@ -91,6 +114,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
           acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
         }
     }
+    if (!ASYNC && t + 1 < tiles) put(t + 1);
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
