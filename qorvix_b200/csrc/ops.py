@@ -595,6 +595,15 @@ DIFF_ROWS_WORK = 3 << 18
 DIFF_ROWS_BYTES = 1 << 30                  # the most that both maps' float32 rows may take
 
 
+def diff_rows_first(lens) -> int:
+    """The first segment that the tcgen05 kernel takes, that of the first portion of DIFF_ROWS_FROM tokens; all of them left out where it and
+    those behind it would fill less than half of the kernel's tiles of 128 queries.  A short segment costs it a whole tile per map: eight
+    of 20 tokens behind 900 ahead of 600, 16 heads, took 173 us a layer with all of them there, 150 with none."""
+    first = next((i for i, n in enumerate(lens) if n >= DIFF_ROWS_FROM), len(lens))
+    rest = lens[first:]
+    return first if sum(-(-n // 128) for n in rest) * 64 <= sum(rest) else len(lens)
+
+
 def _pairs(ctx, from_tokens: int, window: int) -> int:
     """(query, key) pairs of the step's segments of at least `from_tokens` tokens (the keys of a segment's middle token for all of them)."""
     return sum(n * min(p + n // 2 + 1, window or p + n) for n, p in zip(ctx.seg_len, ctx.seg_start_pos) if n >= from_tokens)
@@ -639,10 +648,14 @@ def diff_attention(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, win
         if n1:
             splits = diff_attention_splits(n1, H, G, window, ctx.max_ctx_len)
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start, ctx.seg_pos0, block_table, n1, 1, *args, splits=splits)
-        rows = ctx.max_q_len >= DIFF_ROWS_FROM and _pairs(ctx, DIFF_ROWS_FROM, window) * H >= DIFF_ROWS_WORK
-        if ok and n1 < S and not (rows and diff_attention_rows(out, q, cache_layer, ctx, block_table, n1, *args)):
-            ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start[n1:], ctx.seg_pos0[n1:], block_table[n1:], S - n1,
-                                   max(ctx.seg_len[n1:]), *args)
+        end = S                                      # segments from here on: the tcgen05 kernel
+        if ctx.max_q_len >= DIFF_ROWS_FROM and _pairs(ctx, DIFF_ROWS_FROM, window) * H >= DIFF_ROWS_WORK:
+            end = diff_rows_first(ctx.seg_len)
+        if ok and end < S and not diff_attention_rows(out, q, cache_layer, ctx, block_table, end, *args):
+            end = S
+        if ok and n1 < end:
+            ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start[n1:], ctx.seg_pos0[n1:], block_table[n1:], end - n1,
+                                   max(ctx.seg_len[n1:end]), *args)
         if ok:
             return
     diff_attention_generic(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, window, scale, lam, eps, post)

@@ -98,3 +98,26 @@ def test_rows_that_nobody_sees_may_hold_anything(lens, past, window):
         cache[table[s].long()] = rows.view(blocks, 16, -1)
     assert bool(torch.isfinite(clean).all())
     assert torch.equal(run(lens, past, window, H, G, cache, table, q, 0.3), clean)
+
+
+@pytest.mark.parametrize("lens,past,window,first", [([1, 1, 200], [40, 700, 60], 64, 2), ([1, 20, 33, 130, 9], [5, 300, 0, 90, 40], 0, 3),
+                                                    ([20, 300], [900, 0], 100, 1), ([64, 3, 3, 3], [0, 9, 9, 9], 0, 4), ([40, 63], [0, 0], 0, 2)])
+def test_a_step_is_shared_by_the_kernels(monkeypatch, lens, past, window, first):
+    """One call over single tokens, short segments and portions: each kernel takes its segments, and no row is left out."""
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    H, G = 4, 2
+    blocks = -(-max(a + b for a, b in zip(lens, past)) // 16)
+    table = torch.randperm(len(lens) * blocks, generator=g, device="cuda").to(torch.int32).view(len(lens), blocks)
+    cache = torch.randn((len(lens) * blocks, 16, G * (2 * N + DV)), generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn((sum(lens), H * 2 * N), generator=g, device="cuda").to(torch.bfloat16)
+    taken = []
+    inner = ops.diff_attention_rows
+    monkeypatch.setattr(ops, "diff_attention_rows", lambda *a: taken.append(a[5]) or inner(*a))
+    monkeypatch.setattr(ops, "DIFF_ROWS_WORK", 0)
+    ctx = context(lens, past)
+    out = torch.full((sum(lens), H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.diff_attention(out, q, cache, ctx, table, H, G, N, DV, 16, window, 0.125, 0.3, 1e-5, 0.8)
+    ops.check_kernel_errors()
+    assert taken == ([first] if first < len(lens) else [])
+    ref = want(lens, past, window, H, G, cache, table, q, 0.3)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3

@@ -170,3 +170,9 @@ def test_delta_rule_segments_that_go_token_by_token():
     assert ops.delta_lead([300, 2], 128) == 0 and ops.delta_lead([1, 300, 2], 256) == 1
     assert ops.delta_lead([1, 200], 64) == 2 and ops.delta_lead([200], 130) == 1  # short keys, keys that are no multiple of four
     assert ops.delta_lead([200], 128, blocks=False) == 1 and ops.delta_lead([200], 260) == 1
+
+
+def test_differential_attention_segments_that_share_tiles_of_portions():
+    assert ops.diff_rows_first([1, 1, 600]) == 2 and ops.diff_rows_first([20] * 8 + [600]) == 8       # short segments ahead keep their kernel
+    assert ops.diff_rows_first([64]) == 0 and ops.diff_rows_first([63, 20]) == 2
+    assert ops.diff_rows_first([600, 3]) == 0 and ops.diff_rows_first([300] + [20] * 8) == 9          # behind: a tile each
