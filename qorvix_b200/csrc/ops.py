@@ -143,6 +143,14 @@ def _lib(name: str):
     return lib
 
 
+def _room(shape, dtype, device):
+    """Workspace of a path that another one can stand in for, or None where the device has no room left for it."""
+    try:
+        return torch.empty(shape, device=device, dtype=dtype)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
@@ -612,7 +620,7 @@ def _pairs(ctx, from_tokens: int, window: int) -> int:
 def diff_attention_rows(out, q, cache_layer, ctx, block_table, first: int, H, G, n, dv, page, window, scale, lam, eps, post) -> bool:
     """Differential attention of the step's segments from `first` on with every map as an attention of its own on the tcgen05 tensor cores
     (weights in three bfloat16 terms, rows left in float32) and a pass that joins the maps.  For a portion of DIFF_ROWS_FROM tokens or
-    more, maps of 64 and values of 128; False, nothing written, otherwise."""
+    more, maps of 64 and values of 128; False, nothing written, otherwise and where the device has no room for the rows."""
     lens = ctx.seg_len[first:]
     T = q.shape[0]
     if (n != 64 or dv != 128 or page % 16 or max(lens) < DIFF_ROWS_FROM or q.stride(0) % 8 or out.stride(0) % 4 or q.data_ptr() % 16
@@ -621,7 +629,9 @@ def diff_attention_rows(out, q, cache_layer, ctx, block_table, first: int, H, G,
     _need_cuda(out, q, cache_layer, block_table)
     assert q.stride(1) == 1 and out.stride(1) == 1 and out.dtype == cache_layer.dtype == torch.bfloat16
     assert cache_layer.is_contiguous() and tuple(cache_layer.shape[1:]) == (page, G * (2 * n + dv))
-    rows = torch.empty((T, 2 * H, dv), device=q.device, dtype=torch.float32)
+    rows = _room((T, 2 * H, dv), torch.float32, q.device)
+    if rows is None:
+        return False
     rc = _lib("attention_tc").qv_diff_attention_rows_tc(
         _ptr(out), out.stride(0), _ptr(q), q.stride(0), T, _ptr(cache_layer), cache_layer.shape[0] * page, _ptr(ctx.seg_q_start) + first * 4,
         _ptr(ctx.seg_pos0) + first * 4, _ptr(block_table) + first * 4 * block_table.shape[-1], block_table.shape[-1], len(lens), sum(lens),
@@ -796,7 +806,7 @@ def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table
     [all heads' key matrices; all heads' value matrices], applied to the rows that the portions see) and flash attention on the tensor
     cores over them.  A query then multiplies dn + dr + dv entries a key instead of 2 rank + dr.  Takes the segments from the first of
     LATENT_EXPAND_FROM tokens on; returns how many leading segments it left out (all of them: nothing was done, where a size, a type or
-    the room for the rows does not allow it)."""
+    the room for the rows does not allow it, by LATENT_EXPAND_BYTES or on the device)."""
     S = ctx.num_segments
     lens, pos0 = getattr(ctx, "seg_len", None), getattr(ctx, "seg_start_pos", None)
     if (kv_up is None or q.dtype != torch.bfloat16 or not lens or not pos0 or getattr(ctx, "captured", False) or dn != 128 or dv != 128 or dr != 64
@@ -817,9 +827,11 @@ def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table
     _need_cuda(out, q, gate, cache_layer, block_table)
     _i32(block_table, "block_table")
     dev = q.device
-    c = torch.empty((rows, rank), device=dev, dtype=torch.bfloat16)
-    kv = torch.empty((rows, features), device=dev, dtype=torch.bfloat16)
-    room = torch.empty(rows * dr * 2 + (S - first) * 8, device=dev, dtype=torch.uint8)   # the rotated parts, then two lists of row numbers
+    kv = _room((rows, features), torch.bfloat16, dev)
+    c = _room((rows, rank), torch.bfloat16, dev) if kv is not None else None
+    room = _room(rows * dr * 2 + (S - first) * 8, torch.uint8, dev) if c is not None else None   # the rotated parts, then two lists of row numbers
+    if room is None:
+        return S
     kr = _ptr(room)
     starts_row, firsts_row = kr + rows * dr * 2, kr + rows * dr * 2 + (S - first) * 4
     skip = first * 4                                                                     # bytes of the left-out segments' entries (int32)
@@ -1037,7 +1049,10 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lead = delta_lead(lens, dk, blocks)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
     lib = _lib("channel_scan")
-    ws = torch.empty(int(lib.qv_channel_delta_workspace_floats(tokens, T - tokens, H, dk)), device=q.device, dtype=torch.float32)
+    ws = _room(int(lib.qv_channel_delta_workspace_floats(tokens, T - tokens, H, dk)), torch.float32, q.device) if lead < S else None
+    if ws is None:                                    # token by token, which takes three quarters of the blocks' room
+        lead, tokens, longest = S, T, int(ctx.max_q_len)
+        ws = torch.empty(int(lib.qv_channel_delta_workspace_floats(T, 0, H, dk)), device=q.device, dtype=torch.float32)
     rc = lib.qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
                               _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0), _ptr(ctx.tok_seg),
                               _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, H, G, dk, dv, _ptr(ws), _stream())

@@ -104,3 +104,20 @@ def test_short_segments_ahead_keep_their_kernel(dk, dv, lens):
     state, alone = start.clone(), torch.empty_like(ref)
     ops.channel_scan(alone, qh, kb, v, decay, kb, ug, 1.0, state, ctx, H, dk, dv)
     assert torch.equal(alone, ref) and torch.equal(state, ref_state)
+
+
+def test_without_room_for_the_blocks(monkeypatch):
+    """No room for the blocks' operands on the device: token by token."""
+    lens, H, dk, dv = [1, 40], 2, 128, 40
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, ctx = sum(lens), context(lens)
+    q, k, v, b, decay = rnd(T, dk), rnd(T, dk), rnd(T, H * dv), rnd(T, H), torch.exp(-rnd(T, H * dk).abs())
+    results = []
+    for blocks in (False, True):
+        state, out = torch.zeros(2, ops.channel_scan_state_floats(H, dk, dv), device="cuda"), torch.empty((T, H * dv), device="cuda")
+        if blocks:
+            monkeypatch.setattr(ops, "_room", lambda *a: None)
+        ops.channel_delta(out, q, k, v, b, decay, state, ctx, H, 1, dk, dv, 1e-6, dk ** -0.5, blocks=blocks)
+        results.append((out, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])

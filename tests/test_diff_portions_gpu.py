@@ -121,3 +121,18 @@ def test_a_step_is_shared_by_the_kernels(monkeypatch, lens, past, window, first)
     assert taken == ([first] if first < len(lens) else [])
     ref = want(lens, past, window, H, G, cache, table, q, 0.3)
     assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3
+
+
+def test_without_room_for_the_rows(monkeypatch):
+    """No room for the float32 rows on the device: the kernel that needs none takes the portions too."""
+    lens, past, H, G = [1, 200], [40, 60], 4, 2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    table = torch.arange(2 * 17, dtype=torch.int32, device="cuda").view(2, 17)
+    cache = torch.randn((2 * 17, 16, G * (2 * N + DV)), generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn((sum(lens), H * 2 * N), generator=g, device="cuda").to(torch.bfloat16)
+    monkeypatch.setattr(ops, "DIFF_ROWS_WORK", 0)
+    monkeypatch.setattr(ops, "_room", lambda *a: None)
+    out = torch.full((sum(lens), H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.diff_attention(out, q, cache, context(lens, past), table, H, G, N, DV, 16, 0, 0.125, 0.3, 1e-5, 0.8)
+    ref = want(lens, past, 0, H, G, cache, table, q, 0.3)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3

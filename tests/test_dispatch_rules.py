@@ -176,3 +176,13 @@ def test_differential_attention_segments_that_share_tiles_of_portions():
     assert ops.diff_rows_first([1, 1, 600]) == 2 and ops.diff_rows_first([20] * 8 + [600]) == 8       # short segments ahead keep their kernel
     assert ops.diff_rows_first([64]) == 0 and ops.diff_rows_first([63, 20]) == 2
     assert ops.diff_rows_first([600, 3]) == 0 and ops.diff_rows_first([300] + [20] * 8) == 9          # behind: a tile each
+
+
+def test_no_room_is_an_answer(monkeypatch):
+    import torch
+    assert ops._room((2, 3), torch.float32, "cpu").shape == (2, 3)
+
+    def full(*a, **k):
+        raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(ops.torch, "empty", full)
+    assert ops._room((2, 3), torch.float32, "cpu") is None

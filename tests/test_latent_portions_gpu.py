@@ -100,3 +100,41 @@ def test_rows_that_nobody_sees_may_hold_anything(lens, past, window):
         cache[table[s].long()] = rows.view(blocks, 16, -1)
     assert bool(torch.isfinite(clean).all())
     assert torch.equal(run(), clean)
+
+
+def mixed(lens, past, rank=64, seed=1):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    ctx, T = context(lens, past), sum(lens)
+    blocks = -(-ctx.max_ctx_len // 16)
+    table = torch.randperm(len(lens) * blocks, generator=g, device="cuda").to(torch.int32).view(len(lens), blocks)
+    cache, q, gate = rnd(len(lens) * blocks, 16, rank + DR), rnd(T, H * (DN + DR)), rnd(T, H * DV)
+    wuk, wuv = rnd(H * DN, rank).mul_(rank ** -0.5), rnd(H * DV, rank).mul_(rank ** -0.5)
+    up = torch.cat([wuk, wuv])
+    args = (q, gate, cache, wuk, wuv, ctx, table, H, DN, DR, DV, rank, 16, 0, (DN + DR) ** -0.5)
+
+    def call(kv_up=True):
+        out = torch.full((T, H * DV), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.latent_attention(out, *args, wuk_t=wuk.view(H, DN, rank).transpose(1, 2).contiguous(),
+                             kv_up=(ops.pack_weight(up), up.shape[0]) if kv_up else None)
+        ops.check_kernel_errors()
+        return out.float()
+    return call
+
+
+def test_without_room_for_the_rows(monkeypatch):
+    """No room for the rows on the device, at any of the three allocations: the kernels over the latents take the whole step, bit for bit."""
+    call = mixed([1, 200], [40, 60])
+    want = call(kv_up=False)
+    monkeypatch.setattr(ops, "LATENT_EXPAND_WORK", 0)
+    monkeypatch.setattr(ops, "latent_expand_pays", lambda *a: True)
+    inner = ops._room
+    for fits in (0, 1, 2):
+        left = [fits]
+
+        def room(*a):
+            left[0] -= 1
+            return inner(*a) if left[0] >= 0 else None
+        monkeypatch.setattr(ops, "_room", room)
+        assert torch.equal(call(), want)
+        assert left[0] == -1
