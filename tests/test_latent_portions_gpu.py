@@ -138,3 +138,59 @@ def test_without_room_for_the_rows(monkeypatch):
         monkeypatch.setattr(ops, "_room", room)
         assert torch.equal(call(), want)
         assert left[0] == -1
+
+
+@pytest.mark.parametrize("lens,past,lead", [([1, 1, 200], [40, 700, 60], 2), ([1, 5, 40, 9], [30, 0, 17, 50], 2), ([130], [2500], 0), ([31, 64], [9, 1200], 1)])
+def test_a_step_is_shared_by_the_kernels(monkeypatch, lens, past, lead):
+    """One call over single tokens and portions: the segments ahead of the first portion stay with the kernels over the latents, and no row is
+    left out."""
+    call = mixed(lens, past)
+    want = call(kv_up=False)
+    taken = []
+    inner = ops.latent_attention_expanded
+    monkeypatch.setattr(ops, "latent_attention_expanded", lambda *a: taken.append(inner(*a)) or taken[-1])
+    monkeypatch.setattr(ops, "LATENT_EXPAND_WORK", 0)
+    monkeypatch.setattr(ops, "latent_expand_pays", lambda *a: True)
+    got = call()
+    assert taken == [lead]
+    n = sum(lens[:lead])
+    # other slices of keys ahead, keys and values rounded per head behind: a few bfloat16 roundings either way
+    for a, b in ((got[:n], want[:n]), (got[n:], want[n:])):
+        assert a.numel() == 0 or float((a - b).norm() / b.norm()) < 1.2e-2
+
+
+def test_a_layer_with_a_single_token_ahead_of_a_portion(monkeypatch):
+    """The mixer at the sizes of this path, which packs both matrices at load: a step that holds one request's next token and another's
+    first portion, against float64."""
+    import deganex_helpers as dh
+    import plain_deganex as plain
+    from qorvix_b200.engine.batch import BatchBuilder
+    from test_deganex_gpu import close, mixer_setup, rnd
+    layer = dh.attn(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=64, scale=192 ** -0.5)
+    part, cache, w = mixer_setup(layer, torch.bfloat16, sharp=3.0)
+    assert part.kv_up is not None
+    taken = []
+    inner = ops.latent_attention_expanded
+    monkeypatch.setattr(ops, "latent_attention_expanded", lambda *a: taken.append(inner(*a)) or taken[-1])
+    monkeypatch.setattr(ops, "LATENT_EXPAND_WORK", 0)
+    monkeypatch.setattr(ops, "latent_expand_pays", lambda *a: True)
+    builder, at = BatchBuilder("cuda"), {"a": 0, "b": 0}
+    xs = {r: rnd(95, 72, seed=s).to(torch.bfloat16).float() for r, s in (("a", 3), ("b", 4))}
+    want = {r: plain.latent_attention(xs[r].double(), w, layer["mixer"], 2e-5) for r in xs}
+    for step in ([("a", 40)], [("a", 1), ("b", 60)], [("a", 1), ("b", 1)], [("a", 3), ("b", 34)]):
+        segs, tables = [], {g: [] for g in cache.paged_groups()}
+        for r, n in step:
+            if not cache.has(r):
+                cache.admit(r)
+            assert cache.reserve(r, n)
+            segs.append(dict(tokens=[0] * n, pos0=at[r], slot=cache.slot(r), want=[], first=at[r] == 0))
+            for g in tables:
+                tables[g].append(cache.block_table(r, g))
+        ctx = builder.build(segs, tables, cache.scratch_page)
+        x = torch.cat([xs[r][at[r]: at[r] + n] for r, n in step]).to(torch.bfloat16).to("cuda")
+        got = part.forward(x, ctx, cache.layer_view(0)).float()
+        close(got, torch.cat([want[r][at[r]: at[r] + n] for r, n in step]), torch.bfloat16, str(step), loose=2.0)
+        for r, n in step:
+            cache.commit(r, n)
+            at[r] += n
+    assert taken == [0, 1, 1]

@@ -73,6 +73,9 @@ def test_chunks_against_float64(kind, dk, dv, H, qg, lens, shift):
         block = state[s].view(H, tiles, per)[h].double()
         S = block[:, : dk * vt].reshape(tiles, dk, vt).permute(1, 0, 2).reshape(dk, tiles * vt)[:, :dv]
         return S, block[0, dk * vt: dk * vt + dk] if gated else torch.zeros(dk, dtype=F64, device="cuda"), block[0, -1] if gated else None
+    def normalisers(state, s, h):                               # n of every value tile, and m
+        block = state[s].view(H, tiles, dk * vt + dk + 1)[h].double()
+        return block[:, dk * vt: dk * vt + dk], block[:, -1]
     errors = torch.zeros(2, 2, dtype=F64)
     norms = torch.zeros(2, dtype=F64)
     at = 0
@@ -81,11 +84,14 @@ def test_chunks_against_float64(kind, dk, dv, H, qg, lens, shift):
         for h in range(H):
             rows, kh = slice(at, at + n_tok), slice((h // qg) * dk, (h // qg) * dk + dk)
             S0, n0, m0 = state_of(start, slot, h)
-            y, S1, _, _ = plain(kind, q[rows, kh].double(), k[rows, kh].double(), v[rows, h * dv:(h + 1) * dv].double(), g1[rows, h].double(),
+            y, S1, n1, m1 = plain(kind, q[rows, kh].double(), k[rows, kh].double(), v[rows, h * dv:(h + 1) * dv].double(), g1[rows, h].double(),
                                 g2[rows, h].double(), p1[h].double(), p2[h].double(), p3[h].double(), cap, scale, S0, n0, m0)
             norms += torch.stack([(y ** 2).sum(), (S1 ** 2).sum()]).cpu()
             for i in range(2):
                 errors[i] += torch.stack([((outs[i][rows, h * dv:(h + 1) * dv] - y) ** 2).sum(), ((state_of(states[i], slot, h)[0] - S1) ** 2).sum()]).cpu()
+                if gated:                                       # float32 sums and a float32 running maximum, in every tile's own copy
+                    n, m = normalisers(states[i], slot, h)
+                    assert float((n - n1).norm() / (n1.norm() * tiles ** 0.5)) < 2e-6 and float((m - m1).abs().max()) < 2e-6 * (1 + abs(float(m1)))
         at += n_tok
     rel = (errors / norms).sqrt()
     # a float32 sum of some 64 to 256 products that cancel: a few 1e-7; the chunks may not be further off than token by token
