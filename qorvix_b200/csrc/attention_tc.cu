@@ -69,7 +69,7 @@ struct AttnArgs {
   const int* row_off = nullptr;
   const int* row_key = nullptr;
   const bf16* gate = nullptr;
-  int ld_gate = 0, v_col = 0, min_len = 0;           // segments of fewer than min_len tokens are left out
+  int ld_gate = 0, v_col = 0;
   const bf16* cache = nullptr;                       // DIFF: the cache's rows, and how many there are
   int cache_rows = 0;
 };
@@ -98,7 +98,7 @@ __device__ __forceinline__ bool item_at(const AttnArgs& a, int idx, Item& t) {
   t.q0 = a.seg_q_start[seg];
   t.qlen = a.seg_q_start[seg + 1] - t.q0;
   t.tile0 = (a.q_pairs - 1 - y) * (PAIRED ? 2 * QT : QT);
-  if (t.tile0 >= t.qlen || t.qlen < a.min_len) return false;
+  if (t.tile0 >= t.qlen) return false;
   t.pos0 = a.seg_pos0[seg];
   t.kvh = t.h / (a.H / a.Hkv);
   t.bt = a.block_table + (size_t)seg * a.max_blocks;
@@ -745,12 +745,12 @@ extern "C" int qv_attn_prefill_tc(void* out, int ld_out, const void* q, int ld_q
 // Prompt portions whose keys and values lie as rows of one matrix `kv` [rows][ld_kv]: the H heads' keys of 128 entries from column 0,
 // their values of 128 from column v_col, and a rotated key part of 64 that all heads share in `kr` [rows][64]; queries of 192 a head (the
 // rotated part behind).  Segment s has keys row_key[s] .. in rows row_off[s] .., padded with zeros to a multiple of 128 rows (row_key a
-// multiple of 128 too).  Segments of fewer than min_len tokens are left out.  gate [T][ld_gate]: its sigmoid multiplies the output.
+// multiple of 128 too).  gate [T][ld_gate]: its sigmoid multiplies the output.
 // One query tile an item (two with their rotated parts do not fit shared memory).  Bounded like the paged kernel, by a tile's chain of
 // softmax and products.
 extern "C" int qv_attn_rows_tc(void* out, int ld_out, const void* q, int ld_q, int T, const void* kv, long long ld_kv, int v_col, const void* kr,
                                long long rows, const int* row_off, const int* row_key, const void* gate, int ld_gate,
-                               const int* seg_q_start, const int* seg_pos0, int S, int max_q_len, int min_len, int H, int window, float scale,
+                               const int* seg_q_start, const int* seg_pos0, int S, int max_q_len, int H, int window, float scale,
                                int* err, void* stream) {
   if (S <= 0 || max_q_len <= 0 || rows <= 0) return 0;
   if (H <= 0 || (ld_q & 7) || (ld_out & 7) || (ld_kv & 7) || (v_col & 7) || (gate && ((ld_gate & 7) || ((uintptr_t)gate & 15))) ||
@@ -766,7 +766,7 @@ extern "C" int qv_attn_rows_tc(void* out, int ld_out, const void* q, int ld_q, i
   a.ld_out = ld_out; a.max_blocks = 0; a.H = H; a.Hkv = H; a.page = KT; a.window = window;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.segments = S; a.q_pairs = (int)q_tiles; a.items = (int)(H * S * q_tiles); a.paired = 0;
-  a.row_off = row_off; a.row_key = row_key; a.gate = (const bf16*)gate; a.ld_gate = ld_gate; a.v_col = v_col; a.min_len = min_len;
+  a.row_off = row_off; a.row_key = row_key; a.gate = (const bf16*)gate; a.ld_gate = ld_gate; a.v_col = v_col;
   return launch<128, false, 64>(mq, mkv, mkr, a, (cudaStream_t)stream);
 }
 

@@ -444,9 +444,8 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 // that is, the eight products with S_0 do not wait for one another, and a block costs one chain of sums and shuffles instead of four.
 // Only products of decays (each at most one) occur, no quotients; everything is float32.
 //   channel_delta_operands   x [T][H][3][n] = P_t k_t, P_t q_t, (g_(t+1) .. g_end) kb_t;  pall [T][H][n] = P_end, at a block's first token;
-//                            coef [T][H][8] = A_t0 A_t1 A_t2 -, B_t0 .. B_t3.  A warp per (token, head).
-//   channel_delta_blocks     the recurrence; a lane holds 16 rows of two columns, two warps a CTA work and two fetch (one column a lane and
-//                            four working warps: 496 us where this takes 426).
+//                            coef [T][H][8] = A_t0 A_t1 A_t2 -, B_t0 .. B_t3.  A warp per (block, head).
+//   channel_delta_blocks     the recurrence; a lane holds 16 rows of two columns, two warps a CTA work and two fetch.
 // 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 426 in blocks, the operands 14 and 34.  Bound by a block's chain (dots,
 // shuffles, the triangular sums, the update) in one warp a scheduler.
 // Blocks are counted from the start of a request's portion, so cuts agree to rounding (the 32-bit path takes channel_scan_kernel).
@@ -556,10 +555,12 @@ struct ChannelDeltaArgs {
   int H, dk, dv;
 };
 
-// NB: blocks a stage, two stages.  C: columns a lane, so 4 / C warps work; two more fetch.
-template <int LPC, int NB, int C = 2>
-__global__ void __launch_bounds__(32 * (4 / C + 2)) channel_delta_blocks_kernel(ChannelDeltaArgs a) {
+// NB: blocks a stage, two stages.  Two columns a lane (one column a lane and four working warps: 496 us where this takes 426), so two warps
+// work; two more fetch.
+template <int LPC, int NB>
+__global__ void __launch_bounds__(128) channel_delta_blocks_kernel(ChannelDeltaArgs a) {
   extern __shared__ __align__(16) float cd_ring[];
+  constexpr int C = 2;
   constexpr int CPT = 32 / LPC, CTA_COLS = 4 * CPT, VEC = CS_PAD * LPC, W = 4 / C;
   constexpr int ROW = 3 * VEC + 8 + CTA_COLS;                        // floats a token takes: three vectors, factors, values
   constexpr int BLK = CD_BLOCK * ROW + VEC;                          // a block: its tokens, then P_end
@@ -706,14 +707,14 @@ extern "C" long long qv_channel_delta_workspace_floats(int lead, int rest, int H
 
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
 // beta, g [T, H * dk] the decays, v [T, H * dv].  The first S_lead segments (T_lead tokens, the longest of them max_lead) go token by token, the
-// others in blocks, for which dk is a multiple of 4, at most 256.
+// others in blocks, for which dk is a multiple of 4 above 64, at most 256.
 extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                                 const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
                                 long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,
                                 int T_lead, int max_lead, int H, int G, int dk, int dv, float* workspace, void* stream) {
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || S_lead < 0 || S_lead > S || T_lead < 0 || T_lead > T) return QV_ERR_UNSUPPORTED;
-  if (S_lead < S && (dk % 4 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
+  if (S_lead < S && (dk % 4 || dk <= 64 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
   if (dk > 256) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   if (S_lead > 0) {
@@ -747,14 +748,12 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
 #define CD_LAUNCH(LPC, NB)                                                                                                       \
   do {                                                                                                                           \
     constexpr int smem = 2 * NB * (CD_BLOCK * (3 * CS_PAD * LPC + 8 + 4 * 32 / LPC) + CS_PAD * LPC) * 4;                         \
-    cudaFuncSetAttribute(channel_delta_blocks_kernel<LPC, NB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB, 2>, dim3(S - S_lead, H, ctas), dim3(128), (size_t)smem, st, a);           \
+    cudaFuncSetAttribute(channel_delta_blocks_kernel<LPC, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
+    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB>, dim3(S - S_lead, H, ctas), dim3(128), (size_t)smem, st, a);           \
   } while (0)
-  if (lpc == 1) CD_LAUNCH(1, 4);
-  if (lpc == 2) CD_LAUNCH(2, 4);
-  if (lpc == 4) CD_LAUNCH(4, 4);
   if (lpc == 8) CD_LAUNCH(8, 4);
-  CD_LAUNCH(16, 2);
+  if (lpc == 16) CD_LAUNCH(16, 2);
+  return QV_ERR_UNSUPPORTED;                // shorter keys: token by token is the faster scan
 #undef CD_LAUNCH
 }
 

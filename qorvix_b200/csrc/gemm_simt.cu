@@ -12,7 +12,7 @@
 // types, odd strides) through registers, all of a thread's elements of the next tile in flight under the present one's multiply-adds; and
 // a thread reads four k of a row at a time.  Two tile shapes: 16 x 32 (64 k, 2 x 2 outputs a thread) where 64 x 64 tiles would be few
 // or mostly padding, else 64 x 64 (32 k, 4 x 4 a thread).  Few CTAs are bound by the chain of K dependent multiply-adds and the
-// staging around it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (now 5 / 9 us, 3 rows x 192).
+// staging around it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (now 5 / 10 us, 3 rows).
 #include "common.cuh"
 
 __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live) {

@@ -714,7 +714,7 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
 }
 
 // ---------------------------------------------------------------- portions: the latents as rows, for keys and values formed per head
-// Copies the cached rows that the segments of at least min_len tokens see into c [rows][rank] and kr [rows][dr], a warp a row: segment s
+// Copies the cached rows that the segments see into c [rows][rank] and kr [rows][dr], a warp a row: segment s
 // from key row_key[s] (the window's first key, rounded down to a multiple of 128; 0 without a window) in rows row_off[s] .., padded with
 // rows of zeros to a multiple of 128 (and ahead of the window: those pages may have another owner by now, and a weight of zero does not keep
 // an infinity out of a sum).  The first block also writes row_off and row_key [S].
@@ -722,7 +722,7 @@ __device__ __forceinline__ int lt_first_key(int pos0, int window) { return windo
 __global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict__ c, uint4* __restrict__ kr, int* __restrict__ row_off,
                                                               int* __restrict__ row_key, const uint4* __restrict__ cache, int rank16, int dr16,
                                                               const int* __restrict__ seg_q_start, const int* __restrict__ seg_pos0,
-                                                              const int* __restrict__ block_table, int max_blocks, int S, int min_len, int page,
+                                                              const int* __restrict__ block_table, int max_blocks, int S, int page,
                                                               int window, int rows) {
   pdl_wait();
   pdl_launch_dependents();
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict_
     int off = 0, key = -1, seg = 0;                 // key -1: a row of zeros
     for (int s = 0; s < S; ++s) {
       const int len = seg_q_start[s + 1] - seg_q_start[s], pos0 = seg_pos0[s], first = lt_first_key(pos0, window);
-      const int n = len >= min_len ? pos0 + len - first : 0, padded = (n + 127) & ~127;
+      const int n = pos0 + len - first, padded = (n + 127) & ~127;
       if (r >= off && r < off + padded) { seg = s; key = r - off < n && (window <= 0 || first + r - off > pos0 - window) ? first + r - off : -1; }
       if (r == 0 && lane == 0) { row_off[s] = off; row_key[s] = first; }
       off += padded;
@@ -745,12 +745,12 @@ __global__ void __launch_bounds__(256) latent_rows_out_kernel(uint4* __restrict_
 }
 
 extern "C" int qv_latent_rows_out(void* c, void* kr, int* row_off, int* row_key, const void* cache, int rank, int dr, const int* seg_q_start,
-                                  const int* seg_pos0, const int* block_table, int max_blocks, int S, int min_len, int page, int window, int rows,
+                                  const int* seg_pos0, const int* block_table, int max_blocks, int S, int page, int window, int rows,
                                   void* stream) {
   if (S <= 0 || rows <= 0) return 0;
   if (rank % 8 || dr % 8 || (((uintptr_t)c | (uintptr_t)kr | (uintptr_t)cache) & 15)) return QV_ERR_UNSUPPORTED;
   const int blocks = (rows + 7) / 8;
   return qv_launch(latent_rows_out_kernel, dim3(blocks < 148 * 8 ? blocks : 148 * 8), dim3(256), 0, (cudaStream_t)stream, (uint4*)c, (uint4*)kr,
-                   row_off, row_key, (const uint4*)cache, rank / 8, dr / 8, seg_q_start, seg_pos0, block_table, max_blocks, S, min_len, page, window,
+                   row_off, row_key, (const uint4*)cache, rank / 8, dr / 8, seg_q_start, seg_pos0, block_table, max_blocks, S, page, window,
                    rows);
 }

@@ -64,8 +64,8 @@ _ARGTYPES = {
     "qv_latent_attention_generic": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V, _V],
     "qv_latent_tc_workspace_bytes": [_I, _I, _I, _I, _I],
     "qv_latent_attention_tc": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _V, _V, _I, _V],
-    "qv_latent_rows_out": [_V, _V, _V, _V, _V, _I, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V],
-    "qv_attn_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _I, _V, _L, _V, _V, _V, _I, _V, _V, _I, _I, _I, _I, _I, _F, _V, _V],
+    "qv_latent_rows_out": [_V, _V, _V, _V, _V, _I, _I, _V, _V, _V, _I, _I, _I, _I, _I, _V],
+    "qv_attn_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _I, _V, _L, _V, _V, _V, _I, _V, _V, _I, _I, _I, _I, _F, _V, _V],
     "qv_diff_attention_rows_tc": [_V, _I, _V, _I, _I, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _V, _V, _V],
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
@@ -808,8 +808,8 @@ def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table
     LATENT_EXPAND_FROM tokens on; returns how many leading segments it left out (all of them: nothing was done, where a size, a type or
     the room for the rows does not allow it, by LATENT_EXPAND_BYTES or on the device)."""
     S = ctx.num_segments
-    lens, pos0 = getattr(ctx, "seg_len", None), getattr(ctx, "seg_start_pos", None)
-    if (kv_up is None or q.dtype != torch.bfloat16 or not lens or not pos0 or getattr(ctx, "captured", False) or dn != 128 or dv != 128 or dr != 64
+    lens, pos0 = ctx.seg_len, ctx.seg_start_pos
+    if (kv_up is None or q.dtype != torch.bfloat16 or ctx.captured or dn != 128 or dv != 128 or dr != 64
             or rank % 8 or q.stride(0) % 8 or out.stride(0) % 8 or cache_layer.dtype != torch.bfloat16
             or (gate is not None and (gate.dtype != torch.bfloat16 or gate.stride(0) % 8 or gate.data_ptr() % 16))
             or q.data_ptr() % 16 or out.data_ptr() % 16):
@@ -837,12 +837,12 @@ def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table
     skip = first * 4                                                                     # bytes of the left-out segments' entries (int32)
     starts, firsts, tables = _ptr(ctx.seg_q_start) + skip, _ptr(ctx.seg_pos0) + skip, _ptr(block_table) + skip * block_table.shape[-1]
     _check(_lib("latent_attention").qv_latent_rows_out(
-        _ptr(c), kr, starts_row, firsts_row, _ptr(cache_layer), rank, dr, starts, firsts, tables, block_table.shape[-1], S - first, 1, page,
+        _ptr(c), kr, starts_row, firsts_row, _ptr(cache_layer), rank, dr, starts, firsts, tables, block_table.shape[-1], S - first, page,
         window, rows, _stream()), "latent_rows_out")
     gemm(kv, c, None, packed, features)
     _check(_lib("attention_tc").qv_attn_rows_tc(
         _ptr(out), out.stride(0), _ptr(q), q.stride(0), q.shape[0], _ptr(kv), kv.stride(0), H * dn, kr, rows, starts_row, firsts_row,
-        _ptr(gate), gate.stride(0) if gate is not None else 0, starts, firsts, S - first, max(lens[first:]), 1, H, window, scale,
+        _ptr(gate), gate.stride(0) if gate is not None else 0, starts, firsts, S - first, max(lens[first:]), H, window, scale,
         _ptr(_tc_buffers(dev)["err"]), _stream()), "attn_rows_tc")
     return first
 

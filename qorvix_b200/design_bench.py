@@ -144,8 +144,10 @@ def latent_attention_case(seg_lens, ctx_len, peaks, page=16, window=0, gated=Tru
                                                        ATTN["scale"], wuk_t=wuk_t, kv_up=kv_up, **more), launches=8)
     seen = lambda pos: min(pos + 1, window) if window else pos + 1                      # keys a query at `pos` sees
     pairs = sum(seen(ctx_len - n + i) for n in seg_lens for i in range(n))              # (query, key) pairs per head
-    flops = H * pairs * (2.0 * (rank + dr) + 2.0 * rank) + T * H * 2.0 * rank * (dn + dv)
+    carried = H * pairs * (2.0 * (rank + dr) + 2.0 * rank) + T * H * 2.0 * rank * (dn + dv)        # queries carried into the latent space
     rows = sum(min(ctx_len, window + n - 1) if window else ctx_len for n in seg_lens)   # cache rows the step must read
+    expanded = H * pairs * 2.0 * (dn + dr + dv) + 2.0 * rows * rank * H * (dn + dv)                # or every head's keys and values formed
+    flops = carried if sinks else min(carried, expanded)                                           # what the work needs, whichever path is taken
     return kb._figures(us, rows * row_bytes + (q.numel() + (gate.numel() if gated else 0) + out.numel()) * 2, flops, peaks)
 
 

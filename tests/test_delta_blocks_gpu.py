@@ -1,5 +1,6 @@
-"""The delta rule four tokens at a time against float64 token by token, over every size of lane groups, segments that end anywhere in a block,
-strong and weak decays; and no further off than the token-by-token kernel."""
+"""The delta rule as a step takes it (keys above 64 entries four tokens at a time from the first portion on, others token by token) against
+float64 token by token, over every size of lane groups, segments that end anywhere in a block, strong and weak decays; and no further off
+than the token-by-token kernel."""
 from types import SimpleNamespace
 
 import pytest
