@@ -510,67 +510,86 @@ template <int VT, int NK> struct LcShape {
 };
 
 __device__ __forceinline__ bool lc_finite(float4 v) { return (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w)) <= 3.4028234e38f; }
-// The share of W v in token t's output at columns cc .. cc + 3, tokens behind t left out instead of weighted by zero: for chunks with an
-// infinite or NaN value, which may reach its own token's output and later ones but no earlier one (a weight of zero does not keep it out).
-template <int KIND, int DKP, int LDQ, int LDV>
-__device__ float4 lc_values_up_to(const bf16* qs, const bf16* vc, const LcGates& gt, int t, int cc) {
-  const bf16* ks = qs + LC_C * LDQ;
-  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int j = 0; j <= t; ++j) {
-    float dot = 0.f;
-    for (int i = 0; i < DKP; ++i) dot = fmaf(to_f(qs[t * LDQ + i]), to_f(ks[j * LDQ + i]), dot);
-    const float w = dot * (lc_exp_sum(gt.G[t], gt.H[j]) * (KIND == SCAN_DECAY ? gt.b[j] : 1.f));
-    const bf16* v = vc + j * LDV + cc;
-    y.x = fmaf(w, to_f(v[0]), y.x); y.y = fmaf(w, to_f(v[1]), y.y); y.z = fmaf(w, to_f(v[2]), y.z); y.w = fmaf(w, to_f(v[3]), y.w);
-  }
-  return y;
-}
-
-template <int LDR>
-__device__ __forceinline__ float4 lc_sums(float4 y, const float* red, int from, int to, int t, int cc) {
-#pragma unroll
-  for (int sl = from; sl < to; ++sl) {
-    const float4 z = *(const float4*)(red + ((size_t)sl * LC_C + t) * LDR + cc);
-    y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
-  }
-  return y;
-}
-// Four output columns of token t from their sums; v: the token's values there.
-template <int KIND, int VT, int SLICES>
-__device__ __forceinline__ float4 lc_output(float4 y, const float* rowsum, const float* nq, const bf16* v, const LcGates& gt, int t, float q_scale,
-                                            float b3) {
-  y.x *= q_scale; y.y *= q_scale; y.z *= q_scale; y.w *= q_scale;
-  if (KIND == SCAN_GATED_MAX) {
-    float dot = rowsum[2 * t] + rowsum[2 * t + 1];
-#pragma unroll
-    for (int sl = 0; sl < SLICES; ++sl) dot += nq[sl * LC_C + t];
-    dot *= q_scale;
-    const float den = fmaxf(fabsf(dot), gt.em[t]) + 1e-6f;
-    y.x /= den; y.y /= den; y.z /= den; y.w /= den;
-  } else {
-    y.x = fmaf(b3, to_f(v[0]), y.x); y.y = fmaf(b3, to_f(v[1]), y.y); y.z = fmaf(b3, to_f(v[2]), y.z); y.w = fmaf(b3, to_f(v[3]), y.w);
-  }
-  return y;
-}
-// A chunk's outputs where only the chunk's own values made them infinite or NaN, once more: tokens behind each left out.
-template <int KIND, int VT, int NK>
-__device__ __noinline__ void lc_write_again(float* out, int ld_out, int tokens, int cols, const float* red, const bf16* qs, const bf16* vc,
-                                            const LcGates& gt, const float* rowsum, const float* nq, float q_scale, float b3) {
-  typedef LcShape<VT, NK> Sh;
-  for (int i = threadIdx.x - 256; i < LC_C * VT / 4; i += 256) {
-    const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
-    if (t >= tokens || cc >= cols) continue;
-    const float4 past = lc_sums<Sh::LDR>(*(const float4*)(red + (size_t)t * Sh::LDR + cc), red, 1, Sh::SLICES, t, cc);
-    if (!lc_finite(past) || lc_finite(lc_sums<Sh::LDR>(past, red, Sh::SLICES, Sh::SLICES + 2, t, cc))) continue;
-    const float4 z = lc_values_up_to<KIND, Sh::DKP, Sh::LDQ, Sh::LDV>(qs, vc, gt, t, cc);
-    *(float4*)(out + (size_t)t * ld_out + cc) = lc_output<KIND, VT, Sh::SLICES>(
-        make_float4(past.x + z.x, past.y + z.y, past.z + z.z, past.w + z.w), rowsum, nq, vc + t * Sh::LDV + cc, gt, t, q_scale, b3);
-  }
-}
-
 #define LC_THREADS 512
+// A segment's share (one head, one tile of value columns) token by token, from the state as the step found it: for outputs that came out
+// infinite or NaN.  Within a chunk the weights of later tokens are set to zero, which does not keep their infinities out of earlier tokens'
+// sums; here a token sees its own and earlier ones only.  Slow (some microseconds a token), and apart from the chunks' loop, which it
+// would cost registers: with the chunk's own sums formed once more in place 2,048 tokens of 4 heads of 256 x 512 took 271 us a layer, so 263.
+template <int KIND, int VT>
+__device__ __noinline__ void lc_token_by_token(const ScanArgs& a, int s, int h, int tile, float* S) {
+  constexpr int PARTS = LC_THREADS / VT;
+  const int dk = a.dk, tid = threadIdx.x, col = tid % VT, part = tid / VT;
+  float* qs = S + dk * VT;                           // S [dk][VT]
+  float* ks = qs + dk;
+  float* ns = ks + dk;
+  float* sums = ns + dk;                             // [PARTS][VT]
+  float* sc = sums + LC_THREADS;                     // n . q
+  const int tiles = (a.dv + VT - 1) / VT, q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk, VT);
+  for (int i = tid; i < dk * VT; i += LC_THREADS) S[i] = st[i];
+  float m = 0.f;
+  if (KIND == SCAN_GATED_MAX) {
+    for (int i = tid; i < dk; i += LC_THREADS) ns[i] = st[dk * VT + i];
+    m = st[dk * VT + dk];
+  }
+  const bool live = tile * VT + col < a.dv;
+  const float b1 = a.p1 ? a.p1[h] : 0.f, b2 = a.p2 ? a.p2[h] : 0.f, b3 = a.p3 ? a.p3[h] : 0.f;
+  for (int j = 0; j < len; ++j) {
+    const size_t t = (size_t)(q0 + j);
+    for (int i = tid; i < dk; i += LC_THREADS) {
+      qs[i] = to_f(((const bf16*)a.q)[t * a.ld_q + (size_t)(h / a.q_group) * dk + i]) * a.q_scale;
+      ks[i] = to_f(((const bf16*)a.k)[t * a.ld_k + (size_t)(h / a.q_group) * dk + i]);
+    }
+    const float v = live ? to_f(((const bf16*)a.v)[t * a.ld_v + (size_t)h * a.dv + tile * VT + col]) : 0.f;
+    float keep, take;
+    if (KIND == SCAN_GATED_MAX) {
+      const float li = a.cap * tanhf((a.g1[t * a.ld_g1 + h] + b1) / a.cap), zf = a.cap * tanhf((a.g2[t * a.ld_g2 + h] + b2) / a.cap);
+      const float lf = fminf(zf, 0.f) - log1pf(expf(-fabsf(zf)));
+      const float m_new = fmaxf(lf + m, li);
+      keep = expf(lf + m - m_new);
+      take = expf(li - m_new);
+      m = m_new;
+    } else {
+      const float z = a.g1[t * a.ld_g1 + h] + b1;
+      take = z > 20.f ? z : log1pf(expf(z));
+      keep = expf(-expf(b2) * take);
+    }
+    __syncthreads();                                 // q and k are in place; the last token's sums have been read
+    if (KIND == SCAN_GATED_MAX && tid < 32) {
+      float dot = 0.f;
+      for (int i = tid; i < dk; i += 32) {
+        const float n = keep * ns[i] + take * ks[i];
+        ns[i] = n;
+        dot = fmaf(n, qs[i], dot);
+      }
+      dot = warp_sum(dot);
+      if (tid == 0) *sc = dot;
+    }
+    float acc = 0.f;
+    for (int i = part; i < dk; i += PARTS) {
+      const float x = fmaf(keep, S[i * VT + col], take * v * ks[i]);
+      S[i * VT + col] = x;
+      acc = fmaf(x, qs[i], acc);
+    }
+    sums[part * VT + col] = acc;
+    __syncthreads();
+    if (part == 0 && live) {
+      float y = 0.f;
+      for (int i = 0; i < PARTS; ++i) y += sums[i * VT + col];
+      y = KIND == SCAN_GATED_MAX ? y / (fmaxf(fabsf(*sc), expf(-m)) + 1e-6f) : fmaf(b3, v, y);
+      a.out[t * a.ld_out + (size_t)h * a.dv + tile * VT + col] = y;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < dk * VT; i += LC_THREADS) st[i] = S[i];
+  if (KIND == SCAN_GATED_MAX) {
+    for (int i = tid; i < dk; i += LC_THREADS) st[dk * VT + i] = ns[i];
+    if (tid == 0) st[dk * VT + dk] = m;
+  }
+}
+
 template <int KIND, int VT, int NK>
-__global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const __grid_constant__ ScanArgs a) {
   typedef LcShape<VT, NK> Sh;
   constexpr int SLICES = Sh::SLICES, DKP = Sh::DKP, LDQ = Sh::LDQ, LDV = Sh::LDV, LDR = Sh::LDR;
   extern __shared__ __align__(16) unsigned char lc_smem[];
@@ -726,6 +745,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
       }
   }
 
+  bool finite = true;                                // of this thread's outputs
   for (int c = 0; c < nchunks; ++c) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                 // chunk c and its gates are in place; everyone is done with chunk c - 1
@@ -916,22 +936,35 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(ScanAr
         np[0] = fmaf(gt.A_end, np[0], a0);
         np[1] = fmaf(gt.A_end, np[1], a1);
       }
-      bool finite = true;
       for (int i = tid - 256; i < LC_C * VT / 4; i += 256) {
         const int t = i / (VT / 4), cc = (i - t * (VT / 4)) * 4;
         if (c * LC_C + t >= len || tile * VT + cc >= dv) continue;
-        const float4 y = lc_output<KIND, VT, SLICES>(lc_sums<LDR>(*(const float4*)(red + (size_t)t * LDR + cc), red, 1, SLICES + 2, t, cc),
-                                                     rowsum, nq, vc + t * LDV + cc, gt, t, a.q_scale, b3);
+        float4 y = *(const float4*)(red + (size_t)t * LDR + cc);
+#pragma unroll
+        for (int sl = 1; sl < SLICES + 2; ++sl) {
+          const float4 z = *(const float4*)(red + ((size_t)sl * LC_C + t) * LDR + cc);
+          y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
+        }
+        y.x *= a.q_scale; y.y *= a.q_scale; y.z *= a.q_scale; y.w *= a.q_scale;
+        if (KIND == SCAN_GATED_MAX) {
+          float dot = rowsum[2 * t] + rowsum[2 * t + 1];
+#pragma unroll
+          for (int sl = 0; sl < SLICES; ++sl) dot += nq[sl * LC_C + t];
+          dot *= a.q_scale;
+          const float den = fmaxf(fabsf(dot), gt.em[t]) + 1e-6f;
+          y.x /= den; y.y /= den; y.z /= den; y.w /= den;
+        } else {
+          const bf16* vr = vc + t * LDV + cc;
+          y.x = fmaf(b3, to_f(vr[0]), y.x); y.y = fmaf(b3, to_f(vr[1]), y.y); y.z = fmaf(b3, to_f(vr[2]), y.z); y.w = fmaf(b3, to_f(vr[3]), y.w);
+        }
         *(float4*)(a.out + (size_t)(q0 + c * LC_C + t) * a.ld_out + (size_t)h * dv + tile * VT + cc) = y;
         finite = finite && lc_finite(y);
       }
-      if (!finite)                                   // (apart, and in a function, so that the loop above is free of it)
-        lc_write_again<KIND, VT, NK>(a.out + (size_t)(q0 + c * LC_C) * a.ld_out + (size_t)h * dv + tile * VT, a.ld_out, len - c * LC_C, dv - tile * VT, red,
-                                     qs, vc, gt, rowsum, nq, a.q_scale, b3);
     }
     // the logarithms of the batch that begins with chunk c + 2 (the present one's last gates were worked out ahead of the barrier)
     if ((c + 2) % (LC_BATCH / LC_C) == 0) work_logs((c + 2) * LC_C);
   }
+  if (__syncthreads_or(!finite)) return lc_token_by_token<KIND, VT>(a, s, h, tile, (float*)lc_smem);
   if (warp < 8) {
 #pragma unroll
     for (int nt = 0; nt < 2 * NK; ++nt)
