@@ -700,14 +700,10 @@ __global__ void __launch_bounds__(128) channel_delta_blocks_kernel(ChannelDeltaA
       for (int i = 0; i < CS_ROWS; ++i) st[c * CS_ROWS * 32 + i * 32] = S[c][i];
 }
 
-// Floats of workspace: `lead` tokens token by token (operands of qv_channel_scan), `rest` tokens in blocks (x, pall and coef in this order).
-extern "C" long long qv_channel_delta_workspace_floats(int lead, int rest, int H, int dk) {
-  return ((long long)lead * 3 * dk + (long long)rest * (4 * (long long)dk + 8)) * H;
-}
-
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
 // beta, g [T, H * dk] the decays, v [T, H * dv].  The first S_lead segments (T_lead tokens, the longest of them max_lead) go token by token, the
-// others in blocks, for which dk is a multiple of 4 above 64, at most 256.
+// others in blocks, for which dk is a multiple of 4 above 64, at most 256.  workspace: H x 3 dk floats a token of the first (operands of
+// qv_channel_scan), then H x (4 dk + 8) a token of the others (x, pall and coef in this order).
 extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                                 const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
                                 long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,

@@ -107,7 +107,6 @@ _ARGTYPES = {
     "qv_unit_keys": [_V, _V, _V, _I, _V, _I, _V, _I, _I, _I, _F, _V],
     "qv_channel_scan_state_floats": [_I, _I, _I],
     "qv_channel_scan": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _V],
-    "qv_channel_delta_workspace_floats": [_I, _I, _I, _I],
     "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V],
     "qv_head_norm_gate": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _F, _I, _V],
     "qv_bias_attn_prepare": [_V, _I, _V, _I, _I, _I, _I, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V],
@@ -125,7 +124,7 @@ _ARGTYPES = {
 }
 _RESTYPES = {"qv_error_string": ctypes.c_char_p, "qv_packed_weight_bytes": c_longlong, "qv_gemm_bf16_split_slot_bytes": c_longlong,
              "qv_linear_scan_state_floats": c_longlong, "qv_latent_tc_workspace_bytes": c_longlong, "qv_diff_partial_floats": c_longlong,
-             "qv_channel_scan_state_floats": c_longlong, "qv_channel_delta_workspace_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
+             "qv_channel_scan_state_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
 _typed_libs = {}
 
 
@@ -763,42 +762,53 @@ LATENT_EXPAND_BYTES = 1 << 30              # the most that their rows may take
 LATENT_EXPAND_WORK = 1 << 29
 
 
-def _latent_carried_us(lens, pos0, H: int, window: int, sms: int) -> float:
+def _latent_carried_us(tiles: int, longest: int, seen: int, walk: float, sms: int) -> float:
     """About what the kernels over the latents take beside the layer's other work: tiles of 32 (token, head) rows walk over blocks of 64
-    keys, 6.6 us a block, cut into slices of keys where the tiles leave SMs idle; 19 us of merge and value matrices."""
-    if not lens:
-        return 0.0
-    tiles = sum(-(-n * H // 32) for n in lens)
-    seen = [min(p + n, window + n) if window > 0 else p + n for n, p in zip(lens, pos0)]
-    splits = max(1, min(sms // max(tiles, 1), -(-max(p + n for n, p in zip(lens, pos0)) // 64)))
-    total = sum(-(-n * H // 32) * min(p + n / 2, window or p + n) / 64 for n, p in zip(lens, pos0))
-    return 19.0 + 6.6 * max(-(-max(seen) // 64 // splits), total / sms)
+    keys, 6.6 us a block, cut into slices of keys where the tiles leave SMs idle; 19 us of merge and value matrices.  longest: the longest
+    context, seen: the most keys a segment sees, walk: keys x tiles."""
+    splits = max(1, min(sms // tiles, -(-longest // 64)))
+    return 19.0 + 6.6 * max(-(-seen // 64 // splits), walk / (64 * sms))
 
 
-def _latent_expanded_us(lens, pos0, H: int, rank: int, features: int, window: int, sms: int) -> float:
-    """About what forming every head's keys and values takes (the product, and its rows on their way to memory) and the attention over
-    them: tiles of 128 queries walk over tiles of 128 keys, 2.1 us a tile, no slices of keys."""
-    rows, longest, total = 0, 0, 0.0
-    for n, p in zip(lens, pos0):
-        lo = (p + 1 - window) & ~127 if window > 0 and p + 1 > window else 0
-        rows += (p + n - lo + 127) & ~127
-        longest = max(longest, -(-min(p + n, window + 128 if window > 0 else p + n) // 128))
-        total += -(-n // 128) * H * (min(p + n / 2, window or p + n) / 128 + 0.5)
-    return 2.1 * max(longest, total / sms) + rows * features * (rank / 0.6e9 + 1 / 2.5e6)
-
-
-def latent_expand_pays(lens, pos0, H: int, rank: int, features: int, window: int, sms: int) -> bool:
-    """Whether the segments from the first of LATENT_EXPAND_FROM tokens on are faster with keys and values formed per head.  A few tokens
-    far into a request are not: the rows to form and the walk over them grow with the cached tokens, however few the new ones are, while the
-    kernels over the latents cut the keys over the SMs.  us a layer on the device over the latents and with keys and values formed,
+def latent_expand_pays(lens, pos0, H: int, rank: int, features: int, window: int, sms: int, least_pairs: float = 0.0) -> bool:
+    """Whether the segments from the first of LATENT_EXPAND_FROM tokens on (of at least `least_pairs` query-key pairs a head) are faster with keys
+    and values formed per head.  That takes the product and its rows on their way to memory, and an attention whose tiles of 128 queries walk
+    over tiles of 128 keys, 2.1 us a tile, without slices of keys.  A few tokens far into a request do not pay: the rows to form and
+    the walk over them grow with the cached tokens, however few the new ones are, while the kernels over the latents cut the keys over the
+    SMs.  us a layer on the device over the latents and with keys and values formed,
     16 heads of rank 512: 32 tokens behind 2,000 78 and 85, behind 8,000 140 and 216; 64 behind 2,000 115 and 90, behind 8,000 258 and
     218; 128 behind 8,000 469 and 190.  8 heads of rank 256: 32 behind 8,000 88 and 175, 64 141 and 179, 128 256 and 142.  64 heads of
     rank 512: 32 behind 2,000 176 and 151, behind 8,000 465 and 391."""
-    first = next((i for i, n in enumerate(lens) if n >= LATENT_EXPAND_FROM), len(lens))
-    if first == len(lens):
+    first, i, ahead = -1, 0, None
+    tiles, longest, seen, walk = 0, 0, 0, 0.0                 # over the latents, of all segments so far
+    rows, chain, steps, pairs = 0, 0, 0.0, 0.0                # with keys and values formed, from `first` on
+    for n, p in zip(lens, pos0):                              # (one pass, on the host's way to the launch)
+        if first < 0 and n >= LATENT_EXPAND_FROM:
+            first, ahead = i, (tiles, longest, seen, walk)
+        i += 1
+        end = keys = p + n
+        mid = p + n // 2 + 1                                  # keys that the middle token sees
+        lo, span = 0, end
+        if window > 0:
+            keys, mid, span = min(keys, window + n), min(mid, window), min(end, window + 128)
+            if p + 1 > window:
+                lo = (p + 1 - window) & ~127
+        t = -(-n * H // 32)
+        tiles += t
+        walk += t * mid
+        longest, seen = max(longest, end), max(seen, keys)
+        if first >= 0:
+            rows += (end - lo + 127) & ~127
+            chain = max(chain, -(-span // 128))
+            steps += -(-n // 128) * (mid / 128 + 0.5)
+            if n >= LATENT_EXPAND_FROM:
+                pairs += n * mid
+    if first < 0 or pairs < least_pairs:
         return False
-    apart = _latent_expanded_us(lens[first:], pos0[first:], H, rank, features, window, sms) + _latent_carried_us(lens[:first], pos0[:first], H, window, sms)
-    return apart < 0.9 * _latent_carried_us(lens, pos0, H, window, sms)
+    formed = 2.1 * max(chain, steps * H / sms) + rows * features * (rank / 0.6e9 + 1 / 2.5e6)
+    if first:
+        formed += _latent_carried_us(*ahead, sms)
+    return formed < 0.9 * _latent_carried_us(tiles, longest, seen, walk, sms)
 
 
 def latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale) -> int:
@@ -855,8 +865,7 @@ def latent_attention(out, q, gate, cache_layer, wuk, wuv, ctx, block_table, H, d
     entries = H * (2 * rank + dr)
     if (kv_up is not None and sink is None and weight_terms == 1 and ctx.max_q_len >= LATENT_EXPAND_FROM and not ctx.captured
             and ctx.num_tokens * ctx.max_ctx_len * entries >= LATENT_EXPAND_WORK
-            and _pairs(ctx, LATENT_EXPAND_FROM, window) * entries >= LATENT_EXPAND_WORK
-            and latent_expand_pays(ctx.seg_len, ctx.seg_start_pos, H, rank, H * (dn + dv), window, sm_count())):
+            and latent_expand_pays(ctx.seg_len, ctx.seg_start_pos, H, rank, H * (dn + dv), window, sm_count(), LATENT_EXPAND_WORK / entries)):
         left = latent_attention_expanded(out, q, gate, cache_layer, kv_up, ctx, block_table, H, dn, dr, dv, rank, page, window, scale)
         if left == 0:
             return
@@ -1048,12 +1057,11 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lens = ctx.seg_len
     lead = delta_lead(lens, dk, blocks)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
-    lib = _lib("channel_scan")
-    ws = _room(int(lib.qv_channel_delta_workspace_floats(tokens, T - tokens, H, dk)), torch.float32, q.device) if lead < S else None
+    ws = _room(H * (tokens * 3 * dk + (T - tokens) * (4 * dk + 8)), torch.float32, q.device) if lead < S else None
     if ws is None:                                    # token by token, which takes three quarters of the blocks' room
         lead, tokens, longest = S, T, int(ctx.max_q_len)
-        ws = torch.empty(int(lib.qv_channel_delta_workspace_floats(T, 0, H, dk)), device=q.device, dtype=torch.float32)
-    rc = lib.qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
+        ws = torch.empty(H * T * 3 * dk, device=q.device, dtype=torch.float32)
+    rc = _lib("channel_scan").qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
                               _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0), _ptr(ctx.tok_seg),
                               _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, H, G, dk, dv, _ptr(ws), _stream())
     _check(rc, "channel_delta")

@@ -162,6 +162,7 @@ def test_latent_portions_choose_by_what_either_path_costs():
     assert not pays([1, 1, 32], [700, 900, 8000], 16, 512)                      # behind single tokens
     assert pays([512, 8], [0, 8000], 16, 512)                                   # one CTA a tile over the latents: 900 us and 278
     assert ops.latent_expand_pays([64], [8000], 8, 256, 2048, 500, 148)         # a window leaves few rows to form
+    assert ops.latent_expand_pays([64], [2000], 16, 512, 4096, 0, 148, 64 * 2033) and not ops.latent_expand_pays([64], [2000], 16, 512, 4096, 0, 148, 64 * 2034)
 
 
 def test_delta_rule_segments_that_go_token_by_token():
