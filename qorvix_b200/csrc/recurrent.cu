@@ -509,12 +509,11 @@ template <int VT, int NK> struct LcShape {
   static constexpr int BYTES = 2 * STAGE + RED + 5 * V + 2 * (int)sizeof(LcGates) + LC_C * 2 * 4 + SLICES * LC_C * 4 + 2 * LC_BATCH * 4 + 2 * DKP * 4;
 };
 
-__device__ __forceinline__ bool lc_finite(float4 v) { return (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w)) <= 3.4028234e38f; }
 #define LC_THREADS 512
-// A segment's share (one head, one tile of value columns) token by token, from the state as the step found it: for outputs that came out
-// infinite or NaN.  Within a chunk the weights of later tokens are set to zero, which does not keep their infinities out of earlier tokens'
-// sums; here a token sees its own and earlier ones only.  Slow (some microseconds a token), and apart from the chunks' loop, which it
-// would cost registers: with the chunk's own sums formed once more in place 2,048 tokens of 4 heads of 256 x 512 took 271 us a layer, so 263.
+// A segment's share (one head, one tile of value columns) token by token, from the state as the step found it: for values that are infinite
+// or NaN.  Within a chunk the weights of later tokens are set to zero, which does not keep their infinities out of earlier tokens' sums;
+// here a token sees its own and earlier ones only.  Slow (some microseconds a token), and apart from the chunks' loop, which it would
+// cost registers (2,048 tokens of 4 heads of 256 x 512: 271 us a layer with the chunk's own sums formed once more in place, 264 so).
 template <int KIND, int VT>
 __device__ __noinline__ void lc_token_by_token(const ScanArgs& a, int s, int h, int tile, float* S) {
   constexpr int PARTS = LC_THREADS / VT;
@@ -745,7 +744,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
       }
   }
 
-  bool finite = true;                                // of this thread's outputs
+  uint32_t odd = 0;                                  // bits 15 and 31: a value of this thread's had an exponent of all ones
+  int any_odd = 0;                                   // some thread's had
   for (int c = 0; c < nchunks; ++c) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                 // chunk c and its gates are in place; everyone is done with chunk c - 1
@@ -759,6 +759,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
       for (int i = tid; i < LC_C * VT / 2; i += 256) {
         const int t = i / (VT / 2), cc = (i - t * (VT / 2)) * 2;
         const float cj = gt.c[t];
+        odd |= (*(const uint32_t*)(vc + t * LDV + cc) & 0x7fff7fffu) + 0x00800080u;
         uint32_t w[3];
         lc_split3(cj * to_f(vc[t * LDV + cc]), cj * to_f(vc[t * LDV + cc + 1]), w);
 #pragma unroll
@@ -891,7 +892,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
         *(float2*)(d + 8 * LDR) = make_float2(hi[nb][2] + lo[nb][2], hi[nb][3] + lo[nb][3]);
       }
     }
-    __syncthreads();                                 // the terms of c v and all sums are in place
+    any_odd |= __syncthreads_or(odd & 0x80008000u);  // the terms of c v and all sums are in place
     if (warp < 8) {
       float up[2 * NK][4] = {}, lo[2 * NK][4] = {};
 #pragma unroll
@@ -958,13 +959,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
           y.x = fmaf(b3, to_f(vr[0]), y.x); y.y = fmaf(b3, to_f(vr[1]), y.y); y.z = fmaf(b3, to_f(vr[2]), y.z); y.w = fmaf(b3, to_f(vr[3]), y.w);
         }
         *(float4*)(a.out + (size_t)(q0 + c * LC_C + t) * a.ld_out + (size_t)h * dv + tile * VT + cc) = y;
-        finite = finite && lc_finite(y);
       }
     }
     // the logarithms of the batch that begins with chunk c + 2 (the present one's last gates were worked out ahead of the barrier)
     if ((c + 2) % (LC_BATCH / LC_C) == 0) work_logs((c + 2) * LC_C);
   }
-  if (__syncthreads_or(!finite)) return lc_token_by_token<KIND, VT>(a, s, h, tile, (float*)lc_smem);
+  if (any_odd) {
+    __syncthreads();                                 // all are done with shared memory and with their outputs
+    return lc_token_by_token<KIND, VT>(a, s, h, tile, (float*)lc_smem);
+  }
   if (warp < 8) {
 #pragma unroll
     for (int nt = 0; nt < 2 * NK; ++nt)
