@@ -658,8 +658,14 @@ def diff_attention(out, q, cache_layer, ctx, block_table, H, G, n, dv, page, win
             splits = diff_attention_splits(n1, H, G, window, ctx.max_ctx_len)
             ok = diff_attention_tc(out, q, cache_layer, ctx.seg_q_start, ctx.seg_pos0, block_table, n1, 1, *args, splits=splits)
         end = S                                      # segments from here on: the tcgen05 kernel
-        if ctx.max_q_len >= DIFF_ROWS_FROM and _pairs(ctx, DIFF_ROWS_FROM, window) * H >= DIFF_ROWS_WORK:
-            end = diff_rows_first(ctx.seg_len)
+        if ctx.max_q_len >= DIFF_ROWS_FROM:
+            work = _pairs(ctx, DIFF_ROWS_FROM, window) * H
+            if work >= DIFF_ROWS_WORK:
+                end = diff_rows_first(ctx.seg_len)
+                # short segments between the single tokens and the first portion are a launch of their own beside it, which small portions
+                # do not pay for: eight of 20 tokens ahead of 600, 8 heads (1.4 M), 93 us a layer in one launch and 99; 16 heads 150 and 138
+                if n1 < end < S and work < 2 * DIFF_ROWS_WORK:
+                    end = S
         if ok and end < S and not diff_attention_rows(out, q, cache_layer, ctx, block_table, end, *args):
             end = S
         if ok and n1 < end:

@@ -100,7 +100,7 @@ def test_rows_that_nobody_sees_may_hold_anything(lens, past, window):
     assert torch.equal(run(lens, past, window, H, G, cache, table, q, 0.3), clean)
 
 
-@pytest.mark.parametrize("lens,past,window,first", [([1, 1, 200], [40, 700, 60], 64, 2), ([1, 20, 33, 130, 9], [5, 300, 0, 90, 40], 0, 3),
+@pytest.mark.parametrize("lens,past,window,first", [([1, 1, 200], [40, 700, 60], 64, 2), ([1, 20, 33, 200, 9], [5, 300, 0, 90, 40], 0, 3),
                                                     ([20, 300], [900, 0], 100, 1), ([64, 3, 3, 3], [0, 9, 9, 9], 0, 4), ([40, 63], [0, 0], 0, 2)])
 def test_a_step_is_shared_by_the_kernels(monkeypatch, lens, past, window, first):
     """One call over single tokens, short segments and portions: each kernel takes its segments, and no row is left out."""
