@@ -465,12 +465,13 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(int* __restrict__ row_t
 
 // Rows of a tile of grouped rows.  Tensor cores: a tile is the narrow operand of one accumulator and every tile of an expert reads the
 // expert's matrices once, so a tile should hold all rows of a usual expert; the shared memory that its room takes is taken from the
-// stages in flight.  R rows over E experts (0: not known): 32 for steps of up to 32 tokens (there the tokens themselves are the operand),
-// else the first of 64, 128, 256 that holds 4/3 of the mean (counts scatter around it).
+// stages in flight.  R rows over E experts (0: not known): for steps of up to MOE_DIRECT tokens the first of 32, 64, 128 that holds them all
+// (there the tokens themselves are the operand), else the first of 64, 128, 256 that holds 4/3 of the mean (counts scatter around it).
+#define MOE_DIRECT 128
 extern "C" int qv_moe_tile_rows(int tensor_cores, int tokens, int R, int E) {
   if (!tensor_cores) return MOE_BM;
   if (tokens <= 0 || E <= 0) return 64;
-  if (tokens <= 32) return 32;
+  if (tokens <= MOE_DIRECT) return tokens <= 32 ? 32 : tokens <= 64 ? 64 : 128;
   const long long want = (4LL * R + 3LL * E - 1) / (3LL * E);
   return want <= 64 ? 64 : want <= 128 ? 128 : 256;
 }
@@ -599,7 +600,7 @@ extern "C" int qv_moe_experts(int up, void* out, int ld_out, const void* a, int 
 }
 
 // ---------------------------------------------------------------- the experts' products on the tensor cores (bfloat16)
-// Weights are the 128-row operand of tcgen05.mma, a tile's grouped rows (or, for steps of up to 32 tokens, all tokens) the narrow one,
+// Weights are the 128-row operand of tcgen05.mma, a tile's grouped rows (or, for steps of up to MOE_DIRECT tokens, all tokens) the narrow one,
 // so an expert's matrices are read once per tile of rows whatever the number of rows, and rows are padded to 16 only.  One CTA per SM
 // walks over (tile, block of features) items, features fastest: the CTAs at work share a tile's rows in L2 and stream different weights.
 //   warp 0      weights by contiguous bulk copies (packed tiles), rows by TMA in boxes of 32 rows x 64 k, through a ring of STAGES
@@ -850,14 +851,14 @@ extern "C" int qv_moe_pack_experts(void* out, const void* w, int E, int N, int K
 // As qv_moe_experts for bfloat16 operands, on the tensor cores, with the experts' matrices packed in tiles of 64 x 64
 // ([E][ceil(N/64)][ceil(K/64)][64][64], zero-padded, the eight 16-byte chunks of row r at chunk ^ (r % 8): the image the product
 // reads from shared memory).  tile_rows: what the tile table was made for (32, 64, 128 or 256).  a_rows: the rows of `a`.
-// gathered: room for R rows of K elements, for up products of more than 32 tokens.  Refuses rows of `a` that do not start on 16 bytes.
+// gathered: room for R rows of K elements, for up products of more tokens than MOE_DIRECT or a tile's rows.  Refuses rows of `a` that do not start on 16 bytes.
 extern "C" int qv_moe_experts_tc(int up, void* out, int ld_out, const void* a, int ld_a, int a_rows, const void* w1, const void* w2,
                                  const int* row_token, const int* tiles, int R, int E, int N, int K, int act, float limit, float slope,
                                  int tile_rows, void* gathered, int* err, void* stream) {
   if (R <= 0) return 0;
   if (act < 0 || act > 2 || up < 0 || up > 2 || N <= 0 || K < 8 || (K & 7)) return QV_ERR_UNSUPPORTED;
   if ((ld_a & 7) || (((uintptr_t)a | (uintptr_t)w1 | (uintptr_t)w2) & 15)) return QV_ERR_UNSUPPORTED;
-  const bool direct = up && a_rows <= 32;
+  const bool direct = up && a_rows <= MOE_DIRECT && a_rows <= tile_rows;
   cudaStream_t st = (cudaStream_t)stream;
   ExpertsArgs p;
   p.out = out; p.w1 = (const uint8_t*)w1; p.w2 = (const uint8_t*)w2; p.row_token = row_token; p.tiles = tiles; p.err = err;

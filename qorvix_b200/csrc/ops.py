@@ -1386,6 +1386,9 @@ def moe_route(top_idx, top_w, gate_out, h, w_router, w_gate, correction=None, w_
         add_launches(1)
 
 
+MOE_DIRECT = 128                           # steps of up to this many tokens: the tokens themselves are the products' narrow operand
+
+
 @functools.lru_cache(maxsize=256)           # of the sizes alone; a step asks for each of its layers
 def moe_tile_rows(tensor_cores: bool, tokens: int = 0, rows: int = 0, experts: int = 0) -> int:
     """Rows of a tile of grouped rows: what the tile table is made for (the two experts' kernels differ, and the tensor-core kernel
@@ -1424,7 +1427,7 @@ def moe_pack_experts(w: torch.Tensor) -> torch.Tensor:
 def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, limit: float = 0.0, slope: float = 0.0, tile_rows: int = 0, room=None) -> None:
     """The experts' products on the tensor cores (bfloat16); up as for moe_experts.  p1, p2: matrices packed by moe_pack_experts; the sizes
     follow from out [R, N] and a [., K]; the tile table was made for tiles of `tile_rows` rows (0: moe_tile_rows(True)).  room: a tensor
-    of at least R * K * 2 bytes that up products of more than 32 tokens may write their rows in grouped order to (the down product's
+    of at least R * K * 2 bytes that up products of more tokens than MOE_DIRECT or a tile's rows may write their rows in grouped order to (the down product's
     output will do: it is written when they are done with)."""
     _need_cuda(out, a, p1, p2, row_token, tiles, room)
     R, N = out.shape
@@ -1435,7 +1438,7 @@ def moe_experts_tc(up, out, a, p1, p2, row_token, tiles, act: int = GLU_SILU, li
     assert p2 is None or (p2.is_contiguous() and p2.shape == p1.shape and p2.dtype == p1.dtype)
     assert out.dtype == (torch.bfloat16 if up else torch.float32) and (up or a.shape[0] == R)
     tile_rows = tile_rows or moe_tile_rows(True)
-    gathers = bool(up) and a.shape[0] > 32                     # the rows in grouped order, for the up products of longer steps
+    gathers = bool(up) and a.shape[0] > min(MOE_DIRECT, tile_rows)       # the rows in grouped order, for the up products of longer steps
     if gathers and (room is None or not room.is_contiguous() or room.nbytes < R * K * 2):
         room = torch.empty((R, K), device=a.device, dtype=a.dtype)
     rc = _lib("moe").qv_moe_experts_tc(int(up), _ptr(out), out.stride(0), _ptr(a), a.stride(0), a.shape[0], _ptr(p1), _ptr(p2),

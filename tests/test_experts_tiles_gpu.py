@@ -50,3 +50,23 @@ def test_products_at_tile_edges(T, E, top, K, N, up):
     # K float32 products of order 1/sqrt(K): an absolute error of some K^0.5 * 2^-24, twice that behind a product of two; bfloat16 rounding
     bound = 2e-5 * (1 + want.abs()) + (2.0 ** -8 * want.abs() if up else 0.0)
     assert bool(((got - want).abs() <= bound).all()), float((got - want).abs().max())
+
+
+@pytest.mark.parametrize("T", [33, 64, 65, 128, 129])
+def test_the_tokens_themselves_as_the_narrow_operand(T):
+    """Up to 128 tokens the up product reads the tokens where they lie: the same bits as from rows in grouped order, with an expert that has
+    all tokens and one that has none."""
+    E, top, K, N = 5, 2, 72, 72
+    g = torch.Generator(device="cuda").manual_seed(T)
+    idx = torch.stack([torch.zeros(T, device="cuda"), torch.randint(1, E - 1, (T,), generator=g, device="cuda")], dim=1).to(torch.int32).contiguous()
+    w = ops.moe_pack_experts(torch.randn((E, N, K), generator=g, device="cuda").to(torch.bfloat16))
+    x = torch.randn((T, K + 8), generator=g, device="cuda").to(torch.bfloat16)[:, :K]
+    rows = []
+    for tile_rows in (ops.moe_tile_rows(True, T, T * top, E), 32):          # (a table of 32 rows a tile: 33 tokens and more are gathered)
+        row_token, slot_row, tiles = grouped(idx, E, tile_rows)
+        out = torch.empty((T * top, N), device="cuda", dtype=torch.bfloat16)
+        ops.moe_experts_tc(2, out, x, w, None, row_token, tiles, tile_rows=tile_rows)
+        ops.check_kernel_errors()
+        rows.append(out[slot_row.long()])
+    assert ops.moe_tile_rows(True, T, T * top, E) >= min(T, 128)
+    assert torch.equal(rows[0], rows[1])
