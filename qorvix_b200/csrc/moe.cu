@@ -467,6 +467,8 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(int* __restrict__ row_t
 // expert's matrices once, so a tile should hold all rows of a usual expert; the shared memory that its room takes is taken from the
 // stages in flight.  R rows over E experts (0: not known): for steps of up to MOE_DIRECT tokens the first of 32, 64, 128 that holds them all
 // (there the tokens themselves are the operand), else the first of 64, 128, 256 that holds 4/3 of the mean (counts scatter around it).
+// us a layer with rows gathered and with the tokens themselves, 32 experts of 704 x 1,024: 33 tokens 98 and 95, 128 tokens 98 and 95; 64 of
+// 1,408 x 2,048: 33 tokens 210 and 206, 128 tokens 227 and 224.  Beyond 128 tokens the operand would take more of a stage than the weights.
 #define MOE_DIRECT 128
 extern "C" int qv_moe_tile_rows(int tensor_cores, int tokens, int R, int E) {
   if (!tensor_cores) return MOE_BM;
