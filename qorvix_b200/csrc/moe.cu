@@ -465,15 +465,16 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(int* __restrict__ row_t
 
 // Rows of a tile of grouped rows.  Tensor cores: a tile is the narrow operand of one accumulator and every tile of an expert reads the
 // expert's matrices once, so a tile should hold all rows of a usual expert; the shared memory that its room takes is taken from the
-// stages in flight.  R rows over E experts (0: not known): for steps of up to MOE_DIRECT tokens the first of 32, 64, 128 that holds them all
+// stages in flight.  R rows over E experts (0: not known): for steps of up to MOE_DIRECT tokens the first of 32, 64 that holds them all
 // (there the tokens themselves are the operand), else the first of 64, 128, 256 that holds 4/3 of the mean (counts scatter around it).
-// us a layer with rows gathered and with the tokens themselves, 32 experts of 704 x 1,024: 33 tokens 98 and 95, 128 tokens 98 and 95; 64 of
-// 1,408 x 2,048: 33 tokens 210 and 206, 128 tokens 227 and 224.  Beyond 128 tokens the operand would take more of a stage than the weights.
-#define MOE_DIRECT 128
+// us a layer with rows gathered and with the tokens themselves, 32 experts of 704 x 1,024: 33 tokens 98 and 94, 64 tokens 98 and 94; 64 of
+// 1,408 x 2,048: 33 tokens 210 and 206, 64 tokens 219 and 218, but 100 tokens, inputs not in L2, 223 and 229: there the operand is as many
+// bytes of a stage as the weights.
+#define MOE_DIRECT 64
 extern "C" int qv_moe_tile_rows(int tensor_cores, int tokens, int R, int E) {
   if (!tensor_cores) return MOE_BM;
   if (tokens <= 0 || E <= 0) return 64;
-  if (tokens <= MOE_DIRECT) return tokens <= 32 ? 32 : tokens <= 64 ? 64 : 128;
+  if (tokens <= MOE_DIRECT) return tokens <= 32 ? 32 : 64;
   const long long want = (4LL * R + 3LL * E - 1) / (3LL * E);
   return want <= 64 ? 64 : want <= 128 ? 128 : 256;
 }

@@ -1018,6 +1018,7 @@ def unit_keys(u, au, k, a, a_bias, H: int, n: int, eps: float) -> None:
     _check(rc, "unit_keys")
 
 
+@functools.lru_cache(maxsize=256)           # of the sizes alone
 def channel_scan_state_floats(H: int, dk: int, dv: int) -> int:
     """How many float32 values channel_scan keeps per request for H heads of dk x dv."""
     return int(_lib("channel_scan").qv_channel_scan_state_floats(H, dk, dv))
@@ -1386,7 +1387,7 @@ def moe_route(top_idx, top_w, gate_out, h, w_router, w_gate, correction=None, w_
         add_launches(1)
 
 
-MOE_DIRECT = 128                           # steps of up to this many tokens: the tokens themselves are the products' narrow operand
+MOE_DIRECT = 64                            # steps of up to this many tokens: the tokens themselves are the products' narrow operand
 
 
 @functools.lru_cache(maxsize=256)           # of the sizes alone; a step asks for each of its layers
