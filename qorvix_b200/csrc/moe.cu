@@ -159,6 +159,8 @@ __device__ __forceinline__ void route_dot_tile(const TW* const (&w)[ROUTE_ROWS],
 // Many tokens: a CTA takes ROUTE_TOKENS tokens and walks over all rows, four rows a warp at a time.  What bounds it is the
 // multiply-adds with the conversions around them: a row alone (eight tokens in float32 in shared memory, so 16 bytes read there for
 // four multiply-adds) took 170 us for 2,048 tokens x 65 rows x 2,048.
+// Router as a whole (us, 2,048 wide, 65 / 256 rows), with a row alone over tokens x groups of rows and with this kernel: 257 tokens 35 / 87
+// and 26 / 58, 512 tokens 59 / 147 and 26 / 58, 1,024 tokens 89 / 267 and 27 / 59, 2,048 tokens 164 / 493 and 39 / 99.
 template <typename T, typename TW>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_logits_tokens_kernel(float* __restrict__ logits, const T* __restrict__ h, int ld_h,
                                                                              const TW* __restrict__ wr, const TW* __restrict__ wg, int d,
