@@ -142,7 +142,8 @@ struct ScanArgs {
   float* state; long long slot_stride;    // per slot: [H][tiles][dk * 32 (+ dk + 1 for GATED_MAX)]
   const int* seg_q_start; const int* seg_slot;
   int H, dk, dv;
-  int chunk_from;                         // segments of at least this many tokens are linear_scan_chunk_kernel's (INT_MAX: none)
+  int chunk_from;                         // segments of at least this many tokens are linear_scan_chunk_kernel's (INT_MAX: none),
+  int parallel_from;                      // of at least this many lp_states_kernel's and lp_outputs_kernel's
 };
 
 __host__ __device__ inline int scan_tile_floats(int kind, int dk, int vt = SCAN_VT) { return dk * vt + (kind == SCAN_GATED_MAX ? dk + 1 : 0); }
@@ -465,6 +466,15 @@ __device__ __forceinline__ void lc_mma(float* c, const uint32_t* a, uint32_t b0,
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same from zero.
+__device__ __forceinline__ void lc_mma0(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void lc_mma(bool first, float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  if (first) lc_mma0(c, a, b0, b1);
+  else lc_mma(c, a, b0, b1);
+}
 // x and y as three bfloat16 terms each (x in the lower half of a word)
 __device__ __forceinline__ void lc_split3(float x, float y, uint32_t (&t)[3]) {
 #pragma unroll
@@ -514,28 +524,34 @@ template <int VT, int NK> struct LcShape {
 // or NaN.  Within a chunk the weights of later tokens are set to zero, which does not keep their infinities out of earlier tokens' sums;
 // here a token sees its own and earlier ones only.  Slow (some microseconds a token), and apart from the chunks' loop, which it would
 // cost registers (2,048 tokens of 4 heads of 256 x 512: 271 us a layer with the chunk's own sums formed once more in place, 264 so).
-template <int KIND, int VT>
-__device__ __noinline__ void lc_token_by_token(const ScanArgs& a, int s, int h, int tile, float* S) {
-  constexpr int PARTS = LC_THREADS / VT;
+// n0: n ahead of the first token, n_parts sums of n_ld entries.
+template <int KIND, int VT, int THREADS>
+__device__ __noinline__ void lc_token_by_token(const ScanArgs& a, const float* n0, int n_parts, int n_ld, int s, int q0, int len, int h, int tile,
+                                               float* S) {
+  constexpr int PARTS = THREADS / VT;
   const int dk = a.dk, tid = threadIdx.x, col = tid % VT, part = tid / VT;
   float* qs = S + dk * VT;                           // S [dk][VT]
   float* ks = qs + dk;
   float* ns = ks + dk;
   float* sums = ns + dk;                             // [PARTS][VT]
-  float* sc = sums + LC_THREADS;                     // n . q
-  const int tiles = (a.dv + VT - 1) / VT, q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  float* sc = sums + THREADS;                     // n . q
+  const int tiles = (a.dv + VT - 1) / VT;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk, VT);
-  for (int i = tid; i < dk * VT; i += LC_THREADS) S[i] = st[i];
+  for (int i = tid; i < dk * VT; i += THREADS) S[i] = st[i];
   float m = 0.f;
   if (KIND == SCAN_GATED_MAX) {
-    for (int i = tid; i < dk; i += LC_THREADS) ns[i] = st[dk * VT + i];
+    for (int i = tid; i < dk; i += THREADS) {
+      float n = 0.f;
+      for (int p = 0; p < n_parts; ++p) n += n0[(size_t)p * n_ld + i];
+      ns[i] = n;
+    }
     m = st[dk * VT + dk];
   }
   const bool live = tile * VT + col < a.dv;
   const float b1 = a.p1 ? a.p1[h] : 0.f, b2 = a.p2 ? a.p2[h] : 0.f, b3 = a.p3 ? a.p3[h] : 0.f;
   for (int j = 0; j < len; ++j) {
     const size_t t = (size_t)(q0 + j);
-    for (int i = tid; i < dk; i += LC_THREADS) {
+    for (int i = tid; i < dk; i += THREADS) {
       qs[i] = to_f(((const bf16*)a.q)[t * a.ld_q + (size_t)(h / a.q_group) * dk + i]) * a.q_scale;
       ks[i] = to_f(((const bf16*)a.k)[t * a.ld_k + (size_t)(h / a.q_group) * dk + i]);
     }
@@ -580,11 +596,12 @@ __device__ __noinline__ void lc_token_by_token(const ScanArgs& a, int s, int h, 
     }
   }
   __syncthreads();
-  for (int i = tid; i < dk * VT; i += LC_THREADS) st[i] = S[i];
+  for (int i = tid; i < dk * VT; i += THREADS) st[i] = S[i];
   if (KIND == SCAN_GATED_MAX) {
-    for (int i = tid; i < dk; i += LC_THREADS) st[dk * VT + i] = ns[i];
+    for (int i = tid; i < dk; i += THREADS) st[dk * VT + i] = ns[i];
     if (tid == 0) st[dk * VT + dk] = m;
   }
+  __syncthreads();
 }
 
 template <int KIND, int VT, int NK>
@@ -607,7 +624,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
   const int s = blockIdx.x, h = blockIdx.y, tile = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  if (len < a.chunk_from) return;
+  if (len < a.chunk_from || len >= a.parallel_from) return;
   const int dk = a.dk, dv = a.dv;
   const int tiles = (dv + VT - 1) / VT;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile) * scan_tile_floats(KIND, dk, VT);
@@ -966,7 +983,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
   }
   if (any_odd) {
     __syncthreads();                                 // all are done with shared memory and with their outputs
-    return lc_token_by_token<KIND, VT>(a, s, h, tile, (float*)lc_smem);
+    return lc_token_by_token<KIND, VT, LC_THREADS>(a, st + dk * VT, 1, 0, s, q0, len, h, tile, (float*)lc_smem);
   }
   if (warp < 8) {
 #pragma unroll
@@ -996,6 +1013,648 @@ static int launch_scan_chunk(const ScanArgs& a, dim3 grid, cudaStream_t st) {
   return qv_launch(kernel, grid, dim3(LC_THREADS), (size_t)LcShape<VT, NK>::BYTES, st, a);
 }
 
+// ---------------------------------------------------------------- long portions: the chunks' outputs side by side
+// Of a chunk only S_end = A S_0 + ... goes to the next one.  So for long portions the chunks' arithmetic (above) is dealt to three launches:
+//   lp_gates_kernel     what a chunk's gates amount to (LpGates), a warp a chunk
+//   lp_states_kernel    a CTA owns 64 keys x 64 value columns of a (segment, head) and walks the chunks; the state ahead of each goes to a
+//                       workspace
+//   lp_outputs_kernel   a CTA per (chunk, head, up to 256 value columns) forms q S_0 and W v, all chunks at once
+// The states lie in the workspace as the products' accumulators lie in the lanes, and S^T's accumulators are S's operand for q S_0, so a
+// state is written and read in whole 512-byte pieces and passes through no shared memory.  The update's arithmetic is that of
+// linear_scan_chunk_kernel to the bit.  2,048 tokens of 4 heads of 256 x 512: 173 us in one kernel (32 chunks in a row, W formed again for each
+// tile of 16 columns); gates 8, states 48, outputs 44 here.  Bound by the states' chain of chunks and, in the outputs, by the instructions that
+// split float32 into three terms; the workspace (2 MB a chunk) is read from L2.
+#define LP_KEYS 64                         // keys and value columns a CTA of lp_states_kernel holds
+#define LP_COLS 256                        // value columns a CTA of lp_outputs_kernel forms
+#define LP_THREADS 256
+#define LP_NPARTS 4                        // sums that n is kept in
+struct LpGates {                           // what a chunk's gates amount to; 16-byte pieces
+  float2 G[LC_C], H[LC_C];                 // a number and what rounding it to float32 left over
+  float A[LC_C], em[LC_C];                 // em: exp(-m_t)
+  float R[3][LC_C], E[LC_C];               // blocks of 16 tokens, M_i the largest H in block i: exp(G_t + M_i) for t behind it, exp(H_j - M)
+  float c[LC_C], A_end, m_end, pad[2];     // what the states' kernel reads
+};
+
+// The workspace of one launch of the three: chunks c0 ... c0 + P - 1 of every segment, a slot each.
+struct LpWork {
+  float* S;                                // [slots][H][col tiles of 16][key tiles of 8][32 lanes][4]
+  float* n;                                // [slots][H][LP_NPARTS][dkp], n as sums
+  LpGates* gates;                          // [slots][H]
+  double* m;                               // [segments][H]: the running maximum behind chunk c0 + P - 1
+  int* odd;                                // [segments][H][blocks of 64 columns]: some value was infinite or NaN
+  int P, c0, dkp, ct, vt;                  // dkp: dk in whole runs of 32; ct: column tiles of 16; vt: columns a tile of the state
+};
+static inline size_t lp_slot_bytes(int H, int dk, int dv) {
+  const size_t dkp = (dk + 31) / 32 * 32, ct = (dv + 15) / 16;
+  return (size_t)H * (ct * dkp * 64 + LP_NPARTS * dkp * 4 + sizeof(LpGates));
+}
+static inline size_t lp_segment_bytes(int H, int dv) { return (size_t)H * (8 + (size_t)((dv + 63) / 64) * 4); }
+
+// grid (segments, heads); a warp takes a chunk: two neighbouring tokens a lane, sums and maxima by scans over the warp.  Bound by the
+// latency of its scans and functions.  In lp_states_kernel itself they cost more: a ninth warp there takes 2.5 us a chunk, which otherwise
+// takes 1.4.
+#define LP_GATE_WARPS 32
+__global__ void __launch_bounds__(32 * LP_GATE_WARPS) lp_gates_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ LpWork w) {
+  __shared__ double ends[LP_GATE_WARPS][2];          // F_63 and max H of the warps' chunks
+  pdl_wait();
+  pdl_launch_dependents();
+  const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len < a.parallel_from) return;
+  const int nchunks = (len + LC_C - 1) / LC_C, last = nchunks < w.c0 + w.P ? nchunks : w.c0 + w.P;
+  const float b1 = a.p1 ? a.p1[h] : 0.f, b2 = a.p2 ? a.p2[h] : 0.f;
+  const int tiles = (a.dv + w.vt - 1) / w.vt;
+  double m_next = w.c0 ? w.m[(size_t)s * a.H + h]
+                       : (double)a.state[(size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * scan_tile_floats(SCAN_GATED_MAX, a.dk, w.vt) +
+                                         (size_t)a.dk * w.vt + a.dk];
+  for (int c1 = w.c0; c1 < last; c1 += LP_GATE_WARPS) {
+    const int c = c1 + warp;
+    double lf[2], li[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = c * LC_C + 2 * lane + i;
+      lf[i] = 0.0; li[i] = -1e30;                    // a token beyond the segment: keeps all, adds nothing
+      if (c < last && t < len) {
+        const size_t row = (size_t)(q0 + t);
+        const float zf = a.cap * tanhf((a.g2[row * a.ld_g2 + h] + b2) / a.cap);
+        lf[i] = (double)(fminf(zf, 0.f) - log1pf(expf(-fabsf(zf))));
+        li[i] = (double)(a.cap * tanhf((a.g1[row * a.ld_g1 + h] + b1) / a.cap));
+      }
+    }
+    double sum = lf[0] + lf[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+    }
+    const double sum_ahead = __shfl_up_sync(0xffffffffu, sum, 1);
+    double F[2], Hh[2], G[2], m[2], m_run = 0.0;
+    F[1] = sum;
+    F[0] = (lane ? sum_ahead : 0.0) + lf[0];         // (not sum - lf[1]: a token's gates say nothing about the token ahead of it)
+    Hh[0] = li[0] - F[0]; Hh[1] = li[1] - F[1];
+    double mx = fmax(Hh[0], Hh[1]);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, mx, o);
+      if (lane >= o) mx = fmax(mx, up);
+    }
+    if (lane == 31) { ends[warp][0] = F[1]; ends[warp][1] = mx; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < LP_GATE_WARPS; ++i) {
+      if (i == warp) m_run = m_next;
+      m_next = ends[i][0] + fmax(m_next, ends[i][1]);
+    }
+    const double ahead = __shfl_up_sync(0xffffffffu, mx, 1);
+    const double before = lane ? fmax(m_run, ahead) : m_run;
+    m[0] = F[0] + fmax(before, Hh[0]);
+    m[1] = F[1] + fmax(m_run, mx);
+    G[0] = F[0] - m[0]; G[1] = F[1] - m[1];
+    const double G_end = __shfl_sync(0xffffffffu, G[1], 31), m_end = __shfl_sync(0xffffffffu, m[1], 31);
+    double M = fmax(Hh[0], Hh[1]);                   // of the 16 tokens of eight lanes
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) M = fmax(M, __shfl_xor_sync(0xffffffffu, M, o));
+    double Mi[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Mi[i] = __shfl_sync(0xffffffffu, M, 8 * i);
+    if (c < last) {
+      LpGates& gt = w.gates[((size_t)s * w.P + c - w.c0) * a.H + h];
+      float2 pair[2];
+      pair[0] = lc_pair(G[0]); pair[1] = lc_pair(G[1]);
+      *(float4*)(gt.G + 2 * lane) = make_float4(pair[0].x, pair[0].y, pair[1].x, pair[1].y);
+      pair[0] = lc_pair(Hh[0]); pair[1] = lc_pair(Hh[1]);
+      *(float4*)(gt.H + 2 * lane) = make_float4(pair[0].x, pair[0].y, pair[1].x, pair[1].y);
+      *(float2*)(gt.A + 2 * lane) = make_float2(expf((float)(G[0] + m_run)), expf((float)(G[1] + m_run)));
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        *(float2*)(gt.R[i] + 2 * lane) = lane >= 8 * i + 8 ? make_float2(expf((float)(G[0] + Mi[i])), expf((float)(G[1] + Mi[i]))) : make_float2(0.f, 0.f);
+      *(float2*)(gt.E + 2 * lane) = make_float2(expf((float)(Hh[0] - M)), expf((float)(Hh[1] - M)));
+      *(float2*)(gt.c + 2 * lane) = make_float2(expf((float)(G_end + Hh[0])), expf((float)(G_end + Hh[1])));
+      *(float2*)(gt.em + 2 * lane) = make_float2(expf((float)-m[0]), expf((float)-m[1]));
+      if (lane == 0) { gt.A_end = expf((float)(G_end + m_run)); gt.m_end = (float)m_end; }
+    }
+    __syncthreads();                                 // the ends have been read
+  }
+  if (threadIdx.x == 0) w.m[(size_t)s * a.H + h] = m_next;
+}
+
+// grid (segments, heads, key blocks x column blocks, then the key blocks once more for n).  Eight warps hold the state as S^T, 16
+// columns x 32 keys each.  The terms of c v are formed once a CTA, a chunk ahead of the products that read them, so a chunk is one stretch
+// between barriers; k, v and the gates arrive ahead of that (cp.async).  Bound by the latency of a chunk's products and of the terms' way
+// through shared memory: 1.4 us a chunk.  (With the terms formed in registers by both warps that share columns, and n by a ninth warp, three
+// warps on one scheduler: 1.75.)
+struct LpStatesSmem {
+  bf16 k[3][LC_C][LP_KEYS + 8], v[2][LC_C][LP_KEYS + 8], terms[2][3][LC_C][LP_KEYS + 8];
+  float c[3][LC_C + 4];                    // then A_end
+};
+__global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ LpWork w) {
+  extern __shared__ __align__(16) unsigned char lp_smem[];
+  LpStatesSmem& sm = *(LpStatesSmem*)lp_smem;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int s = blockIdx.x, h = blockIdx.y;
+  const int nkb = (a.dk + LP_KEYS - 1) / LP_KEYS, ncb = (a.dv + LP_KEYS - 1) / LP_KEYS, kb = blockIdx.z % nkb, cb = blockIdx.z / nkb;
+  const bool is_n = cb == ncb;                       // this CTA sums n
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len < a.parallel_from) return;
+  const int dk = a.dk, dv = a.dv, vt = w.vt, tiles = (dv + vt - 1) / vt, tf = scan_tile_floats(SCAN_GATED_MAX, dk, vt);
+  const int nchunks = (len + LC_C - 1) / LC_C, count = (nchunks < w.c0 + w.P ? nchunks : w.c0 + w.P) - w.c0;
+  if (count <= 0) return;
+  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * tf;
+  const int g8 = lane >> 2, t4 = lane & 3, mi = lane >> 3, r8 = lane & 7;
+  const int kw = kb * LP_KEYS + (warp >> 2) * 32, cw = cb * LP_KEYS + (warp & 3) * 16;        // a warp's keys and columns
+  const bool holds = !is_n && cw < dv && kw < w.dkp;
+  const LpGates* gates = w.gates + (size_t)s * w.P * a.H + h;
+
+  // a thread copies, and splits, the same 16 bytes of every 32nd row
+  const int row = tid >> 3, pc = tid & 7;
+  const int token0 = q0 + w.c0 * LC_C, left0 = len - w.c0 * LC_C;
+  const bf16* kp = (const bf16*)a.k + (size_t)(token0 + row) * a.ld_k + (size_t)(h / a.q_group) * dk + kb * LP_KEYS + pc * 8;
+  const bf16* vp = (const bf16*)a.v + (size_t)(token0 + row) * a.ld_v + (size_t)h * dv + cb * LP_KEYS + pc * 8;
+  const bool k_in = kb * LP_KEYS + pc * 8 < dk, v_in = !is_n && cb * LP_KEYS + pc * 8 < dv;
+  auto issue = [&](int c) {
+    if (c < count) {
+      const int left = left0 - c * LC_C;
+#pragma unroll
+      for (int i = 0; i < LC_C; i += 32) {
+        const bool lk = k_in && row + i < left, lv = v_in && row + i < left;
+        lc_cp16(&sm.k[c % 3][row + i][pc * 8], lk ? kp + (size_t)(c * LC_C + i) * a.ld_k : (const bf16*)a.k, lk);
+        if (!is_n) lc_cp16(&sm.v[c & 1][row + i][pc * 8], lv ? vp + (size_t)(c * LC_C + i) * a.ld_v : (const bf16*)a.v, lv);
+      }
+      if (tid < (LC_C + 4) / 4) lc_cp16(sm.c[c % 3] + tid * 4, gates[(size_t)c * a.H].c + tid * 4, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint32_t odd = 0;                                  // bits 15 and 31: a value had an exponent of all ones
+  auto split = [&](int c) {                          // c_j v_j in three terms
+#pragma unroll
+    for (int i = 0; i < LC_C; i += 32) {
+      const uint4 raw4 = *(const uint4*)&sm.v[c & 1][row + i][pc * 8];
+      const uint32_t raw[4] = {raw4.x, raw4.y, raw4.z, raw4.w};
+      const float cj = sm.c[c % 3][row + i];
+      uint32_t t[4][3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        odd |= (raw[e] & 0x7fff7fffu) + 0x00800080u;
+        const __nv_bfloat162 vv = *(const __nv_bfloat162*)&raw[e];
+        lc_split3(cj * __low2float(vv), cj * __high2float(vv), t[e]);
+      }
+#pragma unroll
+      for (int x = 0; x < 3; ++x) *(uint4*)&sm.terms[c & 1][x][row + i][pc * 8] = make_uint4(t[0][x], t[1][x], t[2][x], t[3][x]);
+    }
+  };
+  issue(0);
+  issue(1);
+  float sT[4][4] = {};                               // S^T: value columns cw + g8 (+ 8), keys kw + 8 nt + 2 t4 (+ 1)
+  if (holds) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = kw + nt * 8 + 2 * t4 + (i & 1), col = cw + g8 + (i >> 1) * 8;
+        if (k < dk && col < tiles * vt) sT[nt][i] = st[(size_t)(col / vt) * tf + k * vt + col % vt];
+      }
+  }
+  const int nk = kb * LP_KEYS + 2 * lane;            // n: two keys a lane, a quarter of the tokens a warp
+  float n0 = 0.f, n1 = 0.f;
+  if (is_n && warp == 0 && nk < dk) { n0 = st[dk * vt + nk]; n1 = st[dk * vt + nk + 1]; }
+  if (!is_n) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    split(0);
+  }
+  for (int c = 0; c < count; ++c) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // chunk c + 1 is in place, and chunk c's terms; everyone is done with chunk c - 1
+    issue(c + 2);
+    const float* cs = sm.c[c % 3];
+    const bf16(*ks)[LP_KEYS + 8] = sm.k[c % 3];
+    const size_t slot = ((size_t)s * w.P + c) * a.H + h;
+    if (is_n) {
+      if (warp < LP_NPARTS) {
+        if (nk < w.dkp) *(float2*)(w.n + (slot * LP_NPARTS + warp) * w.dkp + nk) = make_float2(n0, n1);
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < LC_C / LP_NPARTS; j += 4) {
+          const float4 c4 = *(const float4*)(cs + warp * (LC_C / LP_NPARTS) + j);
+          const float cc[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const __nv_bfloat162 kv = *(const __nv_bfloat162*)&ks[warp * (LC_C / LP_NPARTS) + j + u][2 * lane];
+            a0 = fmaf(cc[u], __low2float(kv), a0);
+            a1 = fmaf(cc[u], __high2float(kv), a1);
+          }
+        }
+        n0 = fmaf(cs[LC_C], n0, a0);
+        n1 = fmaf(cs[LC_C], n1, a1);
+      }
+      continue;
+    }
+    if ((warp & 4) && c + 1 < count) split(c + 1);   // (half of the warps ahead of their products, the others behind them)
+    if (holds) {
+      float* ws = w.S + ((slot * w.ct + (cw >> 4)) * (w.dkp >> 3) + (kw >> 3)) * 128 + lane * 4;
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) *(float4*)(ws + nt * 128) = make_float4(sT[nt][0], sT[nt][1], sT[nt][2], sT[nt][3]);
+      float up[4][4], lo[4][4];
+#pragma unroll
+      for (int kk = 0; kk < LC_C; kk += 16) {
+        uint32_t af[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) lc_ldsm4t(af[x], &sm.terms[c & 1][x][kk + (mi >> 1) * 8 + r8][(warp & 3) * 16 + (mi & 1) * 8]);
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          uint32_t bk[4];
+          lc_ldsm4t(bk, &ks[kk + (mi & 1) * 8 + r8][(warp >> 2) * 32 + nb * 16 + (mi >> 1) * 8]);
+#pragma unroll
+          for (int x = 2; x >= 0; --x) {
+            lc_mma(kk == 0 && x != 1, x ? lo[2 * nb] : up[2 * nb], af[x], bk[0], bk[1]);
+            lc_mma(kk == 0 && x != 1, x ? lo[2 * nb + 1] : up[2 * nb + 1], af[x], bk[2], bk[3]);
+          }
+        }
+      }
+      const float ae = cs[LC_C];
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) sT[nt][x] = fmaf(ae, sT[nt][x], up[nt][x] + lo[nt][x]);
+    }
+    if (!(warp & 4) && c + 1 < count) split(c + 1);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (is_n) {
+    float2* sums = (float2*)sm.terms;                // [LP_NPARTS][32]: the terms' place, which these CTAs do not use
+    if (warp < LP_NPARTS) sums[warp * 32 + lane] = make_float2(n0, n1);
+    __syncthreads();
+    if (nk < dk) {
+      const float2 x0 = sums[lane], x1 = sums[32 + lane], x2 = sums[64 + lane], x3 = sums[96 + lane];
+      n0 = (x0.x + x1.x) + (x2.x + x3.x);
+      n1 = (x0.y + x1.y) + (x2.y + x3.y);
+      for (int tile = warp; tile < tiles; tile += LP_THREADS / 32) {
+        float* np = st + (size_t)tile * tf + dk * vt;
+        np[nk] = n0;
+        np[nk + 1] = n1;
+      }
+    }
+    return;
+  }
+  const int any_odd = __syncthreads_or(odd & 0x80008000u);
+  if (kb == 0 && tid == 0) w.odd[((size_t)s * a.H + h) * ncb + cb] = any_odd != 0;
+  if (any_odd) return;                               // the outputs' kernel goes token by token from the state as it is
+  if (holds) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = kw + nt * 8 + 2 * t4 + (i & 1), col = cw + g8 + (i >> 1) * 8;
+        if (k < dk && col < tiles * vt) st[(size_t)(col / vt) * tf + k * vt + col % vt] = sT[nt][i];
+      }
+  }
+  if (kb == 0) {
+    const int tile = cb * LP_KEYS / vt + tid;
+    if (tid < LP_KEYS / vt && tile < tiles) st[(size_t)tile * tf + dk * vt + dk] = gates[(size_t)(count - 1) * a.H].m_end;
+  }
+}
+
+// grid (slots, heads, blocks of LP_COLS value columns).  The warps form W's blocks of 16 x 16 tokens (above the diagonal there is nothing):
+// a warp the diagonal's block of 16 rows, with an exponential an entry, another those ahead of it, with two factors an entry (G_t + M and
+// H_j - M are <= 0 for M the largest H of tokens all ahead of t); the one with nothing to do forms n . q.  W takes k's place in shared
+// memory in three terms.  Then a warp takes 16 columns: q S_0 in runs of 32 keys, the next run's state in flight, then W v.
+struct LpOutShape {
+  int ldq, ldv, k_bytes, bytes;
+  __host__ __device__ LpOutShape(int dkp, int cols) {
+    ldq = dkp + 8;
+    ldv = cols + 8;
+    const int wterms = 3 * LC_C * (LC_C + 8) * 2, kb = LC_C * ldq * 2;
+    k_bytes = kb > wterms ? kb : wterms;
+    bytes = LC_C * ldq * 2 + k_bytes + LC_C * ldv * 2 + (int)sizeof(LpGates) + LC_C * 3 * 4 + dkp * 4;
+  }
+};
+__global__ void __launch_bounds__(LP_THREADS, 2) lp_outputs_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ LpWork w) {
+  extern __shared__ __align__(16) unsigned char lp_smem[];
+  constexpr int LDW = LC_C + 8;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int s = blockIdx.x / w.P, cr = blockIdx.x % w.P, c = w.c0 + cr, h = blockIdx.y;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
+  if (len < a.parallel_from || c * LC_C >= len) return;
+  const int dk = a.dk, dv = a.dv, dkp = w.dkp;
+  const int col0 = blockIdx.z * LP_COLS, cols = dv - col0 < LP_COLS ? (dv - col0 + 15) / 16 * 16 : LP_COLS;
+  const LpOutShape sh(dkp, cols);
+  bf16* qs = (bf16*)lp_smem;                                         // [64][ldq]
+  bf16* ks = qs + LC_C * sh.ldq;                                     // [64][ldq], then
+  bf16* wt = ks;                                                     // [3][64][LDW] the terms of W
+  bf16* vs = (bf16*)(lp_smem + LC_C * sh.ldq * 2 + sh.k_bytes);      // [64][ldv]
+  LpGates& gt = *(LpGates*)(vs + LC_C * sh.ldv);
+  float* rowsum = (float*)(&gt + 1);                                 // [64][2]
+  float* nq = rowsum + 2 * LC_C;                                     // [64] n_0 . q_t
+  float* ns = nq + LC_C;                                             // [dkp]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g8 = lane >> 2, t4 = lane & 3, mi = lane >> 3, r8 = lane & 7;
+  const size_t slot = (size_t)blockIdx.x * a.H + h;
+  const size_t t0 = (size_t)q0 + (size_t)c * LC_C;
+  const int left = len - c * LC_C;
+  {
+    const int pq = dkp >> 3, pv = cols >> 3;
+    const bool q_in = lane * 8 < dk, v_in = col0 + lane * 8 < dv;
+    const bf16* qp = (const bf16*)a.q + (t0 + warp) * a.ld_q + (size_t)(h / a.q_group) * dk + lane * 8;
+    const bf16* kp = (const bf16*)a.k + (t0 + warp) * a.ld_k + (size_t)(h / a.q_group) * dk + lane * 8;
+    const bf16* vp = (const bf16*)a.v + (t0 + warp) * a.ld_v + (size_t)h * dv + col0 + lane * 8;
+    bf16 *qd = qs + warp * sh.ldq + lane * 8, *kd = ks + warp * sh.ldq + lane * 8, *vd = vs + warp * sh.ldv + lane * 8;
+#pragma unroll
+    for (int i = 0; i < LC_C; i += 8) {
+      const bool live = warp + i < left, lq = live && q_in, lv = live && v_in;
+      if (lane < pq) {
+        lc_cp16(qd + i * sh.ldq, lq ? qp + (size_t)(i * a.ld_q) : (const bf16*)a.q, lq);
+        lc_cp16(kd + i * sh.ldq, lq ? kp + (size_t)(i * a.ld_k) : (const bf16*)a.k, lq);
+      }
+      if (lane < pv) lc_cp16(vd + i * sh.ldv, lv ? vp + (size_t)(i * a.ld_v) : (const bf16*)a.v, lv);
+    }
+    for (int i = tid; i < (int)sizeof(LpGates) / 16; i += LP_THREADS) lc_cp16((char*)&gt + i * 16, (const char*)(w.gates + slot) + i * 16, true);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // a warp's first runs of 32 keys of the state, on their way meanwhile
+  const int ncg = cols >> 4;
+  int cg = warp;
+  const float* Sp = w.S + (slot * w.ct + (col0 >> 4) + cg) * (size_t)(dkp >> 3) * 128 + lane * 4;
+  float4 next[4];
+  if (cg < ncg) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) next[i] = *(const float4*)(Sp + i * 128);
+  }
+  if (tid < dkp / 4) {
+    const float4* np = (const float4*)(w.n + slot * LP_NPARTS * dkp) + tid;
+    const float4 x0 = np[0], x1 = np[dkp / 4], x2 = np[dkp / 2], x3 = np[dkp / 4 * 3];
+    *(float4*)(ns + tid * 4) = make_float4((x0.x + x1.x) + (x2.x + x3.x), (x0.y + x1.y) + (x2.y + x3.y), (x0.z + x1.z) + (x2.z + x3.z),
+                                           (x0.w + x1.w) + (x2.w + x3.w));
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  {
+    const int mt = warp >> 1;
+    const bool diag = warp & 1;
+    const int jb0 = diag ? mt : 0, nblk = diag ? 1 : mt;
+    float f[3][2][4] = {};
+    if (nblk) {
+      for (int k4 = 0; k4 < dkp; k4 += 32) {         // runs of two products, added up in float32
+        float part[3][2][4];
+#pragma unroll
+        for (int kk = k4; kk < k4 + 32; kk += 16) {
+          uint32_t af[4], bq[4];
+          lc_ldsm4(af, qs + (mt * 16 + (mi & 1) * 8 + r8) * sh.ldq + kk + (mi >> 1) * 8);
+#pragma unroll
+          for (int b = 0; b < 3; ++b)
+            if (b < nblk) {
+              lc_ldsm4(bq, ks + ((jb0 + b) * 16 + (mi >> 1) * 8 + r8) * sh.ldq + kk + (mi & 1) * 8);
+              lc_mma(kk == k4, part[b][0], af, bq[0], bq[1]);
+              lc_mma(kk == k4, part[b][1], af, bq[2], bq[3]);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+          if (b < nblk) {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+              for (int x = 0; x < 4; ++x) f[b][nt][x] += part[b][nt][x];
+          }
+      }
+    }
+    float rs[2] = {0.f, 0.f};
+    if (diag) {
+      const float2 Gt[2] = {gt.G[mt * 16 + g8], gt.G[mt * 16 + g8 + 8]};
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const int jr = nt * 8 + 2 * t4 + jj;
+          const float2 Hj = gt.H[mt * 16 + jr];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float x = jr <= g8 + r * 8 ? f[0][nt][2 * r + jj] * lc_exp_sum(Gt[r], Hj) : 0.f;
+            f[0][nt][2 * r + jj] = x;
+            rs[r] += x;
+          }
+        }
+    } else {
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+        if (b < nblk) {
+          const float R[2] = {gt.R[b][mt * 16 + g8], gt.R[b][mt * 16 + g8 + 8]};
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            const float2 E = *(const float2*)(gt.E + b * 16 + nt * 8 + 2 * t4);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              f[b][nt][2 * r] *= R[r] * E.x;
+              f[b][nt][2 * r + 1] *= R[r] * E.y;
+              rs[r] += f[b][nt][2 * r] + f[b][nt][2 * r + 1];
+            }
+          }
+        }
+    }
+    if (warp == 0) {                               // n . q, two tokens a lane
+      float sum[2] = {0.f, 0.f};
+      for (int k4 = 0; k4 < dkp; k4 += 32) {         // runs of 32 keys, two sums each
+        float part[2][2] = {};
+#pragma unroll
+        for (int k = k4; k < k4 + 32; k += 8) {
+          const float4 na = *(const float4*)(ns + k), nb = *(const float4*)(ns + k + 4);
+          const float nn[8] = {na.x, na.y, na.z, na.w, nb.x, nb.y, nb.z, nb.w};
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const uint4 qv = *(const uint4*)(qs + (u * 32 + lane) * sh.ldq + k);
+            const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const __nv_bfloat162 q2 = *(const __nv_bfloat162*)&qw[i];
+              part[u][0] = fmaf(nn[2 * i], __low2float(q2), part[u][0]);
+              part[u][1] = fmaf(nn[2 * i + 1], __high2float(q2), part[u][1]);
+            }
+          }
+        }
+        sum[0] += part[0][0] + part[0][1];
+        sum[1] += part[1][0] + part[1][1];
+      }
+      nq[lane] = sum[0];
+      nq[32 + lane] = sum[1];
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 1);
+      rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 2);
+      if (t4 == 0) rowsum[(mt * 16 + g8 + x * 8) * 2 + (warp & 1)] = rs[x];
+    }
+    __syncthreads();                                 // all are done with k
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (b < nblk) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            uint32_t t[3];
+            lc_split3(f[b][nt][2 * r], f[b][nt][2 * r + 1], t);
+#pragma unroll
+            for (int x = 0; x < 3; ++x) *(uint32_t*)(wt + (x * LC_C + mt * 16 + g8 + r * 8) * LDW + (jb0 + b) * 16 + nt * 8 + 2 * t4) = t[x];
+          }
+      }
+  }
+  __syncthreads();                                   // W's terms, its rows' sums and n . q are in place
+  const int* odd = w.odd + ((size_t)s * a.H + h) * ((dv + LP_KEYS - 1) / LP_KEYS);
+  for (; cg < ncg; cg += LP_THREADS / 32) {
+    float acc[4][2][4] = {};
+    const float* Snext = Sp + (size_t)(LP_THREADS / 32) * (dkp >> 3) * 128;    // the warp's next 16 columns
+    for (int run = 0; run < dkp >> 5; ++run) {
+      uint32_t b0[2][2][3], b1[2][2][3];             // [key step][column tile][term]
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk) {
+        lc_split3(next[2 * kk].x, next[2 * kk].y, b0[kk][0]);
+        lc_split3(next[2 * kk].z, next[2 * kk].w, b0[kk][1]);
+        lc_split3(next[2 * kk + 1].x, next[2 * kk + 1].y, b1[kk][0]);
+        lc_split3(next[2 * kk + 1].z, next[2 * kk + 1].w, b1[kk][1]);
+      }
+      const bool more = run + 1 < dkp >> 5;
+      const float* np = more ? Sp + (run + 1) * 512 : Snext;
+      if (more || cg + LP_THREADS / 32 < ncg) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) next[i] = *(const float4*)(np + i * 128);
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float hi[2][4], lo[2][4];
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          uint32_t af[4];
+          lc_ldsm4(af, qs + (m * 16 + (mi & 1) * 8 + r8) * sh.ldq + run * 32 + kk * 16 + (mi >> 1) * 8);
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) {
+            lc_mma(kk == 0, lo[nb], af, b0[kk][nb][2], b1[kk][nb][2]);
+            lc_mma(kk == 0, hi[nb], af, b0[kk][nb][0], b1[kk][nb][0]);
+            lc_mma(lo[nb], af, b0[kk][nb][1], b1[kk][nb][1]);
+          }
+        }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[m][nb][x] += hi[nb][x] + lo[nb][x];
+      }
+    }
+    Sp = Snext;
+    const bool skip = odd[(col0 + cg * 16) / LP_KEYS] != 0;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      float yw[2][4] = {};
+#pragma unroll
+      for (int run = 0; run < 2; ++run) {            // runs of 32 tokens
+        if (2 * run > mt) break;
+        float hi[2][4], lo[2][4];
+#pragma unroll
+        for (int kk = 2 * run; kk < 2 * run + 2; ++kk) {
+          if (kk > mt) break;
+          uint32_t bv[4];
+          lc_ldsm4t(bv, vs + (kk * 16 + (mi & 1) * 8 + r8) * sh.ldv + cg * 16 + (mi >> 1) * 8);
+#pragma unroll
+          for (int x = 2; x >= 0; --x) {
+            uint32_t af[4];
+            lc_ldsm4(af, wt + (x * LC_C + mt * 16 + (mi & 1) * 8 + r8) * LDW + kk * 16 + (mi >> 1) * 8);
+            lc_mma(kk == 2 * run && x != 1, x ? lo[0] : hi[0], af, bv[0], bv[1]);
+            lc_mma(kk == 2 * run && x != 1, x ? lo[1] : hi[1], af, bv[2], bv[3]);
+          }
+        }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) yw[nb][x] += hi[nb][x] + lo[nb][x];
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = mt * 16 + g8 + r * 8;
+        if (t >= left || skip) continue;
+        const float At = gt.A[t];
+        const float den = fmaxf(fabsf((rowsum[2 * t] + rowsum[2 * t + 1] + At * nq[t]) * a.q_scale), gt.em[t]) + 1e-6f;
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          const int col = cg * 16 + nb * 8 + 2 * t4;
+          if (col0 + col >= dv) continue;
+          const float y0 = fmaf(At, acc[mt][nb][2 * r], yw[nb][2 * r]) * a.q_scale, y1 = fmaf(At, acc[mt][nb][2 * r + 1], yw[nb][2 * r + 1]) * a.q_scale;
+          *(float2*)(a.out + (t0 + t) * a.ld_out + (size_t)h * dv + col0 + col) = make_float2(y0 / den, y1 / den);
+        }
+      }
+    }
+  }
+  if (cr == 0) {
+    const int end = (c + w.P) * LC_C < len ? (c + w.P) * LC_C : len;
+    const int tiles = (dv + w.vt - 1) / w.vt;
+    for (int b = col0 / LP_KEYS; b * LP_KEYS < col0 + cols; ++b) {
+      if (!odd[b]) continue;
+      __syncthreads();                               // all are done with shared memory
+      for (int tile = b * LP_KEYS / w.vt; tile < (b + 1) * LP_KEYS / w.vt && tile < tiles; ++tile) {
+        if (w.vt == 16) lc_token_by_token<SCAN_GATED_MAX, 16, LP_THREADS>(a, w.n + slot * LP_NPARTS * dkp, LP_NPARTS, dkp, s, (int)t0, end - c * LC_C, h, tile, (float*)lp_smem);
+        else lc_token_by_token<SCAN_GATED_MAX, 32, LP_THREADS>(a, w.n + slot * LP_NPARTS * dkp, LP_NPARTS, dkp, s, (int)t0, end - c * LC_C, h, tile, (float*)lp_smem);
+      }
+    }
+  }
+}
+
+template <typename F>
+static int lp_configure(F kernel, int bytes, bool* configured) {
+  if (*configured) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  *configured = e == cudaSuccess;
+  return (int)e;
+}
+#define LP_MAX_OUT_BYTES (112 * 1024)      // two CTAs an SM
+
+static int launch_scan_parallel(const ScanArgs& a, int S, int max_len, void* ws, size_t ws_bytes, cudaStream_t st) {
+  static bool configured[2] = {};
+  const int nchunks = (max_len + LC_C - 1) / LC_C;
+  LpWork w;
+  w.dkp = (a.dk + 31) / 32 * 32;
+  w.ct = (a.dv + 15) / 16;
+  w.vt = scan_vt(a.dk);
+  const size_t slot = lp_slot_bytes(a.H, a.dk, a.dv), seg = lp_segment_bytes(a.H, a.dv);
+  size_t P = (ws_bytes - S * seg) / (slot * S);
+  if (P > (size_t)nchunks) P = nchunks;
+  w.P = (int)P;
+  const size_t slots = P * S, cells = slots * a.H;
+  w.m = (double*)ws;
+  w.S = (float*)(w.m + ((size_t)S * a.H + 1) / 2 * 2);
+  w.gates = (LpGates*)(w.S + cells * w.ct * w.dkp * 16);
+  w.n = (float*)(w.gates + cells);
+  w.odd = (int*)(w.n + cells * LP_NPARTS * w.dkp);
+  const int cols = a.dv < LP_COLS ? (a.dv + 15) / 16 * 16 : LP_COLS;
+  const int out_bytes = LpOutShape(w.dkp, cols).bytes, token_bytes = (a.dk * (w.vt + 3) + LP_THREADS + 4) * 4;
+  const int smem = out_bytes > token_bytes ? out_bytes : token_bytes, states = (int)sizeof(LpStatesSmem);
+  const int kblocks = (a.dk + LP_KEYS - 1) / LP_KEYS, cblocks = (a.dv + LP_KEYS - 1) / LP_KEYS;
+  int rc = lp_configure(lp_states_kernel, states, &configured[0]);
+  if (!rc) rc = lp_configure(lp_outputs_kernel, LP_MAX_OUT_BYTES, &configured[1]);
+  for (w.c0 = 0; w.c0 < nchunks && !rc; w.c0 += w.P) {
+    rc = qv_launch(lp_gates_kernel, dim3(S, a.H), dim3(32 * LP_GATE_WARPS), 0, st, a, w);
+    if (!rc) rc = qv_launch(lp_states_kernel, dim3(S, a.H, kblocks * (cblocks + 1)), dim3(LP_THREADS), (size_t)states, st, a, w);
+    const dim3 grid(S * w.P, a.H, (a.dv + LP_COLS - 1) / LP_COLS);
+    if (!rc) rc = qv_launch(lp_outputs_kernel, grid, dim3(LP_THREADS), (size_t)smem, st, a, w);
+  }
+  return rc;
+}
+
+// Segments from this many tokens on take the three launches, if their gates have a running maximum.  By 8 chunks of 4 heads of 256 x 512 the two
+// ways cost the same (a layer 98 us, where launching it from the host is what takes the time), by 32 the one kernel takes 272 and these 200.
+// Scalar decays stay with linear_scan_chunk_kernel: many heads of small states fill the GPU as they are (64 heads of 128 x 64, 1,943 tokens
+// in three segments: a layer 292 us, and 299 with these launches; one segment of 2,048: 282 and 317).
+static inline int scan_parallel_from(int kind) { return kind == SCAN_GATED_MAX ? 640 : 0x7fffffff; }
+// What the three launches take beside qv_linear_scan's operands, for `rest` segments of up to rest_max tokens (0: none of them takes these): the
+// states of as many chunks as LP_ROOM bytes hold, at least one a segment; the next ones follow in launches of their own.
+#define LP_ROOM ((size_t)160 << 20)
+extern "C" long long qv_linear_scan_workspace_bytes(int kind, int rest, int rest_max, int H, int dk, int dv) {
+  if (rest <= 0 || H <= 0 || dk <= 0 || dv <= 0 || rest_max < scan_parallel_from(kind)) return 0;
+  const size_t slot = lp_slot_bytes(H, dk, dv) * rest, seg = lp_segment_bytes(H, dv) * rest;
+  size_t P = (rest_max + LC_C - 1) / LC_C;
+  if (P * slot > LP_ROOM) P = LP_ROOM / slot ? LP_ROOM / slot : 1;
+  return (long long)(P * slot + seg + 32);
+}
+
+
 extern "C" long long qv_linear_scan_state_floats(int kind, int H, int dk, int dv) {
   const int vt = scan_vt(dk);
   return (long long)H * ((dv + vt - 1) / vt) * scan_tile_floats(kind, dk, vt);
@@ -1010,7 +1669,7 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
                               const void* v, int ld_v, const float* g1, int ld_g1, const float* g2, int ld_g2, const float* p1,
                               const float* p2, const float* p3, float cap, float q_scale, float* state, long long slot_stride,
                               const int* seg_q_start, const int* seg_slot, int S, int lead, int rest_max, int rest_min, int H, int dk, int dv, int dt,
-                              void* stream) {
+                              void* ws, long long ws_bytes, void* stream) {
   if (S <= 0) return 0;
   if (kind != SCAN_GATED_MAX && kind != SCAN_DECAY) return QV_ERR_UNSUPPORTED;
   if (H <= 0 || dk <= 0 || dv <= 0 || q_group <= 0 || H > 65535) return QV_ERR_UNSUPPORTED;
@@ -1022,7 +1681,7 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
   a.out = out; a.ld_out = ld_out; a.q = q; a.ld_q = ld_q; a.q_group = q_group; a.k = k; a.ld_k = ld_k; a.v = v; a.ld_v = ld_v;
   a.g1 = g1; a.ld_g1 = ld_g1; a.g2 = g2; a.ld_g2 = ld_g2; a.p1 = p1; a.p2 = p2; a.p3 = p3; a.cap = cap; a.q_scale = q_scale;
   a.state = state; a.slot_stride = slot_stride; a.seg_q_start = seg_q_start; a.seg_slot = seg_slot; a.H = H; a.dk = dk; a.dv = dv;
-  a.chunk_from = 0x7fffffff;
+  a.chunk_from = a.parallel_from = 0x7fffffff;
   dim3 grid(S, H, tiles);
   cudaStream_t st = (cudaStream_t)stream;
   // Portions of SCAN_CHUNK_FROM tokens and more take the tensor cores, the step's other segments the token-by-token kernel: which kernel a
@@ -1034,8 +1693,16 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
     rest.seg_q_start += lead;
     rest.seg_slot += lead;
     const dim3 rest_grid(S - lead, H, tiles);
-    int rc;
-    if (kind == SCAN_GATED_MAX)
+    int rc = 0;
+    const int parallel_from = scan_parallel_from(kind);
+    if (ws && ((uintptr_t)ws & 15) == 0 && rest_max >= parallel_from) {
+      if (ws_bytes < qv_linear_scan_workspace_bytes(kind, S - lead, rest_max, H, dk, dv)) return QV_ERR_UNSUPPORTED;
+      a.parallel_from = rest.parallel_from = parallel_from;
+      rc = launch_scan_parallel(rest, S - lead, rest_max, ws, (size_t)ws_bytes, st);
+      if (rc || (lead == 0 && rest_min >= parallel_from)) return rc;
+    }
+    if (rest.parallel_from <= rest_min) rc = 0;              // none of them is left for the chunks' kernel
+    else if (kind == SCAN_GATED_MAX)
       rc = vt == 16 ? launch_scan_chunk<SCAN_GATED_MAX, 16, 2>(rest, rest_grid, st)
                     : dk <= 64 ? launch_scan_chunk<SCAN_GATED_MAX, 32, 1>(rest, rest_grid, st) : launch_scan_chunk<SCAN_GATED_MAX, 32, 2>(rest, rest_grid, st);
     else

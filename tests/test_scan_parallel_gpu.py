@@ -1,0 +1,54 @@
+"""The gated recurrence over long portions (the chunks' outputs side by side) at the edges of its chunks, key blocks and column blocks, by the
+same measures as the shorter portions' kernel; a workspace that holds a part of the chunks; no room for one."""
+import pytest
+import torch
+
+import test_scan_chunks_gpu as chunks
+from qorvix_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dk,dv,H,qg,lens,shift", [(8, 8, 2, 1, [640], 0.0), (72, 40, 2, 2, [703, 1, 640], 2.0), (128, 272, 1, 1, [705, 20], -3.0),
+                                                   (256, 512, 1, 1, [1027], 3.0)])
+def test_long_portions_against_float64(dk, dv, H, qg, lens, shift):
+    chunks.test_chunks_against_float64(ops.SCAN_GATED_MAX, dk, dv, H, qg, lens, shift)
+
+
+@pytest.mark.parametrize("dk,dv,lens", [(64, 136, [640, 40]), (256, 16, [16, 700])])
+@pytest.mark.parametrize("what", ["value", "gate"])
+def test_what_is_not_finite_reaches_no_earlier_token(dk, dv, lens, what):
+    chunks.test_what_is_not_finite_reaches_no_earlier_token(ops.SCAN_GATED_MAX, dk, dv, lens, what)
+
+
+@pytest.mark.parametrize("lens", [[1, 1, 639, 640], [700, 3, 641]])
+def test_a_segment_does_not_depend_on_its_neighbours(lens):
+    chunks.test_a_segment_does_not_depend_on_its_neighbours(ops.SCAN_GATED_MAX, lens)
+
+
+def test_a_part_of_the_chunks_at_a_time_and_no_room(monkeypatch):
+    """Four segments whose chunks' states are more than the workspace may hold take several launches, each from where the last one ended;
+    without a workspace the shorter portions' kernel takes them.  Against token by token, whose rows are off float64 by some 7e-7 in the median,
+    as the chunks' are by 5e-7 (few rows, with a small n . q, by more): the median row and the states within 2e-6."""
+    H, dk, dv, lens = 8, 256, 512, [704, 640, 650, 900]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T = sum(lens)
+    q, k, v = (rnd(T, H * n).to(torch.bfloat16) for n in (dk, dk, dv))
+    g1, g2, p1, p2 = rnd(T, H), rnd(T, H) + 2, rnd(H), rnd(H)
+    need = ops._lib("recurrent").qv_linear_scan_workspace_bytes(ops.SCAN_GATED_MAX, 4, 900, H, dk, dv)
+    assert need < 15 * 4 * H * dk * dv * 4                      # less than the 15 chunks' states
+
+    def run(chunked):
+        state = torch.zeros(4, ops.linear_scan_state_floats(ops.SCAN_GATED_MAX, H, dk, dv), device="cuda")
+        out = torch.full((T, H * dv), float("nan"), device="cuda")
+        ops.linear_scan(ops.SCAN_GATED_MAX, out, q, k, v, g1, g2, p1, p2, None, 6.0, dk ** -0.5, state, chunks.context(lens, chunked), H, dk, dv)
+        return out.double(), state.double()
+
+    tokens, parts = run(False), run(True)
+    monkeypatch.setattr(ops, "_room", lambda *a: None)
+    one = run(True)
+    for got in (parts, one):
+        rows = (got[0] - tokens[0]).norm(dim=1) / tokens[0].norm(dim=1)
+        assert float(rows.median()) < 2e-6 and bool(torch.isfinite(rows).all())
+        assert float((got[1] - tokens[1]).norm() / tokens[1].norm()) < 2e-6
