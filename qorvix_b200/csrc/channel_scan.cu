@@ -435,282 +435,386 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 #undef CS_LAUNCH
 }
 
-// ---------------------------------------------------------------- delta rule on the decayed state: four tokens at a time
-// With S_0 the state ahead of a block of up to four tokens, P_t the product of the decays of the block's tokens up to t (per channel) and
+// ---------------------------------------------------------------- delta rule on the decayed state: sixteen tokens at a time
+// With S_0 the state ahead of a block of up to 16 tokens, P_t the product of the decays of the block's tokens up to t (per channel) and
 // kb = beta k, the recurrence S_t = diag(g_t) S_(t-1) + kb_t e_t^T, e_t = v_t - S_(t-1)^T (g_t k_t), y_t = S_t^T q_t unrolls to
 //   e_t   = v_t - S_0^T (P_t k_t) - sum_(l < t) A_tl e_l        A_tl = sum_c k_t (g_(l+1) .. g_t) kb_l
 //   y_t   = S_0^T (P_t q_t) + sum_(l <= t) B_tl e_l             B_tl = sum_c q_t (g_(l+1) .. g_t) kb_l
 //   S_end = diag(P_end) S_0 + sum_l (g_(l+1) .. g_end kb_l) e_l^T
-// that is, the eight products with S_0 do not wait for one another, and a block costs one chain of sums and shuffles instead of four.
-// Only products of decays (each at most one) occur, no quotients; everything is float32.
-//   channel_delta_operands   x [T][H][3][n] = P_t k_t, P_t q_t, (g_(t+1) .. g_end) kb_t;  pall [T][H][n] = P_end, at a block's first token;
-//                            coef [T][H][8] = A_t0 A_t1 A_t2 -, B_t0 .. B_t3.  A warp per (block, head).
-//   channel_delta_blocks     the recurrence; a lane holds 16 rows of two columns, two warps a CTA work and two fetch.
-// 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 426 in blocks, the operands 14 and 34.  Bound by a block's chain (dots,
-// shuffles, the triangular sums, the update) in one warp a scheduler.
+// and, the triangular system solved ahead for both of its right sides (X = P k, column by column, and v), to
+//   X'_t  = P_t k_t - sum_(l < t) A_tl X'_l        v'_t = v_t - sum_(l < t) A_tl v'_l
+//   X''_t = P_t q_t - sum_(l <= t) B_tl X'_l       v''_t = sum_(l <= t) B_tl v'_l
+//   e_t   = v'_t - S_0^T X'_t,                     y_t = v''_t + S_0^T X''_t
+// so that all but the products with S_0 and the update is worked out for all blocks at once, and a block costs its recurrence two products
+// and two barriers.  Only products of decays (each at most one) occur, no quotients.
+//   delta_block_operands_kernel   a CTA per (block, head): everything that does not depend on the state, float32 throughout
+//   delta_blocks_kernel           the recurrence: a CTA owns 16 value columns of a (segment, head), a warp 16 of the keys
+// The products with S_0 and of the update are mma.sync on both sides' three bfloat16 terms (the six products that count for 24 bits; the
+// large one's sum apart from the small ones', which the tensor cores would cut off), sums over the keys' slices in float32.
+// 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 460 with four tokens at a time and float32 multiply-adds, and
+// 200 here (operands 61, recurrence 139).
 // Blocks are counted from the start of a request's portion, so cuts agree to rounding (the 32-bit path takes channel_scan_kernel).
-#define CD_BLOCK 4
-// A warp takes a block and a head (the warp of the block's first token; the others have nothing to do): a row of q, k and g is then read
-// once for all of the block's products.
-__global__ void __launch_bounds__(128) channel_delta_operands_kernel(float* __restrict__ x, float* __restrict__ pall, float* __restrict__ coef,
-                                                                    const float* __restrict__ q, int ld_q, const float* __restrict__ k, int ld_k,
-                                                                    const float* __restrict__ b, int ld_b, const float* __restrict__ g, int ld_g,
-                                                                    const int* __restrict__ tok_seg, const int* __restrict__ seg_q_start, int H,
-                                                                    int G, int n, float eps, float q_scale, int t_base, int t_first) {
+#define CD_BLOCK 16
+#define CD_COLS 16
+#define CD_OP_THREADS 256
+struct ChannelDeltaArgs {
+  float* out; int ld_out;                 // [T, H * dv]
+  const float *q, *k, *v, *b, *g; int ld_q, ld_k, ld_v, ld_b, ld_g;
+  float* ws;                              // [slots][H][cd_slot_floats]
+  float* state; long long slot_stride;    // as ChannelScanArgs
+  const int* seg_q_start; const int* seg_slot;
+  int t_base;                             // the first segment's first token
+  int H, G, dk, dv, dkp, dvp;             // dkp, dvp: in whole 16s
+  float eps, q_scale;
+};
+// A block's floats: X', X'' and W = (g_(l+1) .. g_end) kb_l as the products' operands lie in the lanes, P_end, v', v''.
+__host__ __device__ inline size_t cd_slot_floats(int dkp, int dvp) { return (size_t)49 * dkp + 32 * (size_t)dvp; }
+// Blocks of different segments never share a slot: a segment of n tokens has at most n / 16 + 1 of them.
+__device__ __forceinline__ float* cd_slot(const ChannelDeltaArgs& a, int q0, int s, int block, int h) {
+  return a.ws + ((size_t)((q0 - a.t_base) / CD_BLOCK + s + block) * a.H + h) * cd_slot_floats(a.dkp, a.dvp);
+}
+
+// grid (blocks of the longest segment, heads, segments).  Bound by its multiply-adds and the reads of shared memory beside them.
+__global__ void __launch_bounds__(CD_OP_THREADS) delta_block_operands_kernel(const __grid_constant__ ChannelDeltaArgs a) {
+  extern __shared__ __align__(16) float cd_smem[];
   pdl_wait();
   pdl_launch_dependents();
-  const int t = t_first + blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int seg = tok_seg[t], q0 = seg_q_start[seg], j = t - q0, left = seg_q_start[seg + 1] - q0 - j;
-  if (h >= H || j % CD_BLOCK) return;
-  const int nb = left < CD_BLOCK ? left : CD_BLOCK;
-  const int grp = h / (H / G);
-  const float* qr = q + (size_t)t * ld_q + (size_t)grp * n;
-  const float* kr = k + (size_t)t * ld_k + (size_t)grp * n;
-  const float* gr = g + (size_t)t * ld_g + (size_t)h * n;
-  float beta[CD_BLOCK];
+  const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0, j0 = blockIdx.x * CD_BLOCK;
+  if (j0 >= len) return;
+  const int nb = len - j0 < CD_BLOCK ? len - j0 : CD_BLOCK;
+  const int dk = a.dk, dkp = a.dkp, ld = dkp + 4;
+  float* qs = cd_smem;                               // [16][ld] unit vectors, q times q_scale
+  float* ks = qs + CD_BLOCK * ld;
+  float* gs = ks + CD_BLOCK * ld;
+  float* As = gs + CD_BLOCK * ld;                    // [16][16]
+  float* Bs = As + CD_BLOCK * CD_BLOCK;              // [16][16]
+  float* beta = Bs + CD_BLOCK * CD_BLOCK;            // [16]
+  const int grp = h / (a.H / a.G);
+  // two tokens a warp; beyond the segment: keys and queries zero, decays one
 #pragma unroll
-  for (int u = 0; u < CD_BLOCK; ++u) beta[u] = u < nb ? 1.0f / (1.0f + expf(-b[(size_t)(t + u) * ld_b + h])) : 0.f;
-  float qq[CD_BLOCK] = {}, k2[CD_BLOCK] = {}, kk[6] = {}, qk[10] = {};      // pairs (u, l): kk at u (u - 1) / 2 + l, qk at u (u + 1) / 2 + l
-#pragma unroll 2
-  for (int i = lane; i < n; i += 32) {
-    float qv[CD_BLOCK], kv[CD_BLOCK], gv[CD_BLOCK];
+  for (int i = 0; i < 2; ++i) {
+    const int t = warp * 2 + i;
+    const bool in = t < nb;
+    const size_t row = (size_t)(q0 + j0 + (in ? t : 0));
+    const float* qr = a.q + row * a.ld_q + (size_t)grp * dk;
+    const float* kr = a.k + row * a.ld_k + (size_t)grp * dk;
+    const float* gr = a.g + row * a.ld_g + (size_t)h * dk;
+    float qv[8], kv[8], gv[8], sq = 0.f, sk = 0.f;
 #pragma unroll
-    for (int u = 0; u < CD_BLOCK; ++u) {
-      const bool in = u < nb;
-      qv[u] = in ? qr[i + (size_t)u * ld_q] : 0.f;
-      kv[u] = in ? kr[i + (size_t)u * ld_k] : 0.f;
-      gv[u] = in ? gr[i + (size_t)u * ld_g] : 1.f;
+    for (int x = 0; x < 8; ++x) {
+      const int c = lane + 32 * x;
+      const bool ok = in && c < dk;
+      qv[x] = ok ? qr[c] : 0.f;
+      kv[x] = ok ? kr[c] : 0.f;
+      gv[x] = ok ? gr[c] : 1.f;
     }
 #pragma unroll
-    for (int u = 0; u < CD_BLOCK; ++u) {
-      qq[u] = fmaf(qv[u], qv[u], qq[u]);
-      k2[u] = fmaf(kv[u], kv[u], k2[u]);
-      float D = 1.f;                                                 // g_(l+1) .. g_u
+    for (int x = 0; x < 8; ++x) { sq = fmaf(qv[x], qv[x], sq); sk = fmaf(kv[x], kv[x], sk); }
+    const float iq = a.q_scale / sqrtf(warp_sum(sq) + a.eps), ik = 1.0f / sqrtf(warp_sum(sk) + a.eps);
 #pragma unroll
-      for (int l = u; l >= 0; --l) {
-        const float kd = kv[l] * D;
-        qk[u * (u + 1) / 2 + l] = fmaf(qv[u], kd, qk[u * (u + 1) / 2 + l]);
-        if (l < u) kk[u * (u - 1) / 2 + l] = fmaf(kv[u], kd, kk[u * (u - 1) / 2 + l]);
-        D *= gv[l];
+    for (int x = 0; x < 8; ++x) {
+      const int c = lane + 32 * x;
+      if (c < dkp) {
+        qs[t * ld + c] = qv[x] * iq;
+        ks[t * ld + c] = kv[x] * ik;
+        gs[t * ld + c] = gv[x];
       }
     }
+    if (lane == 0) beta[t] = in ? 1.0f / (1.0f + expf(-a.b[row * a.ld_b + h])) : 0.f;
   }
-  float iq[CD_BLOCK], ik[CD_BLOCK];
+  __syncthreads();
+  // columns l and 15 - l of A and B a warp, four channels a lane and pass: 17 tokens' steps for every warp
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i) {
+    const int l = i ? CD_BLOCK - 1 - warp : warp;
+    float sum[2 * CD_BLOCK] = {};                    // A_tl, then B_tl
+    for (int c = lane * 4; c < dkp; c += 128) {
+      const float bl = beta[l];
+      float4 kd = *(const float4*)(ks + l * ld + c);
+      kd.x *= bl; kd.y *= bl; kd.z *= bl; kd.w *= bl;
 #pragma unroll
-  for (int u = 0; u < CD_BLOCK; ++u) {
-    iq[u] = q_scale / sqrtf(warp_sum(qq[u]) + eps);
-    ik[u] = 1.0f / sqrtf(warp_sum(k2[u]) + eps);
-  }
-#pragma unroll
-  for (int i = 0; i < 6; ++i) kk[i] = warp_sum(kk[i]);
-#pragma unroll
-  for (int i = 0; i < 10; ++i) qk[i] = warp_sum(qk[i]);
-  const size_t o = (size_t)(t - t_base) * H + h;
-  for (int i = lane; i < n; i += 32) {
-    float gv[CD_BLOCK], P[CD_BLOCK], suffix[CD_BLOCK];
-#pragma unroll
-    for (int u = 0; u < CD_BLOCK; ++u) gv[u] = u < nb ? gr[i + (size_t)u * ld_g] : 1.f;
-    P[0] = gv[0];
-#pragma unroll
-    for (int u = 1; u < CD_BLOCK; ++u) P[u] = P[u - 1] * gv[u];
-    suffix[CD_BLOCK - 1] = 1.f;
-#pragma unroll
-    for (int u = CD_BLOCK - 2; u >= 0; --u) suffix[u] = suffix[u + 1] * gv[u + 1];
-    pall[o * n + i] = P[CD_BLOCK - 1];
-#pragma unroll
-    for (int u = 0; u < CD_BLOCK; ++u) {
-      if (u >= nb) break;
-      const float ku = kr[i + (size_t)u * ld_k] * ik[u];
-      float* xr = x + (o + (size_t)u * H) * 3 * n + i;
-      xr[0] = P[u] * ku;
-      xr[n] = P[u] * (qr[i + (size_t)u * ld_q] * iq[u]);
-      xr[2 * n] = suffix[u] * (beta[u] * ku);
-    }
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int u = 0; u < CD_BLOCK; ++u) {
-      if (u >= nb) break;
-      float c[8] = {};
-#pragma unroll
-      for (int l = 0; l <= u; ++l) {
-        const float f = ik[l] * beta[l];
-        if (l < u) c[l] = kk[u * (u - 1) / 2 + l] * ik[u] * f;
-        c[4 + l] = qk[u * (u + 1) / 2 + l] * iq[u] * f;
+      for (int t = 0; t < CD_BLOCK; ++t) {
+        if (t < l) continue;
+        const float4 q4 = *(const float4*)(qs + t * ld + c);
+        if (t > l) {
+          const float4 g4 = *(const float4*)(gs + t * ld + c), k4 = *(const float4*)(ks + t * ld + c);
+          kd.x *= g4.x; kd.y *= g4.y; kd.z *= g4.z; kd.w *= g4.w;
+          sum[t] += fmaf(k4.x, kd.x, k4.y * kd.y) + fmaf(k4.z, kd.z, k4.w * kd.w);
+        }
+        sum[CD_BLOCK + t] += fmaf(q4.x, kd.x, q4.y * kd.y) + fmaf(q4.z, kd.z, q4.w * kd.w);
       }
-      float4* dst = (float4*)(coef + (o + (size_t)u * H) * 8);
-      dst[0] = make_float4(c[0], c[1], c[2], c[3]);
-      dst[1] = make_float4(c[4], c[5], c[6], c[7]);
+    }
+    // 32 sums over 32 lanes: a lane ends with its own
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1)
+#pragma unroll
+      for (int x = 0; x < half; ++x) {
+        const bool up = lane & half;
+        const float send = up ? sum[x] : sum[x + half], keep = up ? sum[x + half] : sum[x];
+        sum[x] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+      }
+    (lane < CD_BLOCK ? As : Bs)[(lane & 15) * CD_BLOCK + l] = sum[0];
+  }
+  __syncthreads();
+  float* ws = cd_slot(a, q0, s, blockIdx.x, h);
+  float *X1 = ws, *X2 = X1 + 16 * dkp, *Wf = X2 + 16 * dkp, *Pe = Wf + 16 * dkp, *V1 = Pe + dkp, *V2 = V1 + 16 * a.dvp;
+  for (int col = tid; col < dkp + a.dvp; col += CD_OP_THREADS) {
+    const bool key = col < dkp;
+    float x[CD_BLOCK];
+    float P = 1.f;
+    if (key) {
+#pragma unroll
+      for (int t = 0; t < CD_BLOCK; ++t) {
+        P *= gs[t * ld + col];
+        x[t] = P * ks[t * ld + col];
+      }
+      Pe[col] = P;
+    } else {
+      const int cv = col - dkp;
+      const float* vr = a.v + (size_t)(q0 + j0) * a.ld_v + (size_t)h * a.dv + cv;
+#pragma unroll
+      for (int t = 0; t < CD_BLOCK; ++t) x[t] = t < nb && cv < a.dv ? vr[(size_t)t * a.ld_v] : 0.f;
+    }
+    float y[CD_BLOCK];
+#pragma unroll
+    for (int t = 0; t < CD_BLOCK; ++t) {
+#pragma unroll
+      for (int l = 0; l < t; ++l) x[t] = fmaf(-As[t * CD_BLOCK + l], x[l], x[t]);
+      if (t >= nb) x[t] = 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < CD_BLOCK; ++t) {
+      y[t] = 0.f;
+#pragma unroll
+      for (int l = 0; l <= t; ++l) y[t] = fmaf(Bs[t * CD_BLOCK + l], x[l], y[t]);
+    }
+    if (key) {
+      // X' and X'' as the products' first operand: lane (t % 8) 4 + (key % 8) / 2 holds, of keys 0..7 and then 8..15 of a slice, {even key: t, t + 8;
+      // odd key: t, t + 8}
+      P = 1.f;
+#pragma unroll
+      for (int t = 0; t < CD_BLOCK; ++t) {
+        P *= gs[t * ld + col];
+        y[t] = t < nb ? fmaf(P, qs[t * ld + col], -y[t]) : 0.f;
+      }
+      const size_t at = (size_t)(col >> 3) * 128 + ((col & 7) >> 1) * 4 + (col & 1) * 2;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        *(float2*)(X1 + at + t * 16) = make_float2(x[t], x[t + 8]);
+        *(float2*)(X2 + at + t * 16) = make_float2(y[t], y[t + 8]);
+      }
+      // W as the update's second operand: lane (key % 8) 4 + t4 holds tokens 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9
+      float w[CD_BLOCK], f = 1.f;
+#pragma unroll
+      for (int t = CD_BLOCK - 1; t >= 0; --t) {
+        w[t] = f * (beta[t] * ks[t * ld + col]);
+        f *= gs[t * ld + col];
+      }
+#pragma unroll
+      for (int t4 = 0; t4 < 4; ++t4)
+        *(float4*)(Wf + (size_t)(col >> 3) * 128 + (col & 7) * 16 + t4 * 4) = make_float4(w[2 * t4], w[2 * t4 + 1], w[2 * t4 + 8], w[2 * t4 + 9]);
+    } else {
+      const int cv = col - dkp;
+#pragma unroll
+      for (int t = 0; t < CD_BLOCK; ++t) {
+        V1[t * a.dvp + cv] = x[t];
+        V2[t * a.dvp + cv] = y[t];
+      }
     }
   }
 }
 
-struct ChannelDeltaArgs {
-  float* out; int ld_out;                 // [T, H * dv]
-  const float* x; const float* pall; const float* coef;       // from token t_base on
-  int t_base;
-  const float* v; int ld_v;
-  float* state; long long slot_stride;    // as ChannelScanArgs
-  const int* seg_q_start; const int* seg_slot;
-  int H, dk, dv;
-};
+__device__ __forceinline__ void cd_mma(float* c, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// x and y as three bfloat16 terms each (x in the lower half of a word)
+__device__ __forceinline__ void cd_split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
+  uint32_t t[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    t[i] = *(const uint32_t*)&h;
+    x -= __low2float(h);
+    y -= __high2float(h);
+  }
+  t0 = t[0]; t1 = t[1]; t2 = t[2];
+}
+// c = a b of three terms each
+__device__ __forceinline__ void cd_product(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[3], const uint32_t (&b1)[3]) {
+  float hi[4] = {}, lo[4] = {}, lo2[4] = {};
+  cd_mma(lo, a[0], b0[1], b1[1]);
+  cd_mma(lo2, a[2], b0[0], b1[0]);
+  cd_mma(hi, a[0], b0[0], b1[0]);
+  cd_mma(lo, a[1], b0[0], b1[0]);
+  cd_mma(lo2, a[0], b0[2], b1[2]);
+  cd_mma(lo2, a[1], b0[1], b1[1]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = hi[i] + (lo[i] + lo2[i]);
+}
 
-// NB: blocks a stage, two stages.  Two columns a lane (one column a lane and four working warps: 496 us where this takes 426), so two warps
-// work; two more fetch.
-template <int LPC, int NB>
-__global__ void __launch_bounds__(128) channel_delta_blocks_kernel(ChannelDeltaArgs a) {
-  extern __shared__ __align__(16) float cd_ring[];
-  constexpr int C = 2;
-  constexpr int CPT = 32 / LPC, CTA_COLS = 4 * CPT, VEC = CS_PAD * LPC, W = 4 / C;
-  constexpr int ROW = 3 * VEC + 8 + CTA_COLS;                        // floats a token takes: three vectors, factors, values
-  constexpr int BLK = CD_BLOCK * ROW + VEC;                          // a block: its tokens, then P_end
+// grid (segments, heads, column tiles); NS warps, a slice of 16 keys each, S^T in registers as the accumulators of the update (value columns x
+// keys), which are the second operand of X S_0.  A block: the slices' shares of X' S_0 and X'' S_0 into shared memory, a barrier, their sums
+// (half of the threads e, half y), a barrier, the update.  The next blocks' operands are on their way to registers meanwhile.  Bound by that
+// chain: 1.
+template <int NS>
+__global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_constant__ ChannelDeltaArgs a) {
+  constexpr int EACH = 512 / (32 * NS);              // of the 32 x 16 sums, a thread's
+  constexpr int PER_ROW = CD_COLS / EACH;            // threads a row
+  constexpr int CD_LD = NS == 16 ? 20 : 24;          // (24: the writes of a half warp hit every bank once; 16 slices of that are too much)
+  __shared__ __align__(16) float red[NS][2 * CD_BLOCK][CD_LD];
+  __shared__ __align__(16) float eT[CD_COLS][CD_LD]; // [column][token]
   pdl_wait();
-  const int s = blockIdx.x, h = blockIdx.y;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lic = lane % LPC, cw = lane / LPC;
-  const int dk = a.dk, dv = a.dv, H = a.H;
-  const int tiles = (dv + CPT - 1) / CPT;
+  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CD_COLS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  const bool works = warp < W;
-  const int tile0 = blockIdx.z * 4 + (works ? warp * C : 0);         // of the working warps: C tiles of CPT columns
-  const int cta_col0 = blockIdx.z * CTA_COLS;
-  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + ((size_t)h * tiles + tile0) * (CS_ROWS * 32) + lane;
-  float S[C][CS_ROWS];
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int i = 0; i < CS_ROWS; ++i) S[c][i] = works && tile0 + c < tiles ? st[c * CS_ROWS * 32 + i * 32] : 0.f;
-  auto issue = [&](int ch) {                                         // by the last two warps, a token a warp; zeros beyond the segment
-    float* base = cd_ring + (ch & 1) * NB * BLK;
-#pragma unroll 2
-    for (int tk = warp - W; tk < NB * CD_BLOCK; tk += 2) {
-      const int j = ch * NB * CD_BLOCK + tk;
-      const bool in = j < len;
-      const size_t row = (size_t)(q0 - a.t_base + (in ? j : 0)) * H + h;
-      const float* src = a.x + row * 3 * dk;
-      float* blk = base + (tk / CD_BLOCK) * BLK;
-      float* dst = blk + (tk % CD_BLOCK) * ROW;
-#pragma unroll
-      for (int r = lane * 4; r < CS_ROWS * LPC; r += 128) {
-        const bool ok = in && r < dk;
-        const int off = r + (r / CS_ROWS) * (CS_PAD - CS_ROWS);
-#pragma unroll
-        for (int v = 0; v < 3; ++v) cs_cp16(dst + v * VEC + off, ok ? src + v * dk + r : a.x, ok);
-        if (tk % CD_BLOCK == 0) cs_cp16(blk + CD_BLOCK * ROW + off, ok ? a.pall + row * dk + r : a.x, ok);
-      }
-      if (lane < 2) cs_cp16(dst + 3 * VEC + lane * 4, a.coef + row * 8 + lane * 4, in);
-      for (int cc = lane; cc < CTA_COLS; cc += 32) {
-        const bool ok = in && cta_col0 + cc < dv;
-        cs_cp4(dst + 3 * VEC + 8 + cc, ok ? a.v + (size_t)(q0 + j) * a.ld_v + (size_t)h * dv + cta_col0 + cc : a.v, ok);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  const int dk = a.dk, dv = a.dv, dkp = a.dkp;
+  const int lpc = dk <= 16 ? 1 : dk <= 32 ? 2 : dk <= 64 ? 4 : dk <= 128 ? 8 : 16, cpt = 32 / lpc, tiles = (dv + cpt - 1) / cpt;
+  float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * 512;
+  const int k0 = warp * 16;
+  const bool holds = k0 < dkp;
+  auto at = [&](int nt, int i) -> float* {           // where S^T's entry lies in the state (channel_scan_kernel's layout; rows from dk on: zeros), or null
+    const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = col0 + g8 + (i >> 1) * 8;
+    return k < 16 * lpc && col < tiles * cpt ? st + (size_t)(col / cpt) * 512 + (k & 15) * 32 + (col % cpt) * lpc + (k >> 4) : nullptr;
   };
-  const int nstages = (len + NB * CD_BLOCK - 1) / (NB * CD_BLOCK);
-  if (!works && nstages > 0) issue(0);
-  for (int ch = 0; ch < nstages; ++ch) {
-    if (!works) {
-      if (ch + 1 < nstages) {
-        issue(ch + 1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+  float S[2][4];
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* p = at(nt, i);
+      S[nt][i] = p && k0 + nt * 8 + 2 * t4 + (i & 1) < dk ? *p : 0.f;
+    }
+  const int nblocks = (len + CD_BLOCK - 1) / CD_BLOCK;
+  const int orow = tid / PER_ROW, ocol = (tid % PER_ROW) * EACH;     // the sums this thread forms: rows 0..15 e, 16..31 y
+  struct Operands { float4 x[2][2], w[2]; float2 P[2]; float v[EACH]; };
+  const size_t stride = (size_t)a.H * cd_slot_floats(dkp, a.dvp);
+  const float* ws = cd_slot(a, q0, s, 0, h);
+  const float* wx = ws + (k0 >> 3) * 128 + lane * 4;
+  const float* wP = ws + 48 * (size_t)dkp + k0 + 2 * t4;
+  const float* wv = ws + 49 * (size_t)dkp + (size_t)orow * a.dvp + col0 + ocol;      // (v'' follows v')
+  auto fetch = [&](Operands& o, int blk) {
+    if (blk >= nblocks) return;
+    const size_t off = (size_t)blk * stride;
+    if (holds) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        o.x[0][i] = *(const float4*)(wx + off + i * 128);
+        o.x[1][i] = *(const float4*)(wx + off + 16 * dkp + i * 128);
+        o.w[i] = *(const float4*)(wx + off + 32 * dkp + i * 128);
+        o.P[i] = *(const float2*)(wP + off + i * 8);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) o.v[i] = wv[off + i];
+  };
+  auto step = [&](Operands& o, int blk) {
+    uint32_t w0[2][3], w1[2][3];                     // [key tile][term]
+    if (holds) {
+      uint32_t b0[2][3], b1[2][3];                   // S_0: [column tile][term]
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        cd_split3(S[0][2 * nb], S[0][2 * nb + 1], b0[nb][0], b0[nb][1], b0[nb][2]);
+        cd_split3(S[1][2 * nb], S[1][2 * nb + 1], b1[nb][0], b1[nb][1], b1[nb][2]);
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        uint32_t af[3][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          cd_split3(o.x[m][i].x, o.x[m][i].z, af[0][2 * i], af[1][2 * i], af[2][2 * i]);
+          cd_split3(o.x[m][i].y, o.x[m][i].w, af[0][2 * i + 1], af[1][2 * i + 1], af[2][2 * i + 1]);
+        }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          float c[4];
+          cd_product(c, af, b0[nb], b1[nb]);
+          *(float2*)&red[warp][m * CD_BLOCK + g8][nb * 8 + 2 * t4] = make_float2(c[0], c[1]);
+          *(float2*)&red[warp][m * CD_BLOCK + g8 + 8][nb * 8 + 2 * t4] = make_float2(c[2], c[3]);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        cd_split3(o.w[nt].x, o.w[nt].y, w0[nt][0], w0[nt][1], w0[nt][2]);
+        cd_split3(o.w[nt].z, o.w[nt].w, w1[nt][0], w1[nt][1], w1[nt][2]);
+      }
+    }
+    __syncthreads();                                 // the slices' shares are in place; eT has been read
+    {
+      const int slices = dkp >> 4;
+      float sum[EACH] = {};
+#pragma unroll
+      for (int sl = 0; sl < NS; ++sl)
+        if (sl < slices) {
+#pragma unroll
+          for (int i = 0; i < EACH; ++i) sum[i] += red[sl][orow][ocol + i];
+        }
+      if (orow < CD_BLOCK) {
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) eT[ocol + i][orow] = o.v[i] - sum[i];
       } else {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-      }
-    }
-    __syncthreads();
-    if (works) {
-#pragma unroll 1
-      for (int blk = 0; blk < NB; ++blk) {
-        const int j0 = (ch * NB + blk) * CD_BLOCK;
-        if (j0 >= len) break;
-        const float* d = cd_ring + (ch & 1) * NB * BLK + blk * BLK;
-        float p[CD_BLOCK][C], r[CD_BLOCK][C];
+        const int t = blk * CD_BLOCK + orow - CD_BLOCK;
+        if (t < len) {
+          float* y = a.out + (size_t)(q0 + t) * a.ld_out + (size_t)h * dv + col0 + ocol;
 #pragma unroll
-        for (int t = 0; t < CD_BLOCK; ++t) {
-          const float4* pk = (const float4*)(d + t * ROW + lic * CS_PAD);
-          const float4* pq = (const float4*)(d + t * ROW + VEC + lic * CS_PAD);
-          float ps[C][2] = {}, rs[C][2] = {};                        // two partial sums each
-#pragma unroll
-          for (int i = 0; i < CS_ROWS / 4; ++i) {
-            const float4 k4 = pk[i], q4 = pq[i];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-              ps[c][0] = fmaf(k4.x, S[c][4 * i], ps[c][0]); ps[c][1] = fmaf(k4.y, S[c][4 * i + 1], ps[c][1]);
-              ps[c][0] = fmaf(k4.z, S[c][4 * i + 2], ps[c][0]); ps[c][1] = fmaf(k4.w, S[c][4 * i + 3], ps[c][1]);
-              rs[c][0] = fmaf(q4.x, S[c][4 * i], rs[c][0]); rs[c][1] = fmaf(q4.y, S[c][4 * i + 1], rs[c][1]);
-              rs[c][0] = fmaf(q4.z, S[c][4 * i + 2], rs[c][0]); rs[c][1] = fmaf(q4.w, S[c][4 * i + 3], rs[c][1]);
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < C; ++c) { p[t][c] = ps[c][0] + ps[c][1]; r[t][c] = rs[c][0] + rs[c][1]; }
-        }
-#pragma unroll
-        for (int o = LPC / 2; o > 0; o >>= 1)
-#pragma unroll
-          for (int t = 0; t < CD_BLOCK; ++t)
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-              p[t][c] += __shfl_xor_sync(0xffffffffu, p[t][c], o);
-              r[t][c] += __shfl_xor_sync(0xffffffffu, r[t][c], o);
-            }
-        float e[CD_BLOCK][C];
-#pragma unroll
-        for (int t = 0; t < CD_BLOCK; ++t) {
-          const float4 A4 = *(const float4*)(d + t * ROW + 3 * VEC), B4 = *(const float4*)(d + t * ROW + 3 * VEC + 4);
-          const float A[4] = {A4.x, A4.y, A4.z, A4.w}, B[4] = {B4.x, B4.y, B4.z, B4.w};
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            const int cc = (warp * C + c) * CPT + cw;
-            float ev = d[t * ROW + 3 * VEC + 8 + cc] - p[t][c];
-#pragma unroll
-            for (int l = 0; l < t; ++l) ev = fmaf(-A[l], e[l][c], ev);
-            e[t][c] = ev;
-            float y = r[t][c];
-#pragma unroll
-            for (int l = 0; l <= t; ++l) y = fmaf(B[l], e[l][c], y);
-            if (lic == 0 && cta_col0 + cc < dv && j0 + t < len) a.out[(size_t)(q0 + j0 + t) * a.ld_out + (size_t)h * dv + cta_col0 + cc] = y;
-          }
-        }
-        const float4* pp = (const float4*)(d + CD_BLOCK * ROW + lic * CS_PAD);
-#pragma unroll
-        for (int i = 0; i < CS_ROWS / 4; ++i) {
-          const float4 g4 = pp[i];
-#pragma unroll
-          for (int c = 0; c < C; ++c) { S[c][4 * i] *= g4.x; S[c][4 * i + 1] *= g4.y; S[c][4 * i + 2] *= g4.z; S[c][4 * i + 3] *= g4.w; }
-#pragma unroll
-          for (int t = 0; t < CD_BLOCK; ++t) {
-            const float4 w4 = *(const float4*)(d + t * ROW + 2 * VEC + lic * CS_PAD + 4 * i);
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-              S[c][4 * i] = fmaf(w4.x, e[t][c], S[c][4 * i]); S[c][4 * i + 1] = fmaf(w4.y, e[t][c], S[c][4 * i + 1]);
-              S[c][4 * i + 2] = fmaf(w4.z, e[t][c], S[c][4 * i + 2]); S[c][4 * i + 3] = fmaf(w4.w, e[t][c], S[c][4 * i + 3]);
-            }
-          }
+          for (int i = 0; i < EACH; ++i)
+            if (col0 + ocol + i < dv) y[i] = o.v[i] + sum[i];
         }
       }
     }
-    __syncthreads();
+    __syncthreads();                                 // e is in place; the shares have been read
+    if (holds) {
+      uint32_t af[3][4];                             // e^T: columns g8, g8 + 8; tokens 2 t4, 2 t4 + 1 and 8 further
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 e = *(const float2*)&eT[g8 + (i & 1) * 8][2 * t4 + (i >> 1) * 8];
+        cd_split3(e.x, e.y, af[0][i], af[1][i], af[2][i]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        float c[4];
+        cd_product(c, af, w0[nt], w1[nt]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(i & 1 ? o.P[nt].y : o.P[nt].x, S[nt][i], c[i]);
+      }
+    }
+    fetch(o, blk + 2);
+  };
+  Operands o0, o1;
+  fetch(o0, 0);
+  fetch(o1, 1);
+  for (int blk = 0; blk < nblocks; blk += 2) {
+    step(o0, blk);
+    if (blk + 1 < nblocks) step(o1, blk + 1);
   }
   pdl_launch_dependents();
-  if (!works) return;
 #pragma unroll
-  for (int c = 0; c < C; ++c)
-    if (tile0 + c < tiles)
+  for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int i = 0; i < CS_ROWS; ++i) st[c * CS_ROWS * 32 + i * 32] = S[c][i];
+    for (int i = 0; i < 4; ++i) {
+      float* p = at(nt, i);
+      if (p) *p = S[nt][i];
+    }
+}
+
+// What qv_channel_delta takes beside its operands, in floats: for lead_tokens that go token by token, and for `tokens` of `segs` segments in blocks.
+extern "C" long long qv_channel_delta_workspace_floats(int lead_tokens, int tokens, int segs, int H, int dk, int dv) {
+  const size_t slots = segs > 0 ? (size_t)tokens / CD_BLOCK + segs : 0;
+  return (long long)((size_t)lead_tokens * H * 3 * dk + slots * H * cd_slot_floats((dk + 15) / 16 * 16, (dv + 15) / 16 * 16));
 }
 
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
 // beta, g [T, H * dk] the decays, v [T, H * dv].  The first S_lead segments (T_lead tokens, the longest of them max_lead) go token by token, the
-// others in blocks, for which dk is a multiple of 4 above 64, at most 256.  workspace: H x 3 dk floats a token of the first (operands of
-// qv_channel_scan), then H x (4 dk + 8) a token of the others (x, pall and coef in this order).
+// others (up to max_rest tokens) in blocks, for which dk is a multiple of 4, at most 256.  workspace: qv_channel_delta_workspace_floats, 16-byte
+// aligned.
 extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                                 const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
-                                long long slot_stride, const int* tok_seg, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,
-                                int T_lead, int max_lead, int H, int G, int dk, int dv, float* workspace, void* stream) {
+                                long long slot_stride, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,
+                                int T_lead, int max_lead, int max_rest, int H, int G, int dk, int dv, float* workspace, void* stream) {
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || S_lead < 0 || S_lead > S || T_lead < 0 || T_lead > T) return QV_ERR_UNSUPPORTED;
-  if (S_lead < S && (dk % 4 || dk <= 64 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
+  if (S_lead < S && (dk % 4 || max_rest <= 0 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
   if (dk > 256) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   if (S_lead > 0) {
@@ -723,34 +827,23 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
     if (rc || S_lead == S) return rc;
     workspace += 3 * n;
   }
-  const size_t rest = (size_t)(T - T_lead) * H;
   ChannelDeltaArgs a;
-  float* x = workspace;
-  float* pall = x + rest * 3 * dk;
-  float* coef = pall + rest * dk;
-  for (int done = T_lead; done < T; done += 65535) {
-    const int rows = T - done < 65535 ? T - done : 65535;
-    const int rc = qv_launch(channel_delta_operands_kernel, dim3(rows, (H + 3) / 4), dim3(128), 0, st, x, pall, coef, q, ld_q, k, ld_k, b, ld_b, g,
-                             ld_g, tok_seg, seg_q_start, H, G, dk, eps, q_scale, T_lead, done);
-    if (rc) return rc;
+  a.out = out; a.ld_out = ld_out; a.q = q; a.k = k; a.v = v; a.b = b; a.g = g; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.ld_b = ld_b; a.ld_g = ld_g;
+  a.ws = workspace; a.state = state; a.slot_stride = slot_stride; a.seg_q_start = seg_q_start + S_lead; a.seg_slot = seg_slot + S_lead;
+  a.t_base = T_lead; a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.dkp = (dk + 15) / 16 * 16; a.dvp = (dv + 15) / 16 * 16; a.eps = eps; a.q_scale = q_scale;
+  const int rest = S - S_lead, col_tiles = a.dvp / CD_COLS;
+  if (rest > 65535 || col_tiles > 65535) return QV_ERR_TOO_LARGE;
+  const int smem = (3 * CD_BLOCK * (a.dkp + 4) + 2 * CD_BLOCK * CD_BLOCK + CD_BLOCK) * 4;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(delta_block_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
   }
-  a.out = out; a.ld_out = ld_out; a.x = x; a.pall = pall; a.coef = coef; a.v = v; a.ld_v = ld_v; a.state = state; a.slot_stride = slot_stride;
-  a.seg_q_start = seg_q_start + S_lead; a.seg_slot = seg_slot + S_lead; a.H = H; a.dk = dk; a.dv = dv;
-  a.t_base = T_lead;
-  const int lpc = cs_lanes_per_column(dk);
-  const int cta_cols = 4 * 32 / lpc;
-  const int ctas = (dv + cta_cols - 1) / cta_cols;
-  if (ctas > 65535) return QV_ERR_TOO_LARGE;
-#define CD_LAUNCH(LPC, NB)                                                                                                       \
-  do {                                                                                                                           \
-    constexpr int smem = 2 * NB * (CD_BLOCK * (3 * CS_PAD * LPC + 8 + 4 * 32 / LPC) + CS_PAD * LPC) * 4;                         \
-    cudaFuncSetAttribute(channel_delta_blocks_kernel<LPC, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-    return cs_launch_after(channel_delta_blocks_kernel<LPC, NB>, dim3(S - S_lead, H, ctas), dim3(128), (size_t)smem, st, a);           \
-  } while (0)
-  if (lpc == 8) CD_LAUNCH(8, 4);
-  if (lpc == 16) CD_LAUNCH(16, 2);
-  return QV_ERR_UNSUPPORTED;                // shorter keys: token by token is the faster scan
-#undef CD_LAUNCH
+  const int rc = qv_launch(delta_block_operands_kernel, dim3((max_rest + CD_BLOCK - 1) / CD_BLOCK, H, rest), dim3(CD_OP_THREADS), (size_t)smem, st, a);
+  if (rc) return rc;
+  const dim3 grid(rest, H, col_tiles);
+  if (dk <= 64) return cs_launch_after(delta_blocks_kernel<4>, grid, dim3(128), 0, st, a);
+  if (dk <= 128) return cs_launch_after(delta_blocks_kernel<8>, grid, dim3(256), 0, st, a);
+  return cs_launch_after(delta_blocks_kernel<16>, grid, dim3(512), 0, st, a);
 }
 
 // ---------------------------------------------------------------- unit norm per head, weight, gate, factor

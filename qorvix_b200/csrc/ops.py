@@ -109,7 +109,8 @@ _ARGTYPES = {
     "qv_unit_keys": [_V, _V, _V, _I, _V, _I, _V, _I, _I, _I, _F, _V],
     "qv_channel_scan_state_floats": [_I, _I, _I],
     "qv_channel_scan": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _V],
-    "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V],
+    "qv_channel_delta_workspace_floats": [_I, _I, _I, _I, _I, _I],
+    "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V],
     "qv_head_norm_gate": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _F, _I, _V],
     "qv_bias_attn_prepare": [_V, _I, _V, _I, _I, _I, _I, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V],
     "qv_bias_attention_generic": [_V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _V, _I, _V, _V, _I, _F, _I, _V],
@@ -126,7 +127,7 @@ _ARGTYPES = {
 }
 _RESTYPES = {"qv_error_string": ctypes.c_char_p, "qv_packed_weight_bytes": c_longlong, "qv_gemm_bf16_split_slot_bytes": c_longlong,
              "qv_linear_scan_state_floats": c_longlong, "qv_linear_scan_workspace_bytes": c_longlong, "qv_latent_tc_workspace_bytes": c_longlong, "qv_diff_partial_floats": c_longlong,
-             "qv_channel_scan_state_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
+             "qv_channel_scan_state_floats": c_longlong, "qv_channel_delta_workspace_floats": c_longlong, "qv_head_delta_state_floats": c_longlong}
 _typed_libs = {}
 
 
@@ -1046,23 +1047,20 @@ def channel_scan(out, q, k, v, w, au, u, q_scale: float, state, ctx, H: int, dk:
     _check(rc, "channel_scan")
 
 
-DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go four tokens at a time
+DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go sixteen tokens at a time
 
 
 def delta_lead(lens, dk: int, blocks: bool = True) -> int:
     """How many of a step's leading segments the delta rule takes token by token: those ahead of the first of DELTA_BLOCKS_FROM tokens (single
-    tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries, or of up to 64: there a token has half
-    the work and a block the same chain.  us a layer token by token and in blocks, 16 heads of 128: 4 tokens 43 and 45, 16 tokens 53
-    and 53, 64 tokens 92 and 86, 256 tokens 175 and 147, 63 single tokens beside 4 114 and 155; 8 heads of 64: 64 tokens 66 and 68, 200
-    tokens 109 and 113, eight portions of 256 169 and 178."""
-    if not blocks or dk % 4 or not 64 < dk <= 256:
+    tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries."""
+    if not blocks or dk % 4 or dk > 256:
         return len(lens)
     return next((i for i, n in enumerate(lens) if n >= DELTA_BLOCKS_FROM), len(lens))
 
 
 def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: int, eps: float, q_scale: float, blocks: bool = True) -> bool:
     """The delta rule that reads the decayed state: unit vectors of q and k (q times q_scale), beta = sigmoid(b), decays g, per request and
-    head; state as channel_scan's.  Token by token (delta_operands, channel_scan) or four tokens at a time, see delta_lead.  True."""
+    head; state as channel_scan's.  Token by token (delta_operands, channel_scan) or sixteen tokens at a time, see delta_lead.  True."""
     _need_cuda(out, q, k, v, b, g, state)
     for t in (out, q, k, v, b, g):
         assert t.dtype == torch.float32 and t.stride(1) == 1
@@ -1071,13 +1069,15 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lens = ctx.seg_len
     lead = delta_lead(lens, dk, blocks)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
-    ws = _room(H * (tokens * 3 * dk + (T - tokens) * (4 * dk + 8)), torch.float32, q.device) if lead < S else None
-    if ws is None:                                    # token by token, which takes three quarters of the blocks' room
+    lib = _lib("channel_scan")
+    ws = _room(lib.qv_channel_delta_workspace_floats(tokens, T - tokens, S - lead, H, dk, dv), torch.float32, q.device) if lead < S else None
+    if ws is None:                                    # token by token, which takes less room
         lead, tokens, longest = S, T, int(ctx.max_q_len)
         ws = torch.empty(H * T * 3 * dk, device=q.device, dtype=torch.float32)
-    rc = _lib("channel_scan").qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
-                              _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0), _ptr(ctx.tok_seg),
-                              _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, H, G, dk, dv, _ptr(ws), _stream())
+    rc = lib.qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
+                              _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0),
+                              _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, max(lens[lead:], default=0), H, G, dk, dv,
+                              _ptr(ws), _stream())
     _check(rc, "channel_delta")
     add_launches(3 if 0 < lead < S else 1)
     return True

@@ -1,0 +1,37 @@
+"""The delta rule sixteen tokens at a time at the edges of its blocks, key slices and column tiles, by the measures of the other sizes; and what
+a value that is not finite reaches."""
+import pytest
+import torch
+
+import test_delta_blocks_gpu as blocks
+from qorvix_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dk,dv,H,G,lens,rate", [(4, 1, 2, 1, [16, 17, 1], 0.1), (20, 17, 2, 2, [31, 32, 33], 1.0), (68, 16, 2, 1, [47, 15, 48], 0.05),
+                                                 (132, 33, 1, 1, [49, 16], 0.2)])
+def test_edges_of_blocks_against_float64(dk, dv, H, G, lens, rate):
+    blocks.test_blocks_against_float64(dk, dv, H, G, lens, rate)
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 24), (128, 40)])
+def test_an_infinite_value_reaches_no_earlier_token_and_no_other_column(dk, dv):
+    g = torch.Generator(device="cuda").manual_seed(dk)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    lens, H = [37, 50], 2
+    T, ctx = sum(lens), blocks.context(lens)
+    q, k, v, b, decay = rnd(T, dk), rnd(T, dk), rnd(T, H * dv), rnd(T, H), torch.exp(-rnd(T, H * dk).abs())
+
+    def run():
+        state, out = torch.zeros(2, ops.channel_scan_state_floats(H, dk, dv), device="cuda"), torch.full((T, H * dv), float("nan"), device="cuda")
+        ops.channel_delta(out, q, k, v, b, decay, state, ctx, H, 1, dk, dv, 1e-6, dk ** -0.5)
+        return out
+
+    clean = run()
+    at = 37 + 21                                                # inside the second segment's second block
+    v[at, 3] = float("inf")
+    got = run()
+    others = torch.arange(H * dv, device="cuda") != 3
+    assert bool(torch.isfinite(clean).all()) and torch.equal(got[:at], clean[:at]) and torch.equal(got[:, others], clean[:, others])
+    assert not bool(torch.isfinite(got[at:, 3]).any())
