@@ -1047,15 +1047,20 @@ def channel_scan(out, q, k, v, w, au, u, q_scale: float, state, ctx, H: int, dk:
     _check(rc, "channel_scan")
 
 
-DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go sixteen tokens at a time
+DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go sixteen tokens at a time,
+DELTA_SHORT_KEYS_FROM = 256                # of this many for keys of up to 64 entries
 
 
 def delta_lead(lens, dk: int, blocks: bool = True) -> int:
     """How many of a step's leading segments the delta rule takes token by token: those ahead of the first of DELTA_BLOCKS_FROM tokens (single
-    tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries."""
+    tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries.  Keys of up to 64 entries have
+    half the work a token: portions of up to 256 tokens cost a layer the same either way (8 heads of 64: 64 tokens 149 us token by token
+    and 151 in blocks, four portions of 256 151 and 151, which is the host's time; 1,531 tokens 552 and 204).  16 heads of 128: 16 tokens 153 and
+    151, four portions of 200 252 and 201, 1,531 tokens 637 (four tokens at a time) and 374."""
     if not blocks or dk % 4 or dk > 256:
         return len(lens)
-    return next((i for i, n in enumerate(lens) if n >= DELTA_BLOCKS_FROM), len(lens))
+    first = DELTA_BLOCKS_FROM if dk > 64 else DELTA_SHORT_KEYS_FROM
+    return next((i for i, n in enumerate(lens) if n >= first), len(lens))
 
 
 def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: int, eps: float, q_scale: float, blocks: bool = True) -> bool:

@@ -9,13 +9,13 @@ from qorvix_b200.csrc import ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dk,dv,H,G,lens,rate", [(4, 1, 2, 1, [16, 17, 1], 0.1), (20, 17, 2, 2, [31, 32, 33], 1.0), (68, 16, 2, 1, [47, 15, 48], 0.05),
+@pytest.mark.parametrize("dk,dv,H,G,lens,rate", [(4, 1, 2, 1, [256, 17, 1], 0.1), (20, 17, 2, 2, [257, 32, 33], 1.0), (68, 16, 2, 1, [47, 15, 48], 0.05),
                                                  (132, 33, 1, 1, [49, 16], 0.2)])
 def test_edges_of_blocks_against_float64(dk, dv, H, G, lens, rate):
     blocks.test_blocks_against_float64(dk, dv, H, G, lens, rate)
 
 
-@pytest.mark.parametrize("dk,dv", [(64, 24), (128, 40)])
+@pytest.mark.parametrize("dk,dv", [(72, 24), (128, 40)])
 def test_an_infinite_value_reaches_no_earlier_token_and_no_other_column(dk, dv):
     g = torch.Generator(device="cuda").manual_seed(dk)
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
