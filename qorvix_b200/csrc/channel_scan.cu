@@ -452,7 +452,7 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 // The products with S_0 and of the update are mma.sync on both sides' three bfloat16 terms (the six products that count for 24 bits; the
 // large one's sum apart from the small ones', which the tensor cores would cut off), sums over the keys' slices in float32.
 // 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 460 with four tokens at a time and float32 multiply-adds, and
-// 200 here (operands 61, recurrence 139).
+// 161 here (operands 58, recurrence 103; 61 and 139 with operands of float32 that every CTA split again, read straight to registers).
 // Blocks are counted from the start of a request's portion, so cuts agree to rounding (the 32-bit path takes channel_scan_kernel).
 #define CD_BLOCK 16
 #define CD_COLS 16
@@ -460,27 +460,39 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 struct ChannelDeltaArgs {
   float* out; int ld_out;                 // [T, H * dv]
   const float *q, *k, *v, *b, *g; int ld_q, ld_k, ld_v, ld_b, ld_g;
-  float* ws;                              // [slots][H][cd_slot_floats]
+  float* ws;                              // [segments][blocks][H][cd_slot_floats]: blocks block0 ... block0 + blocks - 1 of every segment
+  int block0, blocks;
   float* state; long long slot_stride;    // as ChannelScanArgs
   const int* seg_q_start; const int* seg_slot;
-  int t_base;                             // the first segment's first token
   int H, G, dk, dv, dkp, dvp;             // dkp, dvp: in whole 16s
   float eps, q_scale;
 };
-// A block's floats: X', X'' and W = (g_(l+1) .. g_end) kb_l as the products' operands lie in the lanes, P_end, v', v''.
-__host__ __device__ inline size_t cd_slot_floats(int dkp, int dvp) { return (size_t)49 * dkp + 32 * (size_t)dvp; }
-// Blocks of different segments never share a slot: a segment of n tokens has at most n / 16 + 1 of them.
-__device__ __forceinline__ float* cd_slot(const ChannelDeltaArgs& a, int q0, int s, int block, int h) {
-  return a.ws + ((size_t)((q0 - a.t_base) / CD_BLOCK + s + block) * a.H + h) * cd_slot_floats(a.dkp, a.dvp);
+// A block's floats: X', X'' and W = (g_(l+1) .. g_end) kb_l in three bfloat16 terms, as the products' operands lie in the lanes, P_end;
+// then per tile of 16 columns v' and v'' ([16 tokens][16 columns] each).
+__host__ __device__ inline size_t cd_slot_floats(int dkp, int dvp) { return (size_t)73 * dkp + 32 * (size_t)dvp; }
+__device__ __forceinline__ float* cd_slot(const ChannelDeltaArgs& a, int s, int block, int h) {
+  return a.ws + (((size_t)s * a.blocks + block - a.block0) * a.H + h) * cd_slot_floats(a.dkp, a.dvp);
+}
+// x and y as three bfloat16 terms each (x in the lower half of a word)
+__device__ __forceinline__ void cd_split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
+  uint32_t t[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    t[i] = *(const uint32_t*)&h;
+    x -= __low2float(h);
+    y -= __high2float(h);
+  }
+  t0 = t[0]; t1 = t[1]; t2 = t[2];
 }
 
 // grid (blocks of the longest segment, heads, segments).  Bound by its multiply-adds and the reads of shared memory beside them.
-__global__ void __launch_bounds__(CD_OP_THREADS) delta_block_operands_kernel(const __grid_constant__ ChannelDeltaArgs a) {
+__global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(const __grid_constant__ ChannelDeltaArgs a) {
   extern __shared__ __align__(16) float cd_smem[];
   pdl_wait();
   pdl_launch_dependents();
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0, j0 = blockIdx.x * CD_BLOCK;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0, block = a.block0 + blockIdx.x, j0 = block * CD_BLOCK;
   if (j0 >= len) return;
   const int nb = len - j0 < CD_BLOCK ? len - j0 : CD_BLOCK;
   const int dk = a.dk, dkp = a.dkp, ld = dkp + 4;
@@ -557,13 +569,14 @@ __global__ void __launch_bounds__(CD_OP_THREADS) delta_block_operands_kernel(con
     (lane < CD_BLOCK ? As : Bs)[(lane & 15) * CD_BLOCK + l] = sum[0];
   }
   __syncthreads();
-  float* ws = cd_slot(a, q0, s, blockIdx.x, h);
-  float *X1 = ws, *X2 = X1 + 16 * dkp, *Wf = X2 + 16 * dkp, *Pe = Wf + 16 * dkp, *V1 = Pe + dkp, *V2 = V1 + 16 * a.dvp;
-  for (int col = tid; col < dkp + a.dvp; col += CD_OP_THREADS) {
+  float* ws = cd_slot(a, s, block, h);
+  uint32_t *X1 = (uint32_t*)ws, *X2 = X1 + 24 * dkp, *Wf = X2 + 24 * dkp;
+  float *Pe = ws + 72 * dkp, *Vs = Pe + dkp;
+  for (int col = tid; col < dkp + a.dvp; col += CD_OP_THREADS) {     // (whole warps: dkp and dvp are multiples of 16, and half warps stay together)
     const bool key = col < dkp;
-    float x[CD_BLOCK];
-    float P = 1.f;
+    float x[CD_BLOCK], y[CD_BLOCK];
     if (key) {
+      float P = 1.f;
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) {
         P *= gs[t * ld + col];
@@ -576,50 +589,73 @@ __global__ void __launch_bounds__(CD_OP_THREADS) delta_block_operands_kernel(con
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) x[t] = t < nb && cv < a.dv ? vr[(size_t)t * a.ld_v] : 0.f;
     }
-    float y[CD_BLOCK];
 #pragma unroll
-    for (int t = 0; t < CD_BLOCK; ++t) {
+    for (int t = 1; t < CD_BLOCK; ++t) {
 #pragma unroll
-      for (int l = 0; l < t; ++l) x[t] = fmaf(-As[t * CD_BLOCK + l], x[l], x[t]);
+      for (int l4 = 0; l4 < t; l4 += 4) {
+        const float4 A4 = *(const float4*)(As + t * CD_BLOCK + l4);
+        const float A[4] = {A4.x, A4.y, A4.z, A4.w};
+#pragma unroll
+        for (int l = l4; l < l4 + 4 && l < t; ++l) x[t] = fmaf(-A[l - l4], x[l], x[t]);
+      }
       if (t >= nb) x[t] = 0.f;
     }
 #pragma unroll
     for (int t = 0; t < CD_BLOCK; ++t) {
       y[t] = 0.f;
 #pragma unroll
-      for (int l = 0; l <= t; ++l) y[t] = fmaf(Bs[t * CD_BLOCK + l], x[l], y[t]);
+      for (int l4 = 0; l4 <= t; l4 += 4) {
+        const float4 B4 = *(const float4*)(Bs + t * CD_BLOCK + l4);
+        const float B[4] = {B4.x, B4.y, B4.z, B4.w};
+#pragma unroll
+        for (int l = l4; l < l4 + 4 && l <= t; ++l) y[t] = fmaf(B[l - l4], x[l], y[t]);
+      }
     }
     if (key) {
-      // X' and X'' as the products' first operand: lane (t % 8) 4 + (key % 8) / 2 holds, of keys 0..7 and then 8..15 of a slice, {even key: t, t + 8;
-      // odd key: t, t + 8}
-      P = 1.f;
+      float P = 1.f;
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) {
         P *= gs[t * ld + col];
         y[t] = t < nb ? fmaf(P, qs[t * ld + col], -y[t]) : 0.f;
       }
-      const size_t at = (size_t)(col >> 3) * 128 + ((col & 7) >> 1) * 4 + (col & 1) * 2;
+      // X' and X'' as the products' first operand: lane (t % 8) 4 + (key % 8) / 2 holds, a term, the words of {t, t + 8} x {key, key + 8}, a word
+      // an even key and the next one.  Of two neighbouring keys the even one's thread makes the words of tokens 0..7, the other 8..15.
+      const int odd = col & 1, lane0 = (col & 7) >> 1, reg = odd + 2 * ((col >> 3) & 1);
+      uint32_t* dst = X1 + (size_t)(col >> 4) * 384 + lane0 * 4 + reg;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        *(float2*)(X1 + at + t * 16) = make_float2(x[t], x[t + 8]);
-        *(float2*)(X2 + at + t * 16) = make_float2(y[t], y[t + 8]);
+      for (int m = 0; m < 2; ++m) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          float* z = m ? y : x;
+          const float other = __shfl_xor_sync(3u << (lane & 30), odd ? z[t] : z[t + 8], 1);
+          uint32_t w0, w1, w2;
+          cd_split3(odd ? other : z[t], odd ? z[t + 8] : other, w0, w1, w2);
+          uint32_t* d = dst + m * 24 * dkp + t * 16;
+          d[0] = w0; d[128] = w1; d[256] = w2;
+        }
       }
-      // W as the update's second operand: lane (key % 8) 4 + t4 holds tokens 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9
-      float w[CD_BLOCK], f = 1.f;
+      // W as the update's second operand: lane (key % 8) 4 + t4 holds, a term, {tokens 2 t4, 2 t4 + 1; 2 t4 + 8, 2 t4 + 9} of key and of key + 8
+      float f = 1.f;
 #pragma unroll
       for (int t = CD_BLOCK - 1; t >= 0; --t) {
-        w[t] = f * (beta[t] * ks[t * ld + col]);
+        x[t] = f * (beta[t] * ks[t * ld + col]);
         f *= gs[t * ld + col];
       }
+      uint32_t* wd = Wf + (size_t)(col >> 4) * 384 + (col & 7) * 16 + 2 * ((col >> 3) & 1);
 #pragma unroll
-      for (int t4 = 0; t4 < 4; ++t4)
-        *(float4*)(Wf + (size_t)(col >> 3) * 128 + (col & 7) * 16 + t4 * 4) = make_float4(w[2 * t4], w[2 * t4 + 1], w[2 * t4 + 8], w[2 * t4 + 9]);
+      for (int t4 = 0; t4 < 4; ++t4) {
+        uint32_t w[2][3];
+        cd_split3(x[2 * t4], x[2 * t4 + 1], w[0][0], w[0][1], w[0][2]);
+        cd_split3(x[2 * t4 + 8], x[2 * t4 + 9], w[1][0], w[1][1], w[1][2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *(uint2*)(wd + i * 128 + t4 * 4) = make_uint2(w[0][i], w[1][i]);
+      }
     } else {
       const int cv = col - dkp;
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) {
-        V1[t * a.dvp + cv] = x[t];
-        V2[t * a.dvp + cv] = y[t];
+        Vs[(cv >> 4) * 512 + t * 16 + (cv & 15)] = x[t];
+        Vs[(cv >> 4) * 512 + 256 + t * 16 + (cv & 15)] = y[t];
       }
     }
   }
@@ -629,47 +665,58 @@ __device__ __forceinline__ void cd_mma(float* c, const uint32_t (&a)[4], uint32_
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// x and y as three bfloat16 terms each (x in the lower half of a word)
-__device__ __forceinline__ void cd_split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
-  uint32_t t[3];
+__device__ __forceinline__ void cd_ldsm4(uint32_t (&r)[4], const void* p) {
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+// c = a b of three terms each, as three sums
+struct CdSums { float hi[4], lo[4], lo2[4]; };
+__device__ __forceinline__ void cd_product(CdSums& c, const uint32_t (&a)[3][4], const uint32_t (&b0)[3], const uint32_t (&b1)[3]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c.hi[i] = c.lo[i] = c.lo2[i] = 0.f;
+  cd_mma(c.lo, a[0], b0[1], b1[1]);
+  cd_mma(c.lo2, a[2], b0[0], b1[0]);
+  cd_mma(c.hi, a[0], b0[0], b1[0]);
+  cd_mma(c.lo, a[1], b0[0], b1[0]);
+  cd_mma(c.lo2, a[0], b0[2], b1[2]);
+  cd_mma(c.lo2, a[1], b0[1], b1[1]);
+}
+__device__ __forceinline__ float cd_sum(const CdSums& c, int i) { return c.hi[i] + (c.lo[i] + c.lo2[i]); }
+__device__ __forceinline__ void cd_words(uint32_t (&a)[3][4], const uint4* p) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    t[i] = *(const uint32_t*)&h;
-    x -= __low2float(h);
-    y -= __high2float(h);
+    const uint4 w = p[i * 32];
+    a[i][0] = w.x; a[i][1] = w.y; a[i][2] = w.z; a[i][3] = w.w;
   }
-  t0 = t[0]; t1 = t[1]; t2 = t[2];
-}
-// c = a b of three terms each
-__device__ __forceinline__ void cd_product(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[3], const uint32_t (&b1)[3]) {
-  float hi[4] = {}, lo[4] = {}, lo2[4] = {};
-  cd_mma(lo, a[0], b0[1], b1[1]);
-  cd_mma(lo2, a[2], b0[0], b1[0]);
-  cd_mma(hi, a[0], b0[0], b1[0]);
-  cd_mma(lo, a[1], b0[0], b1[0]);
-  cd_mma(lo2, a[0], b0[2], b1[2]);
-  cd_mma(lo2, a[1], b0[1], b1[1]);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) c[i] = hi[i] + (lo[i] + lo2[i]);
 }
 
 // grid (segments, heads, column tiles); NS warps, a slice of 16 keys each, S^T in registers as the accumulators of the update (value columns x
-// keys), which are the second operand of X S_0.  A block: the slices' shares of X' S_0 and X'' S_0 into shared memory, a barrier, their sums
-// (half of the threads e, half y), a barrier, the update.  The next blocks' operands are on their way to registers meanwhile.  Bound by that
-// chain: 1.
+// keys), which are the second operand of X S_0.  A block: the slices' shares of X' S_0 into shared memory, a barrier, their sums e (and y of
+// the block ahead), a barrier, the update; X'' S_0 is formed between the two, where the tensor cores have nothing else to do, and summed a
+// block later.  The operands arrive STAGES - 1 blocks ahead (cp.async).  Bound by that chain: two barriers, three rounds through shared memory,
+// two products of three terms a side and the splits between them.
+template <int NS> struct CdShape {
+  static constexpr int LD = NS == 16 ? 20 : 24;      // 24: the writes of a half warp hit every bank once; 16 slices of that are too much
+  static constexpr int STAGES = NS == 16 ? 2 : 4;
+  static constexpr int RED = NS * CD_BLOCK * LD;     // floats
+  __host__ __device__ static int stage_floats(int dkp) { return 73 * dkp + 512; }
+  __host__ __device__ static int bytes(int dkp) { return (STAGES * stage_floats(dkp) + 2 * RED) * 4 + 3 * CD_COLS * CD_BLOCK * 2; }
+};
 template <int NS>
 __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_constant__ ChannelDeltaArgs a) {
-  constexpr int EACH = 512 / (32 * NS);              // of the 32 x 16 sums, a thread's
+  typedef CdShape<NS> Sh;
+  constexpr int THREADS = 32 * NS, STAGES = Sh::STAGES, LD = Sh::LD;
+  constexpr int EACH = THREADS >= 256 ? 1 : 256 / THREADS;           // of the 16 x 16 sums, a thread's
   constexpr int PER_ROW = CD_COLS / EACH;            // threads a row
-  constexpr int CD_LD = NS == 16 ? 20 : 24;          // (24: the writes of a half warp hit every bank once; 16 slices of that are too much)
-  __shared__ __align__(16) float red[NS][2 * CD_BLOCK][CD_LD];
-  __shared__ __align__(16) float eT[CD_COLS][CD_LD]; // [column][token]
+  extern __shared__ __align__(16) float cd_smem[];
   pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CD_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  const int dk = a.dk, dv = a.dv, dkp = a.dkp;
+  const int dk = a.dk, dv = a.dv, dkp = a.dkp, stage_floats = Sh::stage_floats(dkp);
+  float* red = cd_smem + STAGES * stage_floats;      // [NS][16][LD] of e
+  float* red2 = red + Sh::RED;                       // of y
+  bf16* eT = (bf16*)(red2 + Sh::RED);                // [term][column][token], 16-byte halves of a row swapped in every other four columns
   const int lpc = dk <= 16 ? 1 : dk <= 32 ? 2 : dk <= 64 ? 4 : dk <= 128 ? 8 : 16, cpt = 32 / lpc, tiles = (dv + cpt - 1) / cpt;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * 512;
   const int k0 = warp * 16;
@@ -678,6 +725,24 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
     const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = col0 + g8 + (i >> 1) * 8;
     return k < 16 * lpc && col < tiles * cpt ? st + (size_t)(col / cpt) * 512 + (k & 15) * 32 + (col % cpt) * lpc + (k >> 4) : nullptr;
   };
+  const int all = (len + CD_BLOCK - 1) / CD_BLOCK - a.block0, nblocks = all < a.blocks ? all : a.blocks;
+  if (nblocks <= 0) return;
+  const size_t stride = (size_t)a.H * cd_slot_floats(dkp, a.dvp);
+  const float* ws = cd_slot(a, s, a.block0, h);
+  const int pieces = 73 * dkp / 4;
+  auto issue = [&](int blk) {
+    if (blk < nblocks) {
+      float* d = cd_smem + (blk % STAGES) * stage_floats;
+      const float* src = ws + (size_t)blk * stride;
+#pragma unroll
+      for (int i = 0; i < 10; ++i)                   // (73 * 16 NS floats are 9.1 pieces a thread)
+        if (tid + i * THREADS < pieces) cs_cp16(d + (tid + i * THREADS) * 4, src + (tid + i * THREADS) * 4, true);
+      if (tid < 128) cs_cp16(d + 73 * dkp + tid * 4, src + 73 * dkp + blockIdx.z * 512 + tid * 4, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < STAGES - 1; ++i) issue(i);
   float S[2][4];
 #pragma unroll
   for (int nt = 0; nt < 2; ++nt)
@@ -686,108 +751,114 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
       const float* p = at(nt, i);
       S[nt][i] = p && k0 + nt * 8 + 2 * t4 + (i & 1) < dk ? *p : 0.f;
     }
-  const int nblocks = (len + CD_BLOCK - 1) / CD_BLOCK;
-  const int orow = tid / PER_ROW, ocol = (tid % PER_ROW) * EACH;     // the sums this thread forms: rows 0..15 e, 16..31 y
-  struct Operands { float4 x[2][2], w[2]; float2 P[2]; float v[EACH]; };
-  const size_t stride = (size_t)a.H * cd_slot_floats(dkp, a.dvp);
-  const float* ws = cd_slot(a, q0, s, 0, h);
-  const float* wx = ws + (k0 >> 3) * 128 + lane * 4;
-  const float* wP = ws + 48 * (size_t)dkp + k0 + 2 * t4;
-  const float* wv = ws + 49 * (size_t)dkp + (size_t)orow * a.dvp + col0 + ocol;      // (v'' follows v')
-  auto fetch = [&](Operands& o, int blk) {
-    if (blk >= nblocks) return;
-    const size_t off = (size_t)blk * stride;
-    if (holds) {
+  const int orow = (tid / PER_ROW) & 15, ocol = (tid % PER_ROW) * EACH;      // the sums this thread forms
+  const bool sums_e = tid < 256, sums_y = THREADS > 256 ? tid >= 256 : true;
+  float v2[EACH] = {};                               // v'' of the block ahead
+  float* yp = a.out + (size_t)(q0 + a.block0 * CD_BLOCK + orow) * a.ld_out + (size_t)h * dv + col0 + ocol;
+  const size_t ystep = (size_t)CD_BLOCK * a.ld_out;
+  const int yleft = len - a.block0 * CD_BLOCK - orow, ycols = dv - col0 - ocol;
+  for (int i = tid; i < 2 * Sh::RED; i += THREADS) red[i] = 0.f;             // (slices that dk does not reach add nothing)
+  auto finish = [&](int blk) {                       // y of a block, from the shares in red2
+    if (!sums_y) return;
+    float sum[EACH] = {};
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        o.x[0][i] = *(const float4*)(wx + off + i * 128);
-        o.x[1][i] = *(const float4*)(wx + off + 16 * dkp + i * 128);
-        o.w[i] = *(const float4*)(wx + off + 32 * dkp + i * 128);
-        o.P[i] = *(const float2*)(wP + off + i * 8);
-      }
+    for (int sl = 0; sl < NS; ++sl)
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) sum[i] += red2[(sl * CD_BLOCK + orow) * LD + ocol + i];
+    if (blk * CD_BLOCK < yleft) {
+#pragma unroll
+      for (int i = 0; i < EACH; ++i)
+        if (i < ycols) yp[i] = v2[i] + sum[i];
     }
-#pragma unroll
-    for (int i = 0; i < EACH; ++i) o.v[i] = wv[off + i];
+    yp += ystep;
   };
-  auto step = [&](Operands& o, int blk) {
-    uint32_t w0[2][3], w1[2][3];                     // [key tile][term]
+  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+  __syncthreads();                                   // block 0 is in place
+  for (int blk = 0; blk < nblocks; ++blk) {
+    const float* d = cd_smem + (blk % STAGES) * stage_floats;
+    const uint4* words = (const uint4*)d + warp * 96 + lane;
+    uint32_t b0[2][3], b1[2][3];                     // S_0: [column tile][term]
+    CdSums c2[2];
+    float v1[EACH];
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) v1[i] = d[73 * dkp + orow * 16 + ocol + i];
     if (holds) {
-      uint32_t b0[2][3], b1[2][3];                   // S_0: [column tile][term]
+      uint32_t x[3][4];
+      cd_words(x, words);
 #pragma unroll
       for (int nb = 0; nb < 2; ++nb) {
         cd_split3(S[0][2 * nb], S[0][2 * nb + 1], b0[nb][0], b0[nb][1], b0[nb][2]);
         cd_split3(S[1][2 * nb], S[1][2 * nb + 1], b1[nb][0], b1[nb][1], b1[nb][2]);
       }
+      CdSums c[2];
+      cd_product(c[0], x, b0[0], b1[0]);
+      cd_product(c[1], x, b0[1], b1[1]);
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        uint32_t af[3][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          cd_split3(o.x[m][i].x, o.x[m][i].z, af[0][2 * i], af[1][2 * i], af[2][2 * i]);
-          cd_split3(o.x[m][i].y, o.x[m][i].w, af[0][2 * i + 1], af[1][2 * i + 1], af[2][2 * i + 1]);
-        }
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          float c[4];
-          cd_product(c, af, b0[nb], b1[nb]);
-          *(float2*)&red[warp][m * CD_BLOCK + g8][nb * 8 + 2 * t4] = make_float2(c[0], c[1]);
-          *(float2*)&red[warp][m * CD_BLOCK + g8 + 8][nb * 8 + 2 * t4] = make_float2(c[2], c[3]);
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        cd_split3(o.w[nt].x, o.w[nt].y, w0[nt][0], w0[nt][1], w0[nt][2]);
-        cd_split3(o.w[nt].z, o.w[nt].w, w1[nt][0], w1[nt][1], w1[nt][2]);
+      for (int nb = 0; nb < 2; ++nb) {
+        float* r = red + (warp * CD_BLOCK + g8) * LD + nb * 8 + 2 * t4;
+        *(float2*)r = make_float2(cd_sum(c[nb], 0), cd_sum(c[nb], 1));
+        *(float2*)(r + 8 * LD) = make_float2(cd_sum(c[nb], 2), cd_sum(c[nb], 3));
       }
     }
-    __syncthreads();                                 // the slices' shares are in place; eT has been read
-    {
-      const int slices = dkp >> 4;
+    __syncthreads();                                 // the shares of e, and of y of the block ahead, are in place; eT and that block's operands have been read
+    if (sums_e) {
       float sum[EACH] = {};
 #pragma unroll
       for (int sl = 0; sl < NS; ++sl)
-        if (sl < slices) {
 #pragma unroll
-          for (int i = 0; i < EACH; ++i) sum[i] += red[sl][orow][ocol + i];
-        }
-      if (orow < CD_BLOCK) {
+        for (int i = 0; i < EACH; ++i) sum[i] += red[(sl * CD_BLOCK + orow) * LD + ocol + i];
 #pragma unroll
-        for (int i = 0; i < EACH; ++i) eT[ocol + i][orow] = o.v[i] - sum[i];
-      } else {
-        const int t = blk * CD_BLOCK + orow - CD_BLOCK;
-        if (t < len) {
-          float* y = a.out + (size_t)(q0 + t) * a.ld_out + (size_t)h * dv + col0 + ocol;
+      for (int i = 0; i < EACH; ++i) {
+        float e = v1[i] - sum[i];
+        bf16* to = eT + (ocol + i) * CD_BLOCK + (orow ^ (((ocol + i) >> 2) & 1) * 8);
 #pragma unroll
-          for (int i = 0; i < EACH; ++i)
-            if (col0 + ocol + i < dv) y[i] = o.v[i] + sum[i];
+        for (int x = 0; x < 3; ++x) {
+          const bf16 term = __float2bfloat16_rn(e);
+          to[x * CD_COLS * CD_BLOCK] = term;
+          e -= __bfloat162float(term);
         }
       }
     }
-    __syncthreads();                                 // e is in place; the shares have been read
     if (holds) {
-      uint32_t af[3][4];                             // e^T: columns g8, g8 + 8; tokens 2 t4, 2 t4 + 1 and 8 further
+      uint32_t x[3][4];
+      cd_words(x, words + 6 * dkp);
+      cd_product(c2[0], x, b0[0], b1[0]);
+      cd_product(c2[1], x, b0[1], b1[1]);
+    }
+    if (blk) finish(blk - 1);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 e = *(const float2*)&eT[g8 + (i & 1) * 8][2 * t4 + (i >> 1) * 8];
-        cd_split3(e.x, e.y, af[0][i], af[1][i], af[2][i]);
+    for (int i = 0; i < EACH; ++i) v2[i] = d[73 * dkp + 256 + orow * 16 + ocol + i];
+    issue(blk + STAGES - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                 // e is in place, and the next block's operands; the shares have been read
+    if (holds) {
+      uint32_t e[3][4], w[3][4];                     // e^T: columns g8, g8 + 8; tokens 2 t4, 2 t4 + 1 and 8 further
+#pragma unroll
+      for (int x = 0; x < 3; ++x) cd_ldsm4(e[x], eT + x * CD_COLS * CD_BLOCK + (lane & 15) * CD_BLOCK + (((lane >> 4) ^ ((lane >> 2) & 1)) * 8));
+      cd_words(w, words + 12 * dkp);
+      CdSums c[2];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const uint32_t w0[3] = {w[0][2 * nt], w[1][2 * nt], w[2][2 * nt]}, w1[3] = {w[0][2 * nt + 1], w[1][2 * nt + 1], w[2][2 * nt + 1]};
+        cd_product(c[nt], e, w0, w1);
       }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        float c[4];
-        cd_product(c, af, w0[nt], w1[nt]);
+        const float2 P = *(const float2*)(d + 72 * dkp + k0 + nt * 8 + 2 * t4);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(i & 1 ? o.P[nt].y : o.P[nt].x, S[nt][i], c[i]);
+        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(i & 1 ? P.y : P.x, S[nt][i], cd_sum(c[nt], i));
+      }
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        float* r = red2 + (warp * CD_BLOCK + g8) * LD + nb * 8 + 2 * t4;
+        *(float2*)r = make_float2(cd_sum(c2[nb], 0), cd_sum(c2[nb], 1));
+        *(float2*)(r + 8 * LD) = make_float2(cd_sum(c2[nb], 2), cd_sum(c2[nb], 3));
       }
     }
-    fetch(o, blk + 2);
-  };
-  Operands o0, o1;
-  fetch(o0, 0);
-  fetch(o1, 1);
-  for (int blk = 0; blk < nblocks; blk += 2) {
-    step(o0, blk);
-    if (blk + 1 < nblocks) step(o1, blk + 1);
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  finish(nblocks - 1);
   pdl_launch_dependents();
 #pragma unroll
   for (int nt = 0; nt < 2; ++nt)
@@ -798,10 +869,28 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
     }
 }
 
-// What qv_channel_delta takes beside its operands, in floats: for lead_tokens that go token by token, and for `tokens` of `segs` segments in blocks.
-extern "C" long long qv_channel_delta_workspace_floats(int lead_tokens, int tokens, int segs, int H, int dk, int dv) {
-  const size_t slots = segs > 0 ? (size_t)tokens / CD_BLOCK + segs : 0;
-  return (long long)((size_t)lead_tokens * H * 3 * dk + slots * H * cd_slot_floats((dk + 15) / 16 * 16, (dv + 15) / 16 * 16));
+template <int NS>
+static int launch_delta_blocks(const ChannelDeltaArgs& a, dim3 grid, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(delta_blocks_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, CdShape<NS>::bytes(16 * NS));
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int smem = CdShape<NS>::bytes(a.dkp);
+  return cs_launch_after(delta_blocks_kernel<NS>, grid, dim3(32 * NS), (size_t)smem, st, a);
+}
+
+// What qv_channel_delta takes beside its operands, in floats: for lead_tokens that go token by token, and for segs segments of up to max_rest tokens
+// in blocks, of which as many at a time as CD_ROOM floats hold (at least one of each segment).
+#define CD_ROOM ((size_t)48 << 20)
+static inline int cd_blocks_at_a_time(int segs, int max_rest, size_t slot) {
+  const size_t blocks = (max_rest + CD_BLOCK - 1) / CD_BLOCK, fit = CD_ROOM / (slot * segs);
+  return (int)(blocks < fit ? blocks : fit ? fit : 1);
+}
+extern "C" long long qv_channel_delta_workspace_floats(int lead_tokens, int segs, int max_rest, int H, int dk, int dv) {
+  const size_t slot = H * cd_slot_floats((dk + 15) / 16 * 16, (dv + 15) / 16 * 16), lead = (size_t)lead_tokens * H * 3 * dk;
+  return (long long)(segs > 0 && max_rest > 0 ? lead + slot * segs * cd_blocks_at_a_time(segs, max_rest, slot) : lead);
 }
 
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
@@ -830,20 +919,24 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
   ChannelDeltaArgs a;
   a.out = out; a.ld_out = ld_out; a.q = q; a.k = k; a.v = v; a.b = b; a.g = g; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.ld_b = ld_b; a.ld_g = ld_g;
   a.ws = workspace; a.state = state; a.slot_stride = slot_stride; a.seg_q_start = seg_q_start + S_lead; a.seg_slot = seg_slot + S_lead;
-  a.t_base = T_lead; a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.dkp = (dk + 15) / 16 * 16; a.dvp = (dv + 15) / 16 * 16; a.eps = eps; a.q_scale = q_scale;
-  const int rest = S - S_lead, col_tiles = a.dvp / CD_COLS;
+  a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.dkp = (dk + 15) / 16 * 16; a.dvp = (dv + 15) / 16 * 16; a.eps = eps; a.q_scale = q_scale;
+  const int rest = S - S_lead, col_tiles = a.dvp / CD_COLS, blocks = (max_rest + CD_BLOCK - 1) / CD_BLOCK;
   if (rest > 65535 || col_tiles > 65535) return QV_ERR_TOO_LARGE;
   const int smem = (3 * CD_BLOCK * (a.dkp + 4) + 2 * CD_BLOCK * CD_BLOCK + CD_BLOCK) * 4;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(delta_block_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
   }
-  const int rc = qv_launch(delta_block_operands_kernel, dim3((max_rest + CD_BLOCK - 1) / CD_BLOCK, H, rest), dim3(CD_OP_THREADS), (size_t)smem, st, a);
-  if (rc) return rc;
-  const dim3 grid(rest, H, col_tiles);
-  if (dk <= 64) return cs_launch_after(delta_blocks_kernel<4>, grid, dim3(128), 0, st, a);
-  if (dk <= 128) return cs_launch_after(delta_blocks_kernel<8>, grid, dim3(256), 0, st, a);
-  return cs_launch_after(delta_blocks_kernel<16>, grid, dim3(512), 0, st, a);
+  a.blocks = cd_blocks_at_a_time(rest, max_rest, H * cd_slot_floats(a.dkp, a.dvp));
+  for (a.block0 = 0; a.block0 < blocks; a.block0 += a.blocks) {
+    int rc = qv_launch(delta_block_operands_kernel, dim3(blocks - a.block0 < a.blocks ? blocks - a.block0 : a.blocks, H, rest), dim3(CD_OP_THREADS),
+                       (size_t)smem, st, a);
+    if (rc) return rc;
+    const dim3 grid(rest, H, col_tiles);
+    rc = dk <= 64 ? launch_delta_blocks<4>(a, grid, st) : dk <= 128 ? launch_delta_blocks<8>(a, grid, st) : launch_delta_blocks<16>(a, grid, st);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 // ---------------------------------------------------------------- unit norm per head, weight, gate, factor

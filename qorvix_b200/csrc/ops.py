@@ -1055,8 +1055,8 @@ def delta_lead(lens, dk: int, blocks: bool = True) -> int:
     """How many of a step's leading segments the delta rule takes token by token: those ahead of the first of DELTA_BLOCKS_FROM tokens (single
     tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries.  Keys of up to 64 entries have
     half the work a token: portions of up to 256 tokens cost a layer the same either way (8 heads of 64: 64 tokens 149 us token by token
-    and 151 in blocks, four portions of 256 151 and 151, which is the host's time; 1,531 tokens 552 and 204).  16 heads of 128: 16 tokens 153 and
-    151, four portions of 200 252 and 201, 1,531 tokens 637 (four tokens at a time) and 374."""
+    and 151 in blocks, four portions of 256 151 and 151, which is the host's time; 1,531 tokens 552 and 175).  16 heads of 128: 16 tokens 153 and
+    151, four portions of 200 252 and 201, 1,531 tokens 637 (four tokens at a time) and 338."""
     if not blocks or dk % 4 or dk > 256:
         return len(lens)
     first = DELTA_BLOCKS_FROM if dk > 64 else DELTA_SHORT_KEYS_FROM
@@ -1075,7 +1075,7 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lead = delta_lead(lens, dk, blocks)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
     lib = _lib("channel_scan")
-    ws = _room(lib.qv_channel_delta_workspace_floats(tokens, T - tokens, S - lead, H, dk, dv), torch.float32, q.device) if lead < S else None
+    ws = _room(lib.qv_channel_delta_workspace_floats(tokens, S - lead, max(lens[lead:]), H, dk, dv), torch.float32, q.device) if lead < S else None
     if ws is None:                                    # token by token, which takes less room
         lead, tokens, longest = S, T, int(ctx.max_q_len)
         ws = torch.empty(H * T * 3 * dk, device=q.device, dtype=torch.float32)

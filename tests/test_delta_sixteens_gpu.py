@@ -35,3 +35,22 @@ def test_an_infinite_value_reaches_no_earlier_token_and_no_other_column(dk, dv):
     others = torch.arange(H * dv, device="cuda") != 3
     assert bool(torch.isfinite(clean).all()) and torch.equal(got[:at], clean[:at]) and torch.equal(got[:, others], clean[:, others])
     assert not bool(torch.isfinite(got[at:, 3]).any())
+
+
+def test_a_part_of_the_blocks_at_a_time():
+    """Four portions whose blocks' operands are more than the workspace may hold take two rounds of launches, the second from where the first
+    one ended; against token by token, float32 sums of up to 256 products in two orders, some 1e-7 each."""
+    H, dk, dv, lens = 16, 256, 256, [640, 600, 20, 477]
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, ctx = sum(lens), blocks.context(lens)
+    need = ops._lib("channel_scan").qv_channel_delta_workspace_floats
+    assert need(0, 4, 640, H, dk, dv) < 40 * need(0, 4, 16, H, dk, dv)
+    q, k, v, b, decay = rnd(T, dk), rnd(T, dk), rnd(T, H * dv), rnd(T, H), torch.exp(-0.2 * rnd(T, H * dk).abs())
+    results = []
+    for sixteens in (True, False):
+        state, out = torch.zeros(4, ops.channel_scan_state_floats(H, dk, dv), device="cuda"), torch.full((T, H * dv), float("nan"), device="cuda")
+        ops.channel_delta(out, q, k, v, b, decay, state, ctx, H, 1, dk, dv, 1e-6, dk ** -0.5, blocks=sixteens)
+        results.append((out, state))
+    for x, y in zip(*results):
+        assert float((x - y).norm() / y.norm()) < 2e-6
