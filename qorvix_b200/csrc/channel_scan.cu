@@ -35,12 +35,20 @@
 // few tokens still has many loads in flight and the order of a sum depends on R alone.
 // Portions take 16 tokens a CTA and, where R is a multiple of 16, read a token's row four entries at a time (one shared-memory read a
 // multiply-add: 47 us for 1,531 tokens x 64 x 2,048; now 38).  The order of a sum is the same.
+struct CgForm { int kind; float p; const float* rate; };
+__device__ __forceinline__ float cg_gate(float zz, const CgForm& f, int c) {
+  if (f.kind == GATE_POW_SIGMOID) return expf(f.p * (fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))));             // log sigmoid(z)
+  if (f.kind == GATE_EXP_NEG_SIGMOID) return expf(-f.p * (1.0f / (1.0f + expf(-zz))));
+  if (f.kind == GATE_EXP_NEG_SOFTPLUS) return expf(-f.rate[c] * (fmaxf(zz, 0.f) + log1pf(expf(-fabsf(zz)))));  // softplus(z)
+  return zz;
+}
+
 #define CG_CHANNELS 64
 template <int CG_TOKENS>
 __global__ void __launch_bounds__(4 * CG_CHANNELS) channel_gates_kernel(float* __restrict__ out, int ld_out, const float* __restrict__ x1,
                                                                        int ld_x, const float* __restrict__ w2t,
                                                                        const float* __restrict__ bias, int T, int N, int R,
-                                                                       int pre_tanh, int kind, float p, const float* __restrict__ rate) {
+                                                                       int pre_tanh, CgForm form) {
   extern __shared__ __align__(16) float cg_smem[]; // [CG_TOKENS][R] the tokens' low-rank rows, then [4][CG_TOKENS][CG_CHANNELS] partial sums
   float* xs = cg_smem;
   float* part = cg_smem + CG_TOKENS * R;
@@ -98,20 +106,84 @@ __global__ void __launch_bounds__(4 * CG_CHANNELS) channel_gates_kernel(float* _
 #pragma unroll
     for (int q = 1; q < 4; ++q) zz += part[(q * CG_TOKENS + j) * CG_CHANNELS + cl];
     zz += bc;
-    float g;
-    if (kind == GATE_POW_SIGMOID) {
-      const float ls = fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)));          // log sigmoid(z)
-      g = expf(p * ls);
-    } else if (kind == GATE_EXP_NEG_SIGMOID) {
-      g = expf(-p * (1.0f / (1.0f + expf(-zz))));
-    } else if (kind == GATE_EXP_NEG_SOFTPLUS) {
-      const float sp = fmaxf(zz, 0.f) + log1pf(expf(-fabsf(zz)));          // softplus(z)
-      g = expf(-rate[c] * sp);
-    } else {
-      g = zz;
-    }
-    out[(size_t)(t0 + j) * ld_out + c] = g;
+    out[(size_t)(t0 + j) * ld_out + c] = cg_gate(zz, form, c);
   }
+}
+
+// Portions of many tokens with ranks in whole 16s: a tile of 64 tokens x 64 channels a CTA, 8 x 4 of them a thread, whose sums stay in registers (the
+// kernel above has a multiply-add for each entry of x it reads, and meets in shared memory): 1,531 tokens x 64 x 2,048 with softplus 37 us
+// above, 28 here (without a function 30 and 21); bound by the multiply-adds and the gates' functions.  The same sums in the same order: four quarters of a row, added in
+// order.
+#define CT_TOKENS 64
+#define CT_MAX_RANK 128
+__global__ void __launch_bounds__(128, 5) channel_gates_tile_kernel(float* __restrict__ out, int ld_out, const float* __restrict__ x1, int ld_x,
+                                                                 const float* __restrict__ w2t, const float* __restrict__ bias, int T, int N, int R,
+                                                                 int pre_tanh, CgForm form) {
+  extern __shared__ __align__(16) float cg_smem[];   // [64 tokens][R + 4], [R][64 channels]
+  const int ldx = R + 4;
+  float* xs = cg_smem;
+  float* wsm = xs + CT_TOKENS * ldx;
+  const int tid = threadIdx.x, c0 = blockIdx.y * CG_CHANNELS, t0 = blockIdx.x * CT_TOKENS;
+#pragma unroll 8
+  for (int i = tid; i < R * CG_CHANNELS; i += 128) {                 // (weights: no kernel writes them)
+    const int r = i / CG_CHANNELS, c = c0 + i % CG_CHANNELS;
+    wsm[i] = c < N ? w2t[(size_t)r * N + c] : 0.f;
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int r = tid & 31; r < R; r += 32) {           // a token a warp
+    const float* xp = x1 + (size_t)t0 * ld_x + r;
+#pragma unroll 8
+    for (int j = tid >> 5; j < CT_TOKENS; j += 4) {
+      float v = t0 + j < T ? xp[(size_t)j * ld_x] : 0.f;
+      if (pre_tanh) v = tanhf(v);
+      xs[j * ldx + r] = v;
+    }
+  }
+  __syncthreads();
+  const int cl = (tid & 15) * 4, tl = (tid >> 4) * 8;
+  float z[8][4] = {};
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {
+    float part[8][4] = {};
+#pragma unroll 1
+    for (int r = q * (R >> 2); r < (q + 1) * (R >> 2); r += 4) {
+      float w[4][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 v = *(const float4*)(wsm + (r + k) * CG_CHANNELS + cl);
+        w[k][0] = v.x; w[k][1] = v.y; w[k][2] = v.z; w[k][3] = v.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 x = *(const float4*)(xs + (tl + j) * ldx + r);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          part[j][c] = fmaf(x.x, w[0][c], part[j][c]);
+          part[j][c] = fmaf(x.y, w[1][c], part[j][c]);
+          part[j][c] = fmaf(x.z, w[2][c], part[j][c]);
+          part[j][c] = fmaf(x.w, w[3][c], part[j][c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) z[j][c] += part[j][c];
+  }
+  // the gates' functions in a loop over the tile in shared memory: written out for a thread's 32 sums they are more code than the
+  // instruction cache holds
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) *(float4*)(cg_smem + (tl + j) * (CG_CHANNELS + 4) + cl) = make_float4(z[j][0], z[j][1], z[j][2], z[j][3]);
+  __syncthreads();
+  const int c = c0 + (tid & 63);
+  if (c >= N) return;
+  const float bc = bias ? bias[c] : 0.f;
+  const int last = T - t0 < CT_TOKENS ? T - t0 : CT_TOKENS;
+  float* o = out + (size_t)t0 * ld_out + c;
+#pragma unroll 2
+  for (int j = tid >> 6; j < last; j += 2) o[(size_t)j * ld_out] = cg_gate(cg_smem[j * (CG_CHANNELS + 4) + (tid & 63)] + bc, form, c);
 }
 
 // rate [N] float32: the factor per channel of GATE_EXP_NEG_SOFTPLUS (null for the other kinds).
@@ -126,11 +198,23 @@ extern "C" int qv_channel_gates(float* out, int ld_out, const float* x1, int ld_
   const int by = (N + CG_CHANNELS - 1) / CG_CHANNELS;
   if (by > 65535) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
+  const CgForm form = {kind, p, rate};
+  if (T >= 256 && R % 16 == 0 && R <= CT_MAX_RANK) {
+    static bool configured = false;
+    constexpr int most = (CT_TOKENS * (CT_MAX_RANK + 4) + CT_MAX_RANK * CG_CHANNELS) * 4;
+    if (!configured) {
+      const cudaError_t e = cudaFuncSetAttribute(channel_gates_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      if (e != cudaSuccess) return (int)e;
+      configured = true;
+    }
+    return qv_launch(channel_gates_tile_kernel, dim3((T + CT_TOKENS - 1) / CT_TOKENS, by), dim3(128),
+                     (size_t)(CT_TOKENS * (R + 4) + R * CG_CHANNELS) * 4 + (R < 48 ? CT_TOKENS * (CG_CHANNELS + 4) * 4 : 0), st, out, ld_out, x1, ld_x, w2t, bias, T, N, R, pre_tanh, form);
+  }
   const int per = 65535 * tokens;
   for (int done = 0; done < T; done += per) {
     const int rows = T - done < per ? T - done : per;
     const int rc = qv_launch(tokens == 16 ? channel_gates_kernel<16> : channel_gates_kernel<8>, dim3((rows + tokens - 1) / tokens, by), dim3(4 * CG_CHANNELS), smem, st,
-                             out + (size_t)done * ld_out, ld_out, x1 + (size_t)done * ld_x, ld_x, w2t, bias, rows, N, R, pre_tanh, kind, p, rate);
+                             out + (size_t)done * ld_out, ld_out, x1 + (size_t)done * ld_x, ld_x, w2t, bias, rows, N, R, pre_tanh, form);
     if (rc) return rc;
   }
   return 0;
