@@ -12,7 +12,9 @@
 // types, odd strides) through registers, all of a thread's elements of the next tile in flight under the present one's multiply-adds; and
 // a thread reads four k of a row at a time.  Two tile shapes: 16 x 32 (64 k, 2 x 2 outputs a thread) where 64 x 64 tiles would be few
 // or mostly padding, else 64 x 64 (32 k, 4 x 4 a thread).  Few CTAs are bound by the chain of K dependent multiply-adds and the
-// staging around it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (now 5 / 10 us, 3 rows).
+// trips to memory ahead of it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (3 rows), with three
+// tiles of 64 k 3.6 / 8.4 us behind the kernel ahead.  So products of one wave of CTAs get a ring of eight tiles, and the weights' halves of the
+// first ones are asked for ahead of the wait for the kernel ahead (no kernel writes weights): 2.5 / 5.0 us.
 #include "common.cuh"
 
 __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live) {
@@ -25,7 +27,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
                                                                         const TW* __restrict__ W, int M, int N, int K,
                                                                         int lda, int ldw, int ldc, int accumulate) {
   constexpr int THREADS = (BM / TM) * (BN / TN), LD = BK + 4, ROWS = BM + BN, PIECES = BK / 4;
-  __shared__ __align__(16) float ring[STAGES][ROWS * LD];
+  extern __shared__ __align__(16) float gs_ring[];
+  float(*ring)[ROWS * LD] = (float(*)[ROWS * LD])gs_ring;            // [STAGES]
   const int tid = threadIdx.x;
   constexpr int TX = BN / TN, TY = BM / TM;        // a thread's outputs: rows ty + TY * i, columns tx + TX * j
   const int tx = tid % TX, ty = tid / TX;
@@ -36,24 +39,24 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-  pdl_wait();
-  pdl_launch_dependents();
   const int tiles = (K + BK - 1) / BK;
-  auto stage = [&](int t) {                        // tile t into its buffer; zeros beyond the matrices
+  auto stage = [&](int t, int first, int last) {   // rows first .. last - 1 of tile t (A's, then W's) into its buffer; zeros beyond the matrices
     float* dst = ring[t % STAGES];
     const int k0 = t * BK;
-    if (ASYNC) {
-      for (int e = tid; e < ROWS * PIECES; e += THREADS) {
-        const int r = e / PIECES, k = k0 + (e % PIECES) * 4;
-        const bool is_a = r < BM;
-        const int g = is_a ? m0 + r : n0 + r - BM;
-        const bool live = (is_a ? g < M : g < N) && k < K;
-        const float* src = is_a ? (const float*)A + (size_t)g * lda + k : (const float*)W + (size_t)g * ldw + k;
-        gs_cp16(dst + r * LD + (e % PIECES) * 4, live ? src : (const float*)W, live);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 4
+    for (int e = first * PIECES + tid; e < last * PIECES; e += THREADS) {
+      const int r = e / PIECES, k = k0 + (e % PIECES) * 4;
+      const bool is_a = r < BM;
+      const int g = is_a ? m0 + r : n0 + r - BM;
+      const bool live = (is_a ? g < M : g < N) && k < K;
+      const float* src = is_a ? (const float*)A + (size_t)g * lda + k : (const float*)W + (size_t)g * ldw + k;
+      gs_cp16(dst + r * LD + (e % PIECES) * 4, live ? src : (const float*)W, live);
     }
   };
+  if (ASYNC)
+    for (int t = 0; t < STAGES - 1 && t < tiles; ++t) stage(t, BM, ROWS);      // (with the first commit below)
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int PER_A = BM * BK / THREADS, PER_W = BN * BK / THREADS;
   static_assert(BM * BK % THREADS == 0 && BN * BK % THREADS == 0, "every thread stages as many elements");
   TA va[PER_A];
@@ -79,8 +82,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
   };
   if (ASYNC) {
     for (int t = 0; t < STAGES - 1; ++t) {
-      if (t < tiles) stage(t);
-      else asm volatile("cp.async.commit_group;" ::: "memory");
+      if (t < tiles) stage(t, 0, BM);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
   } else if (tiles > 0) {
     fetch(0);
@@ -90,8 +93,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
     if (ASYNC) asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();                               // tile t has landed; the buffer filled next was read a tile ago
     if (ASYNC) {
-      if (t + STAGES - 1 < tiles) stage(t + STAGES - 1);
-      else asm volatile("cp.async.commit_group;" ::: "memory");
+      if (t + STAGES - 1 < tiles) stage(t + STAGES - 1, 0, ROWS);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     } else if (t + 1 < tiles) {
       fetch(t + 1);
     }
@@ -142,13 +145,28 @@ static int launch(void* C, const void* A, const void* W, int M, int N, int K, in
   dim3 grid(small ? (N + 31) / 32 : (N + 63) / 64, small ? (M + 15) / 16 : (M + 63) / 64);
   if (grid.y > 65535) return QV_ERR_TOO_LARGE;
 #define GS_LAUNCH(BM, BN, BK, TM, TN, ST, AS)                                                                                    \
-  return qv_launch(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, grid, dim3((BM / TM) * (BN / TN)), 0, st, (TC*)C,   \
-                   (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, accumulate)
+  do {                                                                                                                           \
+    constexpr size_t smem = (size_t)ST * (BM + BN) * (BK + 4) * 4;                                                               \
+    static bool configured = smem <= 48 * 1024;                                                                                  \
+    if (!configured) {                                                                                                           \
+      const cudaError_t e = cudaFuncSetAttribute(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>,                       \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
+      if (e != cudaSuccess) return (int)e;                                                                                       \
+      configured = true;                                                                                                         \
+    }                                                                                                                            \
+    return qv_launch(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, grid, dim3((BM / TM) * (BN / TN)), smem, st, (TC*)C, \
+                     (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, accumulate);                                            \
+  } while (0)
   if (small) {
-    if (async) GS_LAUNCH(16, 32, 64, 2, 2, 3, true);
+    if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
+      if (async && (long long)grid.x * grid.y <= 148) GS_LAUNCH(16, 32, 64, 2, 2, 8, true);      // a CTA an SM
+      if (async) GS_LAUNCH(16, 32, 64, 2, 2, 3, true);
+    }
     GS_LAUNCH(16, 32, 64, 2, 2, 2, false);
   }
-  if (async) GS_LAUNCH(64, 64, 32, 4, 4, 2, true);
+  if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
+    if (async) GS_LAUNCH(64, 64, 32, 4, 4, 2, true);
+  }
   GS_LAUNCH(64, 64, 32, 4, 4, 2, false);
 #undef GS_LAUNCH
 }
