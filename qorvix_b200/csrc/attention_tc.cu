@@ -22,7 +22,8 @@
 //                 warpgroup has written P, then S = Q K^T of the next keys into the tile's S.
 //   warp 2        TMA: an item's Q tiles, each as soon as the last Q.K^T of the item before has read
 //                 the old one.
-//   warps 4..11   softmax of tile A, warps 12..19 of tile B, two warpgroups each.  A query row is
+//   warps 4..11   softmax of tile A, warps 12..19 of tile B, two warpgroups each (DIFF, ROPE: all four share the one tile, four threads a row
+//                 with 32 keys each; a latent layer of 2,048 tokens 143 us with two threads a row, 136 so).  A query row is
 //                 shared by two threads (one per warpgroup, same lane of tensor memory), each owning 64
 //                 of the tile's 128 keys: it reads its part of the row of S (once for the maximum, on
 //                 which it agrees with its partner through shared memory, and once more, 32 columns
@@ -144,8 +145,8 @@ struct Walk {
 // all three as columns of the cache's rows (map_kv: [rows of all pages][G (2 x 64 + HD)], boxes of 16 rows).  Weights enter P.V as three
 // bfloat16 terms that hold their 24 bits: the large one and the middle one over the thread's share of S, the small one in the room that
 // a second query tile's output would take.  Values of keys that nobody in the item sees enter as zeros: their rows may hold anything (what
-// an earlier owner of the page left behind), and a weight of zero would not keep an infinity or a NaN out of the sums.  All sixteen softmax warps work on the one tile, four threads a row (1,500 tokens behind 500, 16 heads, window 1,024: 106 us; with two
-// threads a row 160, the mma.sync kernel 184).  The normalised rows leave in float32, [tokens][a.H][HD], for diff_rows_kernel.
+// an earlier owner of the page left behind), and a weight of zero would not keep an infinity or a NaN out of the sums.  (1,500 tokens behind 500, 16 heads, window 1,024: 106 us; with two threads a
+// row 160, the mma.sync kernel 184.)  The normalised rows leave in float32, [tokens][a.H][HD], for diff_rows_kernel.
 template <int HD, bool PAIRED, int ROPE, bool DIFF>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                        const __grid_constant__ CUtensorMap map_kv,
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
   constexpr int V_BYTES = KT * HD * 2;               // [NH][128 keys][64]
   constexpr int HALF_BYTES = 128 * 128;              // one [128][64] bf16 tile
   static_assert(2 * KT + 2 * HD <= 512, "S and O of both query tiles must fit tensor memory");
-  constexpr int WGS = DIFF ? 4 : 2;                  // softmax warpgroups that share a query tile's rows (keys KT / WGS each)
+  constexpr int WGS = DIFF || ROPE ? 4 : 2;          // softmax warpgroups that share a query tile's rows (keys KT / WGS each)
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = base;                                // tiles A and B
   constexpr int K_ST = PAIRED || ROPE ? K_ST_PAIRS : K_ST_SINGLE;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         if (!mbar_wait(&v_full[vs], (g / V_ST) & 1, a.err, 16)) return false;
         if (!mbar_wait(&p_full[x], n_pv[x] & 1, a.err, 15)) return false;
         tc_fence_after();
-        // P [128 rows][128 keys] in tensor memory, two keys per column, each softmax warpgroup's 64 keys at the
+        // P [128 rows][128 keys] in tensor memory, two keys per column, each softmax warpgroup's keys at the
         // start of its share of S; V [128 keys][HD] MN-major
         const uint32_t o = tmem_o + (uint32_t)(qx * HD), p = tmem + (uint32_t)(x * KT);
         if (DIFF && leader) {
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk) {
           const uint32_t v_addr = smem_u32(sV + vs * V_BYTES + (kk * 16) * 128);
-          const uint32_t p_col = (uint32_t)(((kk * 16) / 64) * 64 + ((kk * 16) % 64) / 2);
+          const uint32_t p_col = (uint32_t)(((kk * 16) / (KT / WGS)) * (KT / WGS) + ((kk * 16) % (KT / WGS)) / 2);
           umma_f16_ts(o, p + p_col, umma_desc_mn(v_addr, HALF_BYTES), idesc_pv, (kk > 0 || j > 0) ? 1u : 0u);
         }
         umma_commit(&pv_done[x]);
@@ -437,7 +438,8 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
     // softmax: thread = (query row of tile x, half of the tile's keys)
     constexpr int KPT = KT / WGS;                      // keys of a tile per thread
     constexpr int OPT = HD / WGS;                      // output columns per thread
-    const int x = DIFF ? 0 : (warp - 4) >> 3;
+    constexpr int OC = OPT < 32 ? OPT : 32;            // of these at a time
+    const int x = WGS == 4 ? 0 : (warp - 4) >> 3;
     const int wg = ((warp - 4) >> 2) & (WGS - 1);      // which share of the keys and of the output columns
     const int qd = warp & 3;                           // the quarter of tensor memory's lanes this warp may touch
     const int r = qd * 32 + lane;
@@ -467,9 +469,9 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&s_full[buf], phase, a.err, 17));
         // first pass over this thread's part of the row of S: its maximum
         float mx = -INFINITY;
+        uint32_t sv[KPT];
         if (ok) {
           tc_fence_after();
-          uint32_t sv[KPT];
           tmem_ld32(s_addr, sv);
           if (KPT > 32) tmem_ld32(s_addr + 32, sv + KPT - 32);
           tmem_wait_ld();
@@ -521,23 +523,24 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
             tc_fence_after();
           }
 #pragma unroll 1
-          for (int c = 0; c < OPT; c += 32) {
-            uint32_t v[32];
-            tmem_ld32(o_addr + c, v);
+          for (int c = 0; c < OPT; c += OC) {
+            uint32_t v[OC];
+            if constexpr (OC == 32) tmem_ld32(o_addr + c, v);
+            else tmem_ld16(o_addr + c, v);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * corr);
-            tmem_st32(o_addr + c, v);
+            for (int i = 0; i < OC; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * corr);
+            if constexpr (OC == 32) tmem_st32(o_addr + c, v);
+            else tmem_st16(o_addr + c, v);
           }
         }
-        // second pass, 32 columns at a time:
+        // second pass (over the scores as they were read where a thread has 32 of them, else read again, 32 columns at a time):
         // the exponentials, as P over the first half of this thread's columns (a store overwrites
         // only columns that have been read), and their sum
         const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
         float sum = 0.f;
         if (DIFF) {
           // the whole share is read before the first term goes over it; 16 scores at a time become 3 x 8 words
-          uint32_t sv[KPT];
           tmem_ld32(s_addr, sv);
           tmem_wait_ld();
           const uint32_t lo_addr = tmem_lo + lane_base + (uint32_t)(buf * 64 + wg * (KPT / 2));
@@ -569,9 +572,11 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         } else
 #pragma unroll
         for (int c = 0; c < KPT; c += 32) {
-          uint32_t sv[32], w[16];
-          tmem_ld32(s_addr + c, sv);
-          tmem_wait_ld();
+          uint32_t w[16];
+          if (KPT > 32) {                                // (64 scores a thread are too many to keep: they are read again)
+            tmem_ld32(s_addr + c, sv);
+            tmem_wait_ld();
+          }
           if (all_visible) {                             // most tiles: no mask, two instructions per score
             float s4[4] = {0.f, 0.f, 0.f, 0.f};          // the row sum in four chains, added in a fixed order
 #pragma unroll
@@ -624,15 +629,16 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
         bf16* orow = a.out + (size_t)(t.q0 + (store ? row_in_seg : 0)) * a.ld_out + (size_t)t.h * HD + wg * OPT;
         const bf16* grow = ROPE > 0 && a.gate ? a.gate + (size_t)(t.q0 + (store ? row_in_seg : 0)) * a.ld_gate + (size_t)t.h * HD + wg * OPT : nullptr;
 #pragma unroll 1
-        for (int c = 0; c < OPT; c += 32) {
-          uint32_t v[32];
-          tmem_ld32(o_addr + c, v);
+        for (int c = 0; c < OPT; c += OC) {
+          uint32_t v[OC];
+          if constexpr (OC == 32) tmem_ld32(o_addr + c, v);
+          else tmem_ld16(o_addr + c, v);
           tmem_wait_ld();
           if (DIFF) {
             if (store) {
               float* frow = (float*)a.out + ((size_t)(t.q0 + row_in_seg) * a.H + t.h) * HD + wg * OPT;
 #pragma unroll
-              for (int i = 0; i < 32; i += 4)
+              for (int i = 0; i < OC; i += 4)
                 *(float4*)(frow + c + i) = make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv, __uint_as_float(v[i + 2]) * inv,
                                                        __uint_as_float(v[i + 3]) * inv);
             }
@@ -640,7 +646,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           }
           if (ROPE > 0 && grow && store) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
+            for (int i = 0; i < OC; i += 8) {
               const uint4 gv = *(const uint4*)(grow + c + i);
               const bf16* ge = (const bf16*)&gv;
 #pragma unroll
@@ -650,7 +656,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_prefill_tc_kernel(const __g
           }
           if (store) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8)
+            for (int i = 0; i < OC; i += 8)
               *(uint4*)(orow + c + i) = make_uint4(pack2_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv),
                                                    pack2_bf16(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv),
                                                    pack2_bf16(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv),
