@@ -84,6 +84,89 @@ __global__ void __launch_bounds__(256) diff_prepare_kernel(T* __restrict__ q_out
   }
 }
 
+// Portions: a lane holds four neighbouring entries of a map of 4 LANES, so a warp takes 32 / LANES maps at once, straight from the projection; the
+// rotation's other half comes by shuffle, and the lane's weights and angles are the same for all of its maps.  Four warps a token.
+// 1,500 tokens of 16 + 4 heads of 2 x 64 + 128: 21 us with the kernel above (270 instructions a map), 12 here, bound by the
+// projection's 18 MB and the launch around them.
+#define DP_WARPS 4
+template <int LANES>
+__global__ void __launch_bounds__(256) diff_prepare_vec_kernel(bf16* __restrict__ q_out, int ld_q, const float* __restrict__ proj, int ld_p,
+                                                               const float* __restrict__ bias, const float* __restrict__ qw,
+                                                               const float* __restrict__ kw, float eps, const float2* __restrict__ cos_sin,
+                                                               int table_rows, const int* __restrict__ tok_pos, const int* __restrict__ tok_seg,
+                                                               const int* __restrict__ block_table, int max_blocks, bf16* __restrict__ cache, int T,
+                                                               int H, int G, int dv, int rot, int page) {
+  constexpr int N = 4 * LANES, MAPS = 32 / LANES;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int unit0 = blockIdx.x * 8 + (threadIdx.x >> 5), t = unit0 / DP_WARPS, part = unit0 % DP_WARPS, lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const int e = lane % LANES * 4, half = rot >> 1, nq = 2 * H, maps = nq + (cache ? 2 * G : 0);
+  const float* prow = proj + (size_t)t * ld_p;
+  const int pos = tok_pos[t];
+  bf16* crow = nullptr;
+  if (cache) {
+    const int pg = block_table[(size_t)tok_seg[t] * max_blocks + pos / page];
+    crow = cache + ((size_t)pg * page + pos % page) * ((size_t)G * (2 * N + dv));
+  }
+  float cosv[4] = {1.f, 1.f, 1.f, 1.f}, sinv[4] = {0.f, 0.f, 0.f, 0.f};
+  int other = lane;                                          // the lane that holds the other half of the pairs
+  if (e < rot) {
+    const float2* cs = cos_sin + (size_t)(pos < table_rows ? pos : table_rows - 1) * half + (e < half ? e : e - half);
+    other = e < half ? lane + half / 4 : lane - half / 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 c = cs[i];
+      cosv[i] = c.x;
+      sinv[i] = e < half ? -c.y : c.y;
+    }
+  }
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+  const float4 wq = qw ? *(const float4*)(qw + e) : one, wk = kw ? *(const float4*)(kw + e) : one;
+#pragma unroll 2
+  for (int m0 = part * MAPS; m0 < maps; m0 += DP_WARPS * MAPS) {
+    const int m = m0 + lane / LANES;
+    const bool live = m < maps, is_q = m < nq;
+    float x[4] = {};
+    if (live) {
+      const float4 v = *(const float4*)(prow + m * N + e);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+      if (bias) {
+        const float4 b = *(const float4*)(bias + m * N + e);
+        x[0] += b.x; x[1] += b.y; x[2] += b.z; x[3] += b.w;
+      }
+    }
+    if (is_q ? qw != nullptr : kw != nullptr) {
+      float ss = fmaf(x[0], x[0], x[1] * x[1]) + fmaf(x[2], x[2], x[3] * x[3]);
+      const unsigned group = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (lane / LANES * LANES);
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
+      const float inv = 1.0f / sqrtf(ss / (float)N + eps);
+      const float4 w = is_q ? wq : wk;
+      x[0] = x[0] * inv * w.x; x[1] = x[1] * inv * w.y; x[2] = x[2] * inv * w.z; x[3] = x[3] * inv * w.w;
+    }
+    __syncwarp();
+    alignas(8) bf16 o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float y = __shfl_sync(0xffffffffu, x[i], other);
+      o[i] = __float2bfloat16_rn(e < rot ? x[i] * cosv[i] + y * sinv[i] : x[i]);
+    }
+    if (live) *(uint2*)(is_q ? q_out + (size_t)t * ld_q + m * N + e : crow + (size_t)(m - nq) * N + e) = *(const uint2*)o;
+  }
+  if (!crow) return;
+  const float *vs = prow + (nq + 2 * G) * N, *vb = bias ? bias + (nq + 2 * G) * N : nullptr;
+  for (int i = (part * 32 + lane) * 4; i < G * dv; i += DP_WARPS * 128) {
+    float4 v = *(const float4*)(vs + i);
+    if (vb) {
+      const float4 b = *(const float4*)(vb + i);
+      v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
+    alignas(8) const bf16 o[4] = {__float2bfloat16_rn(v.x), __float2bfloat16_rn(v.y), __float2bfloat16_rn(v.z), __float2bfloat16_rn(v.w)};
+    *(uint2*)(crow + (size_t)G * 2 * N + i) = *(const uint2*)o;
+  }
+}
+
 extern "C" int qv_diff_prepare(void* q_out, int ld_q, const void* proj, int ld_p, const float* bias, const float* qw, const float* kw,
                                float eps, const float* cos_sin, int table_rows, const int* tok_pos, const int* tok_seg,
                                const int* block_table, int max_blocks, void* cache, int T, int H, int G, int n, int dv, int rot, int page,
@@ -96,6 +179,13 @@ extern "C" int qv_diff_prepare(void* q_out, int ld_q, const void* proj, int ld_p
   // few tokens: a token's maps are spread over several CTAs (each brings the row in for itself), so that the step fills more SMs
   const int units = 2 * H + 3 * G;
   const int spread = T <= 32 ? ((units + 7) / 8 < 65535 ? (units + 7) / 8 : 65535) : 1;
+  if (T > 32 && proj_dt == QV_DT_F32 && dt == QV_DT_BF16 && (n == 32 || n == 64 || n == 128) && rot % 8 == 0 && dv % 4 == 0 && ld_p % 4 == 0 &&
+      ld_q % 4 == 0 && (((uintptr_t)proj | (uintptr_t)bias | (uintptr_t)qw | (uintptr_t)kw) & 15) == 0 && (((uintptr_t)q_out | (uintptr_t)cache) & 7) == 0 &&
+      T <= 0x7fffffff / DP_WARPS) {
+    auto kernel = n == 32 ? diff_prepare_vec_kernel<8> : n == 64 ? diff_prepare_vec_kernel<16> : diff_prepare_vec_kernel<32>;
+    return qv_launch(kernel, dim3((unsigned)(((long long)T * DP_WARPS + 7) / 8)), dim3(256), 0, st, (bf16*)q_out, ld_q, (const float*)proj, ld_p, bias, qw,
+                     kw, eps, (const float2*)cos_sin, table_rows, tok_pos, tok_seg, block_table, max_blocks, (bf16*)cache, T, H, G, dv, rot, page);
+  }
 #define PREP(TP, TT)                                                                                                              \
   do {                                                                                                                            \
     if (smem > 48 * 1024) cudaFuncSetAttribute(diff_prepare_kernel<TP, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \

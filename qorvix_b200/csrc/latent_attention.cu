@@ -72,6 +72,74 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
   }
 }
 
+// Portions, neighbouring pairs, bfloat16 on 16-byte boundaries: four warps a token, one for the latent (16 bytes a lane, kept in registers
+// between the sum and the write), three for the rotated parts (a pair, one word, a lane).  2,048 tokens of 16 heads, rank 512: 10.4 us with
+// a CTA a token and two bytes a thread, 7.8 here, bound by the trips to memory of its few accesses a warp.
+#define LP_MAX_PIECES 4
+__global__ void __launch_bounds__(256) latent_prepare_vec_kernel(const bf16* __restrict__ proj, int ld, bf16* __restrict__ q, int ld_q, int kv_off,
+                                                                 bf16* __restrict__ cache, const float* __restrict__ norm_w, float eps,
+                                                                 const float2* __restrict__ cos_sin, int table_rows, const int* __restrict__ tok_pos,
+                                                                 const int* __restrict__ tok_seg, const int* __restrict__ block_table, int max_blocks,
+                                                                 int T, int H, int dn, int dr, int rank, int rot, int page) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x * 2 + (threadIdx.x >> 7), part = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const int pos = tok_pos[t];
+  const bf16* lat = proj + (size_t)t * ld + kv_off;
+  bf16* dst = cache + ((size_t)block_table[(size_t)tok_seg[t] * max_blocks + pos / page] * page + (size_t)(pos % page)) * (rank + dr);
+  if (part == 0) {
+    const int pieces = rank >> 3;
+    uint4 v[LP_MAX_PIECES];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < LP_MAX_PIECES; ++k) {
+      const int i = lane + 32 * k;
+      v[k] = i < pieces ? *(const uint4*)(lat + i * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < LP_MAX_PIECES; ++k) {
+      const __nv_bfloat162* e = (const __nv_bfloat162*)&v[k];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float a = __low2float(e[u]), b = __high2float(e[u]);
+        ss = fmaf(a, a, fmaf(b, b, ss));
+      }
+    }
+    const float sc = 1.0f / sqrtf(warp_sum(ss) / (float)rank + eps);
+#pragma unroll
+    for (int k = 0; k < LP_MAX_PIECES; ++k) {
+      const int i = lane + 32 * k;
+      if (i >= pieces) break;
+      const float4 w0 = *(const float4*)(norm_w + i * 8), w1 = *(const float4*)(norm_w + i * 8 + 4);
+      const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+      const __nv_bfloat162* e = (const __nv_bfloat162*)&v[k];
+      uint4 o;
+      __nv_bfloat162* ov = (__nv_bfloat162*)&o;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) ov[u] = __floats2bfloat162_rn(__low2float(e[u]) * sc * w[2 * u], __high2float(e[u]) * sc * w[2 * u + 1]);
+      *(uint4*)(dst + i * 8) = o;
+    }
+    return;
+  }
+  const float2* cs = cos_sin + (size_t)(pos < table_rows ? pos : table_rows - 1) * (rot >> 1);
+  const int pairs = rot >> 1;
+  for (int i = lane; i < pairs; i += 32) {
+    const float2 c = cs[i];
+    auto turn = [&](const bf16* from, bf16* to) {
+      const __nv_bfloat162 x = *(const __nv_bfloat162*)(from + 2 * i);
+      const float a = __low2float(x), b = __high2float(x);
+      *(__nv_bfloat162*)(to + 2 * i) = __floats2bfloat162_rn(a * c.x - b * c.y, b * c.x + a * c.y);
+    };
+    bf16* qr = q + (size_t)t * ld_q + dn;
+#pragma unroll 4
+    for (int h = part - 1; h < H; h += 3) turn(qr + (size_t)h * (dn + dr), qr + (size_t)h * (dn + dr));
+    if (part == 3) turn(lat + rank, dst + rank);
+  }
+  if (part == 3)
+    for (int i = rot + lane; i < dr; i += 32) dst[rank + i] = lat[rank + i];
+}
+
 // The same without a rotated part (dr = 0): a warp per token, the latent read four entries at a time where it lies on the vectors'
 // boundaries; up to 1,024 entries stay in registers between the sum and the write.
 template <typename T>
@@ -130,6 +198,11 @@ extern "C" int qv_latent_prepare(void* proj, int ld, void* q, int ld_q, int kv_o
     QV_DISPATCH_DT(dt, TT,
                    return qv_launch(latent_rows_kernel<TT>, dim3((T + 3) / 4), dim3(128), 0, (cudaStream_t)stream, (const TT*)proj + kv_off, ld, (TT*)cache,
                                     norm_w, eps, tok_pos, tok_seg, block_table, max_blocks, T, rank, page));
+  if (dt == QV_DT_BF16 && T > 32 && !split_half && rank % 8 == 0 && rank <= 256 * LP_MAX_PIECES && (rank + dr) % 8 == 0 && ld % 8 == 0 && kv_off % 8 == 0 &&
+      dn % 2 == 0 && dr % 2 == 0 && ld_q % 2 == 0 && (((uintptr_t)proj | (uintptr_t)cache | (uintptr_t)norm_w) & 15) == 0 && ((uintptr_t)q & 3) == 0)
+    return qv_launch(latent_prepare_vec_kernel, dim3((T + 1) / 2), dim3(256), 0, (cudaStream_t)stream, (const bf16*)proj, ld, (bf16*)q, ld_q, kv_off,
+                     (bf16*)cache, norm_w, eps, (const float2*)cos_sin, table_rows, tok_pos, tok_seg, block_table, max_blocks, T, H, dn, dr, rank, rot,
+                     page);
   QV_DISPATCH_DT(dt, TT,
                  return qv_launch(latent_prepare_kernel<TT>, dim3(T), dim3(256), 0, (cudaStream_t)stream, (TT*)proj, ld, (TT*)q, ld_q,
                                   kv_off, (TT*)cache, norm_w, eps, (const float2*)cos_sin, table_rows, tok_pos, tok_seg, block_table,
