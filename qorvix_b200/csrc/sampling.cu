@@ -88,8 +88,80 @@ __global__ void argmax_kernel(int* __restrict__ out, const float* __restrict__ l
   }
 }
 
+// Long rows: a cluster of eight CTAs a row, each over an eighth of it; their bests meet in the first one's shared memory.  8 rows of 128,256:
+// 20 us with a CTA a row (which waits for its own loads eight times), 13 here.
+#define ARGMAX_CTAS 8
+#define ARGMAX_CLUSTER_FROM 16384
+__global__ void __launch_bounds__(512) argmax_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, int V, long long ld) {
+  __shared__ float sv[16], cv[ARGMAX_CTAS];
+  __shared__ int si[16], ci[ARGMAX_CTAS];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int part = blockIdx.x % ARGMAX_CTAS;
+  const float* row = logits + (size_t)(blockIdx.x / ARGMAX_CTAS) * ld;
+  const int each = ((V + ARGMAX_CTAS - 1) / ARGMAX_CTAS + 3) / 4 * 4, first = part * each, last = first + each < V ? first + each : V;
+  float best = -INFINITY;
+  int besti = 0x7fffffff;
+  auto take = [&](float v, int i) {
+    if (v > best || (v == best && i < besti)) { best = v; besti = i; }
+  };
+  if ((((uintptr_t)row) & 15) == 0) {
+    const int whole = last > first ? first + (last - first) / 4 * 4 : first;
+    for (int i0 = first + threadIdx.x * 4; i0 < whole; i0 += 4 * 512 * 4) {
+      float4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = i0 + k * 512 * 4;
+        v[k] = i < whole ? *(const float4*)(row + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = i0 + k * 512 * 4;
+        if (i >= whole) break;                       // (a row of nothing but NaN must not find the padding's -inf)
+        take(v[k].x, i); take(v[k].y, i + 1); take(v[k].z, i + 2); take(v[k].w, i + 3);
+      }
+    }
+    for (int i = whole + threadIdx.x; i < last; i += 512) take(row[i], i);
+  } else {
+    for (int i = first + threadIdx.x; i < last; i += 512) take(row[i], i);
+  }
+  auto over_warp = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
+      take(ov, oi);
+    }
+  };
+  over_warp();
+  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = besti; }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = threadIdx.x < 16 ? sv[threadIdx.x] : -INFINITY;
+    besti = threadIdx.x < 16 ? si[threadIdx.x] : 0x7fffffff;
+    over_warp();
+    if (threadIdx.x == 0) {                          // into the first CTA's shared memory
+      uint32_t v, i;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(v) : "r"((uint32_t)__cvta_generic_to_shared(cv + part)));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(i) : "r"((uint32_t)__cvta_generic_to_shared(ci + part)));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(v), "f"(best) : "memory");
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(i), "r"(besti) : "memory");
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (part == 0 && threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < ARGMAX_CTAS; ++k) take(cv[k], ci[k]);
+    out[blockIdx.x / ARGMAX_CTAS] = besti == 0x7fffffff ? 0 : besti;
+  }
+}
+
 extern "C" int qv_argmax(int* out, const float* logits, int rows, int V, long long ld, void* stream) {
   if (rows <= 0) return 0;
+  if (V >= ARGMAX_CLUSTER_FROM && rows <= 0x7fffffff / ARGMAX_CTAS)
+    return qv_launch_cluster(argmax_cluster_kernel, dim3(rows * ARGMAX_CTAS), dim3(512), 0, (cudaStream_t)stream, dim3(ARGMAX_CTAS, 1, 1), out, logits, V,
+                             ld);
   return qv_launch(argmax_kernel, dim3(rows), dim3(1024), 0, (cudaStream_t)stream, out, logits, V, ld);
 }
 
