@@ -373,6 +373,10 @@ __device__ __forceinline__ void lt_ldsm2t(uint32_t* r, const void* p) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(s));
 }
+__device__ __forceinline__ void lt_ldsm4t(uint32_t* r, const void* p) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
+}
 __device__ __forceinline__ void lt_mma(float* c, const uint32_t* a, const uint32_t* b) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
@@ -484,6 +488,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
   const int row_first = q0 * H + blockIdx.x * LT_BM;       // global (token, head) row of this tile's first row
   const int rows = min(LT_BM, q1 * H - row_first);
   if (rows <= 0) return;
+  const int mts = rows > 16 ? 2 : 1;                       // halves of the tile that hold rows (a decode step of 16 heads: one)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pos0 = seg_pos0[s];
   const int pos_first = pos0 + row_first / H - q0, pos_last = pos0 + (row_first + rows - 1) / H - q0;
@@ -550,20 +555,31 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     // scores of this warp's eight keys for all 32 rows
     float sc[2][4] = {}, sd[2][4] = {};                      // two chains of dependent products instead of one
     const int nks = kw / 16;
-    for (int ks = 0; ks < nks; ks += 2) {
-      uint32_t a[2][4], b[2];
-      lt_ldsm4(a[0], Qs + (size_t)(lane & 15) * ldk + ks * 16 + (lane >> 4) * 8);
-      lt_ldsm4(a[1], Qs + (size_t)(16 + (lane & 15)) * ldk + ks * 16 + (lane >> 4) * 8);
+    const bf16* qrow = Qs + (size_t)(lane & 15) * ldk + (lane >> 4) * 8;
+    const bf16* krow = Kb + (size_t)(warp * 8 + (lane & 7)) * ldk + (lane >> 3) * 8;
+    int ks = 0;
+    for (; ks + 1 < nks; ks += 2) {                          // 32 entries: one read of the keys, one of each 16 rows and 16 entries
+      uint32_t a[4], c[4], b[4];
+      lt_ldsm4(b, krow + ks * 16);
+      lt_ldsm4(a, qrow + ks * 16);
+      lt_ldsm4(c, qrow + (ks + 1) * 16);
+      lt_mma(sc[0], a, b);
+      lt_mma(sd[0], c, b + 2);
+      if (mts == 2) {
+        lt_ldsm4(a, qrow + (size_t)16 * ldk + ks * 16);
+        lt_ldsm4(c, qrow + (size_t)16 * ldk + (ks + 1) * 16);
+        lt_mma(sc[1], a, b);
+        lt_mma(sd[1], c, b + 2);
+      }
+    }
+    if (ks < nks) {
+      uint32_t a[4], b[2];
       lt_ldsm2(b, Kb + (size_t)(warp * 8 + (lane & 7)) * ldk + ks * 16 + ((lane >> 3) & 1) * 8);
-      lt_mma(sc[0], a[0], b);
-      lt_mma(sc[1], a[1], b);
-      if (ks + 1 < nks) {
-        uint32_t c[2][4], e[2];
-        lt_ldsm4(c[0], Qs + (size_t)(lane & 15) * ldk + (ks + 1) * 16 + (lane >> 4) * 8);
-        lt_ldsm4(c[1], Qs + (size_t)(16 + (lane & 15)) * ldk + (ks + 1) * 16 + (lane >> 4) * 8);
-        lt_ldsm2(e, Kb + (size_t)(warp * 8 + (lane & 7)) * ldk + (ks + 1) * 16 + ((lane >> 3) & 1) * 8);
-        lt_mma(sd[0], c[0], e);
-        lt_mma(sd[1], c[1], e);
+      lt_ldsm4(a, qrow + ks * 16);
+      lt_mma(sc[0], a, b);
+      if (mts == 2) {
+        lt_ldsm4(a, qrow + (size_t)16 * ldk + ks * 16);
+        lt_mma(sc[1], a, b);
       }
     }
 #pragma unroll
@@ -575,6 +591,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
+        if (mt >= mts) break;
         float mx = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -594,6 +611,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
+        if (mt >= mts) break;
         const int r = mt * 16 + hf * 8 + (lane >> 2);
         float bm = st_max[r];
 #pragma unroll
@@ -623,6 +641,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
+        if (mt >= mts) break;
         const int r = mt * 16 + hf * 8 + (lane >> 2);
         float sum = 0.f;
 #pragma unroll
@@ -638,17 +657,21 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
 #pragma unroll
       for (int term = 0; term < WT; ++term) {
         lt_ldsm4(a[term][0], Ps + term * PLANE + (size_t)(lane & 15) * (LT_BK + 8) + kk * 16 + (lane >> 4) * 8);
-        lt_ldsm4(a[term][1], Ps + term * PLANE + (size_t)(16 + (lane & 15)) * (LT_BK + 8) + kk * 16 + (lane >> 4) * 8);
+        if (mts == 2) lt_ldsm4(a[term][1], Ps + term * PLANE + (size_t)(16 + (lane & 15)) * (LT_BK + 8) + kk * 16 + (lane >> 4) * 8);
       }
+      const bf16* vrow = Kb + (size_t)(kk * 16 + (lane & 15)) * ldk + warp * NTW * 8;
 #pragma unroll
-      for (int nt = 0; nt < NTW; ++nt) {
-        uint32_t b[2];
-        lt_ldsm2t(b, Kb + (size_t)(kk * 16 + (lane & 15)) * ldk + (warp * NTW + nt) * 8);
+      for (int nt = 0; nt < NTW; nt += 2) {                  // two tiles of eight columns a read (a last odd one alone)
+        uint32_t b[4];
+        if (nt + 1 < NTW) lt_ldsm4t(b, vrow + nt * 8 + (lane >> 4) * 8);
+        else lt_ldsm2t(b, vrow + nt * 8);
 #pragma unroll
-        for (int term = WT - 1; term >= 0; --term) {         // the small terms first
-          lt_mma(o[0][nt], a[term][0], b);
-          lt_mma(o[1][nt], a[term][1], b);
-        }
+        for (int u = 0; u < 2 && nt + u < NTW; ++u)
+#pragma unroll
+          for (int term = WT - 1; term >= 0; --term) {       // the small terms first
+            lt_mma(o[0][nt + u], a[term][0], b + 2 * u);
+            if (mts == 2) lt_mma(o[1][nt + u], a[term][1], b + 2 * u);
+          }
       }
     }
     __syncthreads();
