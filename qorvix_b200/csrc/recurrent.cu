@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(SCAN_VT * SCAN_WARPS) linear_scan_reg_kernel(S
 // parts apart from its large one, and the update apart from the state.
 // What bounds it: a chunk's chain of products and the two barriers (a prompt has only heads x tiles CTAs); mma.sync issues a product in
 // some 8 clocks a scheduler.  2,048 tokens of 4 heads of 256 x 512: 2,573 us token by token, 175 in chunks; portions of 777, 583 and
-// 583 tokens of 64 heads of 128 x 64: 897 and 130 us.
+// 583 tokens of 64 heads of 128 x 64: 897 and 80 us (90 with an exponential for every entry of W).
 #define LC_C 64
 __device__ __forceinline__ void lc_ldsm4(uint32_t* r, const void* p) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
@@ -604,6 +604,7 @@ __device__ __forceinline__ float lc_exp_sum(float2 x, float2 y) {
 struct LcGates {                           // what a chunk's gates amount to
   float2 G[LC_C], H[LC_C];                           // a number and what rounding it to float32 left over
   float b[LC_C], A[LC_C], c[LC_C], em[LC_C];         // em: exp(-m_t)
+  float R[3][LC_C], E[LC_C];                         // blocks of 16 tokens, M_i the largest H in block i: exp(G_t + M_i) for t behind it, b_j exp(H_j - M)
   float A_end, m_end, pad[2];
 };
 #define LC_GATE_WARP 9                     // of the eight that form W: its 16 x 32 tokens lie above the diagonal
@@ -827,6 +828,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
     }
     const double G_end = __shfl_sync(0xffffffffu, G[1], 31), m_end = __shfl_sync(0xffffffffu, m[1], 31);
     const float c0 = expf((float)(G_end + Hh[0])) * bb[0], c1 = expf((float)(G_end + Hh[1])) * bb[1];
+    double M = fmax(Hh[0], Hh[1]);                   // of the 16 tokens of eight lanes
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) M = fmax(M, __shfl_xor_sync(0xffffffffu, M, o));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double Mi = __shfl_sync(0xffffffffu, M, 8 * i);
+      if (lane >= 8 * i + 8) *(float2*)(gt.R[i] + 2 * lane) = make_float2(expf((float)(G[0] + Mi)), expf((float)(G[1] + Mi)));
+    }
+    *(float2*)(gt.E + 2 * lane) = make_float2(expf((float)(Hh[0] - M)) * bb[0], expf((float)(Hh[1] - M)) * bb[1]);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int t = 2 * lane + i;
@@ -933,8 +943,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
       }
     } else {
       if (warp == LC_GATE_WARP && c + 1 < nchunks) work_gates(c + 1);
-      // W = q k^T of 16 tokens x 32 tokens, decayed, and its product with v
-      const int mt = (warp - 8) >> 1, j0 = (warp & 1) * 32;
+      // W = q k^T of 16 tokens x 32 tokens, decayed, and its product with v: two blocks of 16 x 16, nothing of what lies above the diagonal.  On the
+      // diagonal an exponential an entry; a block below it takes a factor a row and a factor a column (G_t + M and H_j - M are <= 0 for M the
+      // largest H of tokens all ahead of t)
+      const int mt = (warp - 8) >> 1, j0 = (warp & 1) * 32, below = mt - 2 * (warp & 1);         // blocks left of the diagonal's: `below` of the two
       float hi[VT / 8][4] = {}, lo[VT / 8][4] = {};
       float rs[2] = {0.f, 0.f};
       if (j0 <= mt * 16 + 15) {
@@ -948,6 +960,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
             lc_ldsm4(af, qs + (mt * 16 + (mi & 1) * 8 + r8) * LDQ + kk + (mi >> 1) * 8);
 #pragma unroll
             for (int pr = 0; pr < 2; ++pr) {
+              if (pr > below) break;
               lc_ldsm4(bq, ks + (j0 + pr * 16 + (mi >> 1) * 8 + r8) * LDQ + kk + (mi & 1) * 8);
               lc_mma(part[2 * pr], af, bq[0], bq[1]);
               lc_mma(part[2 * pr + 1], af, bq[2], bq[3]);
@@ -958,24 +971,44 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
 #pragma unroll
             for (int x = 0; x < 4; ++x) w[nt][x] += part[nt][x];
         }
-        const float2 Gt[2] = {gt.G[mt * 16 + g8], gt.G[mt * 16 + g8 + 8]};
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int pr = 0; pr < 2; ++pr) {
+          if (pr > below) break;
+          if (pr < below) {
+            const float* Rb = gt.R[2 * (warp & 1) + pr] + mt * 16 + g8;
+            const float R[2] = {Rb[0], Rb[8]};
 #pragma unroll
-          for (int jj = 0; jj < 2; ++jj) {
-            const int j = j0 + nt * 8 + 2 * t4 + jj;
-            const float2 Hj = gt.H[j];
-            const float bj = KIND == SCAN_DECAY ? gt.b[j] : 1.f;
+            for (int h8 = 0; h8 < 2; ++h8) {
+              const float2 E = *(const float2*)(gt.E + j0 + pr * 16 + h8 * 8 + 2 * t4);
+              float* f = w[2 * pr + h8];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const float f = j <= mt * 16 + g8 + r * 8 ? w[nt][2 * r + jj] * (lc_exp_sum(Gt[r], Hj) * bj) : 0.f;
-              w[nt][2 * r + jj] = f;
-              rs[r] += f;
+              for (int r = 0; r < 2; ++r) {
+                f[2 * r] *= R[r] * E.x;
+                f[2 * r + 1] *= R[r] * E.y;
+                rs[r] += f[2 * r] + f[2 * r + 1];
+              }
             }
+          } else {
+            const float2 Gt[2] = {gt.G[mt * 16 + g8], gt.G[mt * 16 + g8 + 8]};
+#pragma unroll
+            for (int h8 = 0; h8 < 2; ++h8)
+#pragma unroll
+              for (int jj = 0; jj < 2; ++jj) {
+                const int jr = h8 * 8 + 2 * t4 + jj;
+                const float2 Hj = gt.H[mt * 16 + jr];
+                const float bj = KIND == SCAN_DECAY ? gt.b[mt * 16 + jr] : 1.f;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const float f = jr <= g8 + r * 8 ? w[2 * pr + h8][2 * r + jj] * (lc_exp_sum(Gt[r], Hj) * bj) : 0.f;
+                  w[2 * pr + h8][2 * r + jj] = f;
+                  rs[r] += f;
+                }
+              }
           }
         }
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
+          if (kk > below) break;
           uint32_t t0[3], t1[3], t2[3], t3[3];
           lc_split3(w[2 * kk][0], w[2 * kk][1], t0);
           lc_split3(w[2 * kk][2], w[2 * kk][3], t1);
