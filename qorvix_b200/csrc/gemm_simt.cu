@@ -22,10 +22,14 @@ __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(live ? 16 : 0) : "memory");
 }
 
-template <typename TA, typename TW, typename TC, int BM, int BN, int BK, int TM, int TN, int STAGES, bool ASYNC>
+// GLU: the rows of W come in groups of 32, 16 gate rows and the 16 up rows of the same features; a thread of a 16 x 32 tile holds both sums of a
+// feature, and C[M, N / 2] = act(gate) * up, as the activation's own kernel has it (the same bits).  Bound as the plain product of its size; a
+// launch and a trip of the sums through memory less: replies of a 32-bit model of three layers (d 192, f 512) 3.7 % faster (0.820 of the time
+// ahead of the ring of eight tiles, 0.851 with two launches).
+template <typename TA, typename TW, typename TC, int BM, int BN, int BK, int TM, int TN, int STAGES, bool ASYNC, bool GLU = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A,
                                                                         const TW* __restrict__ W, int M, int N, int K,
-                                                                        int lda, int ldw, int ldc, int accumulate) {
+                                                                        int lda, int ldw, int ldc, int accumulate, GluAct glu) {
   constexpr int THREADS = (BM / TM) * (BN / TN), LD = BK + 4, ROWS = BM + BN, PIECES = BK / 4;
   extern __shared__ __align__(16) float gs_ring[];
   float(*ring)[ROWS * LD] = (float(*)[ROWS * LD])gs_ring;            // [STAGES]
@@ -123,6 +127,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
   for (int i = 0; i < TM; ++i) {
     const int gm = m0 + ty + TY * i;
     if (gm >= M) continue;
+    if constexpr (GLU) {
+      static_assert(BN == 32 && TN == 2, "a thread's two columns are a gate and its up value");
+      if (n0 < N) C[(size_t)gm * ldc + n0 / 2 + tx] = from_f<TC>(glu_apply(acc[i][0], acc[i][1], glu));
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int gn = n0 + tx + TX * j;
@@ -155,7 +164,7 @@ static int launch(void* C, const void* A, const void* W, int M, int N, int K, in
       configured = true;                                                                                                         \
     }                                                                                                                            \
     return qv_launch(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, grid, dim3((BM / TM) * (BN / TN)), smem, st, (TC*)C, \
-                     (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, accumulate);                                            \
+                     (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, accumulate, GluAct{0, 0.f, 0.f});                   \
   } while (0)
   if (small) {
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
@@ -189,4 +198,25 @@ extern "C" int qv_gemm_simt(void* C, const void* A, const void* W, int M, int N,
     case 7: return launch<bf16, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
   }
   return QV_ERR_UNSUPPORTED;
+}
+
+// C[M, N / 2] = act(gate) * up for W [N, K] with gate and up rows in groups of 16, float32 throughout; act as GluAct::kind.  Products of one wave of
+// 16 x 32 tiles in whole 16-byte pieces only (QV_ERR_UNSUPPORTED else: the product and the activation are then two launches).
+extern "C" int qv_gemm_simt_glu(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int act, float limit, float slope,
+                                void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (act < 0 || act > 2 || N % 32 || ((lda | ldw | K) & 3) || (((uintptr_t)A | (uintptr_t)W) & 15)) return QV_ERR_UNSUPPORTED;
+  if (C < A + (size_t)(M - 1) * lda + K && A < C + (size_t)(M - 1) * ldc + N / 2) return QV_ERR_UNSUPPORTED;      // a result over its own rows: two launches
+  const dim3 grid(N / 32, (M + 15) / 16);
+  const bool small = M <= 32 || (long long)((N + 63) / 64) * ((M + 63) / 64) < 148;
+  if (!small || (long long)grid.x * grid.y > 148) return QV_ERR_UNSUPPORTED;
+  constexpr size_t smem = (size_t)8 * (16 + 32) * (64 + 4) * 4;
+  auto kernel = gemm_simt_kernel<float, float, float, 16, 32, 64, 2, 2, 8, true, true>;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return qv_launch(kernel, grid, dim3(128), smem, (cudaStream_t)stream, C, A, W, M, N, K, lda, ldw, ldc, 0, GluAct{act, limit, slope});
 }

@@ -246,6 +246,10 @@ class Executor {
         if (rc != ERR_UNSUPPORTED) { check(rc, "gemm_bf16_tc (swiglu)"); return; }
       }
     }
+    if (w.interleaved && m.dt == DT_F32 && w.gate_up.rows && w.gate_up.dt == DT_F32) {
+      const int rc = k_->gemm_simt_glu((float*)act, (const float*)xn, (const float*)w.gate_up.rows, T, 2 * m.f, m.d, m.d, m.d, m.f, 0, 0.f, 0.f, st);
+      if (rc != ERR_UNSUPPORTED) { check(rc, "gemm_simt_glu"); return; }
+    }
     void* gu = ws.take((size_t)T * 2 * m.f * dt_size(m.dt));
     gemm(gu, 2 * m.f, m.dt, xn, m.d, w.gate_up, T, st);
     check(k_->swiglu(act, gu, T, m.f, w.interleaved ? 1 : 0, m.dt, st), "swiglu");

@@ -26,6 +26,7 @@ struct Kernels {
   const char* (*error_string)(int) = nullptr;
   // matrix products
   int (*gemm_simt)(void*, const void*, const void*, int, int, int, int, int, int, int, int, int, int, void*) = nullptr;
+  int (*gemm_simt_glu)(float*, const float*, const float*, int, int, int, int, int, int, int, float, float, void*) = nullptr;
   int (*gemm_bf16_tc)(void*, const void*, const void*, int, int, int, int, int, int, int, int*, int, int, void*) = nullptr;
   long long (*packed_weight_bytes)(int, int) = nullptr;
   int (*pack_weight_tiles)(void*, const void*, int, int, int, void*) = nullptr;
@@ -71,7 +72,7 @@ struct Kernels {
     QV_SYM(el, embed, "qv_embed"); QV_SYM(el, add_rmsnorm, "qv_add_rmsnorm"); QV_SYM(el, rope_kv_write, "qv_rope_kv_write");
     QV_SYM(el, swiglu, "qv_swiglu"); QV_SYM(el, cast, "qv_cast"); QV_SYM(el, error_string, "qv_error_string");
     void* gs = open("gemm_simt");
-    QV_SYM(gs, gemm_simt, "qv_gemm_simt");
+    QV_SYM(gs, gemm_simt, "qv_gemm_simt"); QV_SYM(gs, gemm_simt_glu, "qv_gemm_simt_glu");
     void* gb = open("gemm_bf16");
     QV_SYM(gb, gemm_bf16_tc, "qv_gemm_bf16_tc"); QV_SYM(gb, packed_weight_bytes, "qv_packed_weight_bytes");
     QV_SYM(gb, pack_weight_tiles, "qv_pack_weight_tiles"); QV_SYM(gb, gemm_bf16_packed, "qv_gemm_bf16_packed");

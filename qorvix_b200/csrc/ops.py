@@ -41,6 +41,7 @@ _ARGTYPES = {
     "qv_cast": [_V, _V, _L, _I, _I, _V],
     "qv_cast_rows": [_V, _L, _V, _L, _I, _I, _I, _I, _V],
     "qv_gemm_simt": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V],
+    "qv_gemm_simt_glu": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _F, _V],
     "qv_gemm_bf16_tc": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V, _I, _I, _V],
     "qv_packed_weight_bytes": [_I, _I],
     "qv_pack_weight_tiles": [_V, _V, _I, _I, _I, _V],
@@ -1807,8 +1808,8 @@ def gemm_act(out, x, w, packed, n: int, act: int, bias=None) -> None:
 
 def gemm_swiglu(out, x, w_interleaved, packed=None, n: int = 0, act: int = 0, limit: float = 0.0, slope: float = 0.0) -> None:
     """out[M,f] = act(x Wg^T) * (x Wu^T) (act GLU_SILU or GLU_GELU_TANH; GLU_CLAMPED with limit and slope: see glu_act) with gate
-    and up rows interleaved in groups of 16 in w_interleaved [2f, K]: one tensor-core kernel when it takes the shape, else
-    the product followed by the activation kernel."""
+    and up rows interleaved in groups of 16 in w_interleaved [2f, K]: one tensor-core kernel (float32: one kernel of
+    multiply-adds) when it takes the shape, else the product followed by the activation kernel."""
     n = n or w_interleaved.shape[0]
     if act == GLU_CLAMPED:
         if gemm_bf16_glu(out, x, w_interleaved, packed, n, act, limit, slope):
@@ -1818,6 +1819,15 @@ def gemm_swiglu(out, x, w_interleaved, packed=None, n: int = 0, act: int = 0, li
             return
         if (w_interleaved is not None and w_interleaved.dtype == torch.bfloat16
                 and gemm_bf16_tc(out, x, w_interleaved, swiglu=glu_epilogue(act))):
+            return
+    if (w_interleaved is not None and packed is None and x.dtype == out.dtype == w_interleaved.dtype == torch.float32
+            and x.is_cuda and w_interleaved.is_cuda and out.is_cuda and out.is_contiguous()
+            and x.dim() == w_interleaved.dim() == out.dim() == 2 and x.stride(1) == w_interleaved.stride(1) == 1
+            and n == w_interleaved.shape[0] and w_interleaved.shape[1] == x.shape[1] and out.shape == (x.shape[0], n // 2)):
+        rc = _lib("gemm_simt").qv_gemm_simt_glu(_ptr(out), _ptr(x), _ptr(w_interleaved), x.shape[0], n, x.shape[1], x.stride(0), w_interleaved.stride(0),
+                                                out.stride(0), act, float(limit), float(slope), _stream())
+        if rc != -2:
+            _check(rc, "gemm_simt_glu")
             return
     gu = torch.empty((x.shape[0], n), device=x.device, dtype=out.dtype)
     gemm(gu, x, w_interleaved, packed, n)
