@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(512) argmax_cluster_kernel(int* __restrict__ o
   __shared__ int si[16], ci[ARGMAX_CTAS];
   pdl_wait();
   pdl_launch_dependents();
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");             // this CTA runs: its shared memory may be written
   const int part = blockIdx.x % ARGMAX_CTAS;
   const float* row = logits + (size_t)(blockIdx.x / ARGMAX_CTAS) * ld;
   const int each = ((V + ARGMAX_CTAS - 1) / ARGMAX_CTAS + 3) / 4 * 4, first = part * each, last = first + each < V ? first + each : V;
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(512) argmax_cluster_kernel(int* __restrict__ o
   over_warp();
   if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = besti; }
   __syncthreads();
+  asm volatile("barrier.cluster.wait;" ::: "memory");                       // all CTAs of the cluster have started (the row's loads lie between)
   if (threadIdx.x < 32) {
     best = threadIdx.x < 16 ? sv[threadIdx.x] : -INFINITY;
     besti = threadIdx.x < 16 ? si[threadIdx.x] : 0x7fffffff;

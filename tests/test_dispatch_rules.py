@@ -187,3 +187,22 @@ def test_no_room_is_an_answer(monkeypatch):
         raise torch.OutOfMemoryError("no room")
     monkeypatch.setattr(ops.torch, "empty", full)
     assert ops._room((2, 3), torch.float32, "cpu") is None
+
+
+def test_remote_shared_memory_is_touched_behind_a_cluster_barrier_only():
+    """A CTA's shared memory may be read or written by another CTA of its cluster once that CTA is known to run: in every kernel a cluster
+    barrier is arrived at and waited for ahead of the first access (and, so that no CTA leaves early, behind the last one)."""
+    import re
+    from pathlib import Path
+    seen = 0
+    for path in sorted(Path(ops.__file__).parent.glob("*.cu*")):
+        for kernel in re.split(r"__global__", path.read_text())[1:]:
+            remote = [m.start() for m in re.finditer(r"(?:ld|st|red|atom)(?:\.\w+)*\.shared::cluster|dst_smem_cluster|map_shared_rank", kernel)]
+            if not remote:
+                continue
+            seen += 1
+            waits = [m.start() for m in re.finditer(r"barrier\.cluster\.wait|\bcl\.sync\(\)", kernel)]
+            arrives = [m.start() for m in re.finditer(r"barrier\.cluster\.arrive|\bcl\.sync\(\)", kernel)]
+            assert waits and waits[0] < remote[0] and arrives[0] <= waits[0], f"{path.name}: remote shared memory ahead of a cluster barrier"
+            assert waits[-1] > remote[-1], f"{path.name}: a CTA may leave while its shared memory is in use"
+    assert seen >= 2
