@@ -124,13 +124,13 @@ __global__ void __launch_bounds__(128, 5) channel_gates_tile_kernel(float* __res
   float* xs = cg_smem;
   float* wsm = xs + CT_TOKENS * ldx;
   const int tid = threadIdx.x, c0 = blockIdx.y * CG_CHANNELS, t0 = blockIdx.x * CT_TOKENS;
+  pdl_wait();
+  pdl_launch_dependents();
 #pragma unroll 8
-  for (int i = tid; i < R * CG_CHANNELS; i += 128) {                 // (weights: no kernel writes them)
+  for (int i = tid; i < R * CG_CHANNELS; i += 128) {
     const int r = i / CG_CHANNELS, c = c0 + i % CG_CHANNELS;
     wsm[i] = c < N ? w2t[(size_t)r * N + c] : 0.f;
   }
-  pdl_wait();
-  pdl_launch_dependents();
   for (int r = tid & 31; r < R; r += 32) {           // a token a warp
     const float* xp = x1 + (size_t)t0 * ld_x + r;
 #pragma unroll 8

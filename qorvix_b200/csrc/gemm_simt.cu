@@ -14,7 +14,8 @@
 // or mostly padding, else 64 x 64 (32 k, 4 x 4 a thread).  Few CTAs are bound by the chain of K dependent multiply-adds and the
 // trips to memory ahead of it: with one tile of 16 k at a time and no copy in flight, 192 / 512 k took 20 / 51 us (3 rows), with three
 // tiles of 64 k 3.6 / 8.4 us behind the kernel ahead.  So products of one wave of CTAs get a ring of eight tiles, and the weights' halves of the
-// first ones are asked for ahead of the wait for the kernel ahead (no kernel writes weights): 2.5 / 5.0 us.
+// first ones are asked for ahead of the wait for the kernel ahead where the caller says that no launch may still write them (a model's
+// weights): 2.5 / 5.0 us.
 #include "common.cuh"
 
 __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live) {
@@ -29,7 +30,7 @@ __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live)
 template <typename TA, typename TW, typename TC, int BM, int BN, int BK, int TM, int TN, int STAGES, bool ASYNC, bool GLU = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A,
                                                                         const TW* __restrict__ W, int M, int N, int K,
-                                                                        int lda, int ldw, int ldc, int accumulate, GluAct glu) {
+                                                                        int lda, int ldw, int ldc, int accumulate, int settled, GluAct glu) {
   constexpr int THREADS = (BM / TM) * (BN / TN), LD = BK + 4, ROWS = BM + BN, PIECES = BK / 4;
   extern __shared__ __align__(16) float gs_ring[];
   float(*ring)[ROWS * LD] = (float(*)[ROWS * LD])gs_ring;            // [STAGES]
@@ -57,7 +58,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
       gs_cp16(dst + r * LD + (e % PIECES) * 4, live ? src : (const float*)W, live);
     }
   };
-  if (ASYNC)
+  if (ASYNC && settled)
     for (int t = 0; t < STAGES - 1 && t < tiles; ++t) stage(t, BM, ROWS);      // (with the first commit below)
   pdl_wait();
   pdl_launch_dependents();
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
   };
   if (ASYNC) {
     for (int t = 0; t < STAGES - 1; ++t) {
-      if (t < tiles) stage(t, 0, BM);
+      if (t < tiles) stage(t, 0, settled ? BM : ROWS);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
   } else if (tiles > 0) {
@@ -144,9 +145,10 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
   }
 }
 
+#define GS_SETTLED 0x100
 template <typename TA, typename TW, typename TC>
 static int launch(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw,
-                  int ldc, int accumulate, cudaStream_t st) {
+                  int ldc, int flags, cudaStream_t st) {
   const bool async = sizeof(TA) == 4 && sizeof(TW) == 4 && ((lda | ldw | K) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
   // 16 x 32 tiles where most rows of a 64-row tile would be padding, or where 64 x 64 tiles would leave SMs without one
   const long long big = (long long)((N + 63) / 64) * ((M + 63) / 64);
@@ -164,7 +166,7 @@ static int launch(void* C, const void* A, const void* W, int M, int N, int K, in
       configured = true;                                                                                                         \
     }                                                                                                                            \
     return qv_launch(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, grid, dim3((BM / TM) * (BN / TN)), smem, st, (TC*)C, \
-                     (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, accumulate, GluAct{0, 0.f, 0.f});                   \
+                     (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, (flags & 0xff) != 0, flags & GS_SETTLED, GluAct{0, 0.f, 0.f}); \
   } while (0)
   if (small) {
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
@@ -180,30 +182,32 @@ static int launch(void* C, const void* A, const void* W, int M, int N, int K, in
 #undef GS_LAUNCH
 }
 
-// dtypes: a_dt/w_dt/c_dt in {f32, bf16}; accumulate != 0 adds to what C holds.
+// dtypes: a_dt/w_dt/c_dt in {f32, bf16}; flags: 1 adds to what C holds, GS_SETTLED: no launch that may still run writes W, which the
+// kernel then reads ahead of its wait for the launch in front.
 extern "C" int qv_gemm_simt(void* C, const void* A, const void* W, int M, int N, int K, int lda,
-                            int ldw, int ldc, int a_dt, int w_dt, int c_dt, int accumulate,
+                            int ldw, int ldc, int a_dt, int w_dt, int c_dt, int flags,
                             void* stream) {
   if (M <= 0 || N <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   const int key = a_dt * 4 + w_dt * 2 + c_dt;
   switch (key) {
-    case 0: return launch<float, float, float>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 1: return launch<float, float, bf16>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 2: return launch<float, bf16, float>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 3: return launch<float, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 4: return launch<bf16, float, float>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 5: return launch<bf16, float, bf16>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 6: return launch<bf16, bf16, float>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
-    case 7: return launch<bf16, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, accumulate, st);
+    case 0: return launch<float, float, float>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 1: return launch<float, float, bf16>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 2: return launch<float, bf16, float>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 3: return launch<float, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 4: return launch<bf16, float, float>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 5: return launch<bf16, float, bf16>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 6: return launch<bf16, bf16, float>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
+    case 7: return launch<bf16, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, flags, st);
   }
   return QV_ERR_UNSUPPORTED;
 }
 
 // C[M, N / 2] = act(gate) * up for W [N, K] with gate and up rows in groups of 16, float32 throughout; act as GluAct::kind.  Products of one wave of
-// 16 x 32 tiles in whole 16-byte pieces only (QV_ERR_UNSUPPORTED else: the product and the activation are then two launches).
+// 16 x 32 tiles in whole 16-byte pieces only (QV_ERR_UNSUPPORTED else: the product and the activation are then two launches).  settled: as
+// GS_SETTLED.
 extern "C" int qv_gemm_simt_glu(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int act, float limit, float slope,
-                                void* stream) {
+                                int settled, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (act < 0 || act > 2 || N % 32 || ((lda | ldw | K) & 3) || (((uintptr_t)A | (uintptr_t)W) & 15)) return QV_ERR_UNSUPPORTED;
   if (C < A + (size_t)(M - 1) * lda + K && A < C + (size_t)(M - 1) * ldc + N / 2) return QV_ERR_UNSUPPORTED;      // a result over its own rows: two launches
@@ -218,5 +222,6 @@ extern "C" int qv_gemm_simt_glu(float* C, const float* A, const float* W, int M,
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return qv_launch(kernel, grid, dim3(128), smem, (cudaStream_t)stream, C, A, W, M, N, K, lda, ldw, ldc, 0, GluAct{act, limit, slope});
+  return qv_launch(kernel, grid, dim3(128), smem, (cudaStream_t)stream, C, A, W, M, N, K, lda, ldw, ldc, 0, settled,
+                   GluAct{act, limit, slope});
 }

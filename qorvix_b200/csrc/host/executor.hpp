@@ -219,6 +219,8 @@ class Executor {
   }
 
   // out[M, N] (row stride ldc, type c_dt) = x[M, K] (compute dtype, row stride lda) W^T with the kernel that fits
+  // gemm_simt: the model's weights lie still while it runs, so the kernel may read them ahead of its wait for the launch in front
+  static constexpr int SETTLED = 0x100;
   void gemm(void* out, int ldc, int c_dt, const void* x, int lda, const LinearW& w, int M, cudaStream_t st) {
     const int a_dt = m_->dt;
     if (a_dt == DT_BF16 && w.packed) {
@@ -230,7 +232,7 @@ class Executor {
       const int rc = k_->gemm_bf16_tc(out, x, w.rows, M, w.N, w.K, lda, w.K, ldc, c_dt, err_, 0, 0, st);
       if (rc != ERR_UNSUPPORTED) { check(rc, "gemm_bf16_tc"); return; }
     }
-    check(k_->gemm_simt(out, x, w.rows, M, w.N, w.K, lda, w.K, ldc, a_dt, w.dt, c_dt, 0, st), "gemm_simt");
+    check(k_->gemm_simt(out, x, w.rows, M, w.N, w.K, lda, w.K, ldc, a_dt, w.dt, c_dt, SETTLED, st), "gemm_simt");
   }
 
   // act[M, f] = silu(x Wg^T) * (x Wu^T)
@@ -247,7 +249,7 @@ class Executor {
       }
     }
     if (w.interleaved && m.dt == DT_F32 && w.gate_up.rows && w.gate_up.dt == DT_F32) {
-      const int rc = k_->gemm_simt_glu((float*)act, (const float*)xn, (const float*)w.gate_up.rows, T, 2 * m.f, m.d, m.d, m.d, m.f, 0, 0.f, 0.f, st);
+      const int rc = k_->gemm_simt_glu((float*)act, (const float*)xn, (const float*)w.gate_up.rows, T, 2 * m.f, m.d, m.d, m.d, m.f, 0, 0.f, 0.f, 1, st);
       if (rc != ERR_UNSUPPORTED) { check(rc, "gemm_simt_glu"); return; }
     }
     void* gu = ws.take((size_t)T * 2 * m.f * dt_size(m.dt));

@@ -26,7 +26,7 @@ struct Kernels {
   const char* (*error_string)(int) = nullptr;
   // matrix products
   int (*gemm_simt)(void*, const void*, const void*, int, int, int, int, int, int, int, int, int, int, void*) = nullptr;
-  int (*gemm_simt_glu)(float*, const float*, const float*, int, int, int, int, int, int, int, float, float, void*) = nullptr;
+  int (*gemm_simt_glu)(float*, const float*, const float*, int, int, int, int, int, int, int, float, float, int, void*) = nullptr;
   int (*gemm_bf16_tc)(void*, const void*, const void*, int, int, int, int, int, int, int, int*, int, int, void*) = nullptr;
   long long (*packed_weight_bytes)(int, int) = nullptr;
   int (*pack_weight_tiles)(void*, const void*, int, int, int, void*) = nullptr;

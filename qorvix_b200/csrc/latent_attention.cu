@@ -383,8 +383,8 @@ __device__ __forceinline__ void lt_mma(float* c, const uint32_t* a, const uint32
 }
 
 // Per-head products on the tensor cores: for head e, out[t, e*out_off + n] = f(sum_k a[t, e*a_off + k] * w[e][n][k]),
-// t < R, n < N; tiles of 64 tokens x 64 columns, k in steps of 32 through a ring of four stages (cp.async; the weights' first ones ahead of the
-// wait for the kernel ahead), four warps of 32 x 32 (mma.sync m16n8k16, float32 accumulators).  16 tokens, 16 heads, K 512 / 128: 8.8 / 4.5 us
+// t < R, n < N; tiles of 64 tokens x 64 columns, k in steps of 32 through a ring of four stages (cp.async; with early != 0 the weights' first
+// ones ahead of the wait for the kernel ahead, which must not write them), four warps of 32 x 32 (mma.sync m16n8k16, float32 accumulators).  16 tokens, 16 heads, K 512 / 128: 8.8 / 4.5 us
 // with two stages, one trip to memory a step; 7.6 / 3.8 here.  GATED: f multiplies by sigmoid(gate[t, e*gate_off + n]).
 // tail > 0: the `tail` entries that follow a head's K inputs are copied behind its N outputs (the rotated query part
 // rides along with the query's move into the latent space).  K a multiple of 8, rows of a on 16 bytes.
@@ -393,7 +393,7 @@ __device__ __forceinline__ void lt_mma(float* c, const uint32_t* a, const uint32
 template <bool GATED>
 __global__ void __launch_bounds__(128) heads_gemm_kernel(bf16* __restrict__ out, int ld_out, int out_off, const bf16* __restrict__ a, int ld_a,
                                                          int a_off, const bf16* __restrict__ w, const bf16* __restrict__ gate, int ld_gate,
-                                                         int gate_off, int R, int N, int K, int tail) {
+                                                         int gate_off, int R, int N, int K, int tail, int early) {
   __shared__ __align__(16) bf16 As[HG_STAGES][64][HG_LD];
   __shared__ __align__(16) bf16 Bs[HG_STAGES][64][HG_LD];
   const int e = blockIdx.z, row0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
@@ -412,11 +412,12 @@ __global__ void __launch_bounds__(128) heads_gemm_kernel(bf16* __restrict__ out,
     }
   };
   const int nk = (K + 31) / 32;
-  for (int kt = 0; kt < HG_STAGES - 1 && kt < nk; ++kt) stage(kt, true, false);
+  if (early)
+    for (int kt = 0; kt < HG_STAGES - 1 && kt < nk; ++kt) stage(kt, true, false);
   pdl_wait();
   pdl_launch_dependents();
   for (int kt = 0; kt < HG_STAGES - 1; ++kt) {
-    if (kt < nk) stage(kt, false, true);
+    if (kt < nk) stage(kt, !early, true);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   if (tail > 0 && blockIdx.x == 0)
@@ -809,7 +810,7 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
   bf16* lat = (bf16*)(part_ml + (((size_t)splits * rows * 2 + 3) / 4) * 4);
   // the queries' move into the latent space: per head q_plain [T, dn] x Wuk_h [dn, rank], the rotated part copied behind
   int rc = qv_launch(heads_gemm_kernel<false>, dim3((rank + 63) / 64, (T + 63) / 64, H), dim3(128), 0, st, qlat, H * kw, kw,
-                     (const bf16*)q, ld_q, dn + dr, (const bf16*)wuk_t, (const bf16*)nullptr, 0, 0, T, rank, dn, dr);
+                     (const bf16*)q, ld_q, dn + dr, (const bf16*)wuk_t, (const bf16*)nullptr, 0, 0, T, rank, dn, dr, 0);
   if (rc) return rc;
   dim3 grid(((size_t)max_q_len * H + LT_BM - 1) / LT_BM, S, splits);
 #define LT_LAUNCH_WT(N, W)                                                                                                  \
@@ -834,12 +835,13 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
   rc = qv_launch(latent_merge_kernel, dim3((unsigned)rows), dim3(128), (size_t)splits * sizeof(float), st, lat, (const float*)part_o, (const float*)part_ml, rank,
                  splits, (int)rows, sink, H);
   if (rc) return rc;
-  // the heads' value matrices and the gate: per head latent [T, rank] x Wuv_h^T [rank, dv]
+  // the heads' value matrices and the gate: per head latent [T, rank] x Wuv_h^T [rank, dv] (whatever wrote Wuv has ended: the launches above
+  // waited for it)
   if (gate)
     return qv_launch(heads_gemm_kernel<true>, dim3((dv + 63) / 64, (T + 63) / 64, H), dim3(128), 0, st, (bf16*)out, ld_out, dv,
-                     (const bf16*)lat, H * rank, rank, (const bf16*)wuv, (const bf16*)gate, ld_gate, dv, T, dv, rank, 0);
+                     (const bf16*)lat, H * rank, rank, (const bf16*)wuv, (const bf16*)gate, ld_gate, dv, T, dv, rank, 0, 1);
   return qv_launch(heads_gemm_kernel<false>, dim3((dv + 63) / 64, (T + 63) / 64, H), dim3(128), 0, st, (bf16*)out, ld_out, dv,
-                   (const bf16*)lat, H * rank, rank, (const bf16*)wuv, (const bf16*)nullptr, 0, 0, T, dv, rank, 0);
+                   (const bf16*)lat, H * rank, rank, (const bf16*)wuv, (const bf16*)nullptr, 0, 0, T, dv, rank, 0, 1);
 }
 
 // ---------------------------------------------------------------- portions: the latents as rows, for keys and values formed per head

@@ -41,7 +41,7 @@ _ARGTYPES = {
     "qv_cast": [_V, _V, _L, _I, _I, _V],
     "qv_cast_rows": [_V, _L, _V, _L, _I, _I, _I, _I, _V],
     "qv_gemm_simt": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V],
-    "qv_gemm_simt_glu": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _F, _V],
+    "qv_gemm_simt_glu": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _V],
     "qv_gemm_bf16_tc": [_V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V, _I, _I, _V],
     "qv_packed_weight_bytes": [_I, _I],
     "qv_pack_weight_tiles": [_V, _V, _I, _I, _I, _V],
@@ -1510,8 +1510,9 @@ def moe_combine(delta, mix, y, slot_row, top_w, shared, gate, mix_scale=None, ff
 
 # ------------------------------------------------------------------ matrix products
 
-def gemm_simt(c, a, w, accumulate=False) -> None:
-    """c[M,N] (+)= a[M,K] @ w[N,K]^T with float32 multiply-adds on the CUDA cores."""
+def gemm_simt(c, a, w, accumulate=False, settled: bool = False) -> None:
+    """c[M,N] (+)= a[M,K] @ w[N,K]^T with float32 multiply-adds on the CUDA cores.  settled: w is one of a model's weights, which no
+    launch that may still run writes; the kernel then reads it while the launch in front ends."""
     _need_cuda(c, a, w)
     M, K = a.shape
     N = w.shape[0]
@@ -1519,7 +1520,7 @@ def gemm_simt(c, a, w, accumulate=False) -> None:
     assert a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
     rc = _lib("gemm_simt").qv_gemm_simt(
         _ptr(c), _ptr(a), _ptr(w), M, N, K, a.stride(0), w.stride(0), c.stride(0), dt_code(a.dtype),
-        dt_code(w.dtype), dt_code(c.dtype), 1 if accumulate else 0, _stream())
+        dt_code(w.dtype), dt_code(c.dtype), (1 if accumulate else 0) | (0x100 if settled else 0), _stream())
     _check(rc, "gemm_simt")
 
 
@@ -1743,11 +1744,11 @@ def packed_weights_enabled() -> bool:
     return os.environ.get("QORVIX_PACKED_WEIGHTS", "1") != "0"
 
 
-def gemm(out, x, w, packed=None, n: int = 0) -> None:
+def gemm(out, x, w, packed=None, n: int = 0, settled: bool = False) -> None:
     """out = x @ w^T with the kernel that fits the dtypes and the shape.  w is the matrix as rows
     [n, K] (or None when only its packed tiles are kept, `packed` with `n` rows): bfloat16 operands
-    go to the tensor-core kernels (over the packed tiles when there are any), everything else to the
-    CUDA-core kernel."""
+    go to the tensor-core kernels (over the packed tiles when there are any; they take the matrix for
+    a model's weights), everything else to the CUDA-core kernel (settled: see gemm_simt)."""
     if x.dtype == torch.bfloat16 and packed is not None and gemm_bf16_packed(out, x, packed, n or w.shape[0]):
         return
     if w is None:
@@ -1761,7 +1762,7 @@ def gemm(out, x, w, packed=None, n: int = 0) -> None:
         raise KernelError("the product's shape is one the tensor-core kernel refuses and the weight rows were not kept")
     if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and gemm_bf16_tc(out, x, w):
         return
-    gemm_simt(out, x, w)
+    gemm_simt(out, x, w, settled=settled)
 
 
 def glu_epilogue(act: int) -> int:
@@ -1806,10 +1807,10 @@ def gemm_act(out, x, w, packed, n: int, act: int, bias=None) -> None:
     activation(out, out, act, bias=bias)
 
 
-def gemm_swiglu(out, x, w_interleaved, packed=None, n: int = 0, act: int = 0, limit: float = 0.0, slope: float = 0.0) -> None:
+def gemm_swiglu(out, x, w_interleaved, packed=None, n: int = 0, act: int = 0, limit: float = 0.0, slope: float = 0.0, settled: bool = False) -> None:
     """out[M,f] = act(x Wg^T) * (x Wu^T) (act GLU_SILU or GLU_GELU_TANH; GLU_CLAMPED with limit and slope: see glu_act) with gate
     and up rows interleaved in groups of 16 in w_interleaved [2f, K]: one tensor-core kernel (float32: one kernel of
-    multiply-adds) when it takes the shape, else the product followed by the activation kernel."""
+    multiply-adds) when it takes the shape, else the product followed by the activation kernel (settled: see gemm_simt)."""
     n = n or w_interleaved.shape[0]
     if act == GLU_CLAMPED:
         if gemm_bf16_glu(out, x, w_interleaved, packed, n, act, limit, slope):
@@ -1825,12 +1826,12 @@ def gemm_swiglu(out, x, w_interleaved, packed=None, n: int = 0, act: int = 0, li
             and x.dim() == w_interleaved.dim() == out.dim() == 2 and x.stride(1) == w_interleaved.stride(1) == 1
             and n == w_interleaved.shape[0] and w_interleaved.shape[1] == x.shape[1] and out.shape == (x.shape[0], n // 2)):
         rc = _lib("gemm_simt").qv_gemm_simt_glu(_ptr(out), _ptr(x), _ptr(w_interleaved), x.shape[0], n, x.shape[1], x.stride(0), w_interleaved.stride(0),
-                                                out.stride(0), act, float(limit), float(slope), _stream())
+                                                out.stride(0), act, float(limit), float(slope), 1 if settled else 0, _stream())
         if rc != -2:
             _check(rc, "gemm_simt_glu")
             return
     gu = torch.empty((x.shape[0], n), device=x.device, dtype=out.dtype)
-    gemm(gu, x, w_interleaved, packed, n)
+    gemm(gu, x, w_interleaved, packed, n, settled=settled)
     glu_act(out, gu, act, interleaved=True, limit=limit, slope=slope)
 
 

@@ -36,7 +36,7 @@ class Linear:
             out = torch.empty((M, self.out_features), device=x.device, dtype=out_dtype or x.dtype)
         if M == 0:
             return out
-        ops.gemm(out, x, self.weight, self.packed, self.out_features)
+        ops.gemm(out, x, self.weight, self.packed, self.out_features, settled=True)
         return out
 
     __call__ = forward

@@ -55,7 +55,7 @@ class SwiGLU(FeedForward):
             act = torch.empty((x.shape[0], self.f), device=x.device, dtype=self.rt.dtype)
             if self.interleaved:
                 ops.gemm_swiglu(act, x, self.gate_up.weight, self.gate_up.packed, self.gate_up.out_features, act=self.act,
-                               limit=self.limit, slope=self.slope)
+                                limit=self.limit, slope=self.slope, settled=True)
             else:
                 gu = self.gate_up(x, out_dtype=self.rt.dtype)
                 ops.glu_act(act, gu, self.act, limit=self.limit, slope=self.slope)

@@ -206,3 +206,37 @@ def test_remote_shared_memory_is_touched_behind_a_cluster_barrier_only():
             assert waits and waits[0] < remote[0] and arrives[0] <= waits[0], f"{path.name}: remote shared memory ahead of a cluster barrier"
             assert waits[-1] > remote[-1], f"{path.name}: a CTA may leave while its shared memory is in use"
     assert seen >= 2
+
+
+def test_weights_are_read_ahead_of_the_wait_only_where_the_caller_says_they_lie_still(monkeypatch):
+    """A launch may start while the one in front of it still runs; what it reads ahead of its wait must not be what that one writes.  So the
+    32-bit products read w early for a model's layers alone, and the kernels have no other load there."""
+    import re
+    from pathlib import Path
+    from types import SimpleNamespace
+
+    import torch
+    from qorvix_b200.parts.linear import Linear
+
+    flags = []
+    entry = SimpleNamespace(qv_gemm_simt=lambda *a: flags.append(a[12]) or 0)
+    monkeypatch.setattr(ops, "_lib", lambda name: entry)
+    monkeypatch.setattr(ops, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    x, w, out = torch.zeros(2, 8), torch.zeros(4, 8), torch.zeros(2, 4)
+    ops.gemm_simt(out, x, w)
+    ops.gemm_simt(out, x, w, accumulate=True)
+    ops.gemm(out, x, w)
+    layer = object.__new__(Linear)
+    layer.weight, layer.packed, layer.out_features = w, None, 4
+    layer.forward(x)
+    assert flags == [0, 1, 0, 0x100]
+
+    for name, kernel, early in (("gemm_simt.cu", "gemm_simt_kernel", "if (ASYNC && settled)"), ("channel_scan.cu", "channel_gates_tile_kernel", None),
+                                ("latent_attention.cu", "heads_gemm_kernel", "if (early)")):
+        text = (Path(ops.__file__).parent / name).read_text()
+        body = text[re.search(r"__global__[^;{]*\b%s\(" % kernel, text).end():]
+        ahead = body[: body.index("pdl_wait();")]
+        ahead = ahead[ahead.rindex("};") + 2:] if "};" in ahead else ahead            # behind the lambdas that are only defined there
+        loads = re.findall(r"\bstage\(|\bfetch\(|w2t\[", ahead)
+        assert (len(loads) == 1 and early in ahead) if early else not loads, (kernel, ahead)
