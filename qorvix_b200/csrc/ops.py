@@ -71,9 +71,10 @@ _ARGTYPES = {
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
     "qv_linear_scan_chunk_from": [],
+    "qv_linear_scan_parallel_from": [_I],
     "qv_linear_scan_workspace_bytes": [_I, _I, _I, _I, _I, _I],
-    "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V, _L,
-                       _V],
+    "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V,
+                       _L, _V, _V],
     "qv_gated_group_norm": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _I, _V],
     "qv_moe_route": [_V, _V, _V, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _F, _I, _I, _I, _V],
     "qv_moe_max_tiles": [_I, _I, _I],
@@ -905,6 +906,7 @@ class _LeadingSegments:
 
 SCAN_GATED_MAX, SCAN_DECAY = 0, 1
 SCAN_CHUNK_FROM = 16                       # segments of at least this many tokens go in chunks (bfloat16; qv_linear_scan_chunk_from)
+SCAN_CHUNK = 64                            # of so many tokens
 
 
 def _scan_rest(ctx):
@@ -952,17 +954,19 @@ def linear_scan(kind, out, q, k, v, g1, g2, p1, p2, p3, cap, q_scale, state, ctx
     assert state.dtype == torch.float32 and state.stride(-1) == 1
     for p in (p1, p2, p3):
         assert p is None or (p.dtype == torch.float32 and p.numel() >= H)
-    lib, rest = _lib("recurrent"), _scan_rest(ctx)
-    ws = None                              # what long portions' faster kernels need beside their operands; without room the others take them
-    if q.dtype == torch.bfloat16 and rest[1] >= SCAN_CHUNK_FROM:
-        need = lib.qv_linear_scan_workspace_bytes(kind, ctx.num_segments - rest[0], rest[1], H, dk, dv)
-        ws = _room(need, torch.uint8, q.device) if need else None
+    lib, rest, launches = _lib("recurrent"), _scan_rest(ctx), c_int()
+    ws = lens = None                       # what long portions' faster kernels need beside their operands; without room the others take them
+    if q.dtype == torch.bfloat16 and rest[1] >= lib.qv_linear_scan_parallel_from(kind) and getattr(ctx, "seg_len", None):
+        chunks = [-(-n // SCAN_CHUNK) for n in ctx.seg_len[rest[0]:] if n >= lib.qv_linear_scan_parallel_from(kind)]
+        lens = (c_int * ctx.num_segments)(*ctx.seg_len)
+        ws = _room(lib.qv_linear_scan_workspace_bytes(kind, len(chunks), -(-sum(chunks) // len(chunks)) * SCAN_CHUNK, H, dk, dv), torch.uint8, q.device)
     rc = lib.qv_linear_scan(
         kind, _ptr(out), out.stride(0), _ptr(q), q.stride(0), q_group, _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(g1),
         g1.stride(0), _ptr(g2), g2.stride(0) if g2 is not None else 0, _ptr(p1), _ptr(p2), _ptr(p3), float(cap), float(q_scale),
         _ptr(state), state.stride(0), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, *rest,
-        H, dk, dv, dt_code(q.dtype), _ptr(ws), ws.numel() if ws is not None else 0, _stream())
+        H, dk, dv, dt_code(q.dtype), lens, _ptr(ws), ws.numel() if ws is not None else 0, ctypes.byref(launches), _stream())
     _check(rc, "linear_scan")
+    add_launches(launches.value - 1)
 
 
 def gated_group_norm(out, y, gate, w, groups: int, eps: float, gate_first: bool) -> None:

@@ -14,6 +14,7 @@
 //
 // All state arithmetic, gates, decays and norms are float32; q, k and v are read in the compute type.
 #include "common.cuh"
+#include "portion_rounds.h"
 
 #define CONV_MAX_TAPS 16
 #define CONV_CHUNK 16
@@ -1168,22 +1169,28 @@ struct LpGates {                           // what a chunk's gates amount to; 16
   float c[LC_C], A_end, m_end, pad[2];     // what the states' kernel reads
 };
 
-// The workspace of one launch of the three: chunks c0 ... c0 + P - 1 of every segment, a slot each.
+// One round of the three launches: some chunks of some segments, a slot of the workspace each.  What goes from a segment's round to its next
+// one beside the state: the running maximum in its full width and n as the sums it is kept in, so that no bit depends on the rounds.
+#define LP_ITEMS 32
 struct LpWork {
   float* S;                                // [slots][H][col tiles of 16][key tiles of 8][32 lanes][4]
   float* n;                                // [slots][H][LP_NPARTS][dkp], n as sums
   LpGates* gates;                          // [slots][H]
-  double* m;                               // [segments][H]: the running maximum behind chunk c0 + P - 1
-  int* odd;                                // [segments][H][blocks of 64 columns]: some value was infinite or NaN
-  int P, c0, dkp, ct, vt;                  // dkp: dk in whole runs of 32; ct: column tiles of 16; vt: columns a tile of the state
+  double* m;                               // [places][H]: the running maximum behind the round's last chunk
+  float* n_end;                            // [places][H][LP_NPARTS][dkp]: n behind it
+  int* odd;                                // [places][H][blocks of 64 columns]: some value of the round was infinite or NaN
+  int dkp, ct, vt;                         // dkp: dk in whole runs of 32; ct: column tiles of 16; vt: columns a tile of the state
+  PortionRound<LP_ITEMS> round;
 };
 static inline size_t lp_slot_bytes(int H, int dk, int dv) {
   const size_t dkp = (dk + 31) / 32 * 32, ct = (dv + 15) / 16;
   return (size_t)H * (ct * dkp * 64 + LP_NPARTS * dkp * 4 + sizeof(LpGates));
 }
-static inline size_t lp_segment_bytes(int H, int dv) { return (size_t)H * (8 + (size_t)((dv + 63) / 64) * 4); }
+static inline size_t lp_place_bytes(int H, int dk, int dv) {
+  return (size_t)H * (8 + LP_NPARTS * (size_t)((dk + 31) / 32 * 32) * 4 + (size_t)((dv + 63) / 64) * 4);
+}
 
-// grid (segments, heads); a warp takes a chunk: two neighbouring tokens a lane, sums and maxima by scans over the warp.  Bound by the
+// grid (items, heads); a warp takes a chunk: two neighbouring tokens a lane, sums and maxima by scans over the warp.  Bound by the
 // latency of its scans and functions.  In lp_states_kernel itself they cost more: a ninth warp there takes 2.5 us a chunk, which otherwise
 // takes 1.4.
 #define LP_GATE_WARPS 32
@@ -1191,16 +1198,16 @@ __global__ void __launch_bounds__(32 * LP_GATE_WARPS) lp_gates_kernel(const __gr
   __shared__ double ends[LP_GATE_WARPS][2];          // F_63 and max H of the warps' chunks
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const PortionItem& it = w.round.item[blockIdx.x];
+  const int s = it.seg, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  if (len < a.parallel_from) return;
-  const int nchunks = (len + LC_C - 1) / LC_C, last = nchunks < w.c0 + w.P ? nchunks : w.c0 + w.P;
+  const int nchunks = (len + LC_C - 1) / LC_C, last = nchunks < it.first + it.count ? nchunks : it.first + it.count;
   const float b1 = a.p1 ? a.p1[h] : 0.f, b2 = a.p2 ? a.p2[h] : 0.f;
   const int tiles = (a.dv + w.vt - 1) / w.vt;
-  double m_next = w.c0 ? w.m[(size_t)s * a.H + h]
+  double m_next = it.first ? w.m[(size_t)it.place * a.H + h]
                        : (double)a.state[(size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * scan_tile_floats(SCAN_GATED_MAX, a.dk, w.vt) +
                                          (size_t)a.dk * w.vt + a.dk];
-  for (int c1 = w.c0; c1 < last; c1 += LP_GATE_WARPS) {
+  for (int c1 = it.first; c1 < last; c1 += LP_GATE_WARPS) {
     const int c = c1 + warp;
     double lf[2], li[2];
 #pragma unroll
@@ -1251,7 +1258,7 @@ __global__ void __launch_bounds__(32 * LP_GATE_WARPS) lp_gates_kernel(const __gr
 #pragma unroll
     for (int i = 0; i < 3; ++i) Mi[i] = __shfl_sync(0xffffffffu, M, 8 * i);
     if (c < last) {
-      LpGates& gt = w.gates[((size_t)s * w.P + c - w.c0) * a.H + h];
+      LpGates& gt = w.gates[(size_t)(it.slot + c - it.first) * a.H + h];
       float2 pair[2];
       pair[0] = lc_pair(G[0]); pair[1] = lc_pair(G[1]);
       *(float4*)(gt.G + 2 * lane) = make_float4(pair[0].x, pair[0].y, pair[1].x, pair[1].y);
@@ -1268,10 +1275,10 @@ __global__ void __launch_bounds__(32 * LP_GATE_WARPS) lp_gates_kernel(const __gr
     }
     __syncthreads();                                 // the ends have been read
   }
-  if (threadIdx.x == 0) w.m[(size_t)s * a.H + h] = m_next;
+  if (threadIdx.x == 0) w.m[(size_t)it.place * a.H + h] = m_next;
 }
 
-// grid (segments, heads, key blocks x column blocks, then the key blocks once more for n).  Eight warps hold the state as S^T, 16
+// grid (items, heads, key blocks x column blocks, then the key blocks once more for n).  Eight warps hold the state as S^T, 16
 // columns x 32 keys each.  The terms of c v are formed once a CTA, a chunk ahead of the products that read them, so a chunk is one stretch
 // between barriers; k, v and the gates arrive ahead of that (cp.async).  Bound by the latency of a chunk's products and of the terms' way
 // through shared memory: 1.4 us a chunk.  (With the terms formed in registers by both warps that share columns, and n by a ninth warp, three
@@ -1285,24 +1292,24 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_c
   LpStatesSmem& sm = *(LpStatesSmem*)lp_smem;
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x, h = blockIdx.y;
+  const PortionItem& it = w.round.item[blockIdx.x];
+  const int s = it.seg, h = blockIdx.y;
   const int nkb = (a.dk + LP_KEYS - 1) / LP_KEYS, ncb = (a.dv + LP_KEYS - 1) / LP_KEYS, kb = blockIdx.z % nkb, cb = blockIdx.z / nkb;
   const bool is_n = cb == ncb;                       // this CTA sums n
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  if (len < a.parallel_from) return;
   const int dk = a.dk, dv = a.dv, vt = w.vt, tiles = (dv + vt - 1) / vt, tf = scan_tile_floats(SCAN_GATED_MAX, dk, vt);
-  const int nchunks = (len + LC_C - 1) / LC_C, count = (nchunks < w.c0 + w.P ? nchunks : w.c0 + w.P) - w.c0;
+  const int nchunks = (len + LC_C - 1) / LC_C, count = (nchunks < it.first + it.count ? nchunks : it.first + it.count) - it.first;
   if (count <= 0) return;
   float* st = a.state + (size_t)a.seg_slot[s] * a.slot_stride + (size_t)h * tiles * tf;
   const int g8 = lane >> 2, t4 = lane & 3, mi = lane >> 3, r8 = lane & 7;
   const int kw = kb * LP_KEYS + (warp >> 2) * 32, cw = cb * LP_KEYS + (warp & 3) * 16;        // a warp's keys and columns
   const bool holds = !is_n && cw < dv && kw < w.dkp;
-  const LpGates* gates = w.gates + (size_t)s * w.P * a.H + h;
+  const LpGates* gates = w.gates + (size_t)it.slot * a.H + h;
 
   // a thread copies, and splits, the same 16 bytes of every 32nd row
   const int row = tid >> 3, pc = tid & 7;
-  const int token0 = q0 + w.c0 * LC_C, left0 = len - w.c0 * LC_C;
+  const int token0 = q0 + it.first * LC_C, left0 = len - it.first * LC_C;
   const bf16* kp = (const bf16*)a.k + (size_t)(token0 + row) * a.ld_k + (size_t)(h / a.q_group) * dk + kb * LP_KEYS + pc * 8;
   const bf16* vp = (const bf16*)a.v + (size_t)(token0 + row) * a.ld_v + (size_t)h * dv + cb * LP_KEYS + pc * 8;
   const bool k_in = kb * LP_KEYS + pc * 8 < dk, v_in = !is_n && cb * LP_KEYS + pc * 8 < dv;
@@ -1351,7 +1358,11 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_c
   }
   const int nk = kb * LP_KEYS + 2 * lane;            // n: two keys a lane, a quarter of the tokens a warp
   float n0 = 0.f, n1 = 0.f;
-  if (is_n && warp == 0 && nk < dk) { n0 = st[dk * vt + nk]; n1 = st[dk * vt + nk + 1]; }
+  auto n_end = [&]() { return (float2*)(w.n_end + (((size_t)it.place * a.H + h) * LP_NPARTS + warp) * w.dkp + nk); };
+  if (is_n && warp < LP_NPARTS && nk < dk) {
+    if (it.first) { n0 = n_end()->x; n1 = n_end()->y; }
+    else if (warp == 0) { n0 = st[dk * vt + nk]; n1 = st[dk * vt + nk + 1]; }
+  }
   if (!is_n) {
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
@@ -1363,7 +1374,7 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_c
     issue(c + 2);
     const float* cs = sm.c[c % 3];
     const bf16(*ks)[LP_KEYS + 8] = sm.k[c % 3];
-    const size_t slot = ((size_t)s * w.P + c) * a.H + h;
+    const size_t slot = (size_t)(it.slot + c) * a.H + h;
     if (is_n) {
       if (warp < LP_NPARTS) {
         if (nk < w.dkp) *(float2*)(w.n + (slot * LP_NPARTS + warp) * w.dkp + nk) = make_float2(n0, n1);
@@ -1417,7 +1428,10 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_c
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (is_n) {
     float2* sums = (float2*)sm.terms;                // [LP_NPARTS][32]: the terms' place, which these CTAs do not use
-    if (warp < LP_NPARTS) sums[warp * 32 + lane] = make_float2(n0, n1);
+    if (warp < LP_NPARTS) {
+      sums[warp * 32 + lane] = make_float2(n0, n1);
+      if (nk < dk) *n_end() = make_float2(n0, n1);
+    }
     __syncthreads();
     if (nk < dk) {
       const float2 x0 = sums[lane], x1 = sums[32 + lane], x2 = sums[64 + lane], x3 = sums[96 + lane];
@@ -1432,7 +1446,7 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_states_kernel(const __grid_c
     return;
   }
   const int any_odd = __syncthreads_or(odd & 0x80008000u);
-  if (kb == 0 && tid == 0) w.odd[((size_t)s * a.H + h) * ncb + cb] = any_odd != 0;
+  if (kb == 0 && tid == 0) w.odd[((size_t)it.place * a.H + h) * ncb + cb] = any_odd != 0;
   if (any_odd) return;                               // the outputs' kernel goes token by token from the state as it is
   if (holds) {
 #pragma unroll
@@ -1468,9 +1482,12 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_outputs_kernel(const __grid_
   constexpr int LDW = LC_C + 8;
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x / w.P, cr = blockIdx.x % w.P, c = w.c0 + cr, h = blockIdx.y;
+  int i_item = 0;
+  while (i_item + 1 < w.round.items && w.round.item[i_item + 1].slot <= (int)blockIdx.x) ++i_item;
+  const PortionItem& it = w.round.item[i_item];
+  const int s = it.seg, cr = (int)blockIdx.x - it.slot, c = it.first + cr, h = blockIdx.y;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
-  if (len < a.parallel_from || c * LC_C >= len) return;
+  if (c * LC_C >= len) return;
   const int dk = a.dk, dv = a.dv, dkp = w.dkp;
   const int col0 = blockIdx.z * LP_COLS, cols = dv - col0 < LP_COLS ? (dv - col0 + 15) / 16 * 16 : LP_COLS;
   const LpOutShape sh(dkp, cols);
@@ -1634,7 +1651,7 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_outputs_kernel(const __grid_
       }
   }
   __syncthreads();                                   // W's terms, its rows' sums and n . q are in place
-  const int* odd = w.odd + ((size_t)s * a.H + h) * ((dv + LP_KEYS - 1) / LP_KEYS);
+  const int* odd = w.odd + ((size_t)it.place * a.H + h) * ((dv + LP_KEYS - 1) / LP_KEYS);
   for (; cg < ncg; cg += LP_THREADS / 32) {
     float acc[4][2][4] = {};
     const float* Snext = Sp + (size_t)(LP_THREADS / 32) * (dkp >> 3) * 128;    // the warp's next 16 columns
@@ -1717,7 +1734,7 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_outputs_kernel(const __grid_
     }
   }
   if (cr == 0) {
-    const int end = (c + w.P) * LC_C < len ? (c + w.P) * LC_C : len;
+    const int end = (c + it.count) * LC_C < len ? (c + it.count) * LC_C : len;
     const int tiles = (dv + w.vt - 1) / w.vt;
     for (int b = col0 / LP_KEYS; b * LP_KEYS < col0 + cols; ++b) {
       if (!odd[b]) continue;
@@ -1739,34 +1756,31 @@ static int lp_configure(F kernel, int bytes, bool* configured) {
 }
 #define LP_MAX_OUT_BYTES (112 * 1024)      // two CTAs an SM
 
-static int launch_scan_parallel(const ScanArgs& a, int S, int max_len, void* ws, size_t ws_bytes, cudaStream_t st) {
+static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* ws, cudaStream_t st, int* launches) {
   static bool configured[2] = {};
-  const int nchunks = (max_len + LC_C - 1) / LC_C;
   LpWork w;
   w.dkp = (a.dk + 31) / 32 * 32;
   w.ct = (a.dv + 15) / 16;
   w.vt = scan_vt(a.dk);
-  const size_t slot = lp_slot_bytes(a.H, a.dk, a.dv), seg = lp_segment_bytes(a.H, a.dv);
-  size_t P = (ws_bytes - S * seg) / (slot * S);
-  if (P > (size_t)nchunks) P = nchunks;
-  w.P = (int)P;
-  const size_t slots = P * S, cells = slots * a.H;
+  const size_t cells = rounds.slots() * a.H, places = (size_t)rounds.places() * a.H;
   w.m = (double*)ws;
-  w.S = (float*)(w.m + ((size_t)S * a.H + 1) / 2 * 2);
+  w.S = (float*)(w.m + (places + 1) / 2 * 2);
   w.gates = (LpGates*)(w.S + cells * w.ct * w.dkp * 16);
   w.n = (float*)(w.gates + cells);
-  w.odd = (int*)(w.n + cells * LP_NPARTS * w.dkp);
+  w.n_end = w.n + cells * LP_NPARTS * w.dkp;
+  w.odd = (int*)(w.n_end + places * LP_NPARTS * w.dkp);
   const int cols = a.dv < LP_COLS ? (a.dv + 15) / 16 * 16 : LP_COLS;
   const int out_bytes = LpOutShape(w.dkp, cols).bytes, token_bytes = (a.dk * (w.vt + 3) + LP_THREADS + 4) * 4;
   const int smem = out_bytes > token_bytes ? out_bytes : token_bytes, states = (int)sizeof(LpStatesSmem);
   const int kblocks = (a.dk + LP_KEYS - 1) / LP_KEYS, cblocks = (a.dv + LP_KEYS - 1) / LP_KEYS;
   int rc = lp_configure(lp_states_kernel, states, &configured[0]);
   if (!rc) rc = lp_configure(lp_outputs_kernel, LP_MAX_OUT_BYTES, &configured[1]);
-  for (w.c0 = 0; w.c0 < nchunks && !rc; w.c0 += w.P) {
-    rc = qv_launch(lp_gates_kernel, dim3(S, a.H), dim3(32 * LP_GATE_WARPS), 0, st, a, w);
-    if (!rc) rc = qv_launch(lp_states_kernel, dim3(S, a.H, kblocks * (cblocks + 1)), dim3(LP_THREADS), (size_t)states, st, a, w);
-    const dim3 grid(S * w.P, a.H, (a.dv + LP_COLS - 1) / LP_COLS);
+  while (!rc && rounds.next(w.round)) {
+    rc = qv_launch(lp_gates_kernel, dim3(w.round.items, a.H), dim3(32 * LP_GATE_WARPS), 0, st, a, w);
+    if (!rc) rc = qv_launch(lp_states_kernel, dim3(w.round.items, a.H, kblocks * (cblocks + 1)), dim3(LP_THREADS), (size_t)states, st, a, w);
+    const dim3 grid(w.round.slots, a.H, (a.dv + LP_COLS - 1) / LP_COLS);
     if (!rc) rc = qv_launch(lp_outputs_kernel, grid, dim3(LP_THREADS), (size_t)smem, st, a, w);
+    *launches += 3;
   }
   return rc;
 }
@@ -1776,17 +1790,24 @@ static int launch_scan_parallel(const ScanArgs& a, int S, int max_len, void* ws,
 // Scalar decays stay with linear_scan_chunk_kernel: many heads of small states fill the GPU as they are (64 heads of 128 x 64, 1,943 tokens
 // in three segments: a layer 292 us, and 299 with these launches; one segment of 2,048: 282 and 317).
 static inline int scan_parallel_from(int kind) { return kind == SCAN_GATED_MAX ? 640 : 0x7fffffff; }
-// What the three launches take beside qv_linear_scan's operands, for `rest` segments of up to rest_max tokens (0: none of them takes these): the
-// states of as many chunks as LP_ROOM bytes hold, at least one a segment; the next ones follow in launches of their own.
+extern "C" int qv_linear_scan_parallel_from(int kind) { return scan_parallel_from(kind); }
+// What the three launches take beside qv_linear_scan's operands, for `rest` segments that take them, of rest_max tokens each (where they are not
+// alike: of their mean number of chunks): the states of as many chunks as LP_ROOM bytes hold, the next ones follow in launches of their
+// own (so few of a segment, LP_FEW, only where the step has many).
 #define LP_ROOM ((size_t)160 << 20)
+#define LP_FEW 8
+static inline size_t lp_room_slots(int H, int dk, int dv) {
+  const size_t fit = LP_ROOM / lp_slot_bytes(H, dk, dv);
+  return fit ? fit : 1;
+}
+static inline long long lp_bytes(size_t slots, int places, int H, int dk, int dv) {
+  return (long long)(slots * lp_slot_bytes(H, dk, dv) + places * lp_place_bytes(H, dk, dv) + 32);
+}
 extern "C" long long qv_linear_scan_workspace_bytes(int kind, int rest, int rest_max, int H, int dk, int dv) {
   if (rest <= 0 || H <= 0 || dk <= 0 || dv <= 0 || rest_max < scan_parallel_from(kind)) return 0;
-  const size_t slot = lp_slot_bytes(H, dk, dv) * rest, seg = lp_segment_bytes(H, dv) * rest;
-  size_t P = (rest_max + LC_C - 1) / LC_C;
-  if (P * slot > LP_ROOM) P = LP_ROOM / slot ? LP_ROOM / slot : 1;
-  return (long long)(P * slot + seg + 32);
+  const size_t chunks = (size_t)((rest_max + LC_C - 1) / LC_C) * rest, fit = lp_room_slots(H, dk, dv);
+  return lp_bytes(chunks < fit ? chunks : fit, rest, H, dk, dv);
 }
-
 
 extern "C" long long qv_linear_scan_state_floats(int kind, int H, int dk, int dv) {
   const int vt = scan_vt(dk);
@@ -1795,14 +1816,17 @@ extern "C" long long qv_linear_scan_state_floats(int kind, int H, int dk, int dv
 
 // Segments from the first of SCAN_CHUNK_FROM tokens on take the chunks' kernel (those among them that are shorter leave it at once), so
 // that single tokens, which come first in a step, add no CTAs to it: lead, the segments ahead of it; rest_max, rest_min, the longest and the
-// shortest of the others (rest_min 0: not known; that costs a launch).
+// shortest of the others (rest_min 0: not known; that costs a launch).  lens: the segments' tokens (host); ws,
+// ws_bytes: as qv_linear_scan_workspace_bytes says for those of parallel_from tokens and more.  Either null: these take the chunks' kernel
+// like the others.  *launches: how many kernels were launched.
 #define SCAN_CHUNK_FROM 16
 extern "C" int qv_linear_scan_chunk_from(void) { return SCAN_CHUNK_FROM; }
 extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, int ld_q, int q_group, const void* k, int ld_k,
                               const void* v, int ld_v, const float* g1, int ld_g1, const float* g2, int ld_g2, const float* p1,
                               const float* p2, const float* p3, float cap, float q_scale, float* state, long long slot_stride,
                               const int* seg_q_start, const int* seg_slot, int S, int lead, int rest_max, int rest_min, int H, int dk, int dv, int dt,
-                              void* ws, long long ws_bytes, void* stream) {
+                              const int* lens, void* ws, long long ws_bytes, int* launches, void* stream) {
+  *launches = 0;
   if (S <= 0) return 0;
   if (kind != SCAN_GATED_MAX && kind != SCAN_DECAY) return QV_ERR_UNSUPPORTED;
   if (H <= 0 || dk <= 0 || dv <= 0 || q_group <= 0 || H > 65535) return QV_ERR_UNSUPPORTED;
@@ -1828,12 +1852,18 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
     const dim3 rest_grid(S - lead, H, tiles);
     int rc = 0;
     const int parallel_from = scan_parallel_from(kind);
-    if (ws && ((uintptr_t)ws & 15) == 0 && rest_max >= parallel_from) {
-      if (ws_bytes < qv_linear_scan_workspace_bytes(kind, S - lead, rest_max, H, dk, dv)) return QV_ERR_UNSUPPORTED;
-      a.parallel_from = rest.parallel_from = parallel_from;
-      rc = launch_scan_parallel(rest, S - lead, rest_max, ws, (size_t)ws_bytes, st);
+    if (ws && lens && ((uintptr_t)ws & 15) == 0 && rest_max >= parallel_from) {
+      try {
+        PortionRounds rounds(lens + lead, S - lead, LC_C, parallel_from, lp_room_slots(H, dk, dv), LP_FEW);
+        if (ws_bytes < lp_bytes(rounds.slots(), rounds.places(), H, dk, dv)) return QV_ERR_UNSUPPORTED;
+        a.parallel_from = rest.parallel_from = parallel_from;
+        rc = launch_scan_parallel(rest, rounds, ws, st, launches);
+      } catch (...) {
+        return QV_ERR_TOO_LARGE;
+      }
       if (rc || (lead == 0 && rest_min >= parallel_from)) return rc;
     }
+    if (rest.parallel_from > rest_min) ++*launches;
     if (rest.parallel_from <= rest_min) rc = 0;              // none of them is left for the chunks' kernel
     else if (kind == SCAN_GATED_MAX)
       rc = vt == 16 ? launch_scan_chunk<SCAN_GATED_MAX, 16, 2>(rest, rest_grid, st)
@@ -1844,6 +1874,7 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
     if (rest_min >= SCAN_CHUNK_FROM) grid.x = lead;          // none of them is left for the kernel below
     if (rc || grid.x == 0) return rc;
   }
+  ++*launches;
   if (dk <= 8 * 32) {                      // the state fits the registers
     const size_t esz = dt == QV_DT_F32 ? 4 : 2;
     const size_t rowpad = (size_t)((dk + 7) & ~7);

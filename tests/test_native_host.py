@@ -63,3 +63,14 @@ def test_native_scheduler_decisions_with_a_fake_engine(tmp_path):
     assert build.returncode == 0, build.stderr[-3000:]
     run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert run.returncode == 0 and run.stdout.strip() == "ok", run.stderr[-2000:]
+
+
+def test_rounds_of_a_recurrences_chunks(tmp_path):
+    """tests/native/portion_rounds_test.cpp: which chunks share a launch where each takes a slot of a workspace; short neighbours take none."""
+    from qorvix_b200.csrc.build import CSRC, find_host_compiler
+    exe = tmp_path / "portion_rounds_test"
+    build = subprocess.run([find_host_compiler(), "-O1", "-std=c++17", "-I", str(CSRC), "-o", str(exe), str(ROOT / "tests" / "native" / "portion_rounds_test.cpp")],
+                           capture_output=True, text=True, timeout=600)
+    assert build.returncode == 0, build.stderr[-3000:]
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0 and run.stdout.strip() == "ok", run.stdout[-2000:]

@@ -52,3 +52,33 @@ def test_a_part_of_the_chunks_at_a_time_and_no_room(monkeypatch):
         rows = (got[0] - tokens[0]).norm(dim=1) / tokens[0].norm(dim=1)
         assert float(rows.median()) < 2e-6 and bool(torch.isfinite(rows).all())
         assert float((got[1] - tokens[1]).norm() / tokens[1].norm()) < 2e-6
+
+
+@pytest.mark.parametrize("lens", [[32] * 15 + [1100], [1700, 20, 1400, 640, 40, 1200, 1600]])
+def test_a_segment_among_many_does_not_depend_on_them(lens):
+    """One long segment beside many short ones, and five whose chunks' states take several rounds of launches: every segment's outputs and
+    state are, bit for bit, those of a step that holds it alone; short neighbours add no rounds."""
+    H, dk, dv, S, T = 4, 256, 512, len(lens), sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(S)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    q, k, v = (rnd(T, H * n).to(torch.bfloat16) for n in (dk, dk, dv))
+    g1, g2, p1, p2 = rnd(T, H), rnd(T, H) + 2, rnd(H), rnd(H)
+    start = rnd(S, ops.linear_scan_state_floats(ops.SCAN_GATED_MAX, H, dk, dv)) * 0.1
+
+    def run(rows, state, lens):
+        out = torch.full((rows.stop - rows.start, H * dv), float("nan"), device="cuda")
+        before = ops.launch_count()
+        ops.linear_scan(ops.SCAN_GATED_MAX, out, q[rows], k[rows], v[rows], g1[rows], g2[rows], p1, p2, None, 6.0, dk ** -0.5, state, chunks.context(lens),
+                        H, dk, dv)
+        return out, ops.launch_count() - before
+
+    state, at = start.clone(), 0
+    whole, launches = run(slice(0, T), state, lens)
+    assert launches == (4 if S == 16 else 7)                    # (three a round, and the kernel that takes the short ones)
+    for s, n in enumerate(lens):
+        slot = S - 1 - s
+        one = start[slot: slot + 1].clone()
+        alone, launches = run(slice(at, at + n), one, [n])
+        assert launches == (3 if n >= 640 else 1)
+        assert torch.equal(alone, whole[at: at + n]) and torch.equal(one[0], state[slot]), s
+        at += n
