@@ -59,6 +59,7 @@ KERNEL_LIBRARIES = ["elementwise", "gemm_simt", "gemm_bf16", "attention_generic"
 EXTRA_SOURCES = {
     "host_runtime": ["host/dispatch.hpp"],
     "recurrent": ["portion_rounds.h"],
+    "channel_scan": ["portion_rounds.h"],
     "executor": ["host/executor.hpp", "host/kernels.hpp", "host/dispatch.hpp"],
     "ref": ["ref/ref_ops.hpp", "host/json.hpp", "host/safetensors.hpp", "host/model_config.hpp"],
 }

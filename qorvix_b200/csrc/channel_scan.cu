@@ -23,6 +23,7 @@
 // factors and all sums.  The order of every sum depends on the sizes alone, so a token's result does not depend
 // on how its request was cut into steps or on what else is in the batch.
 #include "common.cuh"
+#include "portion_rounds.h"
 
 #define GATE_POW_SIGMOID 0
 #define GATE_EXP_NEG_SIGMOID 1
@@ -541,21 +542,22 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 #define CD_BLOCK 16
 #define CD_COLS 16
 #define CD_OP_THREADS 256
+#define CD_ITEMS 96
 struct ChannelDeltaArgs {
   float* out; int ld_out;                 // [T, H * dv]
   const float *q, *k, *v, *b, *g; int ld_q, ld_k, ld_v, ld_b, ld_g;
-  float* ws;                              // [segments][blocks][H][cd_slot_floats]: blocks block0 ... block0 + blocks - 1 of every segment
-  int block0, blocks;
+  float* ws;                              // [slots][H][cd_slot_floats]: the round's blocks
   float* state; long long slot_stride;    // as ChannelScanArgs
   const int* seg_q_start; const int* seg_slot;
   int H, G, dk, dv, dkp, dvp;             // dkp, dvp: in whole 16s
   float eps, q_scale;
+  PortionRound<CD_ITEMS> round;           // some blocks of some segments, a slot of the workspace each
 };
 // A block's floats: X', X'' and W = (g_(l+1) .. g_end) kb_l in three bfloat16 terms, as the products' operands lie in the lanes, P_end;
 // then per tile of 16 columns v' and v'' ([16 tokens][16 columns] each).
 __host__ __device__ inline size_t cd_slot_floats(int dkp, int dvp) { return (size_t)73 * dkp + 32 * (size_t)dvp; }
-__device__ __forceinline__ float* cd_slot(const ChannelDeltaArgs& a, int s, int block, int h) {
-  return a.ws + (((size_t)s * a.blocks + block - a.block0) * a.H + h) * cd_slot_floats(a.dkp, a.dvp);
+__device__ __forceinline__ float* cd_slot(const ChannelDeltaArgs& a, int slot, int h) {
+  return a.ws + ((size_t)slot * a.H + h) * cd_slot_floats(a.dkp, a.dvp);
 }
 // x and y as three bfloat16 terms each (x in the lower half of a word)
 __device__ __forceinline__ void cd_split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
@@ -570,13 +572,20 @@ __device__ __forceinline__ void cd_split3(float x, float y, uint32_t& t0, uint32
   t0 = t[0]; t1 = t[1]; t2 = t[2];
 }
 
-// grid (blocks of the longest segment, heads, segments).  Bound by its multiply-adds and the reads of shared memory beside them.
+// grid (slots, heads).  Bound by its multiply-adds and the reads of shared memory beside them.
 __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(const __grid_constant__ ChannelDeltaArgs a) {
   extern __shared__ __align__(16) float cd_smem[];
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0, block = a.block0 + blockIdx.x, j0 = block * CD_BLOCK;
+  int first = 0;                                     // whose slot this is
+  for (int last = a.round.items - 1; first < last;) {
+    const int mid = (first + last + 1) >> 1;
+    if (a.round.item[mid].slot <= (int)blockIdx.x) first = mid;
+    else last = mid - 1;
+  }
+  const PortionItem& it = a.round.item[first];
+  const int s = it.seg, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0, j0 = (it.first + (int)blockIdx.x - it.slot) * CD_BLOCK;
   if (j0 >= len) return;
   const int nb = len - j0 < CD_BLOCK ? len - j0 : CD_BLOCK;
   const int dk = a.dk, dkp = a.dkp, ld = dkp + 4;
@@ -653,7 +662,7 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
     (lane < CD_BLOCK ? As : Bs)[(lane & 15) * CD_BLOCK + l] = sum[0];
   }
   __syncthreads();
-  float* ws = cd_slot(a, s, block, h);
+  float* ws = cd_slot(a, blockIdx.x, h);
   uint32_t *X1 = (uint32_t*)ws, *X2 = X1 + 24 * dkp, *Wf = X2 + 24 * dkp;
   float *Pe = ws + 72 * dkp, *Vs = Pe + dkp;
   for (int col = tid; col < dkp + a.dvp; col += CD_OP_THREADS) {     // (whole warps: dkp and dvp are multiples of 16, and half warps stay together)
@@ -774,7 +783,7 @@ __device__ __forceinline__ void cd_words(uint32_t (&a)[3][4], const uint4* p) {
   }
 }
 
-// grid (segments, heads, column tiles); NS warps, a slice of 16 keys each, S^T in registers as the accumulators of the update (value columns x
+// grid (items, heads, column tiles); NS warps, a slice of 16 keys each, S^T in registers as the accumulators of the update (value columns x
 // keys), which are the second operand of X S_0.  A block: the slices' shares of X' S_0 into shared memory, a barrier, their sums e (and y of
 // the block ahead), a barrier, the update; X'' S_0 is formed between the two, where the tensor cores have nothing else to do, and summed a
 // block later.  The operands arrive STAGES - 1 blocks ahead (cp.async).  Bound by that chain: two barriers, three rounds through shared memory,
@@ -794,7 +803,8 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
   constexpr int PER_ROW = CD_COLS / EACH;            // threads a row
   extern __shared__ __align__(16) float cd_smem[];
   pdl_wait();
-  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CD_COLS;
+  const PortionItem& it = a.round.item[blockIdx.x];
+  const int s = it.seg, h = blockIdx.y, col0 = blockIdx.z * CD_COLS, block0 = it.first;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
   const int q0 = a.seg_q_start[s], len = a.seg_q_start[s + 1] - q0;
   const int dk = a.dk, dv = a.dv, dkp = a.dkp, stage_floats = Sh::stage_floats(dkp);
@@ -809,10 +819,10 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
     const int k = k0 + nt * 8 + 2 * t4 + (i & 1), col = col0 + g8 + (i >> 1) * 8;
     return k < 16 * lpc && col < tiles * cpt ? st + (size_t)(col / cpt) * 512 + (k & 15) * 32 + (col % cpt) * lpc + (k >> 4) : nullptr;
   };
-  const int all = (len + CD_BLOCK - 1) / CD_BLOCK - a.block0, nblocks = all < a.blocks ? all : a.blocks;
+  const int all = (len + CD_BLOCK - 1) / CD_BLOCK - block0, nblocks = all < it.count ? all : it.count;
   if (nblocks <= 0) return;
   const size_t stride = (size_t)a.H * cd_slot_floats(dkp, a.dvp);
-  const float* ws = cd_slot(a, s, a.block0, h);
+  const float* ws = cd_slot(a, it.slot, h);
   const int pieces = 73 * dkp / 4;
   auto issue = [&](int blk) {
     if (blk < nblocks) {
@@ -838,9 +848,9 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
   const int orow = (tid / PER_ROW) & 15, ocol = (tid % PER_ROW) * EACH;      // the sums this thread forms
   const bool sums_e = tid < 256, sums_y = THREADS > 256 ? tid >= 256 : true;
   float v2[EACH] = {};                               // v'' of the block ahead
-  float* yp = a.out + (size_t)(q0 + a.block0 * CD_BLOCK + orow) * a.ld_out + (size_t)h * dv + col0 + ocol;
+  float* yp = a.out + (size_t)(q0 + block0 * CD_BLOCK + orow) * a.ld_out + (size_t)h * dv + col0 + ocol;
   const size_t ystep = (size_t)CD_BLOCK * a.ld_out;
-  const int yleft = len - a.block0 * CD_BLOCK - orow, ycols = dv - col0 - ocol;
+  const int yleft = len - block0 * CD_BLOCK - orow, ycols = dv - col0 - ocol;
   for (int i = tid; i < 2 * Sh::RED; i += THREADS) red[i] = 0.f;             // (slices that dk does not reach add nothing)
   auto finish = [&](int blk) {                       // y of a block, from the shares in red2
     if (!sums_y) return;
@@ -965,29 +975,33 @@ static int launch_delta_blocks(const ChannelDeltaArgs& a, dim3 grid, cudaStream_
   return cs_launch_after(delta_blocks_kernel<NS>, grid, dim3(32 * NS), (size_t)smem, st, a);
 }
 
-// What qv_channel_delta takes beside its operands, in floats: for lead_tokens that go token by token, and for segs segments of up to max_rest tokens
-// in blocks, of which as many at a time as CD_ROOM floats hold (at least one of each segment).
+// What qv_channel_delta takes beside its operands, in floats: for lead_tokens that go token by token, and for segs segments of max_rest tokens each
+// (where they are not alike: of their mean number of blocks) in blocks, of which as many at a time as CD_ROOM floats hold.
 #define CD_ROOM ((size_t)48 << 20)
-static inline int cd_blocks_at_a_time(int segs, int max_rest, size_t slot) {
-  const size_t blocks = (max_rest + CD_BLOCK - 1) / CD_BLOCK, fit = CD_ROOM / (slot * segs);
-  return (int)(blocks < fit ? blocks : fit ? fit : 1);
+#define CD_FEW 16                          // blocks of a segment that are worth a round of launches
+static inline size_t cd_slot_all_heads(int H, int dk, int dv) { return H * cd_slot_floats((dk + 15) / 16 * 16, (dv + 15) / 16 * 16); }
+static inline size_t cd_room_slots(int H, int dk, int dv) {
+  const size_t fit = CD_ROOM / cd_slot_all_heads(H, dk, dv);
+  return fit ? fit : 1;
 }
 extern "C" long long qv_channel_delta_workspace_floats(int lead_tokens, int segs, int max_rest, int H, int dk, int dv) {
-  const size_t slot = H * cd_slot_floats((dk + 15) / 16 * 16, (dv + 15) / 16 * 16), lead = (size_t)lead_tokens * H * 3 * dk;
-  return (long long)(segs > 0 && max_rest > 0 ? lead + slot * segs * cd_blocks_at_a_time(segs, max_rest, slot) : lead);
+  const size_t blocks = segs > 0 && max_rest > 0 ? (size_t)((max_rest + CD_BLOCK - 1) / CD_BLOCK) * segs : 0, fit = cd_room_slots(H, dk, dv);
+  return (long long)((size_t)lead_tokens * H * 3 * dk + cd_slot_all_heads(H, dk, dv) * (blocks < fit ? blocks : fit));
 }
 
 // The recurrence over a step's segments: q, k [T, G * dk] float32 (row strides) as the convolutions leave them, b [T, H] the pre-activation of
 // beta, g [T, H * dk] the decays, v [T, H * dv].  The first S_lead segments (T_lead tokens, the longest of them max_lead) go token by token, the
-// others (up to max_rest tokens) in blocks, for which dk is a multiple of 4, at most 256.  workspace: qv_channel_delta_workspace_floats, 16-byte
-// aligned.
+// others (lens [S], host) in blocks, for which dk is a multiple of 4, at most 256.  workspace: qv_channel_delta_workspace_floats, ws_floats of
+// them, 16-byte aligned.  *launches: how many kernels were launched.
 extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                                 const float* b, int ld_b, const float* g, int ld_g, float eps, float q_scale, float* state,
                                 long long slot_stride, const int* seg_q_start, const int* seg_slot, int S, int T, int S_lead,
-                                int T_lead, int max_lead, int max_rest, int H, int G, int dk, int dv, float* workspace, void* stream) {
+                                int T_lead, int max_lead, const int* lens, int H, int G, int dk, int dv, float* workspace, long long ws_floats,
+                                int* launches, void* stream) {
+  *launches = 0;
   if (S <= 0 || T <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || H > 65535 || S_lead < 0 || S_lead > S || T_lead < 0 || T_lead > T) return QV_ERR_UNSUPPORTED;
-  if (S_lead < S && (dk % 4 || max_rest <= 0 || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
+  if (S_lead < S && (dk % 4 || !lens || ((uintptr_t)workspace & 15))) return QV_ERR_UNSUPPORTED;
   if (dk > 256) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   if (S_lead > 0) {
@@ -997,28 +1011,35 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
     if (rc) return rc;
     rc = qv_channel_scan(out, ld_out, qh, H * dk, kb, H * dk, v, ld_v, g, ld_g, kb, H * dk, ug, H * dk, 1.0f, state, slot_stride, seg_q_start,
                          seg_slot, S_lead, max_lead, H, dk, dv, stream);
+    *launches += 2;
     if (rc || S_lead == S) return rc;
     workspace += 3 * n;
+    ws_floats -= 3 * n;
   }
   ChannelDeltaArgs a;
   a.out = out; a.ld_out = ld_out; a.q = q; a.k = k; a.v = v; a.b = b; a.g = g; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.ld_b = ld_b; a.ld_g = ld_g;
   a.ws = workspace; a.state = state; a.slot_stride = slot_stride; a.seg_q_start = seg_q_start + S_lead; a.seg_slot = seg_slot + S_lead;
   a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.dkp = (dk + 15) / 16 * 16; a.dvp = (dv + 15) / 16 * 16; a.eps = eps; a.q_scale = q_scale;
-  const int rest = S - S_lead, col_tiles = a.dvp / CD_COLS, blocks = (max_rest + CD_BLOCK - 1) / CD_BLOCK;
-  if (rest > 65535 || col_tiles > 65535) return QV_ERR_TOO_LARGE;
+  const int col_tiles = a.dvp / CD_COLS;
+  if (col_tiles > 65535) return QV_ERR_TOO_LARGE;
   const int smem = (3 * CD_BLOCK * (a.dkp + 4) + 2 * CD_BLOCK * CD_BLOCK + CD_BLOCK) * 4;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(delta_block_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
   }
-  a.blocks = cd_blocks_at_a_time(rest, max_rest, H * cd_slot_floats(a.dkp, a.dvp));
-  for (a.block0 = 0; a.block0 < blocks; a.block0 += a.blocks) {
-    int rc = qv_launch(delta_block_operands_kernel, dim3(blocks - a.block0 < a.blocks ? blocks - a.block0 : a.blocks, H, rest), dim3(CD_OP_THREADS),
-                       (size_t)smem, st, a);
-    if (rc) return rc;
-    const dim3 grid(rest, H, col_tiles);
-    rc = dk <= 64 ? launch_delta_blocks<4>(a, grid, st) : dk <= 128 ? launch_delta_blocks<8>(a, grid, st) : launch_delta_blocks<16>(a, grid, st);
-    if (rc) return rc;
+  try {
+    PortionRounds rounds(lens + S_lead, S - S_lead, CD_BLOCK, 0, cd_room_slots(H, dk, dv), CD_FEW);
+    if (ws_floats < (long long)(rounds.slots() * cd_slot_all_heads(H, dk, dv))) return QV_ERR_UNSUPPORTED;
+    while (rounds.next(a.round)) {
+      int rc = qv_launch(delta_block_operands_kernel, dim3(a.round.slots, H), dim3(CD_OP_THREADS), (size_t)smem, st, a);
+      if (rc) return rc;
+      const dim3 grid(a.round.items, H, col_tiles);
+      rc = dk <= 64 ? launch_delta_blocks<4>(a, grid, st) : dk <= 128 ? launch_delta_blocks<8>(a, grid, st) : launch_delta_blocks<16>(a, grid, st);
+      if (rc) return rc;
+      *launches += 2;
+    }
+  } catch (...) {
+    return QV_ERR_TOO_LARGE;
   }
   return 0;
 }

@@ -112,7 +112,7 @@ _ARGTYPES = {
     "qv_channel_scan_state_floats": [_I, _I, _I],
     "qv_channel_scan": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _V],
     "qv_channel_delta_workspace_floats": [_I, _I, _I, _I, _I, _I],
-    "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V],
+    "qv_channel_delta": [_V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _I, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _V, _I, _I, _I, _I, _V, _L, _V, _V],
     "qv_head_norm_gate": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _F, _I, _V],
     "qv_bias_attn_prepare": [_V, _I, _V, _I, _I, _I, _I, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V],
     "qv_bias_attention_generic": [_V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _F, _V, _I, _V, _V, _I, _F, _I, _V],
@@ -1052,6 +1052,7 @@ def channel_scan(out, q, k, v, w, au, u, q_scale: float, state, ctx, H: int, dk:
     _check(rc, "channel_scan")
 
 
+DELTA_BLOCK = 16                           # tokens a block
 DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go sixteen tokens at a time,
 DELTA_SHORT_KEYS_FROM = 256                # of this many for keys of up to 64 entries
 
@@ -1079,17 +1080,19 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lens = ctx.seg_len
     lead = delta_lead(lens, dk, blocks)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
-    lib = _lib("channel_scan")
-    ws = _room(lib.qv_channel_delta_workspace_floats(tokens, S - lead, max(lens[lead:]), H, dk, dv), torch.float32, q.device) if lead < S else None
+    lib, launches, rest, ws = _lib("channel_scan"), c_int(), S - lead, None
+    if rest:
+        mean = -(-sum(-(-n // DELTA_BLOCK) for n in lens[lead:]) // rest) * DELTA_BLOCK
+        ws = _room(lib.qv_channel_delta_workspace_floats(tokens, rest, mean, H, dk, dv), torch.float32, q.device)
     if ws is None:                                    # token by token, which takes less room
         lead, tokens, longest = S, T, int(ctx.max_q_len)
         ws = torch.empty(H * T * 3 * dk, device=q.device, dtype=torch.float32)
     rc = lib.qv_channel_delta(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), b.stride(0),
                               _ptr(g), g.stride(0), float(eps), float(q_scale), _ptr(state), state.stride(0),
-                              _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, max(lens[lead:], default=0), H, G, dk, dv,
-                              _ptr(ws), _stream())
+                              _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), S, T, lead, tokens, longest, (c_int * S)(*lens) if lead < S else None,
+                              H, G, dk, dv, _ptr(ws), ws.numel(), ctypes.byref(launches), _stream())
     _check(rc, "channel_delta")
-    add_launches(3 if 0 < lead < S else 1)
+    add_launches(launches.value - 1)
     return True
 
 
