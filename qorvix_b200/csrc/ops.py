@@ -125,6 +125,7 @@ _ARGTYPES = {
     "qv_head_delta_state_floats": [_I, _I, _I],
     "qv_head_delta_scan": [_V, _I, _V, _V, _V, _I, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_argmax": [_V, _V, _I, _I, _L, _V],
+    "qv_argmax_ctas": [_I, _I],
     "qv_sample": [_V, _V, _I, _I, _L, _V, _V, _V, _V, _V, _V, _I, _V, _V, _V, _V],
 }
 _RESTYPES = {"qv_error_string": ctypes.c_char_p, "qv_packed_weight_bytes": c_longlong, "qv_gemm_bf16_split_slot_bytes": c_longlong,

@@ -159,9 +159,16 @@ __global__ void __launch_bounds__(512) argmax_cluster_kernel(int* __restrict__ o
   }
 }
 
+// CTAs a row.  A cluster pays while the rows' clusters are one wave (148 CTAs), and for 64 rows of 65,536 and more; many rows fill the SMs as
+// they are and only get the clusters' start and barriers beside it.  us with a CTA a row and with a cluster, rows in L2: 1 row of
+// 16,384 2.3 and 2.0, of 128,256 7.1 and 2.8; 8 rows 2.3 and 2.3, 7.1 and 3.1; 64 rows 2.4 and 3.7, of 32,768 3.2 and 4.1, of 65,536 4.6 and
+// 4.6, of 128,256 7.4 and 5.8; 256 rows 3.6 and 10.6, of 128,256 21.4 and 25.0.
+extern "C" int qv_argmax_ctas(int rows, int V) {
+  return V >= ARGMAX_CLUSTER_FROM && (rows <= 148 / ARGMAX_CTAS || (V >= 65536 && rows <= 64)) ? ARGMAX_CTAS : 1;
+}
 extern "C" int qv_argmax(int* out, const float* logits, int rows, int V, long long ld, void* stream) {
   if (rows <= 0) return 0;
-  if (V >= ARGMAX_CLUSTER_FROM && rows <= 0x7fffffff / ARGMAX_CTAS)
+  if (qv_argmax_ctas(rows, V) > 1)
     return qv_launch_cluster(argmax_cluster_kernel, dim3(rows * ARGMAX_CTAS), dim3(512), 0, (cudaStream_t)stream, dim3(ARGMAX_CTAS, 1, 1), out, logits, V,
                              ld);
   return qv_launch(argmax_kernel, dim3(rows), dim3(1024), 0, (cudaStream_t)stream, out, logits, V, ld);

@@ -240,3 +240,9 @@ def test_weights_are_read_ahead_of_the_wait_only_where_the_caller_says_they_lie_
         ahead = ahead[ahead.rindex("};") + 2:] if "};" in ahead else ahead            # behind the lambdas that are only defined there
         loads = re.findall(r"\bstage\(|\bfetch\(|w2t\[", ahead)
         assert (len(loads) == 1 and early in ahead) if early else not loads, (kernel, ahead)
+
+
+def test_long_rows_of_logits_share_a_cluster_while_that_is_one_wave():
+    ctas = lambda rows, V: ops._lib("sampling").qv_argmax_ctas(rows, V)
+    assert ctas(1, 16384) == ctas(8, 128256) == ctas(18, 16384) == ctas(64, 65536) == 8
+    assert ctas(8, 16383) == ctas(64, 16384) == ctas(64, 65535) == ctas(65, 128256) == ctas(256, 128256) == 1
