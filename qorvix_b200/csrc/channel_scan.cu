@@ -592,9 +592,9 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
   float* qs = cd_smem;                               // [16][ld] unit vectors, q times q_scale
   float* ks = qs + CD_BLOCK * ld;
   float* gs = ks + CD_BLOCK * ld;
-  float* As = gs + CD_BLOCK * ld;                    // [16][16]
-  float* Bs = As + CD_BLOCK * CD_BLOCK;              // [16][16]
-  float* beta = Bs + CD_BLOCK * CD_BLOCK;            // [16]
+  double* As = (double*)(gs + CD_BLOCK * ld);        // [16][16]
+  double* Bs = As + CD_BLOCK * CD_BLOCK;             // [16][16]
+  float* beta = (float*)(Bs + CD_BLOCK * CD_BLOCK);  // [16]
   const int grp = h / (a.H / a.G);
   // two tokens a warp; beyond the segment: keys and queries zero, decays one
 #pragma unroll
@@ -667,50 +667,51 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
   float *Pe = ws + 72 * dkp, *Vs = Pe + dkp;
   for (int col = tid; col < dkp + a.dvp; col += CD_OP_THREADS) {     // (whole warps: dkp and dvp are multiples of 16, and half warps stay together)
     const bool key = col < dkp;
-    float x[CD_BLOCK], y[CD_BLOCK];
+    // the system's sums in float64 (16 products of numbers of 24 bits in a row, where a block of four had four), their results in float32
+    double xd[CD_BLOCK];
+    float y[CD_BLOCK];
     if (key) {
-      float P = 1.f;
+      float decay = 1.f;
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) {
-        P *= gs[t * ld + col];
-        x[t] = P * ks[t * ld + col];
+        decay *= gs[t * ld + col];
+        xd[t] = decay * ks[t * ld + col];
       }
-      Pe[col] = P;
+      Pe[col] = decay;
     } else {
       const int cv = col - dkp;
       const float* vr = a.v + (size_t)(q0 + j0) * a.ld_v + (size_t)h * a.dv + cv;
 #pragma unroll
-      for (int t = 0; t < CD_BLOCK; ++t) x[t] = t < nb && cv < a.dv ? vr[(size_t)t * a.ld_v] : 0.f;
-    }
-#pragma unroll
-    for (int t = 1; t < CD_BLOCK; ++t) {
-#pragma unroll
-      for (int l4 = 0; l4 < t; l4 += 4) {
-        const float4 A4 = *(const float4*)(As + t * CD_BLOCK + l4);
-        const float A[4] = {A4.x, A4.y, A4.z, A4.w};
-#pragma unroll
-        for (int l = l4; l < l4 + 4 && l < t; ++l) x[t] = fmaf(-A[l - l4], x[l], x[t]);
-      }
-      if (t >= nb) x[t] = 0.f;
+      for (int t = 0; t < CD_BLOCK; ++t) xd[t] = t < nb && cv < a.dv ? vr[(size_t)t * a.ld_v] : 0.f;
     }
 #pragma unroll
     for (int t = 0; t < CD_BLOCK; ++t) {
-      y[t] = 0.f;
+      double sum = xd[t];
 #pragma unroll
-      for (int l4 = 0; l4 <= t; l4 += 4) {
-        const float4 B4 = *(const float4*)(Bs + t * CD_BLOCK + l4);
-        const float B[4] = {B4.x, B4.y, B4.z, B4.w};
-#pragma unroll
-        for (int l = l4; l < l4 + 4 && l <= t; ++l) y[t] = fmaf(B[l - l4], x[l], y[t]);
+      for (int l2 = 0; l2 + 1 < t; l2 += 2) {
+        const double2 A2 = *(const double2*)(As + t * CD_BLOCK + l2);
+        sum = fma(-A2.y, xd[l2 + 1], fma(-A2.x, xd[l2], sum));
       }
+      if (t & 1) sum = fma(-As[t * CD_BLOCK + t - 1], xd[t - 1], sum);
+      xd[t] = t < nb ? (float)sum : 0.f;
+    }
+    float P = 1.f;
+#pragma unroll
+    for (int t = 0; t < CD_BLOCK; ++t) {
+      double sum = 0.0;
+#pragma unroll
+      for (int l2 = 0; l2 + 1 <= t; l2 += 2) {
+        const double2 B2 = *(const double2*)(Bs + t * CD_BLOCK + l2);
+        sum = fma(B2.y, xd[l2 + 1], fma(B2.x, xd[l2], sum));
+      }
+      if (!(t & 1)) sum = fma(Bs[t * CD_BLOCK + t], xd[t], sum);
+      if (key) {
+        P *= gs[t * ld + col];
+        sum = t < nb ? fma((double)P, (double)qs[t * ld + col], -sum) : 0.0;
+      }
+      y[t] = (float)sum;
     }
     if (key) {
-      float P = 1.f;
-#pragma unroll
-      for (int t = 0; t < CD_BLOCK; ++t) {
-        P *= gs[t * ld + col];
-        y[t] = t < nb ? fmaf(P, qs[t * ld + col], -y[t]) : 0.f;
-      }
       // X' and X'' as the products' first operand: lane (t % 8) 4 + (key % 8) / 2 holds, a term, the words of {t, t + 8} x {key, key + 8}, a word
       // an even key and the next one.  Of two neighbouring keys the even one's thread makes the words of tokens 0..7, the other 8..15.
       const int odd = col & 1, lane0 = (col & 7) >> 1, reg = odd + 2 * ((col >> 3) & 1);
@@ -719,10 +720,10 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
       for (int m = 0; m < 2; ++m) {
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-          float* z = m ? y : x;
-          const float other = __shfl_xor_sync(3u << (lane & 30), odd ? z[t] : z[t + 8], 1);
+          const float z0 = m ? y[t] : (float)xd[t], z8 = m ? y[t + 8] : (float)xd[t + 8];
+          const float other = __shfl_xor_sync(3u << (lane & 30), odd ? z0 : z8, 1);
           uint32_t w0, w1, w2;
-          cd_split3(odd ? other : z[t], odd ? z[t + 8] : other, w0, w1, w2);
+          cd_split3(odd ? other : z0, odd ? z8 : other, w0, w1, w2);
           uint32_t* d = dst + m * 24 * dkp + t * 16;
           d[0] = w0; d[128] = w1; d[256] = w2;
         }
@@ -731,15 +732,15 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
       float f = 1.f;
 #pragma unroll
       for (int t = CD_BLOCK - 1; t >= 0; --t) {
-        x[t] = f * (beta[t] * ks[t * ld + col]);
+        y[t] = f * (beta[t] * ks[t * ld + col]);
         f *= gs[t * ld + col];
       }
       uint32_t* wd = Wf + (size_t)(col >> 4) * 384 + (col & 7) * 16 + 2 * ((col >> 3) & 1);
 #pragma unroll
       for (int t4 = 0; t4 < 4; ++t4) {
         uint32_t w[2][3];
-        cd_split3(x[2 * t4], x[2 * t4 + 1], w[0][0], w[0][1], w[0][2]);
-        cd_split3(x[2 * t4 + 8], x[2 * t4 + 9], w[1][0], w[1][1], w[1][2]);
+        cd_split3(y[2 * t4], y[2 * t4 + 1], w[0][0], w[0][1], w[0][2]);
+        cd_split3(y[2 * t4 + 8], y[2 * t4 + 9], w[1][0], w[1][1], w[1][2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) *(uint2*)(wd + i * 128 + t4 * 4) = make_uint2(w[0][i], w[1][i]);
       }
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(CD_OP_THREADS, 3) delta_block_operands_kernel(
       const int cv = col - dkp;
 #pragma unroll
       for (int t = 0; t < CD_BLOCK; ++t) {
-        Vs[(cv >> 4) * 512 + t * 16 + (cv & 15)] = x[t];
+        Vs[(cv >> 4) * 512 + t * 16 + (cv & 15)] = (float)xd[t];
         Vs[(cv >> 4) * 512 + 256 + t * 16 + (cv & 15)] = y[t];
       }
     }
@@ -1022,7 +1023,7 @@ extern "C" int qv_channel_delta(float* out, int ld_out, const float* q, int ld_q
   a.H = H; a.G = G; a.dk = dk; a.dv = dv; a.dkp = (dk + 15) / 16 * 16; a.dvp = (dv + 15) / 16 * 16; a.eps = eps; a.q_scale = q_scale;
   const int col_tiles = a.dvp / CD_COLS;
   if (col_tiles > 65535) return QV_ERR_TOO_LARGE;
-  const int smem = (3 * CD_BLOCK * (a.dkp + 4) + 2 * CD_BLOCK * CD_BLOCK + CD_BLOCK) * 4;
+  const int smem = (3 * CD_BLOCK * (a.dkp + 4) + 4 * CD_BLOCK * CD_BLOCK + CD_BLOCK) * 4;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(delta_block_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
