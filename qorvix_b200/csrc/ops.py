@@ -1054,20 +1054,31 @@ def channel_scan(out, q, k, v, w, au, u, q_scale: float, state, ctx, H: int, dk:
 
 
 DELTA_BLOCK = 16                           # tokens a block
-DELTA_BLOCKS_FROM = 16                     # segments from the first of this many tokens on go sixteen tokens at a time,
-DELTA_SHORT_KEYS_FROM = 256                # of this many for keys of up to 64 entries
+DELTA_SHORT_KEYS_FROM = 256                # keys of up to 64 entries: portions of this many tokens go sixteen tokens at a time
 
 
-def delta_lead(lens, dk: int, blocks: bool = True) -> int:
-    """How many of a step's leading segments the delta rule takes token by token: those ahead of the first of DELTA_BLOCKS_FROM tokens (single
-    tokens come first in a step), all where `blocks` is False and for keys that are no multiple of 4 entries.  Keys of up to 64 entries have
-    half the work a token: portions of up to 256 tokens cost a layer the same either way (8 heads of 64: 64 tokens 149 us token by token
-    and 151 in blocks, four portions of 256 151 and 151, which is the host's time; 1,531 tokens 552 and 175).  16 heads of 128: 16 tokens 153 and
-    151, four portions of 200 252 and 201, 1,531 tokens 637 (four tokens at a time) and 338."""
+def delta_lead(lens, dk: int, blocks: bool = True, heads: int = 128) -> int:
+    """How many of a step's leading segments the delta rule takes token by token (single tokens come first in a step): those ahead of the first
+    portion that pays for sixteen tokens at a time; all where `blocks` is False, for keys that are no multiple of 4 entries or above 256.
+    us token by token and in blocks (rows in L2), one portion and eight: 16 heads of 128, 16 tokens 11.5 and 15.8, 35.9 and 33.5; 24 tokens
+    14.6 and 16.9, 50 and 43; 32 tokens 18.1 and 17.0, 64 and 44; 8 heads 16 tokens x 8 20.5 and 24.3.  4 heads of 256, 32 tokens 21.5 and
+    27.0, 48 tokens 29.7 and 29.2; 16 heads of 256, 32 tokens 42 and 36.  So from 32 tokens on (of 256 entries 48, or 32 where the heads make
+    up for it), from 16 where portions x heads fill the GPU.  Keys of up to 64 entries have half the work a token: 8 heads of 64, 256
+    tokens 84 and 26 (shorter portions were not worth it when they were measured by whole layers); of up to 32 entries a full GPU is faster
+    token by token: 16 heads of 32, 256 tokens x 8 80 and 73, x 16 100 and 153; 64 heads x 8 136 and 287, one portion 75 and 48."""
     if not blocks or dk % 4 or dk > 256:
         return len(lens)
-    first = DELTA_BLOCKS_FROM if dk > 64 else DELTA_SHORT_KEYS_FROM
-    return next((i for i, n in enumerate(lens) if n >= first), len(lens))
+    for i, n in enumerate(lens):
+        if dk <= 64:
+            pays = n >= DELTA_SHORT_KEYS_FROM
+        else:
+            work = (len(lens) - i) * heads
+            pays = n >= (32 if dk <= 128 or work >= 16 else 48) or (n >= 16 and work >= 128)
+        if pays:
+            if dk <= 32 and sum(lens[i:]) * heads > 128 * max(lens[i:]):
+                break
+            return i
+    return len(lens)
 
 
 def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: int, eps: float, q_scale: float, blocks: bool = True) -> bool:
@@ -1079,7 +1090,7 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     assert state.dtype == torch.float32 and state.stride(-1) == 1 and state.shape[-1] >= channel_scan_state_floats(H, dk, dv)
     T, S = q.shape[0], ctx.num_segments
     lens = ctx.seg_len
-    lead = delta_lead(lens, dk, blocks)
+    lead = delta_lead(lens, dk, blocks, H)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
     lib, launches, rest, ws = _lib("channel_scan"), c_int(), S - lead, None
     if rest:

@@ -246,3 +246,13 @@ def test_long_rows_of_logits_share_a_cluster_while_that_is_one_wave():
     ctas = lambda rows, V: ops._lib("sampling").qv_argmax_ctas(rows, V)
     assert ctas(1, 16384) == ctas(8, 128256) == ctas(18, 16384) == ctas(64, 65536) == 8
     assert ctas(8, 16383) == ctas(64, 16384) == ctas(64, 65535) == ctas(65, 128256) == ctas(256, 128256) == 1
+
+
+def test_which_portions_the_delta_rule_takes_in_blocks():
+    lead = ops.delta_lead
+    assert lead([16], 128, heads=16) == 1 and lead([31], 128, heads=32) == 1 and lead([32], 128, heads=1) == 0
+    assert lead([1] * 5 + [16] * 8, 128, heads=16) == 5 and lead([1] * 5 + [16] * 8, 128, heads=8) == 13
+    assert lead([1, 32, 40], 256, heads=4) == 3 and lead([1, 32, 48], 256, heads=4) == 2 and lead([1, 32], 256, heads=16) == 1
+    assert lead([255], 64, heads=8) == 1 and lead([1, 256], 64, heads=8) == 1 and lead([256] * 32, 64, heads=32) == 0
+    assert lead([256] * 8, 32, heads=16) == 0 and lead([256] * 9, 32, heads=16) == 9 and lead([256], 32, heads=64) == 0
+    assert lead([999], 126) == lead([999], 260) == lead([999], 128, blocks=False) == 1
