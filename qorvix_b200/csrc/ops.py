@@ -1063,7 +1063,7 @@ def delta_lead(lens, dk: int, blocks: bool = True, heads: int = 128) -> int:
     us token by token and in blocks (rows in L2), one portion and eight: 16 heads of 128, 16 tokens 11.5 and 15.8, 35.9 and 33.5; 24 tokens
     14.6 and 16.9, 50 and 43; 32 tokens 18.1 and 17.0, 64 and 44; 8 heads 16 tokens x 8 20.5 and 24.3.  4 heads of 256, 32 tokens 21.5 and
     27.0, 48 tokens 29.7 and 29.2; 16 heads of 256, 32 tokens 42 and 36.  So from 32 tokens on (of 256 entries 48, or 32 where the heads make
-    up for it), from 16 where portions x heads fill the GPU.  Keys of up to 64 entries have half the work a token: 8 heads of 64, 256
+    up for it), from 16 where portions x heads fill the GPU or single tokens ahead do (63 beside 16 tokens, 16 heads of 128: 46 and 41).  Keys of up to 64 entries have half the work a token: 8 heads of 64, 256
     tokens 84 and 26 (shorter portions were not worth it when they were measured by whole layers); of up to 32 entries a full GPU is faster
     token by token: 16 heads of 32, 256 tokens x 8 80 and 73, x 16 100 and 153; 64 heads x 8 136 and 287, one portion 75 and 48."""
     if not blocks or dk % 4 or dk > 256:
@@ -1073,7 +1073,7 @@ def delta_lead(lens, dk: int, blocks: bool = True, heads: int = 128) -> int:
             pays = n >= DELTA_SHORT_KEYS_FROM
         else:
             work = (len(lens) - i) * heads
-            pays = n >= (32 if dk <= 128 or work >= 16 else 48) or (n >= 16 and work >= 128)
+            pays = n >= (32 if dk <= 128 or work >= 16 else 48) or (n >= 16 and (work >= 128 or len(lens) * heads >= 512))
         if pays:
             if dk <= 32 and sum(lens[i:]) * heads > 128 * max(lens[i:]):
                 break
