@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(4 * CG_CHANNELS) channel_gates_kernel(float* _
 
 // Portions of many tokens with ranks in whole 16s: a tile of 64 tokens x 64 channels a CTA, 8 x 4 of them a thread, whose sums stay in registers (the
 // kernel above has a multiply-add for each entry of x it reads, and meets in shared memory): 1,531 tokens x 64 x 2,048 with softplus 37 us
-// above, 28 here (without a function 30 and 21); bound by the multiply-adds and the gates' functions.  The same sums in the same order: four quarters of a row, added in
+// above, 28 here (without a function 30 and 21; see qv_channel_gates_tiles); bound by the multiply-adds and the gates' functions.  The same sums in the same order: four quarters of a row, added in
 // order.
 #define CT_TOKENS 64
 #define CT_MAX_RANK 128
@@ -127,14 +127,19 @@ __global__ void __launch_bounds__(128, 5) channel_gates_tile_kernel(float* __res
   const int tid = threadIdx.x, c0 = blockIdx.y * CG_CHANNELS, t0 = blockIdx.x * CT_TOKENS;
   pdl_wait();
   pdl_launch_dependents();
+  if (N % 4 == 0 && ((uintptr_t)w2t & 15) == 0 && c0 + CG_CHANNELS <= N) {
 #pragma unroll 8
-  for (int i = tid; i < R * CG_CHANNELS; i += 128) {
-    const int r = i / CG_CHANNELS, c = c0 + i % CG_CHANNELS;
-    wsm[i] = c < N ? w2t[(size_t)r * N + c] : 0.f;
+    for (int i = tid * 4; i < R * CG_CHANNELS; i += 512) *(float4*)(wsm + i) = *(const float4*)(w2t + (size_t)(i / CG_CHANNELS) * N + c0 + i % CG_CHANNELS);
+  } else {
+#pragma unroll 8
+    for (int i = tid; i < R * CG_CHANNELS; i += 128) {
+      const int r = i / CG_CHANNELS, c = c0 + i % CG_CHANNELS;
+      wsm[i] = c < N ? w2t[(size_t)r * N + c] : 0.f;
+    }
   }
   for (int r = tid & 31; r < R; r += 32) {           // a token a warp
     const float* xp = x1 + (size_t)t0 * ld_x + r;
-#pragma unroll 8
+#pragma unroll 16
     for (int j = tid >> 5; j < CT_TOKENS; j += 4) {
       float v = t0 + j < T ? xp[(size_t)j * ld_x] : 0.f;
       if (pre_tanh) v = tanhf(v);
@@ -187,6 +192,15 @@ __global__ void __launch_bounds__(128, 5) channel_gates_tile_kernel(float* __res
   for (int j = tid >> 6; j < last; j += 2) o[(size_t)j * ld_out] = cg_gate(cg_smem[j * (CG_CHANNELS + 4) + (tid & 63)] + bc, form, c);
 }
 
+// Whether the tiles take a portion: ranks in whole 16s that fit, and tiles enough to hide their loads and functions behind one another: a tile
+// has four times the work in a row that a CTA of the other kernel has.  us with the other kernel and with the tiles (rows in L2): 64 tiles of
+// rank 64 5.2 and 9.7 with softplus (without a function 4.7 and 6.9); 256 tiles 12.7 and 11.6 (11.2 and 8.4), of rank 16 6.9 and 7.9
+// (5.5 and 4.8); 320 of rank 32 0.99 of the other kernel's time; 512 of rank 16 12.3 and 12.6; 1,024 of rank 64 43 and 28 (38 and 21).
+extern "C" int qv_channel_gates_tiles(int T, int N, int R, int kind) {
+  const long long tiles = (long long)((T + CT_TOKENS - 1) / CT_TOKENS) * ((N + CG_CHANNELS - 1) / CG_CHANNELS);
+  return T >= 256 && R % 16 == 0 && R <= CT_MAX_RANK && tiles >= (kind == GATE_LINEAR ? 256 : R >= 32 ? 320 : 640);
+}
+
 // rate [N] float32: the factor per channel of GATE_EXP_NEG_SOFTPLUS (null for the other kinds).
 extern "C" int qv_channel_gates(float* out, int ld_out, const float* x1, int ld_x, const float* w2t, const float* bias, int T, int N,
                                 int R, int pre_tanh, int kind, float p, const float* rate, void* stream) {
@@ -200,7 +214,7 @@ extern "C" int qv_channel_gates(float* out, int ld_out, const float* x1, int ld_
   if (by > 65535) return QV_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   const CgForm form = {kind, p, rate};
-  if (T >= 256 && R % 16 == 0 && R <= CT_MAX_RANK) {
+  if (qv_channel_gates_tiles(T, N, R, kind)) {
     static bool configured = false;
     constexpr int most = (CT_TOKENS * (CT_MAX_RANK + 4) + CT_MAX_RANK * CG_CHANNELS) * 4;
     if (!configured) {

@@ -103,6 +103,7 @@ _ARGTYPES = {
     "qv_sigmoid_gate": [_V, _V, _I, _V, _I, _V, _I, _I, _I, _V],
     "qv_depth_mix": [_V, _V, _V, _L, _V, _I, _V],
     "qv_scale": [_V, _L, _F, _V],
+    "qv_channel_gates_tiles": [_I, _I, _I, _I],
     "qv_channel_gates": [_V, _I, _V, _I, _V, _V, _I, _I, _I, _I, _I, _F, _V, _V],
     "qv_delta_operands": [_V, _V, _V, _V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _I, _I, _F, _F, _V],
     "qv_post_rmsnorm_add": [_V, _V, _I, _V, _F, _V, _I, _I, _I, _I, _V, _F, _V],

@@ -251,8 +251,17 @@ def test_long_rows_of_logits_share_a_cluster_while_that_is_one_wave():
 def test_which_portions_the_delta_rule_takes_in_blocks():
     lead = ops.delta_lead
     assert lead([16], 128, heads=16) == 1 and lead([31], 128, heads=32) == 1 and lead([32], 128, heads=1) == 0
+    assert lead([1] * 63 + [16], 128, heads=16) == 63 and lead([1] * 32 + [16], 128, heads=8) == 33
     assert lead([1] * 5 + [16] * 8, 128, heads=16) == 5 and lead([1] * 5 + [16] * 8, 128, heads=8) == 13
     assert lead([1, 32, 40], 256, heads=4) == 3 and lead([1, 32, 48], 256, heads=4) == 2 and lead([1, 32], 256, heads=16) == 1
     assert lead([255], 64, heads=8) == 1 and lead([1, 256], 64, heads=8) == 1 and lead([256] * 32, 64, heads=32) == 0
     assert lead([256] * 8, 32, heads=16) == 0 and lead([256] * 9, 32, heads=16) == 9 and lead([256], 32, heads=64) == 0
     assert lead([999], 126) == lead([999], 260) == lead([999], 128, blocks=False) == 1
+
+
+def test_gates_take_tiles_where_there_are_enough_of_them():
+    tiles = lambda *a: ops._lib("channel_scan").qv_channel_gates_tiles(*a)
+    softplus, linear = ops.GATE_EXP_NEG_SOFTPLUS, ops.GATE_LINEAR
+    assert tiles(1531, 2048, 64, softplus) and tiles(1531, 2048, 64, linear) and tiles(512, 2048, 16, linear) and tiles(300, 4096, 32, softplus)
+    assert not tiles(2048, 128, 64, softplus) and not tiles(512, 2048, 32, softplus) and not tiles(512, 4096, 16, softplus) and not tiles(300, 2048, 64, linear)
+    assert not tiles(255, 65536, 64, linear) and not tiles(2048, 2048, 40, linear) and not tiles(2048, 2048, 144, linear)
