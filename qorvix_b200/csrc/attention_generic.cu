@@ -45,6 +45,9 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
   const size_t v_off = (size_t)Hkv * page * hd;
   const size_t head_off = (size_t)kvh * page * hd;
 
+  // Of heads above 128 entries two keys' values are all that fits, which does not pay for holding them over the scores (256 entries, float32:
+  // 5 % more): they are fetched behind the scores, for the keys whose weight is not zero.
+  constexpr bool AHEAD = NREG <= 4;
   constexpr int KEYS = NREG <= 1 ? 32 : NREG <= 2 ? 16 : NREG <= 4 ? 8 : 2;      // keys whose values are fetched together
   float o[NREG];
 #pragma unroll
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
         }
       }
     };
-    values(0);
+    if constexpr (AHEAD) values(0);
     if (valid) {
       const T* kp = cache + base;
       float dot = 0.f;
@@ -102,13 +105,28 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(
 #pragma unroll
     for (int j = 0; j < NREG; ++j) o[j] *= corr;
     for (int j0 = 0; j0 < nk; j0 += KEYS) {
-      if (j0) values(j0);
+      float pj[KEYS];
+      if constexpr (AHEAD) {
+        if (j0) values(j0);
+      }
 #pragma unroll
       for (int j = 0; j < KEYS; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, p, (j0 + j) & 31);
-        if (j0 + j >= nk || pj == 0.f) continue;     // masked (before the window) or underflowed: adds nothing
+        pj[j] = __shfl_sync(0xffffffffu, p, (j0 + j) & 31);
+        if (j0 + j >= nk) pj[j] = 0.f;
+        if constexpr (!AHEAD) {
+          const T* vp = cache + __shfl_sync(0xffffffffu, (unsigned long long)base, (j0 + j) & 31) + v_off;
 #pragma unroll
-        for (int r = 0; r < NREG; ++r) o[r] = fmaf(pj, to_f(v[j][r]), o[r]);
+          for (int r = 0; r < NREG; ++r) {
+            const int i = lane + 32 * r;
+            v[j][r] = pj[j] != 0.f && i < hd ? vp[i] : from_f<T>(0.f);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < KEYS; ++j) {
+        if (pj[j] == 0.f) continue;                  // masked (before the window) or underflowed: adds nothing
+#pragma unroll
+        for (int r = 0; r < NREG; ++r) o[r] = fmaf(pj[j], to_f(v[j][r]), o[r]);
       }
     }
     m = m_new;
