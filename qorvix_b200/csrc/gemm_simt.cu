@@ -87,7 +87,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(TC* __
   };
   if (ASYNC) {
     for (int t = 0; t < STAGES - 1; ++t) {
-      if (t < tiles) stage(t, 0, settled ? BM : ROWS);
+      if (t < tiles) stage(t, 0, BM);
+      if (t < tiles && !settled) stage(t, BM, ROWS);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
   } else if (tiles > 0) {
