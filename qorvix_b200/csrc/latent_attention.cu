@@ -696,6 +696,9 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
 // e^(sink[head] - M) where there are sinks)
 // The slices' factors are worked out once by all threads, then every thread reads its columns of four slices at a time.
 #define MERGE_SLICES 16
+// FEW: 2 .. MERGE_SLICES slices of up to 512 columns; a kernel of its own, since its 64 registers of partial results would halve the CTAs an SM
+// holds for the others (2,048 rows of one slice 5.5 us, and 7.2 in one kernel).
+template <bool FEW>
 __global__ void __launch_bounds__(128) latent_merge_kernel(bf16* __restrict__ lat, const float* __restrict__ part_o,
                                                            const float* __restrict__ part_ml, int rank, int splits, int total_rows,
                                                            const float* __restrict__ sink, int H) {
@@ -706,7 +709,7 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(bf16* __restrict__ la
   const size_t row = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float sk = sink ? sink[row % H] : -INFINITY;
-  if (splits == 1) {                                       // nothing to merge: divide (and take the sink in)
+  if (!FEW && splits == 1) {                               // nothing to merge: divide (and take the sink in)
     const float2 ml = *(const float2*)(part_ml + 2 * row);
     const float top = fmaxf(ml.x, sk), w = expf(ml.x - top);
     const float f = w / (w * ml.y + (sink ? expf(sk - top) : 0.f));
@@ -716,7 +719,7 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(bf16* __restrict__ la
     }
     return;
   }
-  if (splits <= MERGE_SLICES && rank % 4 == 0 && rank <= 512) {
+  if constexpr (FEW) {
     // few slices: every thread asks for its four columns of all of them at once, every warp works the factors out for itself meanwhile (no
     // barrier); the same sums.  256 rows of 512 from 9 slices: three trips to memory in a row before, one here; the layer
     // of 16 requests behind 1,500 tokens 59.8 us -> 56.7.
@@ -832,7 +835,7 @@ extern "C" int qv_latent_attention_tc(void* out, int ld_out, const void* q, int 
 #undef LT_LAUNCH
 #undef LT_LAUNCH_WT
   if (rc) return rc;
-  rc = qv_launch(latent_merge_kernel, dim3((unsigned)rows), dim3(128), (size_t)splits * sizeof(float), st, lat, (const float*)part_o, (const float*)part_ml, rank,
+  rc = qv_launch(splits > 1 && splits <= MERGE_SLICES ? latent_merge_kernel<true> : latent_merge_kernel<false>, dim3((unsigned)rows), dim3(128), (size_t)splits * sizeof(float), st, lat, (const float*)part_o, (const float*)part_ml, rank,
                  splits, (int)rows, sink, H);
   if (rc) return rc;
   // the heads' value matrices and the gate: per head latent [T, rank] x Wuv_h^T [rank, dv] (whatever wrote Wuv has ended: the launches above
