@@ -71,7 +71,7 @@ _ARGTYPES = {
     "qv_conv_state": [_V, _I, _V, _I, _V, _V, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_linear_scan_state_floats": [_I, _I, _I, _I],
     "qv_linear_scan_chunk_from": [],
-    "qv_linear_scan_parallel_from": [_I],
+    "qv_linear_scan_parallel_from": [_I, _I, _I, _I],
     "qv_linear_scan_workspace_bytes": [_I, _I, _I, _I, _I, _I],
     "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V,
                        _L, _V, _V],
@@ -958,8 +958,9 @@ def linear_scan(kind, out, q, k, v, g1, g2, p1, p2, p3, cap, q_scale, state, ctx
         assert p is None or (p.dtype == torch.float32 and p.numel() >= H)
     lib, rest, launches = _lib("recurrent"), _scan_rest(ctx), c_int()
     ws = lens = None                       # what long portions' faster kernels need beside their operands; without room the others take them
-    if q.dtype == torch.bfloat16 and rest[1] >= lib.qv_linear_scan_parallel_from(kind) and getattr(ctx, "seg_len", None):
-        chunks = [-(-n // SCAN_CHUNK) for n in ctx.seg_len[rest[0]:] if n >= lib.qv_linear_scan_parallel_from(kind)]
+    least = lib.qv_linear_scan_parallel_from(kind, H, dk, dv)
+    if q.dtype == torch.bfloat16 and rest[1] >= least and getattr(ctx, "seg_len", None):
+        chunks = [-(-n // SCAN_CHUNK) for n in ctx.seg_len[rest[0]:] if n >= least]
         lens = (c_int * ctx.num_segments)(*ctx.seg_len)
         ws = _room(lib.qv_linear_scan_workspace_bytes(kind, len(chunks), -(-sum(chunks) // len(chunks)) * SCAN_CHUNK, H, dk, dv), torch.uint8, q.device)
     rc = lib.qv_linear_scan(

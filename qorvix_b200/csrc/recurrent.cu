@@ -1789,8 +1789,22 @@ static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* 
 // ways cost the same (a layer 98 us, where launching it from the host is what takes the time), by 32 the one kernel takes 272 and these 200.
 // Scalar decays stay with linear_scan_chunk_kernel: many heads of small states fill the GPU as they are (64 heads of 128 x 64, 1,943 tokens
 // in three segments: a layer 292 us, and 299 with these launches; one segment of 2,048: 282 and 317).
-static inline int scan_parallel_from(int kind) { return kind == SCAN_GATED_MAX ? 640 : 0x7fffffff; }
-extern "C" int qv_linear_scan_parallel_from(int kind) { return scan_parallel_from(kind); }
+// Which sizes: linear_scan_chunk_kernel forms W again for every tile of value columns, so many tiles a head speak for the three launches; where few
+// tiles of all heads together fill the GPU once (128 CTAs) it is at its best.  A rule on a segment's own length and the sizes, so that its
+// neighbours do not decide which sums it gets.  us with the one kernel and with the three launches, one segment and four of 1,024 tokens: 4 heads
+// of 256 x 512 86 and 64, 333 and 171 (640 tokens: 56 and 56, 213 and 128); 4 heads of 128 x 256 71 and 53, 73 and 64 (768 x 4: 56 and 57);
+// 16 heads of 256 x 64 85 and 54, 170 and 139 (768 x 2: 66 and 72); 32 heads of 128 x 128 73 and 81, 286 and 207 (2,048: 141 and
+// 144, 558 and 419); 16 heads of 64 x 64 61 and 46, 62 and 75; 64 heads of 128 x 64 74 and 98, 288 and 298; 4 heads of 64 x 64 61 and 43, 61
+// and 46 (640 x 8: 40 and 44); 1 head 61 and 44 (640: 39 and 35).
+static inline int scan_parallel_from(int kind, int H, int dk, int dv) {
+  const int never = 0x7fffffff;
+  if (kind != SCAN_GATED_MAX || dk > 256) return never;
+  const int vt = scan_vt(dk), tiles = (dv + vt - 1) / vt;
+  if (tiles >= 16 || (long long)H * tiles <= 4) return 640;
+  if (tiles >= 6 || (tiles >= 4 && vt == 16) || (long long)H * tiles <= 8) return 1024;
+  return tiles >= 4 ? 2048 : never;
+}
+extern "C" int qv_linear_scan_parallel_from(int kind, int H, int dk, int dv) { return scan_parallel_from(kind, H, dk, dv); }
 // What the three launches take beside qv_linear_scan's operands, for `rest` segments that take them, of rest_max tokens each (where they are not
 // alike: of their mean number of chunks): the states of as many chunks as LP_ROOM bytes hold, the next ones follow in launches of their
 // own (so few of a segment, LP_FEW, only where the step has many).
@@ -1804,7 +1818,7 @@ static inline long long lp_bytes(size_t slots, int places, int H, int dk, int dv
   return (long long)(slots * lp_slot_bytes(H, dk, dv) + places * lp_place_bytes(H, dk, dv) + 32);
 }
 extern "C" long long qv_linear_scan_workspace_bytes(int kind, int rest, int rest_max, int H, int dk, int dv) {
-  if (rest <= 0 || H <= 0 || dk <= 0 || dv <= 0 || rest_max < scan_parallel_from(kind)) return 0;
+  if (rest <= 0 || H <= 0 || dk <= 0 || dv <= 0 || rest_max < scan_parallel_from(kind, H, dk, dv)) return 0;
   const size_t chunks = (size_t)((rest_max + LC_C - 1) / LC_C) * rest, fit = lp_room_slots(H, dk, dv);
   return lp_bytes(chunks < fit ? chunks : fit, rest, H, dk, dv);
 }
@@ -1851,7 +1865,7 @@ extern "C" int qv_linear_scan(int kind, float* out, int ld_out, const void* q, i
     rest.seg_slot += lead;
     const dim3 rest_grid(S - lead, H, tiles);
     int rc = 0;
-    const int parallel_from = scan_parallel_from(kind);
+    const int parallel_from = scan_parallel_from(kind, H, dk, dv);
     if (ws && lens && ((uintptr_t)ws & 15) == 0 && rest_max >= parallel_from) {
       try {
         PortionRounds rounds(lens + lead, S - lead, LC_C, parallel_from, lp_room_slots(H, dk, dv), LP_FEW);

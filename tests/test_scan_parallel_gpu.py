@@ -15,6 +15,18 @@ def test_long_portions_against_float64(dk, dv, H, qg, lens, shift):
     chunks.test_chunks_against_float64(ops.SCAN_GATED_MAX, dk, dv, H, qg, lens, shift)
 
 
+@pytest.mark.parametrize("dk,dv,H,qg,lens,shift", [(128, 272, 1, 1, [1025, 20], -3.0), (136, 72, 2, 1, [1024, 16], 1.0)])
+def test_sizes_that_take_them_from_1024_tokens_on(dk, dv, H, qg, lens, shift):
+    assert ops._lib("recurrent").qv_linear_scan_parallel_from(ops.SCAN_GATED_MAX, H, dk, dv) == 1024
+    chunks.test_chunks_against_float64(ops.SCAN_GATED_MAX, dk, dv, H, qg, lens, shift)
+
+
+@pytest.mark.parametrize("what", ["value", "gate"])
+def test_what_is_not_finite_beside_several_blocks_of_columns(what):
+    assert ops._lib("recurrent").qv_linear_scan_parallel_from(ops.SCAN_GATED_MAX, 2, 64, 136) == 2048
+    chunks.test_what_is_not_finite_reaches_no_earlier_token(ops.SCAN_GATED_MAX, 64, 136, [2048, 40], what)
+
+
 @pytest.mark.parametrize("dk,dv,lens", [(64, 136, [640, 40]), (256, 16, [16, 700])])
 @pytest.mark.parametrize("what", ["value", "gate"])
 def test_what_is_not_finite_reaches_no_earlier_token(dk, dv, lens, what):
