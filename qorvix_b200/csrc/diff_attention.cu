@@ -167,6 +167,11 @@ __global__ void __launch_bounds__(256) diff_prepare_vec_kernel(bf16* __restrict_
   }
 }
 
+// Whether portions of these sizes take diff_prepare_vec_kernel: all but up to 148 tokens (one wave of a CTA a token) with many maps of 128
+// entries, of which a warp takes one at a time (32 + 8 heads: 33 tokens 10.4 us with a CTA a token and 11.2 with four warps a token, 128 11.0
+// and 11.3, 300 faster; of 64 entries, 64 + 16 heads, 33 tokens no slower).
+extern "C" int qv_diff_prepare_vec(int T, int H, int G, int n) { return T > 32 && (n < 128 || T > 148 || 2 * (H + G) < 64); }
+
 extern "C" int qv_diff_prepare(void* q_out, int ld_q, const void* proj, int ld_p, const float* bias, const float* qw, const float* kw,
                                float eps, const float* cos_sin, int table_rows, const int* tok_pos, const int* tok_seg,
                                const int* block_table, int max_blocks, void* cache, int T, int H, int G, int n, int dv, int rot, int page,
@@ -179,7 +184,7 @@ extern "C" int qv_diff_prepare(void* q_out, int ld_q, const void* proj, int ld_p
   // few tokens: a token's maps are spread over several CTAs (each brings the row in for itself), so that the step fills more SMs
   const int units = 2 * H + 3 * G;
   const int spread = T <= 32 ? ((units + 7) / 8 < 65535 ? (units + 7) / 8 : 65535) : 1;
-  if (T > 32 && proj_dt == QV_DT_F32 && dt == QV_DT_BF16 && (n == 32 || n == 64 || n == 128) && rot % 8 == 0 && dv % 4 == 0 && ld_p % 4 == 0 &&
+  if (qv_diff_prepare_vec(T, H, G, n) && proj_dt == QV_DT_F32 && dt == QV_DT_BF16 && (n == 32 || n == 64 || n == 128) && rot % 8 == 0 && dv % 4 == 0 && ld_p % 4 == 0 &&
       ld_q % 4 == 0 && (((uintptr_t)proj | (uintptr_t)bias | (uintptr_t)qw | (uintptr_t)kw) & 15) == 0 && (((uintptr_t)q_out | (uintptr_t)cache) & 7) == 0 &&
       T <= 0x7fffffff / DP_WARPS) {
     auto kernel = n == 32 ? diff_prepare_vec_kernel<8> : n == 64 ? diff_prepare_vec_kernel<16> : diff_prepare_vec_kernel<32>;

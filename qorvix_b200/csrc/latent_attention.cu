@@ -188,6 +188,12 @@ __global__ void __launch_bounds__(128) latent_rows_kernel(const T* __restrict__ 
   }
 }
 
+// Whether portions of these sizes take latent_prepare_vec_kernel.  Its three warps a token turn the heads' queries one after the other, so few heads
+// suit it: us with a CTA a token and with it, 8 heads of rank 256: 33 tokens 2.8 and 2.5, 128 2.8 and 2.7, 2,048 7.0 and 4.9; 16 heads of
+// rank 512: 64 tokens 3.7 and 3.7, 128 3.4 and 3.8, 300 3.6 and 2.9, 2,048 8.8 and 6.8; 32 heads of rank 1,024: 128 4.6 and 5.0, 300 4.9 and
+// 3.8; 64 heads 128 5.0 and 8.1, 2,048 15.2 and 15.4; 128 heads 23.4 and 26.9.  (Up to 148 tokens a CTA a token is one wave.)
+extern "C" int qv_latent_prepare_vec(int T, int H) { return T > 32 && (H <= 8 || (T > 148 && H <= 32)); }
+
 extern "C" int qv_latent_prepare(void* proj, int ld, void* q, int ld_q, int kv_off, void* cache, const float* norm_w, float eps,
                                  const float* cos_sin, int table_rows, const int* tok_pos, const int* tok_seg,
                                  const int* block_table, int max_blocks, int T, int H, int dn, int dr, int rank, int rot,
@@ -198,7 +204,7 @@ extern "C" int qv_latent_prepare(void* proj, int ld, void* q, int ld_q, int kv_o
     QV_DISPATCH_DT(dt, TT,
                    return qv_launch(latent_rows_kernel<TT>, dim3((T + 3) / 4), dim3(128), 0, (cudaStream_t)stream, (const TT*)proj + kv_off, ld, (TT*)cache,
                                     norm_w, eps, tok_pos, tok_seg, block_table, max_blocks, T, rank, page));
-  if (dt == QV_DT_BF16 && T > 32 && !split_half && rank % 8 == 0 && rank <= 256 * LP_MAX_PIECES && (rank + dr) % 8 == 0 && ld % 8 == 0 && kv_off % 8 == 0 &&
+  if (dt == QV_DT_BF16 && qv_latent_prepare_vec(T, H) && !split_half && rank % 8 == 0 && rank <= 256 * LP_MAX_PIECES && (rank + dr) % 8 == 0 && ld % 8 == 0 && kv_off % 8 == 0 &&
       dn % 2 == 0 && dr % 2 == 0 && ld_q % 2 == 0 && (((uintptr_t)proj | (uintptr_t)cache | (uintptr_t)norm_w) & 15) == 0 && ((uintptr_t)q & 3) == 0)
     return qv_launch(latent_prepare_vec_kernel, dim3((T + 1) / 2), dim3(256), 0, (cudaStream_t)stream, (const bf16*)proj, ld, (bf16*)q, ld_q, kv_off,
                      (bf16*)cache, norm_w, eps, (const float2*)cos_sin, table_rows, tok_pos, tok_seg, block_table, max_blocks, T, H, dn, dr, rank, rot,

@@ -61,6 +61,7 @@ _ARGTYPES = {
     "qv_add_rmsnorm2": [_V, _V, _V, _V, _V, _V, _I, _I, _F, _I, _I, _V],
     "qv_sum2": [_V, _V, _V, _L, _I, _I, _V],
     "qv_softcap": [_V, _L, _F, _V],
+    "qv_latent_prepare_vec": [_I, _I],
     "qv_latent_prepare": [_V, _I, _V, _I, _I, _V, _V, _F, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_latent_attention_generic": [_V, _I, _V, _I, _V, _I, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _V, _V],
     "qv_latent_tc_workspace_bytes": [_I, _I, _I, _I, _I],
@@ -76,6 +77,7 @@ _ARGTYPES = {
     "qv_linear_scan": [_I, _V, _I, _V, _I, _I, _V, _I, _V, _I, _V, _I, _V, _I, _V, _V, _V, _F, _F, _V, _L, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _V, _V,
                        _L, _V, _V],
     "qv_gated_group_norm": [_V, _I, _V, _I, _V, _I, _V, _I, _I, _I, _F, _I, _I, _V],
+    "qv_moe_route_rows": [_I, _I, _I],
     "qv_moe_route": [_V, _V, _V, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _F, _I, _I, _I, _V],
     "qv_moe_max_tiles": [_I, _I, _I],
     "qv_moe_tile_rows": [_I, _I, _I, _I],
@@ -91,6 +93,7 @@ _ARGTYPES = {
     "qv_activation": [_V, _V, _V, _L, _I, _I, _I, _V],
     "qv_stream_pass": [_V, _V, _V, _V, _I, _V, _V, _V, _V, _F, _V, _I, _I, _I, _I, _I, _I, _V],
     "qv_cache_rows": [_V, _V, _I, _V, _V, _V, _I, _I, _I, _I, _I, _V],
+    "qv_diff_prepare_vec": [_I, _I, _I, _I],
     "qv_diff_prepare": [_V, _I, _V, _I, _V, _V, _V, _F, _V, _I, _V, _V, _V, _I, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _V],
     "qv_diff_partial_floats": [_I],
     "qv_diff_attention_tc": [_V, _I, _V, _I, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _V, _I, _V],

@@ -274,3 +274,12 @@ def test_from_where_long_segments_of_the_gated_recurrence_take_three_launches():
     assert least(ops.SCAN_GATED_MAX, 4, 128, 256) == least(ops.SCAN_GATED_MAX, 16, 256, 64) == least(ops.SCAN_GATED_MAX, 4, 64, 64) == 1024
     assert least(ops.SCAN_GATED_MAX, 32, 128, 128) == 2048 and least(ops.SCAN_GATED_MAX, 64, 128, 64) == least(ops.SCAN_GATED_MAX, 16, 64, 64) == never
     assert least(ops.SCAN_DECAY, 4, 256, 512) == least(ops.SCAN_GATED_MAX, 1, 264, 64) == never
+
+
+def test_which_portions_take_the_passes_of_several_warps_a_token():
+    latent = lambda *a: ops._lib("latent_attention").qv_latent_prepare_vec(*a)
+    assert latent(33, 8) and latent(149, 16) and latent(2048, 32)
+    assert not latent(32, 8) and not latent(148, 16) and not latent(2048, 64)
+    diff = lambda *a: ops._lib("diff_attention").qv_diff_prepare_vec(*a)
+    assert diff(33, 64, 16, 64) and diff(33, 16, 4, 128) and diff(149, 32, 8, 128)
+    assert not diff(32, 8, 4, 64) and not diff(148, 32, 8, 128)
