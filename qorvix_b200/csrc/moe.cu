@@ -413,6 +413,12 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(int* __rest
 // logits_ws: room for T * (E + 1) floats, or null.  With it, the logits are formed in a launch of their own: for steps of up to
 // 256 tokens over (tokens x groups of eight rows) CTAs, for longer ones a CTA per eight tokens; the
 // result is the same whichever kernel forms them (same sums, same order).
+// Whether moe_logits_rows_kernel forms the logits (where types and alignment let it): not of few rows over many tokens of short rows, whose time
+// is the inputs' way to shared memory (us with moe_logits_tokens_kernel and with rows: 2,048 tokens of 512, 33 rows 14.0 and 15.2, 65 rows 18.0
+// and 17.2, 33 rows of 1,024 entries 17.3 and 18.1, of 2,048 faster; 1,024 tokens of 512, 33 rows 9.7 and 8.2; 300 tokens, 9 rows of 512
+// 6.6 and 6.9, of 1,024 7.8 and 7.6).
+extern "C" int qv_moe_route_rows(int T, int rows, int d) { return T <= 1024 ? rows > 16 || d >= 1024 : rows > 40 || d >= 2048; }
+
 extern "C" int qv_moe_route(int* top_idx, float* top_w, float* gate_out, const void* h, int ld_h, const void* wr, const void* wg,
                             float* logits_ws, int T, int d, int E, int top, int dt, int w_dt, const float* correction, float w_scale,
                             int sigmoid, int groups, int keep, void* stream) {
@@ -428,7 +434,7 @@ extern "C" int qv_moe_route(int* top_idx, float* top_w, float* gate_out, const v
   const bool tokens = logits_ws && !split && d % 4 == 0 && (size_t)ROUTE_TOKENS * d * sizeof(float) <= 160 * 1024;
   const dim3 lgrid(T, (E + (wg ? 1 : 0) + ROUTE_WARPS - 1) / ROUTE_WARPS);
   const dim3 tgrid((T + ROUTE_TOKENS - 1) / ROUTE_TOKENS);
-  const bool rows16 = tokens && dt == QV_DT_BF16 && w_dt == QV_DT_BF16 && d % 8 == 0 && ld_h % 8 == 0 &&
+  const bool rows16 = tokens && qv_moe_route_rows(T, E + (wg ? 1 : 0), d) && dt == QV_DT_BF16 && w_dt == QV_DT_BF16 && d % 8 == 0 && ld_h % 8 == 0 &&
                       (((uintptr_t)h | (uintptr_t)wr | (uintptr_t)wg) & 15) == 0;
   if (rows16) {
     const int rows = route_rows(E + (wg ? 1 : 0));

@@ -283,3 +283,9 @@ def test_which_portions_take_the_passes_of_several_warps_a_token():
     diff = lambda *a: ops._lib("diff_attention").qv_diff_prepare_vec(*a)
     assert diff(33, 64, 16, 64) and diff(33, 16, 4, 128) and diff(149, 32, 8, 128)
     assert not diff(32, 8, 4, 64) and not diff(148, 32, 8, 128)
+
+
+def test_the_routers_rows():
+    rows = lambda *a: ops._lib("moe").qv_moe_route_rows(*a)
+    assert rows(2048, 65, 512) and rows(1024, 33, 512) and rows(2048, 33, 2048) and rows(300, 9, 1024)
+    assert not rows(2048, 33, 512) and not rows(1025, 40, 2040) and not rows(300, 9, 512)
