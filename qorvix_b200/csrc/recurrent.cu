@@ -19,10 +19,6 @@
 #define CONV_MAX_TAPS 16
 #define CONV_CHUNK 16
 
-// SiLU: with the fast functions where the result is rounded to bfloat16 (their error, a few float32 ulp, vanishes in the rounding).
-template <typename TO> __device__ __forceinline__ float conv_silu(float x) { return x / (1.0f + expf(-x)); }
-template <> __device__ __forceinline__ float conv_silu<bf16>(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
 // in/out: [T, channels] with row strides and types of their own; w [channels, taps] (last column: the current token),
 // bias [channels] or null; tail [slots][(taps-1) * channels] float32, oldest input first.  act 1: SiLU of the sum, 0: the sum
 // as it is; add_input 1: the current input is added to the result (out = in + conv(in), after the activation).
@@ -99,7 +95,7 @@ __global__ void __launch_bounds__(128) conv_state_kernel(TO* __restrict__ out, i
       if (i < taps - 2) win[i] = win[i + 1];
       else if (i == taps - 2) win[i] = cur;
     }
-    if (act) acc = conv_silu<TO>(acc);
+    if (act) acc = acc / (1.0f + expf(-acc));
     if (add_input) acc += cur;
     out[(size_t)(q0 + j0 + jj) * ld_out + c] = from_f<TO>(acc);
   }
@@ -181,7 +177,7 @@ __global__ void __launch_bounds__(128) conv_state_vec_kernel(TO* __restrict__ ou
       acc = fmaf(wt[TAPS - 1][k], x, acc);
 #pragma unroll
       for (int i = 0; i < TAPS - 1; ++i) win[i][k] = i < TAPS - 2 ? win[i + 1][k] : x;
-      if (act) acc = conv_silu<TO>(acc);
+      if (act) acc = acc / (1.0f + expf(-acc));
       if (add_input) acc += x;
       o.v[k] = from_f<TO>(acc);
     }
