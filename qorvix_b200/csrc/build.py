@@ -58,8 +58,9 @@ KERNEL_LIBRARIES = ["elementwise", "gemm_simt", "gemm_bf16", "attention_generic"
 # what a library is built from beside its source and HEADERS (their bytes are part of its name's hash)
 EXTRA_SOURCES = {
     "host_runtime": ["host/dispatch.hpp"],
-    "recurrent": ["portion_rounds.h"],
-    "channel_scan": ["portion_rounds.h"],
+    "gemm_simt": ["per_device.h"],
+    "recurrent": ["portion_rounds.h", "per_device.h"],
+    "channel_scan": ["portion_rounds.h", "per_device.h"],
     "executor": ["host/executor.hpp", "host/kernels.hpp", "host/dispatch.hpp"],
     "ref": ["ref/ref_ops.hpp", "host/json.hpp", "host/safetensors.hpp", "host/model_config.hpp"],
 }

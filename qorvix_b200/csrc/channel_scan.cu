@@ -23,6 +23,7 @@
 // factors and all sums.  The order of every sum depends on the sizes alone, so a token's result does not depend
 // on how its request was cut into steps or on what else is in the batch.
 #include "common.cuh"
+#include "per_device.h"
 #include "portion_rounds.h"
 
 #define GATE_POW_SIGMOID 0
@@ -215,13 +216,9 @@ extern "C" int qv_channel_gates(float* out, int ld_out, const float* x1, int ld_
   cudaStream_t st = (cudaStream_t)stream;
   const CgForm form = {kind, p, rate};
   if (qv_channel_gates_tiles(T, N, R, kind)) {
-    static bool configured = false;
-    constexpr int most = (CT_TOKENS * (CT_MAX_RANK + 4) + CT_MAX_RANK * CG_CHANNELS) * 4;
-    if (!configured) {
-      const cudaError_t e = cudaFuncSetAttribute(channel_gates_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (e != cudaSuccess) return (int)e;
-      configured = true;
-    }
+    static PerDevice allowed;
+    const int rc = qv_allow_smem(channel_gates_tile_kernel, (CT_TOKENS * (CT_MAX_RANK + 4) + CT_MAX_RANK * CG_CHANNELS) * 4, allowed);
+    if (rc) return rc;
     return qv_launch(channel_gates_tile_kernel, dim3((T + CT_TOKENS - 1) / CT_TOKENS, by), dim3(128),
                      (size_t)(CT_TOKENS * (R + 4) + R * CG_CHANNELS) * 4 + (R < 48 ? CT_TOKENS * (CG_CHANNELS + 4) * 4 : 0), st, out, ld_out, x1, ld_x, w2t, bias, T, N, R, pre_tanh, form);
   }
@@ -980,12 +977,9 @@ __global__ void __launch_bounds__(32 * NS, 1) delta_blocks_kernel(const __grid_c
 
 template <int NS>
 static int launch_delta_blocks(const ChannelDeltaArgs& a, dim3 grid, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(delta_blocks_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, CdShape<NS>::bytes(16 * NS));
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice allowed;
+  const int rc = qv_allow_smem(delta_blocks_kernel<NS>, CdShape<NS>::bytes(16 * NS), allowed);
+  if (rc) return rc;
   const int smem = CdShape<NS>::bytes(a.dkp);
   return cs_launch_after(delta_blocks_kernel<NS>, grid, dim3(32 * NS), (size_t)smem, st, a);
 }

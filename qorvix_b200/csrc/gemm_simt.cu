@@ -17,6 +17,7 @@
 // first ones are asked for ahead of the wait for the kernel ahead where the caller says that no launch may still write them (a model's
 // weights): 2.5 / 5.0 us.
 #include "common.cuh"
+#include "per_device.h"
 
 __device__ __forceinline__ void gs_cp16(float* dst, const float* src, bool live) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(dst);
@@ -159,12 +160,10 @@ static int launch(void* C, const void* A, const void* W, int M, int N, int K, in
 #define GS_LAUNCH(BM, BN, BK, TM, TN, ST, AS)                                                                                    \
   do {                                                                                                                           \
     constexpr size_t smem = (size_t)ST * (BM + BN) * (BK + 4) * 4;                                                               \
-    static bool configured = smem <= 48 * 1024;                                                                                  \
-    if (!configured) {                                                                                                           \
-      const cudaError_t e = cudaFuncSetAttribute(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>,                       \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
-      if (e != cudaSuccess) return (int)e;                                                                                       \
-      configured = true;                                                                                                         \
+    static PerDevice allowed;                                                                                                    \
+    if (smem > 48 * 1024) {                                                                                                      \
+      const int rc = qv_allow_smem(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, smem, allowed);                     \
+      if (rc) return rc;                                                                                                         \
     }                                                                                                                            \
     return qv_launch(gemm_simt_kernel<TA, TW, TC, BM, BN, BK, TM, TN, ST, AS>, grid, dim3((BM / TM) * (BN / TN)), smem, st, (TC*)C, \
                      (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, (flags & 0xff) != 0, flags & GS_SETTLED, GluAct{0, 0.f, 0.f}); \
@@ -217,12 +216,9 @@ extern "C" int qv_gemm_simt_glu(float* C, const float* A, const float* W, int M,
   if (!small || (long long)grid.x * grid.y > 148) return QV_ERR_UNSUPPORTED;
   constexpr size_t smem = (size_t)8 * (16 + 32) * (64 + 4) * 4;
   auto kernel = gemm_simt_kernel<float, float, float, 16, 32, 64, 2, 2, 8, true, true>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice allowed;
+  const int rc = qv_allow_smem(kernel, smem, allowed);
+  if (rc) return rc;
   return qv_launch(kernel, grid, dim3(128), smem, (cudaStream_t)stream, C, A, W, M, N, K, lda, ldw, ldc, 0, settled,
                    GluAct{act, limit, slope});
 }

@@ -14,6 +14,7 @@
 //
 // All state arithmetic, gates, decays and norms are float32; q, k and v are read in the compute type.
 #include "common.cuh"
+#include "per_device.h"
 #include "portion_rounds.h"
 
 #define CONV_MAX_TAPS 16
@@ -1134,12 +1135,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_scan_chunk_kernel(const 
 template <int KIND, int VT, int NK>
 static int launch_scan_chunk(const ScanArgs& a, dim3 grid, cudaStream_t st) {
   auto kernel = linear_scan_chunk_kernel<KIND, VT, NK>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LcShape<VT, NK>::BYTES);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static PerDevice allowed;
+  const int rc = qv_allow_smem(kernel, LcShape<VT, NK>::BYTES, allowed);
+  if (rc) return rc;
   return qv_launch(kernel, grid, dim3(LC_THREADS), (size_t)LcShape<VT, NK>::BYTES, st, a);
 }
 
@@ -1743,17 +1741,10 @@ __global__ void __launch_bounds__(LP_THREADS, 2) lp_outputs_kernel(const __grid_
   }
 }
 
-template <typename F>
-static int lp_configure(F kernel, int bytes, bool* configured) {
-  if (*configured) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  *configured = e == cudaSuccess;
-  return (int)e;
-}
 #define LP_MAX_OUT_BYTES (112 * 1024)      // two CTAs an SM
 
 static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* ws, cudaStream_t st, int* launches) {
-  static bool configured[2] = {};
+  static PerDevice allowed[2];
   LpWork w;
   w.dkp = (a.dk + 31) / 32 * 32;
   w.ct = (a.dv + 15) / 16;
@@ -1769,8 +1760,8 @@ static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* 
   const int out_bytes = LpOutShape(w.dkp, cols).bytes, token_bytes = (a.dk * (w.vt + 3) + LP_THREADS + 4) * 4;
   const int smem = out_bytes > token_bytes ? out_bytes : token_bytes, states = (int)sizeof(LpStatesSmem);
   const int kblocks = (a.dk + LP_KEYS - 1) / LP_KEYS, cblocks = (a.dv + LP_KEYS - 1) / LP_KEYS;
-  int rc = lp_configure(lp_states_kernel, states, &configured[0]);
-  if (!rc) rc = lp_configure(lp_outputs_kernel, LP_MAX_OUT_BYTES, &configured[1]);
+  int rc = qv_allow_smem(lp_states_kernel, states, allowed[0]);
+  if (!rc) rc = qv_allow_smem(lp_outputs_kernel, LP_MAX_OUT_BYTES, allowed[1]);
   while (!rc && rounds.next(w.round)) {
     rc = qv_launch(lp_gates_kernel, dim3(w.round.items, a.H), dim3(32 * LP_GATE_WARPS), 0, st, a, w);
     if (!rc) rc = qv_launch(lp_states_kernel, dim3(w.round.items, a.H, kblocks * (cblocks + 1)), dim3(LP_THREADS), (size_t)states, st, a, w);

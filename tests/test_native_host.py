@@ -74,3 +74,16 @@ def test_rounds_of_a_recurrences_chunks(tmp_path):
     assert build.returncode == 0, build.stderr[-3000:]
     run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert run.returncode == 0 and run.stdout.strip() == "ok", run.stdout[-2000:]
+
+
+def test_what_is_set_once_a_device(tmp_path):
+    """tests/native/per_device_test.cpp; and the kernels that any device of a process could run with their static shared memory use it."""
+    from qorvix_b200.csrc.build import CSRC, find_host_compiler
+    exe = tmp_path / "per_device_test"
+    build = subprocess.run([find_host_compiler(), "-O1", "-std=c++17", "-pthread", "-I", str(CSRC), "-o", str(exe),
+                            str(ROOT / "tests" / "native" / "per_device_test.cpp")], capture_output=True, text=True, timeout=600)
+    assert build.returncode == 0, build.stderr[-3000:]
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0 and run.stdout.strip() == "ok", run.stdout[-2000:]
+    for name in ("gemm_simt.cu", "channel_scan.cu", "recurrent.cu"):
+        assert "static bool configured" not in (CSRC / name).read_text(), name
