@@ -23,7 +23,7 @@
 //   warp 2        TMA: an item's Q tiles, each as soon as the last Q.K^T of the item before has read
 //                 the old one.
 //   warps 4..11   softmax of tile A, warps 12..19 of tile B, two warpgroups each (DIFF, ROPE: all four share the one tile, four threads a row
-//                 with 32 keys each; a latent layer of 2,048 tokens 143 us with two threads a row, 136 so).  A query row is
+//                 with 32 keys each; a latent layer of 2,048 tokens 145 us with two threads a row, 141 so).  A query row is
 //                 shared by two threads (one per warpgroup, same lane of tensor memory), each owning 64
 //                 of the tile's 128 keys: it reads its part of the row of S (once for the maximum, on
 //                 which it agrees with its partner through shared memory, and once more, 32 columns

@@ -36,7 +36,7 @@
 // is cut into four quarters (r ascending in each, by four groups of threads) that are added in order, so that a step of
 // few tokens still has many loads in flight and the order of a sum depends on R alone.
 // Portions take 16 tokens a CTA and, where R is a multiple of 16, read a token's row four entries at a time (one shared-memory read a
-// multiply-add: 47 us for 1,531 tokens x 64 x 2,048; now 38).  The order of a sum is the same.
+// multiply-add: 47 us for 1,531 tokens x 64 x 2,048, which now take the tiles below; 38 so).  The order of a sum is the same.
 struct CgForm { int kind; float p; const float* rate; };
 __device__ __forceinline__ float cg_gate(float zz, const CgForm& f, int c) {
   if (f.kind == GATE_POW_SIGMOID) return expf(f.p * (fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))));             // log sigmoid(z)
@@ -543,12 +543,14 @@ extern "C" int qv_channel_scan(float* out, int ld_out, const float* q, int ld_q,
 //   e_t   = v'_t - S_0^T X'_t,                     y_t = v''_t + S_0^T X''_t
 // so that all but the products with S_0 and the update is worked out for all blocks at once, and a block costs its recurrence two products
 // and two barriers.  Only products of decays (each at most one) occur, no quotients.
-//   delta_block_operands_kernel   a CTA per (block, head): everything that does not depend on the state, float32 throughout
+//   delta_block_operands_kernel   a CTA per (block, head): everything that does not depend on the state, float32, the triangular system's sums float64
 //   delta_blocks_kernel           the recurrence: a CTA owns 16 value columns of a (segment, head), a warp 16 of the keys
 // The products with S_0 and of the update are mma.sync on both sides' three bfloat16 terms (the six products that count for 24 bits; the
 // large one's sum apart from the small ones', which the tensor cores would cut off), sums over the keys' slices in float32.
 // 1,531 tokens of 16 heads of 128 x 128: 607 us token by token, 460 with four tokens at a time and float32 multiply-adds, and
-// 161 here (operands 58, recurrence 103; 61 and 139 with operands of float32 that every CTA split again, read straight to registers).
+// 168 here (operands 65, recurrence 103; operands 58 with the triangular system's sums in float32, which left portions of 16 to 100 tokens
+// further off float64 than four tokens at a time had; 61 and 139 with operands of float32 that every CTA split again, read straight to
+// registers).
 // Blocks are counted from the start of a request's portion, so cuts agree to rounding (the 32-bit path takes channel_scan_kernel).
 #define CD_BLOCK 16
 #define CD_COLS 16

@@ -1772,8 +1772,8 @@ static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* 
   return rc;
 }
 
-// Segments from this many tokens on take the three launches, if their gates have a running maximum.  By 8 chunks of 4 heads of 256 x 512 the two
-// ways cost the same (a layer 98 us, where launching it from the host is what takes the time), by 32 the one kernel takes 272 and these 200.
+// Segments from this many tokens on take the three launches, if their gates have a running maximum (2,048 tokens of 4 heads of 256 x 512: a layer
+// 272 us with the one kernel, 200 with these).
 // Scalar decays stay with linear_scan_chunk_kernel: many heads of small states fill the GPU as they are (64 heads of 128 x 64, 1,943 tokens
 // in three segments: a layer 292 us, and 299 with these launches; one segment of 2,048: 282 and 317).
 // Which sizes: linear_scan_chunk_kernel forms W again for every tile of value columns, so many tiles a head speak for the three launches; where few

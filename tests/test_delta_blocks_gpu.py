@@ -1,4 +1,4 @@
-"""The delta rule as a step takes it (keys above 64 entries four tokens at a time from the first portion on, others token by token) against
+"""The delta rule as a step takes it (sixteen tokens at a time from the first portion on that pays for it, others token by token) against
 float64 token by token, over every size of lane groups, segments that end anywhere in a block, strong and weak decays; and no further off
 than the token-by-token kernel."""
 from types import SimpleNamespace
@@ -74,7 +74,7 @@ def test_blocks_against_float64(dk, dv, H, G, lens, rate):
                 err[i] += torch.stack([((outs[i][rows, h * dv:(h + 1) * dv] - ys) ** 2).sum(), ((matrix(states[i], slot, h) - S) ** 2).sum()]).cpu()
         at += n
     rel = (err / norm).sqrt()
-    # sums of up to 256 float32 products: some 1e-7; four tokens at a time may not be further off than one at a time
+    # sums of up to 256 float32 products: some 1e-7; sixteen tokens at a time may not be further off than one at a time
     assert bool((rel[0] <= torch.maximum(1.2 * rel[1], torch.full((2,), 2.5e-7, dtype=torch.float64))).all()), rel.tolist()
 
 

@@ -94,3 +94,30 @@ def test_a_segment_among_many_does_not_depend_on_them(lens):
         assert launches == (3 if n >= 640 else 1)
         assert torch.equal(alone, whole[at: at + n]) and torch.equal(one[0], state[slot]), s
         at += n
+
+
+def test_an_infinite_value_ahead_of_a_later_round():
+    """An infinite value in the first of two rounds of launches, whose block of columns then goes token by token: tokens ahead of it, other columns
+    and the normaliser stay what they are, through the second round too (float32 sums of up to 64 products in another order: 2e-5)."""
+    H, dk, dv, lens = 8, 256, 512, [1700, 1500]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T = sum(lens)
+    q, k, v = (rnd(T, H * n).to(torch.bfloat16) for n in (dk, dk, dv))
+    g1, g2, p1, p2 = rnd(T, H), rnd(T, H) + 2, rnd(H), rnd(H)
+
+    def run():
+        state = torch.zeros(2, ops.linear_scan_state_floats(ops.SCAN_GATED_MAX, H, dk, dv), device="cuda")
+        out, before = torch.full((T, H * dv), float("nan"), device="cuda"), ops.launch_count()
+        ops.linear_scan(ops.SCAN_GATED_MAX, out, q, k, v, g1, g2, p1, p2, None, 6.0, dk ** -0.5, state, chunks.context(lens), H, dk, dv)
+        assert ops.launch_count() - before == 6
+        return out, state.view(2, H, dv // 16, dk * 16 + dk + 1)[:, :, :, dk * 16:]        # n and m of every value tile
+
+    (clean, clean_n), at = run(), 133
+    assert bool(torch.isfinite(clean).all())
+    v[at, 3] = float("inf")
+    got, n = run()
+    others, scale = torch.arange(H * dv, device="cuda") != 3, clean.abs().max()
+    assert bool(((got[:, others] - clean[:, others]).abs() <= 2e-5 * scale).all()) and bool(((got[:at] - clean[:at]).abs() <= 2e-5 * scale).all())
+    assert torch.equal(got[1700:], clean[1700:]) and not bool(torch.isfinite(got[at:1700, 3]).any())
+    assert float((n - clean_n).norm() / clean_n.norm()) < 2e-6
