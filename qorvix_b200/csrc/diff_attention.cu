@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(256) diff_prepare_kernel(T* __restrict__ q_out
 }
 
 // Portions: a lane holds four neighbouring entries of a map of 4 LANES, so a warp takes 32 / LANES maps at once, straight from the projection; the
-// rotation's other half comes by shuffle, and the lane's weights and angles are the same for all of its maps.  Four warps a token.
+// rotation's other half comes by shuffle, and the lane's weights and angles are the same for all of its maps.  Four warps a token.  The same
+// sums in the same order.
 // 1,500 tokens of 16 + 4 heads of 2 x 64 + 128: 21 us with the kernel above (270 instructions a map), 12 here, bound by the
 // projection's 18 MB and the launch around them.
 #define DP_WARPS 4
@@ -137,10 +138,21 @@ __global__ void __launch_bounds__(256) diff_prepare_vec_kernel(bf16* __restrict_
       }
     }
     if (is_q ? qw != nullptr : kw != nullptr) {
-      float ss = fmaf(x[0], x[0], x[1] * x[1]) + fmaf(x[2], x[2], x[3] * x[3]);
+      // the sums of the kernel above: its lane 4 (lane % 8) + i adds up every 32nd entry, which lie eight lanes apart, then its warp's tree
       const unsigned group = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (lane / LANES * LANES);
+      float s[4];
 #pragma unroll
-      for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
+      for (int i = 0; i < 4; ++i) {
+        s[i] = x[i] * x[i];
+#pragma unroll
+        for (int k = 1; k < LANES / 8; ++k) {
+          const float ahead = __shfl_up_sync(group, s[i], 8, LANES);
+          if (lane % LANES >= 8 * k) s[i] = fmaf(x[i], x[i], ahead);
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s[i] += __shfl_xor_sync(group, s[i], o);
+      }
+      const float ss = __shfl_sync(group, (s[0] + s[2]) + (s[1] + s[3]), LANES - 8, LANES);
       const float inv = 1.0f / sqrtf(ss / (float)N + eps);
       const float4 w = is_q ? wq : wk;
       x[0] = x[0] * inv * w.x; x[1] = x[1] * inv * w.y; x[2] = x[2] * inv * w.z; x[3] = x[3] * inv * w.w;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
 }
 
 // Portions, neighbouring pairs, bfloat16 on 16-byte boundaries: four warps a token, one for the latent (16 bytes a lane, kept in registers
-// between the sum and the write), three for the rotated parts (a pair, one word, a lane).  2,048 tokens of 16 heads, rank 512: 10.4 us with
+// between the sum and the write), three for the rotated parts (a pair, one word, a lane).  The same sums in the same order.  2,048 tokens of 16 heads, rank 512: 10.4 us with
 // a CTA a token and two bytes a thread, 7.8 here, bound by the trips to memory of its few accesses a warp.
 #define LP_MAX_PIECES 4
 __global__ void __launch_bounds__(256) latent_prepare_vec_kernel(const bf16* __restrict__ proj, int ld, bf16* __restrict__ q, int ld_q, int kv_off,
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256) latent_prepare_vec_kernel(const bf16* __r
   if (part == 0) {
     const int pieces = rank >> 3;
     uint4 v[LP_MAX_PIECES];
-    float ss = 0.f;
+    float s[8] = {};
 #pragma unroll
     for (int k = 0; k < LP_MAX_PIECES; ++k) {
       const int i = lane + 32 * k;
@@ -103,10 +103,19 @@ __global__ void __launch_bounds__(256) latent_prepare_vec_kernel(const bf16* __r
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float a = __low2float(e[u]), b = __high2float(e[u]);
-        ss = fmaf(a, a, fmaf(b, b, ss));
+        s[2 * u] = fmaf(a, a, s[2 * u]);
+        s[2 * u + 1] = fmaf(b, b, s[2 * u + 1]);
       }
     }
-    const float sc = 1.0f / sqrtf(warp_sum(ss) / (float)rank + eps);
+    // s[e]: what thread 8 lane + e of the kernel above sums; its warps' trees, then the block's
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+    float ss = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float sc = 1.0f / sqrtf(ss / (float)rank + eps);
 #pragma unroll
     for (int k = 0; k < LP_MAX_PIECES; ++k) {
       const int i = lane + 32 * k;
@@ -126,10 +135,10 @@ __global__ void __launch_bounds__(256) latent_prepare_vec_kernel(const bf16* __r
   const int pairs = rot >> 1;
   for (int i = lane; i < pairs; i += 32) {
     const float2 c = cs[i];
-    auto turn = [&](const bf16* from, bf16* to) {
+    auto turn = [&](const bf16* from, bf16* to) {            // (the multiply-adds as the kernel above's are fused)
       const __nv_bfloat162 x = *(const __nv_bfloat162*)(from + 2 * i);
       const float a = __low2float(x), b = __high2float(x);
-      *(__nv_bfloat162*)(to + 2 * i) = __floats2bfloat162_rn(a * c.x - b * c.y, b * c.x + a * c.y);
+      *(__nv_bfloat162*)(to + 2 * i) = __floats2bfloat162_rn(fmaf(a, c.x, -(b * c.y)), fmaf(b, c.x, a * c.y));
     };
     bf16* qr = q + (size_t)t * ld_q + dn;
 #pragma unroll 4

@@ -1,5 +1,5 @@
 """The passes ahead of differential and latent attention over portions (vector accesses, several warps a token) against the steps of up to 32 tokens,
-which take the general kernels: float32 arithmetic in another order, so at most one rounding of the stored type apart, and seldom."""
+which take the general kernels: at most one rounding of the stored type apart, and seldom; and, with the sums in their order, the same bits."""
 from types import SimpleNamespace
 
 import pytest
@@ -67,3 +67,38 @@ def test_latent(rank, dr, rot, dn):
 
     for got, want in zip(run([(0, T)]), run(parts(T))):
         close(got, want)
+
+
+@pytest.mark.parametrize("n,dv,rot", [(32, 36, 32), (64, 128, 64), (128, 20, 96)])
+def test_a_token_of_differential_attention_does_not_depend_on_its_step(n, dv, rot):
+    T, page, H, G = 170, 16, 4, 2
+    rnd, bt, pos, seg, pages = setup(T, page, n)
+    proj, b, w = rnd(T, (H + G) * 2 * n + G * dv), rnd((H + G) * 2 * n + G * dv), rnd(n)
+    table = rnd(T, rot // 2, 2)
+
+    def run(cuts):
+        q, cache = torch.empty(T, H * 2 * n, device="cuda", dtype=BF16), torch.zeros(pages, page, G * (2 * n + dv), device="cuda", dtype=BF16)
+        for a, e in cuts:
+            ctx = SimpleNamespace(tok_pos=pos[a:e], tok_seg=seg[a:e])
+            ops.diff_prepare(q[a:e], proj[a:e], b, w, w, 1e-5, table, ctx, bt, cache, H, G, n, dv, rot, page)
+        return q, cache
+
+    assert all(torch.equal(x, y) for x, y in zip(run([(0, T)]), run(parts(T))))
+
+
+@pytest.mark.parametrize("rank,dr,rot,dn", [(8, 8, 8, 2), (256, 64, 64, 128), (512, 64, 32, 64), (1024, 72, 70, 6)])
+def test_a_token_of_latent_attention_does_not_depend_on_its_step(rank, dr, rot, dn):
+    T, page, H = 170, 16, 7
+    rnd, bt, pos, seg, pages = setup(T, page, rank)
+    width = H * (dn + dr)
+    kv_off = -(-width // 8) * 8
+    source, w, table = rnd(T, -(-(kv_off + rank + dr) // 8) * 8).to(BF16), rnd(rank), rnd(T, rot // 2, 2)
+
+    def run(cuts):
+        proj, cache = source.clone(), torch.zeros(pages, page, rank + dr, device="cuda", dtype=BF16)
+        for a, e in cuts:
+            ctx = SimpleNamespace(tok_pos=pos[a:e], tok_seg=seg[a:e])
+            ops.latent_prepare(proj[a:e], proj[a:e, :width], kv_off, cache, w, 1e-5, table, ctx, bt, H, dn, dr, rank, rot, page)
+        return proj, cache
+
+    assert all(torch.equal(x, y) for x, y in zip(run([(0, T)]), run(parts(T))))
