@@ -1065,6 +1065,7 @@ DELTA_SHORT_KEYS_FROM = 256                # keys of up to 64 entries: portions 
 def delta_lead(lens, dk: int, blocks: bool = True, heads: int = 128) -> int:
     """How many of a step's leading segments the delta rule takes token by token (single tokens come first in a step): those ahead of the first
     portion that pays for sixteen tokens at a time; all where `blocks` is False, for keys that are no multiple of 4 entries or above 256.
+    heads: as many as fill the GPU if not given.
     us token by token and in blocks (rows in L2), one portion and eight: 16 heads of 128, 16 tokens 11.5 and 15.8, 35.9 and 33.5; 24 tokens
     14.6 and 16.9, 50 and 43; 32 tokens 18.1 and 17.0, 64 and 44; 8 heads 16 tokens x 8 20.5 and 24.3.  4 heads of 256, 32 tokens 21.5 and
     27.0, 48 tokens 29.7 and 29.2; 16 heads of 256, 32 tokens 42 and 36.  So from 32 tokens on (of 256 entries 48, or 32 where the heads make
