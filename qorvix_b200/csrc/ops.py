@@ -949,6 +949,12 @@ def linear_scan_state_floats(kind: int, H: int, dk: int, dv: int) -> int:
     return int(_lib("recurrent").qv_linear_scan_state_floats(kind, H, dk, dv))
 
 
+@functools.lru_cache(maxsize=256)           # of the sizes alone
+def scan_parallel_from(kind: int, H: int, dk: int, dv: int) -> int:
+    """From how many tokens on a segment takes the launches that need a workspace."""
+    return int(_lib("recurrent").qv_linear_scan_parallel_from(kind, H, dk, dv))
+
+
 def linear_scan(kind, out, q, k, v, g1, g2, p1, p2, p3, cap, q_scale, state, ctx, H, dk, dv, q_group=1) -> None:
     """Per request and head: S = a S + b k v^T, out = S^T q (see csrc/recurrent.cu for the two kinds of gates);
     state [slots, n] float32 is read and left up to date.  q, k: [T, (H/q_group)*dk], v: [T, H*dv] (column slices
@@ -961,7 +967,7 @@ def linear_scan(kind, out, q, k, v, g1, g2, p1, p2, p3, cap, q_scale, state, ctx
         assert p is None or (p.dtype == torch.float32 and p.numel() >= H)
     lib, rest, launches = _lib("recurrent"), _scan_rest(ctx), c_int()
     ws = lens = None                       # what long portions' faster kernels need beside their operands; without room the others take them
-    least = lib.qv_linear_scan_parallel_from(kind, H, dk, dv)
+    least = scan_parallel_from(kind, H, dk, dv)
     if q.dtype == torch.bfloat16 and rest[1] >= least and getattr(ctx, "seg_len", None):
         chunks = [-(-n // SCAN_CHUNK) for n in ctx.seg_len[rest[0]:] if n >= least]
         lens = (c_int * ctx.num_segments)(*ctx.seg_len)
@@ -1087,6 +1093,14 @@ def delta_lead(lens, dk: int, blocks: bool = True, heads: int = 128) -> int:
     return len(lens)
 
 
+@functools.lru_cache(maxsize=256)           # of the sizes alone
+def _delta_room(H: int, dk: int, dv: int):
+    """The workspace's floats a block of all heads, and how many of these it holds at most."""
+    floats = _lib("channel_scan").qv_channel_delta_workspace_floats
+    block = int(floats(0, 1, DELTA_BLOCK, H, dk, dv))
+    return block, int(floats(0, 1, 1 << 30, H, dk, dv)) // block
+
+
 def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: int, eps: float, q_scale: float, blocks: bool = True) -> bool:
     """The delta rule that reads the decayed state: unit vectors of q and k (q times q_scale), beta = sigmoid(b), decays g, per request and
     head; state as channel_scan's.  Token by token (delta_operands, channel_scan) or sixteen tokens at a time, see delta_lead.  True."""
@@ -1098,10 +1112,10 @@ def channel_delta(out, q, k, v, b, g, state, ctx, H: int, G: int, dk: int, dv: i
     lens = ctx.seg_len
     lead = delta_lead(lens, dk, blocks, H)
     tokens, longest = (T, int(ctx.max_q_len)) if lead == S else (sum(lens[:lead]), max(lens[:lead], default=0))
-    lib, launches, rest, ws = _lib("channel_scan"), c_int(), S - lead, None
-    if rest:
-        mean = -(-sum(-(-n // DELTA_BLOCK) for n in lens[lead:]) // rest) * DELTA_BLOCK
-        ws = _room(lib.qv_channel_delta_workspace_floats(tokens, rest, mean, H, dk, dv), torch.float32, q.device)
+    lib, launches, ws = _lib("channel_scan"), c_int(), None
+    if lead < S:
+        block, room = _delta_room(H, dk, dv)
+        ws = _room(tokens * H * 3 * dk + block * min(room, sum([-(-n // DELTA_BLOCK) for n in lens[lead:]])), torch.float32, q.device)
     if ws is None:                                    # token by token, which takes less room
         lead, tokens, longest = S, T, int(ctx.max_q_len)
         ws = torch.empty(H * T * 3 * dk, device=q.device, dtype=torch.float32)

@@ -1772,22 +1772,23 @@ static int launch_scan_parallel(const ScanArgs& a, PortionRounds& rounds, void* 
   return rc;
 }
 
-// Segments from this many tokens on take the three launches, if their gates have a running maximum (2,048 tokens of 4 heads of 256 x 512: a layer
-// 272 us with the one kernel, 200 with these).
+// Segments from this many tokens on take the three launches, if their gates have a running maximum.  A layer with 4 heads of 256 x 512, us with the
+// one kernel and with these: 768 tokens 121 and 127 (two launches more of a step that is not captured), 900 150 and 144, 1,024 159 and 148, 2,048
+// 271 and 201; with 4 heads of 128 x 256 1,024 tokens 117 and 102, 2,048 203 and 140.
 // Scalar decays stay with linear_scan_chunk_kernel: many heads of small states fill the GPU as they are (64 heads of 128 x 64, 1,943 tokens
 // in three segments: a layer 292 us, and 299 with these launches; one segment of 2,048: 282 and 317).
 // Which sizes: linear_scan_chunk_kernel forms W again for every tile of value columns, so many tiles a head speak for the three launches; where few
 // tiles of all heads together fill the GPU once (128 CTAs) it is at its best.  A rule on a segment's own length and the sizes, so that its
-// neighbours do not decide which sums it gets.  us with the one kernel and with the three launches, one segment and four of 1,024 tokens: 4 heads
-// of 256 x 512 86 and 64, 333 and 171 (640 tokens: 56 and 56, 213 and 128); 4 heads of 128 x 256 71 and 53, 73 and 64 (768 x 4: 56 and 57);
+// neighbours do not decide which sums it gets.  us with the one kernel and with the three launches, captured, one segment and four of 1,024
+// tokens: 4 heads of 256 x 512 86 and 64, 333 and 171; 4 heads of 128 x 256 71 and 53, 73 and 64 (768 x 4: 56 and 57);
 // 16 heads of 256 x 64 85 and 54, 170 and 139 (768 x 2: 66 and 72); 32 heads of 128 x 128 73 and 81, 286 and 207 (2,048: 141 and
 // 144, 558 and 419); 16 heads of 64 x 64 61 and 46, 62 and 75; 64 heads of 128 x 64 74 and 98, 288 and 298; 4 heads of 64 x 64 61 and 43, 61
-// and 46 (640 x 8: 40 and 44); 1 head 61 and 44 (640: 39 and 35).
+// and 46; 1 head 61 and 44.
 static inline int scan_parallel_from(int kind, int H, int dk, int dv) {
   const int never = 0x7fffffff;
   if (kind != SCAN_GATED_MAX || dk > 256) return never;
   const int vt = scan_vt(dk), tiles = (dv + vt - 1) / vt;
-  if (tiles >= 16 || (long long)H * tiles <= 4) return 640;
+  if (tiles >= 16) return 896;
   if (tiles >= 6 || (tiles >= 4 && vt == 16) || (long long)H * tiles <= 8) return 1024;
   return tiles >= 4 ? 2048 : never;
 }

@@ -270,7 +270,7 @@ def test_gates_take_tiles_where_there_are_enough_of_them():
 def test_from_where_long_segments_of_the_gated_recurrence_take_three_launches():
     least = lambda *a: ops._lib("recurrent").qv_linear_scan_parallel_from(*a)
     never = 2 ** 31 - 1
-    assert least(ops.SCAN_GATED_MAX, 4, 256, 512) == least(ops.SCAN_GATED_MAX, 16, 256, 256) == least(ops.SCAN_GATED_MAX, 1, 64, 64) == 640
+    assert least(ops.SCAN_GATED_MAX, 4, 256, 512) == least(ops.SCAN_GATED_MAX, 16, 256, 256) == 896 and least(ops.SCAN_GATED_MAX, 1, 64, 64) == 1024
     assert least(ops.SCAN_GATED_MAX, 4, 128, 256) == least(ops.SCAN_GATED_MAX, 16, 256, 64) == least(ops.SCAN_GATED_MAX, 4, 64, 64) == 1024
     assert least(ops.SCAN_GATED_MAX, 32, 128, 128) == 2048 and least(ops.SCAN_GATED_MAX, 64, 128, 64) == least(ops.SCAN_GATED_MAX, 16, 64, 64) == never
     assert least(ops.SCAN_DECAY, 4, 256, 512) == least(ops.SCAN_GATED_MAX, 1, 264, 64) == never
